@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
                         double *__restrict__ part) {
     constexpr int K4 = (NBK - 2) * NBK;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = slice_twiddles<NBK, SlicePlan<NBK>::wide>(S, tw);
     const int kind = blockIdx.x;
     const double sg = kind ? -1.0 : 1.0, beta = 1.0 / T, tE = kind ? beta : 0.0;
     const int nb = nw0 / 2 + 1;
@@ -713,7 +713,7 @@ __global__ void k_hbwd_table(const double *__restrict__ ek, const double *__rest
 // cotangent of h_j (2 V u_j, plus the boundary's at tau = 0, beta) through
 // T^T into the parameter directions.  tmpU: [nb][K4p] scratch.
 template <int NBK>
-__global__ void __launch_bounds__(kSliceThreads, 1)
+__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
     k_cond_slice_bwd(const double *__restrict__ htab, const double *__restrict__ V, const double *__restrict__ hVb,
                      const double *__restrict__ preb, const double2 *__restrict__ tw, int nw0, int K4p, double T,
                      double *__restrict__ tmpU, double *__restrict__ vcond, double *__restrict__ part) {
@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
         // u = T^T hVb(j)
         for (int c = threadIdx.x; c < K4; c += blockDim.x) S[c] = hVb[bidx2(j, c, nw0 + 1)] / edge_w(c % NBK, NBK);
         __syncthreads();
-        dst_dct_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+        dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
         for (int c = threadIdx.x; c < K4; c += blockDim.x) u[c] = S[c] * edge_w(c % NBK, NBK);
         __syncthreads();
         // h_j = T (A E(t))
@@ -742,7 +742,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
             S[c] = xa.y * h_E(xa.x, t, beta);
         }
         __syncthreads();
-        dst_dct_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+        dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
         for (int c = threadIdx.x; c < K4; c += blockDim.x) {
             const int l = c / NBK, m = c % NBK;
             const double uc = u[c];
@@ -754,7 +754,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
             S[c] = hb / edge_w(m, NBK);
         }
         __syncthreads();
-        dst_dct_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+        dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
         for (int c = threadIdx.x; c < K4; c += blockDim.x) {
             const double s = S[c] * edge_w(c % NBK, NBK);
             const double *tc = htab + 8 * (size_t)c;
@@ -920,13 +920,13 @@ __global__ void __launch_bounds__(256, 2)
 // G(r, tau)'s cotangent contracted with its two tangents.
 // ---------------------------------------------------------------------------
 template <int NBK>
-__global__ void __launch_bounds__(kSliceThreads, 1)
+__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
     k_sigma_slice_bwd(const double *__restrict__ stb, const double *__restrict__ Grt, const double *__restrict__ V,
                       const double *__restrict__ dGrt1, const double *__restrict__ dGrt2,
                       const double *__restrict__ vcond, const double *__restrict__ vbk, const double2 *__restrict__ tw,
                       int nw0, int K4p, double *__restrict__ Vb, double *__restrict__ part) {
     constexpr int n8 = NBK * (NBK + 1) / 2;
-    constexpr int NR = (n8 + kSliceThreads - 1) / kSliceThreads;
+    constexpr int NR = (n8 + SlicePlan<NBK>::threads - 1) / SlicePlan<NBK>::threads;
     extern __shared__ __align__(16) double S[];
     const auto *tws = slice_twiddles<NBK>(S, tw);
     const int jv = blockIdx.x, nb = nw0 / 2 + 1;
@@ -944,7 +944,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
             put_sym<NBK>(S, l, m, stb[bidx(j, o, nw0 + 1)] / oct_tw(l, m, NBK));
         }
         __syncthreads();
-        dct2_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+        dct2_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
         int k = 0;
         const size_t rj = (size_t)j * n8;
         for (int o = threadIdx.x; o < n8; o += blockDim.x, ++k) {
@@ -1004,7 +1004,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
     constexpr int n8 = NBK * (NBK + 1) / 2;
     constexpr int NR = (n8 + kSliceThreads - 1) / kSliceThreads;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = slice_twiddles<NBK, SlicePlan<NBK>::wide>(S, tw);
     const int nb = nw0 / 2 + 1;
     double u[2][NR];
 #pragma unroll 1
@@ -1128,7 +1128,7 @@ __global__ void __launch_bounds__(256, 2)
 // A^T (transposed V-bar column), then the RPA factors' derivatives: chi0's
 // cotangent contracted with its two tangents, and Usp, Uch, U.
 template <int NBK>
-__global__ void __launch_bounds__(kSliceThreads, 1)
+__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
     k_vertex_q_bwd(const double *__restrict__ Vb, const double *__restrict__ chiq, const double *__restrict__ dchiq1,
                    const double *__restrict__ dchiq2, const double2 *__restrict__ tw, int nb, double normFact,
                    double U, double Usp, double Uch, double *__restrict__ part) {
@@ -1142,7 +1142,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
         put_sym<NBK>(S, l, m, Vb[bidx(n, o, nb)] / oct_tw(l, m, NBK));
     }
     __syncthreads();
-    dct2_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+    dct2_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
     const double nU = normFact * U;
     double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // th1, th2, Usp, Uch, U
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
@@ -1208,18 +1208,18 @@ template <int NBK>
 struct RunCondSliceBwd {
     static cudaError_t run(const GridDev *g, const CondDev *c, const AdjDev *a, const double *V,
                            const double *dchirt0, double mu0, double T, double fact4, double dmu0_2, cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes;
-        cudaError_t e = set_smem(k_cond_boundary_bwd<NBK>, sm);
+        const size_t sm = SliceSmem<NBK>::bytes, smw = SliceSmem<NBK, SlicePlan<NBK>::wide>::bytes;
+        cudaError_t e = set_smem(k_cond_boundary_bwd<NBK>, smw);
         if (e != cudaSuccess) return e;
         if ((e = set_smem(k_cond_slice_bwd<NBK>, sm)) != cudaSuccess) return e;
         const double nf = 1.0 / ((double)g->nk0 * g->nk0);
-        k_cond_boundary_bwd<NBK><<<2, kSliceThreads, sm, st>>>(g->ek, c->dek, V, dchirt0, c->pre, g->tw_k, a->dbb,
+        k_cond_boundary_bwd<NBK><<<2, kSliceThreads, smw, st>>>(g->ek, c->dek, V, dchirt0, c->pre, g->tw_k, a->dbb,
                                                                 g->nw0, c->K4p, mu0, T, nf, fact4, dmu0_2, a->tmpB,
                                                                 a->vbk, a->preb, a->dchb, a->part + a->row_cb * kAdjW);
         if ((e = launched()) != cudaSuccess) return e;
         k_hbwd_table<<<(c->K4 + 255) / 256, 256, 0, st>>>(g->ek, c->dek, c->K4, g->nbk, mu0, T, nf, dmu0_2, a->htab);
         if ((e = launched()) != cudaSuccess) return e;
-        k_cond_slice_bwd<NBK><<<g->nb, kSliceThreads, sm, st>>>(a->htab, V, a->hVb, a->preb, g->tw_k, g->nw0, c->K4p,
+        k_cond_slice_bwd<NBK><<<g->nb, SlicePlan<NBK>::threads, sm, st>>>(a->htab, V, a->hVb, a->preb, g->tw_k, g->nw0, c->K4p,
                                                                  T, a->tmpU, a->vcond, a->part + a->row_cs * kAdjW);
         return launched();
     }
@@ -1240,15 +1240,15 @@ struct RunSigmaSliceBwd {
     static cudaError_t run(const GridDev *g, const CondDev *c, const AdjDev *a, const double *Grt, const double *V,
                            const double *dchirt0, const double *dG0p, double mu0, double fact8, double dmu0_2,
                            cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes;
+        const size_t sm = SliceSmem<NBK>::bytes, smw = SliceSmem<NBK, SlicePlan<NBK>::wide>::bytes;
         cudaError_t e = set_smem(k_sigma_slice_bwd<NBK>, sm);
         if (e != cudaSuccess) return e;
-        if ((e = set_smem(k_sigma_boundary_bwd<NBK>, sm)) != cudaSuccess) return e;
-        k_sigma_slice_bwd<NBK><<<g->nb, kSliceThreads, sm, st>>>(a->stb, Grt, V, a->dGrt[0], a->dGrt[1], a->vcond,
+        if ((e = set_smem(k_sigma_boundary_bwd<NBK>, smw)) != cudaSuccess) return e;
+        k_sigma_slice_bwd<NBK><<<g->nb, SlicePlan<NBK>::threads, sm, st>>>(a->stb, Grt, V, a->dGrt[0], a->dGrt[1], a->vcond,
                                                                   a->vbk, g->tw_k, g->nw0, c->K4p, a->Vb,
                                                                   a->part + a->row_ss * kAdjW);
         if ((e = launched()) != cudaSuccess) return e;
-        k_sigma_boundary_bwd<NBK><<<1, kSliceThreads, sm, st>>>(
+        k_sigma_boundary_bwd<NBK><<<1, kSliceThreads, smw, st>>>(
             a->dSb, Grt, V, dchirt0, dG0p, g->er, a->dchb, a->dGrt[0], a->dGrt[1], a->ddG0p[0], a->ddG0p[1],
             a->ddchir[0], a->ddchir[1], a->der2, g->tw_k, g->nw0, g->n8p, c->K4p, mu0, fact8, dmu0_2, a->Vb,
             a->part + a->row_sb * kAdjW);
@@ -1275,7 +1275,7 @@ struct RunVertexQBwd {
         cudaError_t e = set_smem(k_vertex_q_bwd<NBK>, sm);
         if (e != cudaSuccess) return e;
         const double normFact = T / ((double)g->nk0 * g->nk0);
-        k_vertex_q_bwd<NBK><<<g->nb, kSliceThreads, sm, st>>>(a->Vb, chiq, a->dchiq[0], a->dchiq[1], g->tw_k, g->nb,
+        k_vertex_q_bwd<NBK><<<g->nb, SlicePlan<NBK>::threads, sm, st>>>(a->Vb, chiq, a->dchiq[0], a->dchiq[1], g->tw_k, g->nb,
                                                                normFact, U, Usp, Uch, a->part + a->row_vq * kAdjW);
         return launched();
     }

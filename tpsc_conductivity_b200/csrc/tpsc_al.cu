@@ -71,7 +71,7 @@ __device__ __forceinline__ double2 half_twiddle_conj(const TwoLevelTw *ht2, int 
 // table (src/cond_opt.cpp:4304-4330), DST x DCT, times G(r, -tau_j), DST x DCT
 // (src/cond_opt.cpp:5220-5248); h(r, 0) and h(r, beta) kept for the end slopes.
 template <int NBK>
-__global__ void __launch_bounds__(kSliceThreads, 1)
+__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
     k_al_hg_slice(const double *__restrict__ tab, const double *__restrict__ Grt, const double2 *__restrict__ tw,
                   int nw0, int n8, double T, double *__restrict__ hGt, double *__restrict__ pre) {
     constexpr int K4 = (NBK - 2) * NBK;
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
         S[c] = xa.y * exp(xa.x > 0 ? -xa.x * t : xa.x * bt);
     }
     __syncthreads();
-    dst_dct_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+    dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
     for (int c = threadIdx.x; c < K4; c += blockDim.x) {
         const int l = c / NBK, m = c % NBK;
         const double v = S[c];
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
         S[c] = v * g_minus(Grt, nw0, n8, j, oct_index(l + 1, m));
     }
     __syncthreads();
-    dst_dct_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+    dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
     for (int c = threadIdx.x; c < K4; c += blockDim.x) hGt[bidx2(j, c, nw0 + 1)] = S[c];
 }
 
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
                   double *__restrict__ dhG) {
     constexpr int K4 = (NBK - 2) * NBK;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = slice_twiddles<NBK, SlicePlan<NBK>::wide>(S, tw);
     const int kind = blockIdx.x;
     for (int c = threadIdx.x; c < K4; c += blockDim.x) {
         const int l = c / NBK, m = c % NBK;
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(256, 1) k_al_hq(const AlHqArgs a) {
 // (src/cond_opt.cpp:5628-5716); blocks Nw0 + 1 and Nw0 + 2 transform the two
 // end slopes.
 template <int NBK>
-__global__ void __launch_bounds__(kSliceThreads, 1)
+__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
     k_al_q2r(const double2 *__restrict__ HQ, const double2 *__restrict__ dHQ, const double2 *__restrict__ tw,
              int nw0, double nf, double2 *__restrict__ HR, double2 *__restrict__ dHR) {
     constexpr int K4 = (NBK - 2) * NBK;
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
     for (int part = 0; part < 2; ++part) {
         for (int c = threadIdx.x; c < K4; c += blockDim.x) S[c] = nf * (part == 0 ? src[c].x : src[c].y);
         __syncthreads();
-        dst_dct_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+        dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
         for (int c = threadIdx.x; c < K4; c += blockDim.x) dst[2 * c + part] = S[c];
         __syncthreads();
     }
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
 //   k = 2, 3: the same for H2, whose end values are H(r, beta), H(r, 0) and
 //   whose end slopes are -dH(r, beta), -dH(r, 0).
 template <int NBK>
-__global__ void __launch_bounds__(kSliceThreads, 1)
+__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
     k_al_r2k(const double2 *__restrict__ HR, const double2 *__restrict__ dHR, const double *__restrict__ Grt,
              const double *__restrict__ er, const double *__restrict__ dG0p, const double2 *__restrict__ tw, int nw0,
              int n8, double mu0, double2 *__restrict__ HK, double2 *__restrict__ H2K, double2 *__restrict__ dHK) {
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
             S[c] = v;
         }
         __syncthreads();
-        dst_dct_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+        dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
         for (int c = threadIdx.x; c < K4; c += blockDim.x) {
             double *dst;
             if (b < NJ)
@@ -586,15 +586,15 @@ template <int NBK>
 struct RunAlHg {
     static cudaError_t run(const GridDev *g, const CondDev *c, const AlDev *a, const double *dG0p, double mu0,
                            double T, cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes;
+        const size_t sm = SliceSmem<NBK>::bytes, smw = SliceSmem<NBK, SlicePlan<NBK>::wide>::bytes;
         cudaError_t e = set_smem(k_al_hg_slice<NBK>, sm);
         if (e != cudaSuccess) return e;
-        if ((e = set_smem(k_al_hg_bound<NBK>, sm)) != cudaSuccess) return e;
+        if ((e = set_smem(k_al_hg_bound<NBK>, smw)) != cudaSuccess) return e;
         const double nf = 1.0 / ((double)g->nk0 * g->nk0);
-        k_al_hg_slice<NBK><<<g->nw0 + 1, kSliceThreads, sm, st>>>(c->tab, a->Grt, g->tw_k, g->nw0, g->n8, T, a->hGt,
+        k_al_hg_slice<NBK><<<g->nw0 + 1, SlicePlan<NBK>::threads, sm, st>>>(c->tab, a->Grt, g->tw_k, g->nw0, g->n8, T, a->hGt,
                                                                    a->pre);
         if ((e = launched()) != cudaSuccess) return e;
-        k_al_hg_bound<NBK><<<2, kSliceThreads, sm, st>>>(g->ek, c->dek, g->er, dG0p, a->Grt, g->tw_k, a->pre, g->nw0,
+        k_al_hg_bound<NBK><<<2, kSliceThreads, smw, st>>>(g->ek, c->dek, g->er, dG0p, a->Grt, g->tw_k, a->pre, g->nw0,
                                                           g->n8, mu0, T, nf, a->dhG);
         return launched();
     }
@@ -630,9 +630,9 @@ struct RunAlSlices {
         if (e != cudaSuccess) return e;
         if ((e = set_smem(k_al_r2k<NBK>, sm)) != cudaSuccess) return e;
         const double nf = 1.0 / ((double)g->nk0 * g->nk0);
-        k_al_q2r<NBK><<<g->nw0 + 3, kSliceThreads, sm, st>>>(a->HQ, a->dHQ, g->tw_k, g->nw0, nf, a->HR, a->dHR);
+        k_al_q2r<NBK><<<g->nw0 + 3, SlicePlan<NBK>::threads, sm, st>>>(a->HQ, a->dHQ, g->tw_k, g->nw0, nf, a->HR, a->dHR);
         if ((e = launched()) != cudaSuccess) return e;
-        k_al_r2k<NBK><<<g->nw0 + 5, kSliceThreads, sm, st>>>(a->HR, a->dHR, a->Grt, g->er, dG0p, g->tw_k, g->nw0,
+        k_al_r2k<NBK><<<g->nw0 + 5, SlicePlan<NBK>::threads, sm, st>>>(a->HR, a->dHR, a->Grt, g->er, dG0p, g->tw_k, g->nw0,
                                                               g->n8, mu0, a->HK, a->H2K, a->dHK);
         return launched();
     }

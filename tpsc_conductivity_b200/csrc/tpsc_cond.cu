@@ -118,7 +118,7 @@ __global__ void k_cond_table(const double *__restrict__ ek, const double *__rest
 // DST x DCT again.  The first transform at tau = 0 and beta is kept in
 // `pre` for the boundary kernel.
 template <int NBK>
-__global__ void __launch_bounds__(kSliceThreads, 1)
+__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
     k_cond_slice(const double *__restrict__ tab, const double *__restrict__ V, const double2 *__restrict__ tw,
                  int nw0, double T, int K4p, double *__restrict__ hV, double *__restrict__ f0V,
                  double *__restrict__ pre) {
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
         S[c] = (y == 0) ? xa.y * E : (xa.y * t + b) * E;  // row l, column m: c = l NBK + m
     }
     __syncthreads();
-    dst_dct_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+    dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
     const int jv = j < nb ? j : nw0 - j;
     const bool edge = (j == 0 || j == nw0);
     double *pe = pre + (size_t)(2 * y + (j == nw0 ? 1 : 0)) * K4p;
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
         S[c] = v * (2.0 * V[bidx(jv, oct_index(l + 1, m), nb)]);
     }
     __syncthreads();
-    dst_dct_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+    dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
     double *out = (y == 0) ? hV : f0V;
     for (int c = threadIdx.x; c < K4; c += blockDim.x) out[bidx2(j, c, nw0 + 1)] = S[c];
 }
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
                     int nw0, int K4p, double mu0, double T, double nf, double fact, double *__restrict__ dbound) {
     constexpr int K4 = (NBK - 2) * NBK;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = slice_twiddles<NBK, SlicePlan<NBK>::wide>(S, tw);
     const int kind = blockIdx.x;
     const int nb = nw0 / 2 + 1;
     for (int c = threadIdx.x; c < K4; c += blockDim.x) {
@@ -722,21 +722,21 @@ struct RunCondSlices {
     // ny = 2: the h and f0 slices and all four end conditions; ny = 1: h only
     static cudaError_t run(const GridDev *g, const CondDev *c, const double *V, const double *dchirt0, double mu0,
                            double T, double fact, int ny, bool f32, cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes;
+        const size_t sm = SliceSmem<NBK>::bytes, smw = SliceSmem<NBK, SlicePlan<NBK>::wide>::bytes;
         cudaError_t e = set_smem(k_cond_slice<NBK>, sm);
         if (e != cudaSuccess) return e;
-        if ((e = set_smem(k_cond_boundary<NBK>, sm)) != cudaSuccess) return e;
+        if ((e = set_smem(k_cond_boundary<NBK>, smw)) != cudaSuccess) return e;
         const double nf = 1.0 / ((double)g->nk0 * g->nk0);
         k_cond_table<<<(c->K4 + 255) / 256, 256, 0, st>>>(g->ek, c->dek, c->K4, g->nbk, mu0, T, nf, c->tab);
         if ((e = launched()) != cudaSuccess) return e;
         if (f32) {
             if ((e = launch_cond_slice32(*g, *c, V, T, ny, st)) != cudaSuccess) return e;
         } else {
-            k_cond_slice<NBK><<<dim3(g->nw0 + 1, ny), kSliceThreads, sm, st>>>(c->tab, V, g->tw_k, g->nw0, T,
+            k_cond_slice<NBK><<<dim3(g->nw0 + 1, ny), SlicePlan<NBK>::threads, sm, st>>>(c->tab, V, g->tw_k, g->nw0, T,
                                                                                 c->K4p, c->hV, c->f0V, c->pre);
             if ((e = launched()) != cudaSuccess) return e;
         }
-        k_cond_boundary<NBK><<<2 * ny, kSliceThreads, sm, st>>>(g->ek, c->dek, V, dchirt0, g->tw_k, c->pre, g->nw0, c->K4p,
+        k_cond_boundary<NBK><<<2 * ny, kSliceThreads, smw, st>>>(g->ek, c->dek, V, dchirt0, g->tw_k, c->pre, g->nw0, c->K4p,
                                                             mu0, T, nf, fact, c->dbound);
         return launched();
     }

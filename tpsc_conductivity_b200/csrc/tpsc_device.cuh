@@ -145,11 +145,33 @@ cudaError_t finish(Reduce r, int nblocks, double offset0, cudaStream_t st, const
 // ---------------------------------------------------------------------------
 // slice kernels: shared-memory plan of one nbk x nbk slice + FFT scratch
 // ---------------------------------------------------------------------------
+// Threads, FFT groups and CTAs per SM of an FP64 slice kernel.  A pass
+// transforms (NBK + 1)/2 line pairs, one per group of G threads, and the
+// groups' scratch is most of the shared memory, so a block holds the groups
+// that a pass can use and no more: 129 lines take 22 groups (65 pairs in 3
+// rounds, one CTA per SM), smaller slices one group per pair and as many
+// CTAs as the registers allow.  A fixed 352 threads left 25% (65 lines) to
+// 95% (9 lines) of a block idle in the transforms at one CTA per SM.
+// 128^2 x 2048, G slices (2049 per SM-filling launch): 121 -> 100 us, cond
+// slices with both transforms 236 -> 184; 64^2 x 1024, r -> k slices of the
+// Aslamazov-Larkin term 85 -> 60 us.  65 lines in 2 rounds of 17 groups at
+// three CTAs took 104 us, in 3 rounds of 11 groups 119.
 template <int NBK>
+struct SlicePlan {
+    static constexpr int G = FftPlan<2 * (NBK - 1)>::G;
+    static constexpr int ngrp = NBK >= 129 ? kSliceThreads / G : (NBK + 1) / 2;
+    static constexpr int threads = NBK >= 129 ? kSliceThreads : NBK == 17 ? 64 : (ngrp * G + 31) / 32 * 32;
+    static constexpr int blocks = NBK >= 129 ? 1 : NBK == 65 ? 2 : NBK == 33 ? 4 : 8;
+    // groups of a kSliceThreads block: the one- to four-CTA boundary kernels,
+    // whose single slice should be done as soon as possible
+    static constexpr int wide = kSliceThreads / G;
+};
+
+template <int NBK, int NG = SlicePlan<NBK>::ngrp>
 struct SliceSmem {
     static constexpr int L = 2 * (NBK - 1);
     static constexpr int G = FftPlan<L>::G;
-    static constexpr int NGRP = kSliceThreads / G;
+    static constexpr int NGRP = NG;
     static constexpr size_t slice_bytes = (size_t)NBK * NBK * sizeof(double);
     static constexpr size_t scr_off = (slice_bytes + 15) & ~(size_t)15;
     static constexpr size_t tw_off = scr_off + (size_t)NGRP * padded_len(L) * sizeof(double2);
@@ -169,11 +191,11 @@ __device__ __forceinline__ double2 *slice_scratch(double *S) {
 // FFT scratch -- the full table, or where that does not fit the two-level
 // table (entry m = hi[m >> 6] lo[m & 63]); the first __syncthreads of the
 // kernel publishes it.
-template <int NBK>
+template <int NBK, int NG = SlicePlan<NBK>::ngrp>
 __device__ __forceinline__ auto slice_twiddles(double *S, const double2 *__restrict__ tw) {
     constexpr int L = SliceSmem<NBK>::L;
-    char *base = reinterpret_cast<char *>(S) + SliceSmem<NBK>::tw_off;
-    if constexpr (SliceSmem<NBK>::smem_tw) {
+    char *base = reinterpret_cast<char *>(S) + SliceSmem<NBK, NG>::tw_off;
+    if constexpr (SliceSmem<NBK, NG>::smem_tw) {
         double2 *t = reinterpret_cast<double2 *>(base);
         for (int i = threadIdx.x; i < L; i += blockDim.x) t[i] = __ldg(&tw[i]);
         return (const double2 *)t;

@@ -374,7 +374,9 @@ __device__ __forceinline__ void group_fft(C *x, int t, const TW *__restrict__ tw
 // threads of the block must call.  Two lines (rows, then columns) go through
 // one complex FFT of their even extension; the first FFT pass reads the
 // lines straight from S and the last pass writes outputs k < NBK back.
-template <int NBK, class T, class C, class TW>
+// NGRP: groups that transform lines (0: blockDim.x / G); the threads behind
+// them only take part in the barriers.
+template <int NBK, int NGRP = 0, class T, class C, class TW>
 __device__ void dct2_slice(T *S, C *scr, const TW *tw) {
     constexpr int L = 2 * (NBK - 1);
     constexpr int G = FftPlan<L>::G;
@@ -382,7 +384,7 @@ __device__ void dct2_slice(T *S, C *scr, const TW *tw) {
     const int tid = threadIdx.x;
     const int grp = tid / G;
     const int t = tid % G;
-    const int ngrp = blockDim.x / G;
+    const int ngrp = NGRP ? NGRP : blockDim.x / G;
     C *x = scr + grp * padded_len(L);
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
@@ -391,7 +393,7 @@ __device__ void dct2_slice(T *S, C *scr, const TW *tw) {
         const int es = pass == 0 ? 1 : NBK;
         const int ls = pass == 0 ? NBK : 1;
 #pragma unroll 1
-        for (int p = grp; p < NPAIR; p += ngrp) {
+        for (int p = grp; p < NPAIR && grp < ngrp; p += ngrp) {
             const int r0 = 2 * p, r1 = 2 * p + 1;
             const bool two = r1 < NBK;
             T *a = S + r0 * ls;
@@ -421,7 +423,7 @@ __device__ void dct2_slice(T *S, C *scr, const TW *tw) {
 // extension of two packed lines, the DST through the odd extension
 // z = [0, X, 0, -reverse(X)], whose transform is -i Y_a + Y_b for the packed
 // pair a + i b.  Same calling rules as dct2_slice.
-template <int NBK, class T, class C, class TW>
+template <int NBK, int NGRP = 0, class T, class C, class TW>
 __device__ void dst_dct_slice(T *S, C *scr, const TW *tw) {
     constexpr int L = 2 * (NBK - 1);
     constexpr int NR = NBK - 2;
@@ -429,11 +431,11 @@ __device__ void dst_dct_slice(T *S, C *scr, const TW *tw) {
     const int tid = threadIdx.x;
     const int grp = tid / G;
     const int t = tid % G;
-    const int ngrp = blockDim.x / G;
+    const int ngrp = NGRP ? NGRP : blockDim.x / G;
     C *x = scr + grp * padded_len(L);
     // rows: DCT-I along m, NR lines
 #pragma unroll 1
-    for (int p = grp; p < (NR + 1) / 2; p += ngrp) {
+    for (int p = grp; p < (NR + 1) / 2 && grp < ngrp; p += ngrp) {
         const int r0 = 2 * p, r1 = 2 * p + 1;
         const bool two = r1 < NR;
         T *a = S + r0 * NBK;
@@ -454,7 +456,7 @@ __device__ void dst_dct_slice(T *S, C *scr, const TW *tw) {
     __syncthreads();
     // columns: DST-I along l, NBK lines
 #pragma unroll 1
-    for (int p = grp; p < (NBK + 1) / 2; p += ngrp) {
+    for (int p = grp; p < (NBK + 1) / 2 && grp < ngrp; p += ngrp) {
         const int c0 = 2 * p, c1 = 2 * p + 1;
         const bool two = c1 < NBK;
         T *a = S + c0;

@@ -114,7 +114,7 @@ __global__ void k_gk_table(const double *__restrict__ ek, int n8, double mu0, do
 // -G(r, beta - tau), so one table serves both stages.  Plain layout
 // Grt[j * n8 + o].
 template <int NBK>
-__global__ void __launch_bounds__(kSliceThreads, 1)
+__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
     k_gslice(const double2 *__restrict__ gk, const double2 *__restrict__ tw,
              int n8, int nw0, double T, double *__restrict__ Grt) {
     extern __shared__ __align__(16) double S[];
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
         return c.y * exp((c.x > 0 ? -t : bt) * c.x);
     });
     __syncthreads();
-    dct2_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+    dct2_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
     double *out = Grt + (size_t)j * n8;
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
 // j = 0..Nw0/2 (src/chi0.cpp:393-418, 497-517, 545-558).  tau = 0 uses
 // G(r,0-) = G(r,0+) + delta_r0, tau = beta/2 uses 2 G^2.
 template <int NBK>
-__global__ void __launch_bounds__(kSliceThreads, 1)
+__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
     k_chi0_slice(const double *__restrict__ Grt, const double2 *__restrict__ tw,
                  int n8, int nw0, double *__restrict__ chirt, double *__restrict__ chiq) {
     extern __shared__ __align__(16) double S[];
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
     stage_drow<NBK>(gm, Grt + (size_t)(nw0 - j) * n8);
     cp_async_wait_all();
     __syncthreads();
-    fill_from_staged<NBK, kSliceThreads>(S, [&](int o) -> double {
+    fill_from_staged<NBK, SlicePlan<NBK>::threads>(S, [&](int o) -> double {
         const double a = gp[o];
         double c;
         if (j == 0)
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
         return c;
     });
     __syncthreads();
-    dct2_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+    dct2_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
         oct_lm(o, l, m);
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
                     double nk02, double *__restrict__ dG0p, double *__restrict__ dtau_chirt0,
                     double *__restrict__ dtau_chiqt0, Bp b) {
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = slice_twiddles<NBK, SlicePlan<NBK>::wide>(S, tw);
     ek = at(ek, b.arena);
     er = at(er, b.arena);
     Grt = at(Grt, b.arena);
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
 // V(q, iqn) = (T/L^2) U [3 Usp (chisp - chi0) + Uch (chich - chi0)] / 8 and
 // its DCT-I over q, one bosonic frequency per CTA (src/chi.cpp:89-115).
 template <int NBK>
-__global__ void __launch_bounds__(kSliceThreads, 1)
+__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
     k_vertex_q(const double *__restrict__ chiq, const double2 *__restrict__ tw,
                int n8, int nb, double normFact, double U, const double *__restrict__ Usc, double *__restrict__ Vr) {
     extern __shared__ __align__(16) double S[];
@@ -252,14 +252,14 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
     stage_blockrow<NBK>(cs, chiq, j, nb);
     cp_async_wait_all();
     __syncthreads();
-    fill_from_staged<NBK, kSliceThreads>(S, [&](int o) -> double {
+    fill_from_staged<NBK, SlicePlan<NBK>::threads>(S, [&](int o) -> double {
         const double c0 = cs[o];
         const double sp = c0 / (1.0 - Usp * c0 / 2.0);
         const double ch = c0 / (1.0 + Uch * c0 / 2.0);
         return normFact * U * (3.0 * Usp * (sp - c0) + Uch * (ch - c0)) / 8.0;
     });
     __syncthreads();
-    dct2_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+    dct2_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
         oct_lm(o, l, m);
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
                      const double *__restrict__ dG0p, int n8, int nw0, int n8p, double mu0, double U,
                      const double *__restrict__ Usc, double *__restrict__ dS, Bp b) {
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = slice_twiddles<NBK, SlicePlan<NBK>::wide>(S, tw);
     er = at(er, b.arena);
     Grt = at(Grt, b.arena);
     V = at(V, b.arena);
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
 // V(r, tau_j) = V(r, beta - tau_j) for tau_j > beta/2 (src/green.cpp:1822-1885),
 // in FP64 (the mixed form's FP32 slice is k_sigma_slice32).
 template <int NBK>
-__global__ void __launch_bounds__(kSliceThreads, 1)
+__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
     k_sigma_slice(const double *__restrict__ Grt, const double *__restrict__ V,
                   const double2 *__restrict__ tw, int n8, int nw0, int ahead, double *__restrict__ sigt) {
     extern __shared__ __align__(16) double S[];
@@ -342,9 +342,9 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
     stage_drow<NBK>(gs, Grt + (size_t)j * n8);
     cp_async_wait_all();
     __syncthreads();
-    fill_from_staged<NBK, kSliceThreads>(S, [&](int o) -> double { return gs[o] * vs[o]; });
+    fill_from_staged<NBK, SlicePlan<NBK>::threads>(S, [&](int o) -> double { return gs[o] * vs[o]; });
     __syncthreads();
-    dct2_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+    dct2_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
         oct_lm(o, l, m);
@@ -1682,7 +1682,7 @@ struct RunGslice {
         const double nk02 = (double)g->nk0 * g->nk0;
         k_gk_table<<<(g->n8 + 255) / 256, 256, 0, st>>>(g->ek, g->n8, mu0, T, nk02, g->gk, Bp{});
         if ((e = launched()) != cudaSuccess) return e;
-        k_gslice<NBK><<<g->nw0 + 1, kSliceThreads, sm, st>>>(g->gk, g->tw_k, g->n8, g->nw0, T, Grt);
+        k_gslice<NBK><<<g->nw0 + 1, SlicePlan<NBK>::threads, sm, st>>>(g->gk, g->tw_k, g->n8, g->nw0, T, Grt);
         return launched();
     }
 };
@@ -1691,11 +1691,11 @@ struct RunChi0Boundary {
     template <class GT>
     static cudaError_t run(const GridDev *g, const GT *Grt, double mu0, double T, double *dG0p, double *dchirt0,
                            double *dchiqt0, const Bp *b, cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes;
-        cudaError_t e = set_smem(k_chi0_boundary<NBK, GT>, sm);
+        const size_t smw = SliceSmem<NBK, SlicePlan<NBK>::wide>::bytes;
+        cudaError_t e = set_smem(k_chi0_boundary<NBK, GT>, smw);
         if (e != cudaSuccess) return e;
         const double nk02 = (double)g->nk0 * g->nk0;
-        k_chi0_boundary<NBK, GT><<<dim3(1, 1, b->P), kSliceThreads, sm, st>>>(g->ek, g->er, g->tw_k, Grt, g->n8, mu0,
+        k_chi0_boundary<NBK, GT><<<dim3(1, 1, b->P), kSliceThreads, smw, st>>>(g->ek, g->er, g->tw_k, Grt, g->n8, mu0,
                                                                                T, nk02, dG0p, dchirt0, dchiqt0, *b);
         return launched();
     }
@@ -1706,7 +1706,7 @@ struct RunChi0Slice {
         const size_t sm = SliceSmem<NBK>::bytes;
         cudaError_t e = set_smem(k_chi0_slice<NBK>, sm);
         if (e != cudaSuccess) return e;
-        k_chi0_slice<NBK><<<g->nb, kSliceThreads, sm, st>>>(Grt, g->tw_k, g->n8, g->nw0, chirt, chiq);
+        k_chi0_slice<NBK><<<g->nb, SlicePlan<NBK>::threads, sm, st>>>(Grt, g->tw_k, g->n8, g->nw0, chirt, chiq);
         return launched();
     }
 };
@@ -1718,7 +1718,7 @@ struct RunVertexQ {
         cudaError_t e = set_smem(k_vertex_q<NBK>, sm);
         if (e != cudaSuccess) return e;
         const double normFact = T / ((double)g->nk0 * g->nk0);
-        k_vertex_q<NBK><<<g->nb, kSliceThreads, sm, st>>>(chiq, g->tw_k, g->n8, g->nb, normFact, U, Usc, Vr);
+        k_vertex_q<NBK><<<g->nb, SlicePlan<NBK>::threads, sm, st>>>(chiq, g->tw_k, g->n8, g->nb, normFact, U, Usc, Vr);
         return launched();
     }
 };
@@ -1728,10 +1728,10 @@ struct RunSigmaBoundary {
     static cudaError_t run(const GridDev *g, const GT *Grt, const double *V, const double *dchirt0,
                            const double *dG0p, double mu0, double U, const double *Usc, double *dS, const Bp *b,
                            cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes;
-        cudaError_t e = set_smem(k_sigma_boundary<NBK, GT>, sm);
+        const size_t smw = SliceSmem<NBK, SlicePlan<NBK>::wide>::bytes;
+        cudaError_t e = set_smem(k_sigma_boundary<NBK, GT>, smw);
         if (e != cudaSuccess) return e;
-        k_sigma_boundary<NBK, GT><<<dim3(2, 1, b->P), kSliceThreads, sm, st>>>(g->er, g->tw_k, Grt, V, dchirt0, dG0p,
+        k_sigma_boundary<NBK, GT><<<dim3(2, 1, b->P), kSliceThreads, smw, st>>>(g->er, g->tw_k, Grt, V, dchirt0, dG0p,
                                                                                 g->n8, g->nw0, g->n8p, mu0, U, Usc, dS,
                                                                                 *b);
         return launched();
@@ -1743,8 +1743,8 @@ struct RunSigmaSlice {
         const size_t sm = SliceSmem<NBK>::bytes;
         cudaError_t e = set_smem(k_sigma_slice<NBK>, sm);
         if (e != cudaSuccess) return e;
-        const int ahead = resident_ctas(k_sigma_slice<NBK>, kSliceThreads, sm);
-        k_sigma_slice<NBK><<<g->nw0 + 1, kSliceThreads, sm, st>>>(Grt, V, g->tw_k, g->n8, g->nw0, ahead, sigt);
+        const int ahead = resident_ctas(k_sigma_slice<NBK>, SlicePlan<NBK>::threads, sm);
+        k_sigma_slice<NBK><<<g->nw0 + 1, SlicePlan<NBK>::threads, sm, st>>>(Grt, V, g->tw_k, g->n8, g->nw0, ahead, sigt);
         return launched();
     }
 };

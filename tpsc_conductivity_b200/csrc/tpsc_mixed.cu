@@ -32,14 +32,26 @@ namespace {
 
 constexpr int kSlice32Threads = 256;
 
+// Threads, FFT groups and CTAs per SM of an FP32 slice kernel (see SlicePlan):
+// 65 lines in 2 rounds of 17 groups at three CTAs per SM (128^2 x 2048, all
+// five slice kernels: 606 us with 256 threads, 527 so, 554 in one round of 33)
+template <int NBK>
+struct Slice32Plan {
+    static constexpr int G = FftPlan<2 * (NBK - 1)>::G;
+    static constexpr int ngrp = NBK >= 129 ? kSlice32Threads / G : NBK == 65 ? 17 : (NBK + 1) / 2;
+    static constexpr int threads = NBK >= 129 ? kSlice32Threads : NBK == 17 ? 64 : (ngrp * G + 31) / 32 * 32;
+    static constexpr int blocks = NBK >= 129 ? 2 : NBK == 65 ? 3 : NBK == 33 ? 5 : 8;
+};
+
 template <int NBK>
 struct Slice32Smem {
     static constexpr int L = 2 * (NBK - 1);
     static constexpr int G = FftPlan<L>::G;
-    static constexpr int NGRP = kSlice32Threads / G;
+    static constexpr int NGRP = Slice32Plan<NBK>::ngrp;
     static constexpr size_t slice_bytes = (size_t)NBK * NBK * sizeof(float);
     static constexpr size_t scr_off = (slice_bytes + 15) & ~(size_t)15;
-    static constexpr size_t tw_off = scr_off + (size_t)NGRP * padded_len(L) * sizeof(float2);
+    // (the float4 twiddles behind an odd number of 17-point scratch areas)
+    static constexpr size_t tw_off = (scr_off + (size_t)NGRP * padded_len(L) * sizeof(float2) + 15) & ~(size_t)15;
     // the L twiddles, and for L = 256 the second pass's twiddles transposed
     // behind them (15 x 16, see stockham_pass)
     static constexpr int NTW = L + (L == 256 ? 15 * 16 : 0);
@@ -85,7 +97,7 @@ __device__ __forceinline__ const float4 *twiddles32(float *S, const float4 *__re
 // stage, src/green.cpp:1830-1841 and src/chi0.cpp:462-495): G0 formed in
 // FP64, rounded once to float; Grt32[j * n8 + o].
 template <int NBK>
-__global__ void __launch_bounds__(kSlice32Threads, 2)
+__global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::blocks)
     k_gslice32(const double2 *__restrict__ gk, const float4 *__restrict__ tw,
                int n8, int nw0, double T, float *__restrict__ Grt, Bp b) {
     extern __shared__ __align__(16) float S32[];
@@ -101,7 +113,7 @@ __global__ void __launch_bounds__(kSlice32Threads, 2)
         return (float)(c.y * exp((c.x > 0 ? -t : bt) * c.x));
     });
     __syncthreads();
-    dct2_slice<NBK>(S32, scratch32<NBK>(S32), tws);
+    dct2_slice<NBK, Slice32Plan<NBK>::ngrp>(S32, scratch32<NBK>(S32), tws);
     float *out = Grt + (size_t)j * n8;
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
@@ -114,7 +126,7 @@ __global__ void __launch_bounds__(kSlice32Threads, 2)
 // is exact in FP64 and kept there for the tau transforms), its DCT-I in FP32
 // -> chi0(q, tau_j) in FP64 (src/chi0.cpp:393-418, 497-517, 545-558).
 template <int NBK>
-__global__ void __launch_bounds__(kSlice32Threads, 2)
+__global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::blocks)
     k_chi0_slice32(const float *__restrict__ Grt, const float4 *__restrict__ tw,
                    int n8, int nw0, int ahead, double *__restrict__ chirt, double *__restrict__ chiq, Bp b) {
     extern __shared__ __align__(16) float S32[];
@@ -136,7 +148,7 @@ __global__ void __launch_bounds__(kSlice32Threads, 2)
     stage_frow<NBK>(gm, Grt + (size_t)(nw0 - j) * n8);
     cp_async_wait_all();
     __syncthreads();
-    fill_from_staged<NBK, kSlice32Threads>(S32, [&](int o) -> float {
+    fill_from_staged<NBK, Slice32Plan<NBK>::threads>(S32, [&](int o) -> float {
         const double a = gp[o];
         double c;
         if (j == 0)
@@ -149,7 +161,7 @@ __global__ void __launch_bounds__(kSlice32Threads, 2)
         return (float)c;
     });
     __syncthreads();
-    dct2_slice<NBK>(S32, scratch32<NBK>(S32), tws);
+    dct2_slice<NBK, Slice32Plan<NBK>::ngrp>(S32, scratch32<NBK>(S32), tws);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
         oct_lm(o, l, m);
@@ -162,7 +174,7 @@ __global__ void __launch_bounds__(kSlice32Threads, 2)
 //   chi_sp - chi0 = a chi0^2 / (1 - a chi0),  chi_ch - chi0 = -b chi0^2 / (1 + b chi0),
 // so that V takes one FP64 division per point.
 template <int NBK>
-__global__ void __launch_bounds__(kSlice32Threads, 2)
+__global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::blocks)
     k_vertex_q32(const double *__restrict__ chiq, const float4 *__restrict__ tw,
                  int n8, int nb, int ahead, double normFact, double U, const double *__restrict__ Usc,
                  double *__restrict__ Vr, Bp b) {
@@ -181,7 +193,7 @@ __global__ void __launch_bounds__(kSlice32Threads, 2)
     stage_blockrow<NBK>(cs, chiq, j, nb);
     cp_async_wait_all();
     __syncthreads();
-    fill_from_staged<NBK, kSlice32Threads>(S32, [&](int o) -> float {
+    fill_from_staged<NBK, Slice32Plan<NBK>::threads>(S32, [&](int o) -> float {
         const double c0 = cs[o];
         const double a = 0.5 * Usp, b = 0.5 * Uch;
         const double ds = 1.0 - a * c0, dc = 1.0 + b * c0;
@@ -189,7 +201,7 @@ __global__ void __launch_bounds__(kSlice32Threads, 2)
         return (float)(0.125 * normFact * U * c0 * c0 * num / (ds * dc));
     });
     __syncthreads();
-    dct2_slice<NBK>(S32, scratch32<NBK>(S32), tws);
+    dct2_slice<NBK, Slice32Plan<NBK>::ngrp>(S32, scratch32<NBK>(S32), tws);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
         oct_lm(o, l, m);
@@ -221,7 +233,7 @@ struct SigmaSlice32Smem {
 // the Chebyshev recurrence from the FP64 twiddle table entry tw64[t],
 // tw64[m] = exp(-2 pi i m / L), L = 2 (nbk - 1)).
 template <int NBK>
-__global__ void __launch_bounds__(kSlice32Threads, 2)
+__global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::blocks)
     k_sigma_slice32(const float *__restrict__ Grt, const double *__restrict__ V, const float4 *__restrict__ tw,
                     const double2 *__restrict__ tw64, int n8, int nw0, int ahead, double *__restrict__ sigt, Bp b) {
     Grt = at(Grt, b.arena);
@@ -249,7 +261,7 @@ __global__ void __launch_bounds__(kSlice32Threads, 2)
     cp_async_wait_all();
     __syncthreads();
     // octant points o < NOCT are exactly those with l <= R
-    fill_from_staged<NBK, kSlice32Threads>(S32, [&](int o) -> float {
+    fill_from_staged<NBK, Slice32Plan<NBK>::threads>(S32, [&](int o) -> float {
         const double x = (double)gs[o] * vs[o];
         if (o < NOCT) {
             xn[o] = x;
@@ -273,7 +285,7 @@ __global__ void __launch_bounds__(kSlice32Threads, 2)
         u[i] = acc;
     }
     // (the transform's barriers publish u)
-    dct2_slice<NBK>(S32, scratch32<NBK>(S32), tws);
+    dct2_slice<NBK, Slice32Plan<NBK>::ngrp>(S32, scratch32<NBK>(S32), tws);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
         oct_lm(o, l, m);
@@ -293,7 +305,7 @@ __global__ void __launch_bounds__(kSlice32Threads, 2)
 // once; outputs kept in FP64 for the FP64 tau kernel.  h V enters only the
 // Maki-Thompson part of chi_jj and f0 V only its q_n = 0 value.
 template <int NBK>
-__global__ void __launch_bounds__(kSlice32Threads, 2)
+__global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::blocks)
     k_cond_slice32(const double *__restrict__ tab, const double *__restrict__ V, const float4 *__restrict__ tw,
                    int nw0, double T, int K4p, double *__restrict__ hV, double *__restrict__ f0V,
                    double *__restrict__ pre) {
@@ -311,7 +323,7 @@ __global__ void __launch_bounds__(kSlice32Threads, 2)
         S32[c] = (float)((y == 0) ? xa.y * E : (xa.y * t + b) * E);
     }
     __syncthreads();
-    dst_dct_slice<NBK>(S32, scratch32<NBK>(S32), tws);
+    dst_dct_slice<NBK, Slice32Plan<NBK>::ngrp>(S32, scratch32<NBK>(S32), tws);
     const int jv = j < nb ? j : nw0 - j;
     const bool edge = (j == 0 || j == nw0);
     double *pe = pre + (size_t)(2 * y + (j == nw0 ? 1 : 0)) * K4p;
@@ -322,7 +334,7 @@ __global__ void __launch_bounds__(kSlice32Threads, 2)
         S32[c] = (float)(v * (2.0 * V[bidx(jv, oct_index(l + 1, m), nb)]));
     }
     __syncthreads();
-    dst_dct_slice<NBK>(S32, scratch32<NBK>(S32), tws);
+    dst_dct_slice<NBK, Slice32Plan<NBK>::ngrp>(S32, scratch32<NBK>(S32), tws);
     double *out = (y == 0) ? hV : f0V;
     for (int c = threadIdx.x; c < K4; c += blockDim.x) out[bidx2(j, c, nw0 + 1)] = S32[c];
 }
@@ -333,7 +345,7 @@ struct RunCondSlice32 {
         const size_t sm = Slice32Smem<NBK>::bytes;
         cudaError_t e = set_smem(k_cond_slice32<NBK>, sm);
         if (e != cudaSuccess) return e;
-        k_cond_slice32<NBK><<<dim3(g->nw0 + 1, ny), kSlice32Threads, sm, st>>>(c->tab, V, g->tw_k32, g->nw0, T,
+        k_cond_slice32<NBK><<<dim3(g->nw0 + 1, ny), Slice32Plan<NBK>::threads, sm, st>>>(c->tab, V, g->tw_k32, g->nw0, T,
                                                                                c->K4p, c->hV, c->f0V, c->pre);
         return launched();
     }
@@ -350,7 +362,7 @@ struct RunGslice32 {
         cudaError_t e = set_smem(k_gslice32<NBK>, sm);
         if (e != cudaSuccess) return e;
         if ((e = launch_gk_table(*g, mu0, T, st, *b)) != cudaSuccess) return e;
-        k_gslice32<NBK><<<dim3(g->nw0 + 1, 1, b->P), kSlice32Threads, sm, st>>>(g->gk, g->tw_k32, g->n8, g->nw0, T,
+        k_gslice32<NBK><<<dim3(g->nw0 + 1, 1, b->P), Slice32Plan<NBK>::threads, sm, st>>>(g->gk, g->tw_k32, g->n8, g->nw0, T,
                                                                                Grt, *b);
         return launched();
     }
@@ -364,8 +376,8 @@ struct RunChi0Slice32 {
         const size_t sm = Slice32Smem<NBK>::bytes;
         cudaError_t e = set_smem(k_chi0_slice32<NBK>, sm);
         if (e != cudaSuccess) return e;
-        const int ahead = b->P > 1 ? 0 : resident_ctas(k_chi0_slice32<NBK>, kSlice32Threads, sm);
-        k_chi0_slice32<NBK><<<dim3(g->nb, 1, b->P), kSlice32Threads, sm, st>>>(Grt, g->tw_k32, g->n8, g->nw0, ahead,
+        const int ahead = b->P > 1 ? 0 : resident_ctas(k_chi0_slice32<NBK>, Slice32Plan<NBK>::threads, sm);
+        k_chi0_slice32<NBK><<<dim3(g->nb, 1, b->P), Slice32Plan<NBK>::threads, sm, st>>>(Grt, g->tw_k32, g->n8, g->nw0, ahead,
                                                                               chirt, chiq, *b);
         return launched();
     }
@@ -381,8 +393,8 @@ struct RunVertexQ32 {
         cudaError_t e = set_smem(k_vertex_q32<NBK>, sm);
         if (e != cudaSuccess) return e;
         const double normFact = T / ((double)g->nk0 * g->nk0);
-        const int ahead = b->P > 1 ? 0 : resident_ctas(k_vertex_q32<NBK>, kSlice32Threads, sm);
-        k_vertex_q32<NBK><<<dim3(g->nb, 1, b->P), kSlice32Threads, sm, st>>>(chiq, g->tw_k32, g->n8, g->nb, ahead,
+        const int ahead = b->P > 1 ? 0 : resident_ctas(k_vertex_q32<NBK>, Slice32Plan<NBK>::threads, sm);
+        k_vertex_q32<NBK><<<dim3(g->nb, 1, b->P), Slice32Plan<NBK>::threads, sm, st>>>(chiq, g->tw_k32, g->n8, g->nb, ahead,
                                                                             normFact, U, Usc, Vr, *b);
         return launched();
     }
@@ -398,8 +410,8 @@ struct RunSigmaSlice32 {
         const size_t sm = SigmaSlice32Smem<NBK>::bytes;
         cudaError_t e = set_smem(k_sigma_slice32<NBK>, sm);
         if (e != cudaSuccess) return e;
-        const int ahead = b->P > 1 ? 0 : resident_ctas(k_sigma_slice32<NBK>, kSlice32Threads, sm);
-        k_sigma_slice32<NBK><<<dim3(g->nw0 + 1, 1, b->P), kSlice32Threads, sm, st>>>(Grt, V, g->tw_k32, g->tw_k, g->n8,
+        const int ahead = b->P > 1 ? 0 : resident_ctas(k_sigma_slice32<NBK>, Slice32Plan<NBK>::threads, sm);
+        k_sigma_slice32<NBK><<<dim3(g->nw0 + 1, 1, b->P), Slice32Plan<NBK>::threads, sm, st>>>(Grt, V, g->tw_k32, g->tw_k, g->n8,
                                                                                     g->nw0, ahead, sigt, *b);
         return launched();
     }

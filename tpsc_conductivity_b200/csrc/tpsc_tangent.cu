@@ -24,7 +24,7 @@ namespace {
 
 // the tangent of k_gslice: fd[o] = (beta f(xi_o), dxi_o); dGrt[j * n8 + o]
 template <int NBK>
-__global__ void __launch_bounds__(kSliceThreads, 1)
+__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
     k_gslice_tan(const double2 *__restrict__ gk, const double2 *__restrict__ fd, const double2 *__restrict__ tw,
                  int n8, int nw0, double T, double *__restrict__ dGrt) {
     extern __shared__ __align__(16) double S[];
@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
         return c.y * exp((c.x > 0 ? -t : bt) * c.x) * (q.x - t) * q.y;
     });
     __syncthreads();
-    dct2_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+    dct2_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
     double *out = dGrt + (size_t)j * n8;
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
 
 // the tangent of k_chi0_slice (the product rule on each of its three forms)
 template <int NBK>
-__global__ void __launch_bounds__(kSliceThreads, 1)
+__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
     k_chi0_slice_tan(const double *__restrict__ Grt, const double *__restrict__ dGrt,
                      const double2 *__restrict__ tw, int n8, int nw0, double *__restrict__ dchiq) {
     extern __shared__ __align__(16) double S[];
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
         return 2.0 * (dgm[o] * a + gm[o] * da);
     });
     __syncthreads();
-    dct2_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+    dct2_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
         oct_lm(o, l, m);
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
                         double dmu0, double T, double nk02, double *__restrict__ d_dtau_chiqt0,
                         double *__restrict__ out_ddG0p, double *__restrict__ out_ddchir) {
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = slice_twiddles<NBK, SlicePlan<NBK>::wide>(S, tw);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
         oct_lm(o, l, m);
@@ -132,17 +132,17 @@ template <int NBK>
 struct RunChi0Tan {
     static cudaError_t run(const GridDev *g, const TangentBufs *t, double mu0, double dmu0, double T,
                            cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes;
+        const size_t sm = SliceSmem<NBK>::bytes, smw = SliceSmem<NBK, SlicePlan<NBK>::wide>::bytes;
         cudaError_t e;
         if ((e = set_smem(k_gslice_tan<NBK>, sm)) != cudaSuccess) return e;
         if ((e = set_smem(k_chi0_slice_tan<NBK>, sm)) != cudaSuccess) return e;
-        if ((e = set_smem(k_chi0_boundary_tan<NBK>, sm)) != cudaSuccess) return e;
+        if ((e = set_smem(k_chi0_boundary_tan<NBK>, smw)) != cudaSuccess) return e;
         const double nk02 = (double)g->nk0 * g->nk0;
-        k_gslice_tan<NBK><<<g->nw0 + 1, kSliceThreads, sm, st>>>(g->gk, t->fd, g->tw_k, g->n8, g->nw0, T, t->dGrt);
+        k_gslice_tan<NBK><<<g->nw0 + 1, SlicePlan<NBK>::threads, sm, st>>>(g->gk, t->fd, g->tw_k, g->n8, g->nw0, T, t->dGrt);
         if ((e = launched()) != cudaSuccess) return e;
-        k_chi0_slice_tan<NBK><<<g->nb, kSliceThreads, sm, st>>>(t->Grt, t->dGrt, g->tw_k, g->n8, g->nw0, t->dchiq);
+        k_chi0_slice_tan<NBK><<<g->nb, SlicePlan<NBK>::threads, sm, st>>>(t->Grt, t->dGrt, g->tw_k, g->n8, g->nw0, t->dchiq);
         if ((e = launched()) != cudaSuccess) return e;
-        k_chi0_boundary_tan<NBK><<<1, kSliceThreads, sm, st>>>(g->ek, g->er, t->der, t->fd, g->tw_k, t->Grt, t->dGrt,
+        k_chi0_boundary_tan<NBK><<<1, kSliceThreads, smw, st>>>(g->ek, g->er, t->der, t->fd, g->tw_k, t->Grt, t->dGrt,
                                                                t->dG0p, g->n8, mu0, dmu0, T, nk02, t->ddq0,
                                                                t->ddG0p, t->ddchir);
         return launched();
