@@ -546,6 +546,41 @@ __device__ __forceinline__ void sigma_full(double i1, double sinf, double c2, do
     iS = -sinf * i1 + c3 * i2 * i1 + Sv.y * i4;
 }
 
+// The sum rules' Matsubara tail: with x_n = 1/qn^2, chi_n = a x_n + b x_n^2 and h = sgn U/2,
+//   chi/(1 + h chi) - chi = sum_{m>=1} (-h)^m chi^{m+1},
+//   sum_n chi_n^{m+1} = sum_i C(m+1, i) a^{m+1-i} b^i Q_{m+1+i},
+// with the U-independent power sums Q_k = sum_n x_n^k (tailq[k], k <= 2 kTailM + 2).
+// A column whose |h chi_max| >= kTailSeriesMax is summed term by term.
+constexpr int kTailM = 8;
+constexpr double kTailSeriesMax = 0.004;  // (0.004)^8 < 1e-19: series truncation below rounding
+
+__device__ __forceinline__ void tail_series(double a, double b, double h, const double *__restrict__ Q, double &f,
+                                           double &dfdh) {
+    double ap[kTailM + 2], bp[kTailM + 2];
+    ap[0] = bp[0] = 1.0;
+#pragma unroll
+    for (int k = 1; k < kTailM + 2; ++k) {
+        ap[k] = ap[k - 1] * a;
+        bp[k] = bp[k - 1] * b;
+    }
+    f = 0.0;
+    dfdh = 0.0;
+    double hm = 1.0;  // (-h)^(m-1)
+#pragma unroll
+    for (int m = 1; m <= kTailM; ++m) {
+        const int p = m + 1;
+        double Sp = 0.0, coef = 1.0;  // coef = C(p, i)
+#pragma unroll
+        for (int i = 0; i <= p; ++i) {
+            Sp += coef * ap[p - i] * bp[i] * __ldg(&Q[p + i]);
+            coef = coef * (p - i) / (i + 1);
+        }
+        f += (-h) * hm * Sp;           // (-h)^m S_p
+        dfdh += -m * hm * Sp;          // d/dh (-h)^m = -m (-h)^(m-1)
+        hm *= -h;
+    }
+}
+
 // 32-byte streaming load (two 16-byte evict-first loads)
 __device__ __forceinline__ double4 ld_stream4(const double4 *p) {
     const double2 *q = reinterpret_cast<const double2 *>(p);
@@ -572,6 +607,157 @@ __device__ __forceinline__ void trdiff_term(double wn, double rS, double iS, dou
     trdiff_term(wn, rS, iS, e, mu0, pmu, w, v, dv);
     const double x = pmu - e - rS, y = wn - iS, r = 1.0 / (x * x + y * y);
     d2v += 2.0 * w * x * (x * x - 3.0 * y * y) * (r * r * r);
+}
+
+// a row of four: streamed (read once), or left in the caches for the next pass
+template <bool STREAM>
+__device__ __forceinline__ double4 ld_row(const double4 *p) {
+    return STREAM ? ld_stream4(p) : *p;
+}
+
+// a thread's share of column block blk of the sum-rule trace and of its U
+// derivative (k_sumrule; the reference form's root search takes the same
+// values in the same order)
+template <bool STREAM>
+__device__ __forceinline__ void sumrule_block(const double4 *__restrict__ chiq, const double *__restrict__ cinf,
+                                              const double *__restrict__ cinf2, const double *__restrict__ w16,
+                                              const double *__restrict__ tailq, int blk, int nb, int jdir, int tail,
+                                              double Uv, double sgn, double T, double scale, double &out, double &dout) {
+    const double hu = sgn * Uv / 2.0;
+    double v = 0.0, dv = 0.0, tv = 0.0, tdv = 0.0;
+    const int o0 = 4 * blk;
+    const double4 w = *reinterpret_cast<const double4 *>(w16 + o0);
+    const double ww[4] = {w.x, w.y, w.z, w.w};
+    const double4 *col = chiq + (size_t)blk * nb;
+    for (int j = threadIdx.x; j < jdir; j += blockDim.x) {
+        const double4 x = ld_row<STREAM>(&col[j]);
+        const double f = j == 0 ? 0.5 : 1.0;
+        const double xs[4] = {x.x, x.y, x.z, x.w};
+        double sv = 0.0, sd = 0.0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const double q = xs[c] / (1.0 + hu * xs[c]);
+            sv += ww[c] * (q - xs[c]);
+            sd += ww[c] * q * q;
+        }
+        v += f * sv;
+        dv += f * sd;
+    }
+    // tail: n = nwmax+1 .. 2 nwmax
+    const int nwmax = nb - 1;
+    const double tw = 2.0 * 3.141592653589793 * T;
+    const double wn1 = (nwmax + 1) * tw;
+    const double x1 = 1.0 / (wn1 * wn1);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        if (ww[c] == 0.0 || !tail) continue;
+        const double a = cinf[o0 + c], b = cinf2[o0 + c];
+        const double cmax = fabs(a) * x1 + fabs(b) * x1 * x1;
+        if (fabs(hu) * cmax < kTailSeriesMax) {
+            if (threadIdx.x == c) {
+                double f, dfdh;
+                tail_series(a, b, hu, tailq, f, dfdh);
+                tv += ww[c] * f;
+                tdv += ww[c] * dfdh * (0.5 * sgn);
+            }
+        } else {
+            for (int t = threadIdx.x; t < nwmax; t += blockDim.x) {
+                const double wn = (nwmax + 1 + t) * tw;
+                const double i2 = 1.0 / (wn * wn);
+                const double xv = a * i2 + b * i2 * i2;
+                const double q = xv / (1.0 + hu * xv);
+                tv += ww[c] * (q - xv);
+                tdv += ww[c] * (-0.5 * sgn) * q * q;
+            }
+        }
+    }
+    dv *= -0.5 * sgn;
+    out = scale * (v + tv);
+    dout = scale * (dv + tdv);
+}
+
+// a thread's share of column block blk of Tr(G - G0) at pmu and of its
+// derivative (k_trace_diff_G and the reference form's root search)
+template <bool STREAM>
+__device__ __forceinline__ void trace_diff_block(const double2 *__restrict__ S, const double *__restrict__ s2,
+                                                 const double *__restrict__ s3, const double *__restrict__ s4,
+                                                 const double *__restrict__ sinfp, const double *__restrict__ ek,
+                                                 const double *__restrict__ w16, int blk, int nw0, double mu0,
+                                                 double pmu, double T, int jdir, int tail, double &v, double &dv) {
+    const int NO = nw0 / 2;
+    const double sinf = sinfp[0];
+    v = dv = 0.0;
+    const int o0 = 4 * blk;
+    double ww[4], e[4], c2[4], c3[4], c4[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        ww[c] = w16[o0 + c];
+        const bool ok = ww[c] != 0.0;
+        e[c] = ok ? ek[o0 + c] : 0.0;
+        c2[c] = ok ? s2[o0 + c] : 0.0;
+        c3[c] = ok ? s3[o0 + c] : 0.0;
+        c4[c] = ok ? s4[o0 + c] : 0.0;
+    }
+    const double pt = 3.141592653589793 * T;
+    const double4 *row = reinterpret_cast<const double4 *>(S + (size_t)blk * 4 * NO);
+    for (int j = threadIdx.x; j < jdir; j += blockDim.x) {
+        const double wn = (2 * j + 1) * pt;
+        const double i1 = 1.0 / wn;
+        const double4 p = ld_row<STREAM>(&row[2 * j]), q = ld_row<STREAM>(&row[2 * j + 1]);
+        const double2 sv[4] = {make_double2(p.x, p.y), make_double2(p.z, p.w), make_double2(q.x, q.y),
+                               make_double2(q.z, q.w)};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (ww[c] == 0.0) continue;
+            double rS, iS;
+            sigma_full(i1, sinf, c2[c], c3[c], sv[c], rS, iS);
+            trdiff_term(wn, rS, iS, e[c], mu0, pmu, ww[c], v, dv);
+        }
+    }
+    for (int t = threadIdx.x; tail && t <= NO; t += blockDim.x) {
+        const int j = NO + t;
+        const double wn = (2 * j + 1) * pt;
+        const double i1 = 1.0 / wn, i2 = i1 * i1;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (ww[c] == 0.0) continue;
+            const double rS = -c2[c] * i2 + c4[c] * i2 * i2;
+            const double iS = -sinf * i1 + c3[c] * i2 * i1;
+            trdiff_term(wn, rS, iS, e[c], mu0, pmu, ww[c], v, dv);
+        }
+    }
+}
+
+// a thread's share of column block blk of green::traceSelfG2 at mu
+// (src/green.cpp:2929-2976)
+template <bool STREAM>
+__device__ __forceinline__ double trace_self2_block(const double2 *__restrict__ S, const double *__restrict__ s2,
+                                                    const double *__restrict__ s3, const double *__restrict__ sinfp,
+                                                    const double *__restrict__ ek, const double *__restrict__ w16,
+                                                    int blk, int nw0, double mu, double T, double nk02) {
+    const int o0 = 4 * blk, NO = nw0 / 2;
+    const double sinf = sinfp[0];
+    const double pt = 3.141592653589793 * T;
+    KSum v;
+    const double4 *row = reinterpret_cast<const double4 *>(S + (size_t)blk * 4 * NO);
+    for (int j = threadIdx.x; j < NO; j += blockDim.x) {
+        const double wn = (2 * j + 1) * pt;
+        const double i1 = 1.0 / wn;
+        const double4 p = ld_row<STREAM>(&row[2 * j]), q = ld_row<STREAM>(&row[2 * j + 1]);
+        const double2 sv[4] = {make_double2(p.x, p.y), make_double2(p.z, p.w), make_double2(q.x, q.y),
+                               make_double2(q.z, q.w)};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const double w8 = 0.5 * w16[o0 + c];
+            if (w8 == 0.0) continue;
+            double rS, iS;
+            sigma_full(i1, sinf, s2[o0 + c], s3[o0 + c], sv[c], rS, iS);
+            const double a = ek[o0 + c] - mu + rS;
+            const double tmp = w8 * T * 2 / (nk02 * ((wn - iS) * (wn - iS) + a * a));
+            v.add(tmp * (iS * wn - iS * iS - (ek[o0 + c] - mu) * rS - rS * rS));
+        }
+    }
+    return v.value();
 }
 
 // complex division

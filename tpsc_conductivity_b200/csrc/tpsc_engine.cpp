@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "../../include/tpsc_b200.h"
+#include "tpsc_findzero.h"
 #include "tpsc_host.h"
 #include "tpsc_kernels.cuh"
 
@@ -30,247 +31,9 @@ const double PI = std::acos(-1.0);
 const double EPS = std::numeric_limits<double>::epsilon();
 
 // ---------------------------------------------------------------------------
-// Root search with the control flow of generique::find_zero: bracketing
-// inverse-quadratic interpolation with secant and bisection fallbacks, tol
-// 1e-16 and 20 iterations (src/generique.cpp:604-913); with lims, the bounded
-// variant: tol 1e-15, 12 iterations, eps = 2 machine epsilons
-// (src/generique.cpp:917-1234).  The evaluator returns false on a device
-// error, which aborts the search.
-// ---------------------------------------------------------------------------
-template <typename F>
-bool find_zero(F &&func, const double init[3], double *root, const double *lims, int *nev, bool *dev_err) {
-    double tol, eps;
-    int itmax;
-    if (!lims) {
-        tol = 1.0e-16;
-        eps = 10.0 * EPS;
-        itmax = 20;
-    } else {
-        tol = 1.0e-15;
-        eps = 2.0 * EPS;
-        itmax = 12;
-    }
-    *nev = 0;
-    *dev_err = false;
-    auto f = [&](double x, double &y) -> bool {
-        ++*nev;
-        if (!func(x, y)) {
-            *dev_err = true;
-            return false;
-        }
-        return true;
-    };
-    int nbiter = 0;
-    const double dytol = 0.01;
-    double x0 = init[0], xmin = init[1], xmax = init[2];
-    double ymin, ymax;
-    if (!f(xmin, ymin) || !f(xmax, ymax)) return false;
-    double x[3] = {x0, xmin, xmax}, y[3] = {0.0, ymin, ymax};
-    if (std::fabs(ymin) < tol) {
-        *root = xmin;
-        return true;
-    }
-    if (std::fabs(ymax) < tol) {
-        *root = xmax;
-        return true;
-    }
-    if (ymin * ymax > 0) {
-        if (!f(x[0], y[0])) return false;
-        if (std::fabs(y[0]) < tol) {
-            *root = x[0];
-            return true;
-        }
-        if (y[0] * y[2] < 0) {
-            const double xt = x[0];
-            x[0] = (x[0] + x[2]) / 2;
-            x[1] = xt;
-            y[1] = y[0];
-        } else {
-            double ytmp = y[0], xtmp = x[0], xtmp1, ytmp1;
-            if (std::fabs(y[1]) < std::fabs(ytmp)) ytmp = y[1], xtmp = x[1];
-            if (std::fabs(y[2]) < std::fabs(ytmp)) ytmp = y[2], xtmp = x[2];
-            xtmp1 = xtmp + 10 * eps;
-            if (!f(xtmp1, ytmp1)) return false;
-            xtmp1 = xtmp - ytmp * ((xtmp1 - xtmp) / (ytmp1 - ytmp));
-            if (!f(xtmp1, ytmp1)) return false;
-            nbiter++;
-            while (std::fabs(ytmp1) > tol && nbiter < itmax && ytmp1 * ytmp > 0 && std::isfinite(xtmp1)) {
-                xtmp = xtmp1;
-                ytmp = ytmp1;
-                xtmp1 = xtmp + 10 * eps;
-                if (!f(xtmp1, ytmp1)) return false;
-                xtmp1 = xtmp - ytmp * ((xtmp1 - xtmp) / (ytmp1 - ytmp));
-                if (!f(xtmp1, ytmp1)) return false;
-                nbiter++;
-            }
-            if (std::fabs(ytmp1) < tol) {
-                *root = xtmp1;
-                return true;
-            }
-            if (ytmp1 * ytmp < 0) {
-                x[0] = (xtmp + xtmp1) / 2;
-                x[1] = xtmp;
-                y[1] = ytmp;
-                x[2] = xtmp1;
-                y[2] = ytmp1;
-            }
-            if (nbiter >= itmax) return false;
-            if (!std::isfinite(xtmp1)) return false;
-        }
-    }
-    if (lims) {
-        if (x[1] < lims[0] || x[1] > lims[1] || x[2] < lims[0] || x[2] > lims[1]) return false;
-    }
-    if (std::fabs(xmax - xmin) < eps) {
-        *root = xmin;
-        return true;
-    }
-    if (!f(x[0], y[0])) return false;
-    if (std::fabs(y[0]) < tol) {
-        *root = x[0];
-        return true;
-    }
-    int ind1, ind2, ind3, indm = 0, indp = 0, indfar, indmid;
-    auto classify = [&]() {
-        if (y[0] * y[1] > 0)
-            ind1 = 0, ind2 = 1;
-        else if (y[0] * y[2] > 0)
-            ind1 = 0, ind2 = 2;
-        else
-            ind1 = 1, ind2 = 2;
-        ind3 = 3 - ind1 - ind2;
-        if (x[ind3] > x[ind1]) {
-            if (x[ind1] > x[ind2])
-                indfar = ind2, indmid = ind1;
-            else
-                indfar = ind1, indmid = ind2;
-            indm = indmid, indp = ind3;
-        } else {
-            if (x[ind1] < x[ind2])
-                indfar = ind2, indmid = ind1;
-            else
-                indfar = ind1, indmid = ind2;
-            indm = ind3, indp = indmid;
-        }
-    };
-    classify();
-    x[indfar] = -y[indmid] * (x[ind3] - x[indmid]) / (y[ind3] - y[indmid]) + x[indmid];
-    if (!f(x[indfar], y[indfar])) return false;
-    double dy = y[indfar], dyprec;
-    double a = 0.0, b = 0.0, c = 0.0;
-    while (std::fabs(dy) > tol && nbiter < itmax) {
-        classify();
-        const double denom = -x[0] * x[0] * x[2] + x[0] * x[0] * x[1] - x[0] * x[1] * x[1] + x[0] * x[2] * x[2] -
-                             x[2] * x[2] * x[1] + x[2] * x[1] * x[1];
-        if (std::fabs(denom) > 0.0) {
-            a = (x[0] * y[2] - x[0] * y[1] + x[2] * y[1] - y[2] * x[1] - y[0] * x[2] + y[0] * x[1]) / denom;
-            b = -(-y[2] * x[1] * x[1] + x[1] * x[1] * y[0] - x[2] * x[2] * y[0] - y[1] * x[0] * x[0] +
-                  y[2] * x[0] * x[0] + y[1] * x[2] * x[2]) /
-                denom;
-            c = (y[2] * x[0] * x[0] * x[1] - y[1] * x[0] * x[0] * x[2] - x[1] * x[1] * x[0] * y[2] +
-                 x[2] * x[2] * x[0] * y[1] + x[1] * x[1] * y[0] * x[2] - x[2] * x[2] * y[0] * x[1]) /
-                denom;
-        }
-        if ((b * b - 4.0 * a * c) > 0.0 && std::fabs(denom) > 0.0) {
-            const double sq = std::sqrt(b * b - 4.0 * a * c);
-            const double xp = (-b + sq) / (2 * a), xm = (-b - sq) / (2 * a);
-            if (xp > x[indm] && xp < x[indp])
-                x[indfar] = xp;
-            else if (xm > x[indm] && xm < x[indp])
-                x[indfar] = xm;
-            else if (std::fabs(y[ind3] - y[indmid]) > tol)
-                x[indfar] = -y[indmid] * (x[ind3] - x[indmid]) / (y[ind3] - y[indmid]) + x[indmid];
-            else {
-                *root = x[indmid];
-                return true;
-            }
-        } else {
-            if (std::fabs(y[ind3] - y[indmid]) > tol)
-                x[indfar] = -y[indmid] * (x[ind3] - x[indmid]) / (y[ind3] - y[indmid]) + x[indmid];
-            else {
-                *root = x[indmid];
-                return true;
-            }
-        }
-        if (!f(x[indfar], y[indfar])) return false;
-        dyprec = std::fabs(dy);
-        dy = y[indfar];
-        if (std::fabs(dyprec - std::fabs(dy)) < dytol * dyprec || dyprec < std::fabs(dy)) {
-            x[indfar] = (x[ind3] + x[indmid]) / 2.0;
-            if (!f(x[indfar], y[indfar])) return false;
-            dy = y[indfar];
-        }
-        nbiter++;
-    }
-    int best = 0;
-    *root = x[0];
-    if (std::fabs(y[1]) < std::fabs(y[best])) {
-        *root = x[1];
-        best = 1;
-    }
-    if (std::fabs(y[2]) < std::fabs(y[best])) *root = x[2];
-    return true;
-}
-
-// ---------------------------------------------------------------------------
-// Safeguarded Newton root search for the Newton form: f returns the value and
-// the derivative (from the same device pass).  [lo, hi] is the reference's
-// search interval; it shrinks to the side of each evaluation that the
-// derivative's sign and the value's sign rule out, and a Newton step that
-// leaves it is replaced by the midpoint.  Converged when |f| is below tol,
-// when the step is below 1e-14 relative, or when the step stops shrinking
-// (at most half the previous one) while already below 1e-10 relative: f is
-// then at its rounding-noise floor and further steps only dither.
-// ---------------------------------------------------------------------------
-template <typename F>
-bool newton_root(F &&func, double x0, double lo, double hi, double tol, double *root, int *nev, bool *dev_err) {
-    *nev = 0;
-    *dev_err = false;
-    // the start must lie strictly inside the interval (the spin sum rule has
-    // its pole at the upper end: U/2 can lie beyond it)
-    double x = (x0 > lo && x0 < hi) ? x0 : 0.5 * (lo + hi), prev_step = 0.0;
-    for (int it = 0; it < 60; ++it) {
-        double y, dy;
-        ++*nev;
-        if (!func(x, y, dy)) {
-            *dev_err = true;
-            return false;
-        }
-        if (!std::isfinite(y) || !std::isfinite(dy)) return false;
-        if (std::fabs(y) < tol) {
-            *root = x;
-            return true;
-        }
-        // the root lies on the side where f changes sign
-        if ((y > 0) == (dy > 0))
-            hi = std::min(hi, x);
-        else
-            lo = std::max(lo, x);
-        const double scale = std::max(1.0, std::fabs(x));
-        double xn = (dy != 0.0) ? x - y / dy : 0.5 * (lo + hi);
-        // convergence is judged on the Newton step itself, before the bracket
-        // safeguard: at the root the step rounds to (or next to) x, which may
-        // coincide with the bracket end just moved to x
-        if (dy != 0.0 && std::fabs(xn - x) <= 1e-14 * scale) {
-            *root = xn;
-            return true;
-        }
-        if (!(xn >= lo && xn <= hi)) xn = 0.5 * (lo + hi);
-        const double step = std::fabs(xn - x);
-        if (it >= 2 && step < 1e-10 * scale && step > 0.5 * prev_step) {
-            *root = xn;
-            return true;
-        }
-        prev_step = step;
-        x = xn;
-    }
-    return false;
-}
-
-// ---------------------------------------------------------------------------
 // one (nk0, Nw0) grid: tables and arrays
 // ---------------------------------------------------------------------------
-// What a Newton-form solve's launches take beyond the grid's buffers: the
+// What a solve's launches take beyond the grid's buffers: the
 // key of a captured solve graph (tpsc_set_graph_mode)
 struct SolveKey {
     int form = -1, cap = -1;
@@ -328,7 +91,7 @@ struct Grid {
     double tailP_host[kTailP] = {0};
     std::vector<void *> allocs;
     unsigned warm_forms = 0;  // bit f: a direct (uncaptured) Newton solve in form f ran on this grid
-    // the Newton-form solve on this grid as an executable CUDA graph, the key
+    // the solve on this grid as an executable CUDA graph, the key
     // it was captured with and the kernels in it
     cudaGraphExec_t graph_exec = nullptr;
     SolveKey graph_key;
@@ -421,7 +184,7 @@ struct tpsc_ctx {
     size_t snap_bytes[2] = {0, 0};
     int snap_next = 0;
     bool copies_pending = false;
-    // Newton-form solves as CUDA graphs (tpsc_set_graph_mode; the executable
+    // solves as CUDA graphs (tpsc_set_graph_mode; the executable
     // graphs live in the grids)
     int graph_mode = 1;       // 0 off, 1 replay a repeated solve, 2 capture every solve
     bool graph_off = false;   // a capture failed: direct launches from then on
@@ -763,33 +526,17 @@ int grid_set_model(tpsc_ctx *ctx, Grid *g) {
         g->mu0 = 0.0 + ctx->mu_shift;
         return TPSC_OK;
     }
-    int rc = TPSC_OK;
-    if (ctx->form & TPSC_FORM_NEWTON) {
+    // r = (mu0, iterations) of the Newton search or (mu0, success) of find_zero
+    const bool newton = (ctx->form & TPSC_FORM_NEWTON) != 0;
+    if (newton)
         CK(launch_mu0_newton(d, ctx->n, ctx->T, ctx->red, ctx->st));
-        double r[2];
-        if ((rc = read_result(ctx, 2, r))) return rc;
-        if (!std::isfinite(r[0]) || r[1] >= 200) return fail(ctx, TPSC_ERR_NO_ROOT, "mu0 not found");
-        g->mu0 = r[0] + ctx->mu_shift;
-        return TPSC_OK;
-    }
-    auto dens = [&](double mu, double &y) -> bool {
-        cudaError_t e = launch_density(d, mu, ctx->n, ctx->T, ctx->red, ctx->st);
-        if (e != cudaSuccess) {
-            rc = cuda_fail(ctx, e, "launch_density");
-            return false;
-        }
-        rc = read_result(ctx, 1, &y);
-        return rc == TPSC_OK;
-    };
-    const double init[3] = {0.0, -8.0, 8.0};
-    double root = 0;
-    int nev;
-    bool derr;
-    if (!find_zero(dens, init, &root, nullptr, &nev, &derr)) {
-        if (derr) return rc;
-        return fail(ctx, TPSC_ERR_NO_ROOT, "mu0 not found");
-    }
-    g->mu0 = root + ctx->mu_shift;
+    else
+        CK(launch_mu0_zero(d, ctx->n, ctx->T, ctx->red, ctx->st));
+    double r[2];
+    int rc = read_result(ctx, 2, r);
+    if (rc) return rc;
+    if (!std::isfinite(r[0]) || (newton ? r[1] >= 200 : r[1] != 1.0)) return fail(ctx, TPSC_ERR_NO_ROOT, "mu0 not found");
+    g->mu0 = r[0] + ctx->mu_shift;
     return TPSC_OK;
 }
 
@@ -856,12 +603,14 @@ int set_roots(tpsc_ctx *ctx, const double *r, unsigned err) {
     return TPSC_OK;
 }
 // r = (Tr Sigma G0, its asymptotic part, mu, evals, ok, Tr Sigma G at mu, -, Sigma_inf)
-// of the Newton-form mu search, err its barrier flag
-int set_mu(tpsc_ctx *ctx, const double *r, int err) {
+// of the mu search, err its barrier flag; traces: r[0..1] were formed
+int set_mu(tpsc_ctx *ctx, const double *r, int err, bool traces) {
     if (err) return fail(ctx, TPSC_ERR_CUDA, "device mu search: grid barrier timed out");
     ctx->scal[TPSC_S_SIGMA_INF] = r[7];
-    ctx->scal[TPSC_S_TR_SG] = r[0];
-    ctx->scal[TPSC_S_TR_SG_ASYMP] = r[0] + r[1];
+    if (traces) {
+        ctx->scal[TPSC_S_TR_SG] = r[0];
+        ctx->scal[TPSC_S_TR_SG_ASYMP] = r[0] + r[1];
+    }
     if (r[4] != 1.0) return fail(ctx, TPSC_ERR_NO_ROOT, "mu not found");
     ctx->scal[TPSC_S_MU] = r[2];
     ctx->scal[TPSC_S_EVALS_MU] = r[3];
@@ -870,8 +619,8 @@ int set_mu(tpsc_ctx *ctx, const double *r, int err) {
     return TPSC_OK;
 }
 
-// read: take chi0max back now and check it; a Newton-form solve leaves that
-// to its one readback at the end (the root search reads the device value)
+// read: take chi0max back now and check it; a solve leaves that to its one
+// readback at the end (the root search reads the device value)
 int run_chi0(tpsc_ctx *ctx, bool read = true) {
     Grid *g = ctx->cur;
     const GridDev &d = g->d;
@@ -994,94 +743,37 @@ int sumrule(tpsc_ctx *ctx, int channel, double Uv, double *tr, double *dtr) {
 }
 
 // chi::find_Usp_Uch(nq0, nw0, Usc) on the current grid after chi0 (src/chi.cpp:850-876)
-// read: take the roots back now; a Newton-form solve defers that to its one
-// readback at the end, the interval's end then coming from the device chi0max
+// read: take the roots back now; a solve defers that to its one readback at
+// the end, the interval's end then coming from the device chi0max
 int roots_Usp_Uch(tpsc_ctx *ctx, double Usc[2], bool read = true) {
     const double n = ctx->n, U = ctx->U, nsr = ctx->nsr;
-    const bool newton = (ctx->form & TPSC_FORM_NEWTON) != 0;
     int rc = TPSC_OK;
-    if (newton) {
-        // both roots in one cooperative launch (tpsc_roots.cu), into ctx->dres
-        Grid *g = ctx->cur;
-        if ((rc = ensure_moments(ctx, g))) return rc;
-        RootScratch rs = ctx->roots;
-        rs.out = ctx->dres;
-        if (read)
-            CK(launch_sumrule_roots(g->d, g->chiq, g->cinf, g->cinf2, g->d_mom_suf, g->d_cmax_suf, g->d_tailm,
-                                    ctx->T, n, nsr, U, 2.0 / ctx->scal[TPSC_S_CHI0MAX] - 2 * EPS, rs, ctx->st));
-        else
-            CK(launch_sumrule_roots(g->d, g->chiq, g->cinf, g->cinf2, g->d_mom_suf, g->d_cmax_suf, g->d_tailm,
-                                    ctx->T, n, nsr, U, 0.0, rs, ctx->st, ctx->red.result, 2 * EPS));
-        ctx->roots.reset_sr = true;
-        ctx->cur->have_U = true;
-        if (!read) return TPSC_OK;
-        // the results and the barrier's error flag in one readback
-        if ((rc = read_back(ctx, {{ctx->dres, 6 * sizeof(double), 0}, {ctx->roots.bar + 2, sizeof(unsigned), 6}})))
-            return rc;
-        unsigned err;
-        std::memcpy(&err, ctx->h_res + 6, sizeof(unsigned));
-        ctx->roots.reset_sr = err != 0;
-        if ((rc = set_roots(ctx, ctx->h_res, err))) return rc;
-        Usc[0] = ctx->Usp;
-        Usc[1] = ctx->Uch;
-        return TPSC_OK;
-    }
-    // R_sp(Us) = trace + n - n^2/2 - nsr + Us nsr^2/(2U)  (chi::sum_rule_sp, src/chi.cpp:833-836)
-    auto rsp = [&](double Us, double &y, double &dy) -> bool {
-        double tr, dtr;
-        rc = sumrule(ctx, 0, Us, &tr, &dtr);
-        if (rc) return false;
-        y = tr + n - n * n / 2.0 - nsr + Us * nsr * nsr / (2.0 * U);
-        dy = dtr + nsr * nsr / (2.0 * U);
-        return true;
-    };
-    auto rsp1 = [&](double Us, double &y) -> bool {
-        double dy;
-        return rsp(Us, y, dy);
-    };
-    const double init_sp[3] = {U / 2.0, 0.0, 2.0 / ctx->scal[TPSC_S_CHI0MAX] - 2 * EPS};
-    int nev;
-    bool derr, ok;
-    double root = 0;
-    ok = newton ? newton_root(rsp, init_sp[0], init_sp[1], init_sp[2], 1e-16, &root, &nev, &derr)
-                : find_zero(rsp1, init_sp, &root, nullptr, &nev, &derr);
-    if (!ok) {
-        if (derr) return rc;
-        return fail(ctx, TPSC_ERR_NO_ROOT, "Usp not found");
-    }
-    ctx->scal[TPSC_S_EVALS_SP] = nev;
-    Usc[0] = root;
-    ctx->Usp = root;
-    // R_ch(Uc) = trace + n - n^2/2 - (nsr + Usp nsr^2/(2U) - nsr^2)  (src/chi.cpp:840-843)
-    auto rch = [&](double Uc, double &y, double &dy) -> bool {
-        double tr, dtr;
-        rc = sumrule(ctx, 1, Uc, &tr, &dtr);
-        if (rc) return false;
-        y = tr + n - n * n / 2.0 - (nsr + ctx->Usp * nsr * nsr / (2.0 * U) - nsr * nsr);
-        dy = dtr;
-        return true;
-    };
-    auto rch1 = [&](double Uc, double &y) -> bool {
-        double dy;
-        return rch(Uc, y, dy);
-    };
-    const double init_ch[3] = {0.0, 0.0, 1000.0 * U};
-    // the Newton form starts the charge search at U (the interval's lower end
-    // is not an interior point)
-    ok = newton ? newton_root(rch, U, init_ch[1], init_ch[2], 1e-16, &root, &nev, &derr)
-                : find_zero(rch1, init_ch, &root, nullptr, &nev, &derr);
-    if (!ok) {
-        if (derr) return rc;
-        return fail(ctx, TPSC_ERR_NO_ROOT, "Uch not found");
-    }
-    ctx->scal[TPSC_S_EVALS_CH] = nev;
-    Usc[1] = root;
-    ctx->Uch = root;
-    ctx->scal[TPSC_S_USP] = ctx->Usp;
-    ctx->scal[TPSC_S_UCH] = ctx->Uch;
-    ctx->cur->have_U = true;
+    // both roots in one cooperative launch (tpsc_roots.cu), into ctx->dres,
     // where the vertex and Sigma kernels read them
-    CK(launch_store(ctx->dres, Usc, 2, ctx->st));
+    Grid *g = ctx->cur;
+    RootScratch rs = ctx->roots;
+    rs.out = ctx->dres;
+    const double hi = read ? 2.0 / ctx->scal[TPSC_S_CHI0MAX] - 2 * EPS : 0.0, off = read ? 0.0 : 2 * EPS;
+    const double *chi0max = read ? nullptr : ctx->red.result;
+    if (ctx->form & TPSC_FORM_NEWTON) {
+        if ((rc = ensure_moments(ctx, g))) return rc;
+        CK(launch_sumrule_roots(g->d, g->chiq, g->cinf, g->cinf2, g->d_mom_suf, g->d_cmax_suf, g->d_tailm, ctx->T, n,
+                                nsr, U, hi, rs, ctx->st, chi0max, off));
+    } else {
+        CK(launch_sumrule_zero(g->d, g->chiq, g->cinf, g->cinf2, ctx->T, n, nsr, U, hi, rs, ctx->st, chi0max, off));
+    }
+    ctx->roots.reset_sr = true;
+    ctx->cur->have_U = true;
+    if (!read) return TPSC_OK;
+    // the results and the barrier's error flag in one readback
+    if ((rc = read_back(ctx, {{ctx->dres, 6 * sizeof(double), 0}, {ctx->roots.bar + 2, sizeof(unsigned), 6}})))
+        return rc;
+    unsigned err;
+    std::memcpy(&err, ctx->h_res + 6, sizeof(unsigned));
+    ctx->roots.reset_sr = err != 0;
+    if ((rc = set_roots(ctx, ctx->h_res, err))) return rc;
+    Usc[0] = ctx->Usp;
+    Usc[1] = ctx->Uch;
     return TPSC_OK;
 }
 
@@ -1105,8 +797,8 @@ int run_vertex(tpsc_ctx *ctx) {
     return TPSC_OK;
 }
 
-// settle: read Sigma_inf back now; a Newton-form solve leaves it to the
-// readback of the mu search that follows
+// settle: read Sigma_inf back now; a solve leaves it to the readback of the mu
+// search that follows
 int run_self(tpsc_ctx *ctx, bool settle = true) {
     Grid *g = ctx->cur;
     if (!g || !g->have_V) return fail(ctx, TPSC_ERR_STATE, "the vertex V(r, tau) has not been computed");
@@ -1175,35 +867,36 @@ void mu_series_cut(const tpsc_ctx *ctx, int *jc_out, double *wc_out) {
     mu_series_cut(ctx->cur->d.nw0, ctx->T, jc_out, wc_out);
 }
 
-// The Newton form of traceSelfG + find_mu + traceSelfG2: one pass over Sigma
-// for Tr Sigma G0 and the series moments (k_sigma_moments), then the Newton
-// search and Tr Sigma G at mu in one cooperative launch (k_mu_roots), one
-// readback for all of it.
-int queue_mu_newton(tpsc_ctx *ctx) {
+// traceSelfG + find_mu + traceSelfG2.  The Newton form makes one pass over
+// Sigma for Tr Sigma G0 and the series moments (k_sigma_moments), then the
+// Newton search and Tr Sigma G at mu in one cooperative launch (k_mu_roots);
+// the reference form takes find_zero and Tr Sigma G at mu in one cooperative
+// launch (k_mu_zero), and in a solve (traces) Tr Sigma G0 by itself before it.
+// sigma_traces: where the two parts of Tr Sigma G0 are left
+// (ctx->red.result[0..2] holds chi0max).
+const double *sigma_traces(const tpsc_ctx *ctx) {
+    return (ctx->form & TPSC_FORM_NEWTON) ? ctx->redm.result : ctx->red.result + 4;
+}
+int queue_mu_search(tpsc_ctx *ctx, bool traces) {
     Grid *g = ctx->cur;
     const GridDev &d = g->d;
-    int jc;
-    double wc;
-    mu_series_cut(ctx, &jc, &wc);
-    CK(launch_sigma_moments(d, g->S, g->s2, g->s3, g->s4, g->sinf, g->mu0, ctx->T, jc, ctx->redm, ctx->st));
-    CK(launch_mu_roots(d, g->S, g->s2, g->s3, g->s4, g->sinf, ctx->redm.result, g->mu0, ctx->T, jc, wc, ctx->roots,
-                       ctx->st));
+    if (ctx->form & TPSC_FORM_NEWTON) {
+        int jc;
+        double wc;
+        mu_series_cut(ctx, &jc, &wc);
+        CK(launch_sigma_moments(d, g->S, g->s2, g->s3, g->s4, g->sinf, g->mu0, ctx->T, jc, ctx->redm, ctx->st));
+        CK(launch_mu_roots(d, g->S, g->s2, g->s3, g->s4, g->sinf, ctx->redm.result, g->mu0, ctx->T, jc, wc, ctx->roots,
+                           ctx->st));
+    } else {
+        if (traces) {
+            Reduce r = ctx->red;
+            r.result += 4;
+            CK(launch_trace_self_G(d, g->S, g->s2, g->s3, g->sinf, g->mu0, ctx->T, r, ctx->st));
+        }
+        CK(launch_mu_zero(d, g->S, g->s2, g->s3, g->s4, g->sinf, g->mu0, ctx->T, ctx->roots, ctx->st));
+    }
     ctx->roots.reset_mu = true;
     return TPSC_OK;
-}
-
-int self_traces_and_mu_newton(tpsc_ctx *ctx) {
-    int rc = queue_mu_newton(ctx);
-    if (rc) return rc;
-    if ((rc = read_back(ctx, {{ctx->redm.result, 2 * sizeof(double), 0},
-                              {ctx->roots.out, 4 * sizeof(double), 2},
-                              {ctx->roots.bar + 6, sizeof(int), 6},
-                              {ctx->cur->sinf, sizeof(double), 7}})))
-        return rc;
-    int err;
-    std::memcpy(&err, ctx->h_res + 6, sizeof(int));
-    ctx->roots.reset_mu = err != 0;
-    return set_mu(ctx, ctx->h_res, err);
 }
 
 // stage times from ctx->ev[0..5] and the finiteness check of the scalars
@@ -1226,12 +919,12 @@ int mark(tpsc_ctx *ctx, int i) {
     return TPSC_OK;
 }
 
-// The Newton-form solve from the chi0 stage on, queued on ctx->st without a
+// The solve from the chi0 stage on, queued on ctx->st without a
 // host round trip (the roots, the vertex and Sigma read their inputs on the
 // device), ending in the gather of everything the host checks into ctx->h_res;
-// newton_finish waits for it and checks chi0max, the sum-rule roots, the mu
+// solve_finish waits for it and checks chi0max, the sum-rule roots, the mu
 // search and their barrier flags in stage order.
-int newton_queue(tpsc_ctx *ctx) {
+int solve_queue(tpsc_ctx *ctx) {
     double Usc[2];
     int rc;
     if ((rc = mark(ctx, 0))) return rc;
@@ -1243,20 +936,20 @@ int newton_queue(tpsc_ctx *ctx) {
     if ((rc = mark(ctx, 3))) return rc;
     if ((rc = run_self(ctx, false))) return rc;
     if ((rc = mark(ctx, 4))) return rc;
-    if ((rc = queue_mu_newton(ctx))) return rc;
+    if ((rc = queue_mu_search(ctx, true))) return rc;
     if ((rc = mark(ctx, 5))) return rc;
     // h_res: [0..2] chi0max, qmax; [3..8] the sum-rule roots; [9] their flag;
     // [10..11] the Sigma traces; [12..15] the mu search; [16] its flag; [17] Sigma_inf
     return queue_read_back(ctx, {{ctx->red.result, 3 * sizeof(double), 0},
                                  {ctx->dres, 6 * sizeof(double), 3},
                                  {ctx->roots.bar + 2, sizeof(unsigned), 9},
-                                 {ctx->redm.result, 2 * sizeof(double), 10},
+                                 {sigma_traces(ctx), 2 * sizeof(double), 10},
                                  {ctx->roots.out, 4 * sizeof(double), 12},
                                  {ctx->roots.bar + 6, sizeof(int), 16},
                                  {ctx->cur->sinf, sizeof(double), 17}});
 }
 
-int newton_finish(tpsc_ctx *ctx) {
+int solve_finish(tpsc_ctx *ctx) {
     CK(cudaStreamSynchronize(ctx->st));
     int rc;
     const double *h = ctx->h_res;
@@ -1273,19 +966,20 @@ int newton_finish(tpsc_ctx *ctx) {
     for (int i = 0; i < 6; ++i) r[i] = h[10 + i];
     r[6] = 0.0;
     r[7] = h[17];
-    return set_mu(ctx, r, err_mu);
+    return set_mu(ctx, r, err_mu, true);
 }
 
-// the host state newton_queue leaves behind (a replayed graph only launches)
-void newton_state(tpsc_ctx *ctx) {
+// the host state solve_queue leaves behind (a replayed graph only launches)
+void solve_state(tpsc_ctx *ctx) {
     Grid *g = ctx->cur;
     g->g_mixed = mixed(ctx);
-    g->have_chi0 = g->have_mom = g->have_U = g->have_V = g->have_S = true;
+    g->have_chi0 = g->have_U = g->have_V = g->have_S = true;
+    g->have_mom = (ctx->form & TPSC_FORM_NEWTON) != 0;
     g->have_mom_host = false;
     ctx->roots.reset_sr = ctx->roots.reset_mu = true;
 }
 
-// The Newton-form solve on the current grid, queued directly or as a CUDA
+// The solve on the current grid, queued directly or as a CUDA
 // graph (ctx->graph_mode): a solve whose key (grid, form, model, mu0, the
 // root searches' barrier state and grid cap: everything its launches take)
 // equals the captured one replays the executable graph; in mode 1 a key seen
@@ -1294,7 +988,7 @@ void newton_state(tpsc_ctx *ctx) {
 // happen outside a capture); a new capture updates the executable graph in
 // place when its topology allows.  A capture that fails turns graphs off for
 // the context and the solve runs as direct launches.
-int newton_solve(tpsc_ctx *ctx) {
+int run_solve(tpsc_ctx *ctx) {
     Grid *g = ctx->cur;
     const GridDev &d = g->d;
     if (mixed(ctx) && !g->Grt32) CK(dalloc(g, &g->Grt32, (size_t)(d.nw0 + 1) * d.n8));
@@ -1315,14 +1009,14 @@ int newton_solve(tpsc_ctx *ctx) {
         add_launches(g->graph_kernels);
         ctx->graph_kernels = g->graph_kernels;
         ++ctx->graph_replays;
-        newton_state(ctx);
-        return newton_finish(ctx);
+        solve_state(ctx);
+        return solve_finish(ctx);
     }
     if (graphs && (ctx->graph_mode == 2 || (key == ctx->seen_key && ctx->seen_grid == g))) {
         const long long k0 = launches_thread();
         CK(cudaStreamBeginCapture(ctx->st, cudaStreamCaptureModeThreadLocal));
         ctx->capturing = true;
-        rc = newton_queue(ctx);
+        rc = solve_queue(ctx);
         ctx->capturing = false;
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamEndCapture(ctx->st, &graph);
@@ -1346,7 +1040,7 @@ int newton_solve(tpsc_ctx *ctx) {
             ++ctx->graph_captures;
             CK(cudaGraphLaunch(g->graph_exec, ctx->st));
             add_launches(nk);
-            return newton_finish(ctx);
+            return solve_finish(ctx);
         }
         // the capture failed: the same launches, directly, from now on
         cudaGetLastError();
@@ -1357,38 +1051,28 @@ int newton_solve(tpsc_ctx *ctx) {
     }
     ctx->seen_key = key;
     ctx->seen_grid = g;
-    if ((rc = newton_queue(ctx))) return rc;
+    if ((rc = solve_queue(ctx))) return rc;
     g->warm_forms |= fbit;
-    return newton_finish(ctx);
+    return solve_finish(ctx);
 }
 
+// green::find_mu with traceSelfG2 (src/green.cpp:3185-3282); in the Newton form
+// the traces of traceSelfG come with it
 int find_mu(tpsc_ctx *ctx) {
     Grid *g = ctx->cur;
     if (!g || !g->have_S) return fail(ctx, TPSC_ERR_STATE, "the self-energy has not been computed");
-    if (ctx->form & TPSC_FORM_NEWTON) return self_traces_and_mu_newton(ctx);
-    int rc = TPSC_OK;
-    auto f = [&](double m, double &y) -> bool {
-        rc = trace_diff_G(ctx, m, &y);
-        return rc == TPSC_OK;
-    };
-    const double init[3] = {0.0, -10.0, 10.0}, lims[2] = {-20.0, 20.0};
-    double root = 0;
-    int nev;
-    bool derr;
-    if (!find_zero(f, init, &root, lims, &nev, &derr)) {
-        if (derr) return rc;
-        return fail(ctx, TPSC_ERR_NO_ROOT, "mu not found");
-    }
-    ctx->scal[TPSC_S_EVALS_MU] = nev;
-    ctx->scal[TPSC_S_MU] = root;
-    // traceSelfG2 at the new mu (src/green.cpp:3281)
-    CK(launch_trace_self_G2(g->d, g->S, g->s2, g->s3, g->sinf, root, ctx->T, ctx->red, ctx->st));
-    double r;
-    rc = read_result(ctx, 1, &r);
+    const bool traces = (ctx->form & TPSC_FORM_NEWTON) != 0;
+    int rc = queue_mu_search(ctx, traces);
     if (rc) return rc;
-    ctx->scal[TPSC_S_TR_SG2] = r;
-    ctx->scal[TPSC_S_DBLOCC_SG2] = (r + ctx->U * ctx->n * ctx->n / 4.0) / ctx->U;
-    return TPSC_OK;
+    if ((rc = read_back(ctx, {{sigma_traces(ctx), 2 * sizeof(double), 0},
+                              {ctx->roots.out, 4 * sizeof(double), 2},
+                              {ctx->roots.bar + 6, sizeof(int), 6},
+                              {g->sinf, sizeof(double), 7}})))
+        return rc;
+    int err;
+    std::memcpy(&err, ctx->h_res + 6, sizeof(int));
+    ctx->roots.reset_mu = err != 0;
+    return set_mu(ctx, ctx->h_res, err, traces);
 }
 
 // Device state of the correlator on grid g for n_theta bins: the K4 arrays
@@ -2136,38 +1820,9 @@ int tpsc_solve(tpsc_ctx *ctx) {
     int rc = need_model(ctx);
     if (rc) return rc;
     cudaSetDevice(ctx->device);
-    if (ctx->form & TPSC_FORM_NEWTON) {
-        // no host round trip from the chi0 stage to the one readback at the end
-        if ((rc = switch_grid(ctx, ctx->nk0, ctx->Nw0))) return rc;
-        if ((rc = newton_solve(ctx))) return rc;
-        return finish_solve(ctx);
-    }
-    CK(cudaEventRecord(ctx->ev[0], ctx->st));
-    rc = switch_grid(ctx, ctx->nk0, ctx->Nw0);
-    if (rc) return rc;
-    rc = run_chi0(ctx);
-    if (rc) return rc;
-    CK(cudaEventRecord(ctx->ev[1], ctx->st));
-    double Usc[2];
-    rc = roots_Usp_Uch(ctx, Usc);
-    if (rc) return rc;
-    set_dblocc(ctx);
-    CK(cudaEventRecord(ctx->ev[2], ctx->st));
-    rc = run_vertex(ctx);
-    if (rc) return rc;
-    CK(cudaEventRecord(ctx->ev[3], ctx->st));
-    rc = run_self(ctx, !(ctx->form & TPSC_FORM_NEWTON));
-    if (rc) return rc;
-    CK(cudaEventRecord(ctx->ev[4], ctx->st));
-    // the Newton form computes traceSelfG in the same Sigma pass as the find_mu moments
-    if (!(ctx->form & TPSC_FORM_NEWTON)) {
-        double tsg[2];
-        rc = trace_self_G(ctx, tsg);
-        if (rc) return rc;
-    }
-    rc = find_mu(ctx);
-    if (rc) return rc;
-    CK(cudaEventRecord(ctx->ev[5], ctx->st));
+    // no host round trip from the chi0 stage to the one readback at the end
+    if ((rc = switch_grid(ctx, ctx->nk0, ctx->Nw0))) return rc;
+    if ((rc = run_solve(ctx))) return rc;
     return finish_solve(ctx);
 }
 
@@ -2392,7 +2047,7 @@ int group_run(tpsc_ctx *ctx, Group *q, int P, cudaStream_t st, int root_cap) {
 }
 
 // the scalars of point p of the group (the Newton-form solve's checks and
-// results, as newton_finish and switch_grid leave them) -> out; its status
+// results, as solve_finish and switch_grid leave them) -> out; its status
 int group_point_result(const Group *q, int p, const double *prm, double *out, std::string &msg) {
     const double *r = q->h_res + (size_t)p * kGroupRes;
     const double *pp = reinterpret_cast<const double *>(q->h_in + (size_t)p * q->in_bytes +
@@ -3401,7 +3056,7 @@ int tpsc_launch_count(tpsc_ctx *ctx, long long *count) {
 int tpsc_set_form(tpsc_ctx *ctx, int form) {
     if (!ctx) return fail(nullptr, TPSC_ERR_ARG, "null context");
     if (form < 0 || form > (TPSC_FORM_NEWTON | TPSC_FORM_MIXED)) return fail(ctx, TPSC_ERR_ARG, "unknown form");
-    // mu0 comes from the root search of the form (host find_zero or the
+    // mu0 comes from the root search of the form (find_zero or the
     // device Newton kernel; they agree to an ulp or so): when that changes,
     // the next grid switch (every solve and chi0 stage) derives it again, so
     // a result does not depend on whether the form was set before the model

@@ -71,23 +71,6 @@ int grid_for(long long total, int threads) {
 
 
 // ---------------------------------------------------------------------------
-// mu0 of the finite lattice: sum_o w 2 f(eps - mu) / L^2 - n
-// (green0::ddensity_mu_PBC, src/green0.cpp:182-203)
-// ---------------------------------------------------------------------------
-__global__ void k_density(const double *__restrict__ ek, int n8, int nbk,
-                          double mu, double T, double nk2, double *partial) {
-    KSum acc;
-    for (int o = blockIdx.x * blockDim.x + threadIdx.x; o < n8; o += gridDim.x * blockDim.x) {
-        int l, m;
-        oct_lm(o, l, m);
-        const int w = oct_weight(8, l, m, nbk);
-        acc.add(2 * w / ((exp((ek[o] - mu) / T) + 1.0) * nk2));
-    }
-    double v[1] = {acc.value()};
-    block_store<1>(v, partial);
-}
-
-// ---------------------------------------------------------------------------
 // slice kernels
 // ---------------------------------------------------------------------------
 
@@ -845,42 +828,6 @@ constexpr int kRedThreads = 256;
 // block's rows are contiguous 32-byte loads.  w16 holds the octant weights
 // (16 halved on edges and diagonal; 0 on padding columns); the row n = 0
 // carries an extra factor 1/2.
-//
-// Tail: with x_n = 1/qn^2, chi_n = a x_n + b x_n^2 and h = sgn U/2,
-//   chi/(1 + h chi) - chi = sum_{m>=1} (-h)^m chi^{m+1},
-//   sum_n chi_n^{m+1} = sum_i C(m+1, i) a^{m+1-i} b^i Q_{m+1+i},
-// with the U-independent power sums Q_k = sum_n x_n^k (tailq[k], k <= 2 kTailM + 2).
-// A column whose |h chi_max| >= kTailSeriesMax is summed term by term.
-constexpr int kTailM = 8;
-constexpr double kTailSeriesMax = 0.004;  // (0.004)^8 < 1e-19: series truncation below rounding
-
-__device__ __forceinline__ void tail_series(double a, double b, double h, const double *__restrict__ Q, double &f,
-                                           double &dfdh) {
-    double ap[kTailM + 2], bp[kTailM + 2];
-    ap[0] = bp[0] = 1.0;
-#pragma unroll
-    for (int k = 1; k < kTailM + 2; ++k) {
-        ap[k] = ap[k - 1] * a;
-        bp[k] = bp[k - 1] * b;
-    }
-    f = 0.0;
-    dfdh = 0.0;
-    double hm = 1.0;  // (-h)^(m-1)
-#pragma unroll
-    for (int m = 1; m <= kTailM; ++m) {
-        const int p = m + 1;
-        double Sp = 0.0, coef = 1.0;  // coef = C(p, i)
-#pragma unroll
-        for (int i = 0; i <= p; ++i) {
-            Sp += coef * ap[p - i] * bp[i] * __ldg(&Q[p + i]);
-            coef = coef * (p - i) / (i + 1);
-        }
-        f += (-h) * hm * Sp;           // (-h)^m S_p
-        dfdh += -m * hm * Sp;          // d/dh (-h)^m = -m (-h)^(m-1)
-        hm *= -h;
-    }
-}
-
 // Stored frequencies j < jdir are summed term by term (jdir = nb: all of
 // them); the Newton form passes jdir < nb and adds the frequencies above as a
 // power series in h from the moments of k_chi0_moments.
@@ -888,57 +835,8 @@ __global__ void __launch_bounds__(kRedThreads)
     k_sumrule(const double4 *__restrict__ chiq, const double *__restrict__ cinf, const double *__restrict__ cinf2,
               const double *__restrict__ w16, const double *__restrict__ tailq, int nb, int jdir, int tail, double Uv,
               double sgn, double T, double scale, Reduce r) {
-    const double hu = sgn * Uv / 2.0;
-    double v = 0.0, dv = 0.0, tv = 0.0, tdv = 0.0;
-    const int blk = blockIdx.x;
-    const int o0 = 4 * blk;
-    const double4 w = *reinterpret_cast<const double4 *>(w16 + o0);
-    const double ww[4] = {w.x, w.y, w.z, w.w};
-    const double4 *col = chiq + (size_t)blk * nb;
-    for (int j = threadIdx.x; j < jdir; j += blockDim.x) {
-        const double4 x = ld_stream4(&col[j]);
-        const double f = j == 0 ? 0.5 : 1.0;
-        const double xs[4] = {x.x, x.y, x.z, x.w};
-        double sv = 0.0, sd = 0.0;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const double q = xs[c] / (1.0 + hu * xs[c]);
-            sv += ww[c] * (q - xs[c]);
-            sd += ww[c] * q * q;
-        }
-        v += f * sv;
-        dv += f * sd;
-    }
-    // tail: n = nwmax+1 .. 2 nwmax
-    const int nwmax = nb - 1;
-    const double tw = 2.0 * 3.141592653589793 * T;
-    const double wn1 = (nwmax + 1) * tw;
-    const double x1 = 1.0 / (wn1 * wn1);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        if (ww[c] == 0.0 || !tail) continue;
-        const double a = cinf[o0 + c], b = cinf2[o0 + c];
-        const double cmax = fabs(a) * x1 + fabs(b) * x1 * x1;
-        if (fabs(hu) * cmax < kTailSeriesMax) {
-            if (threadIdx.x == c) {
-                double f, dfdh;
-                tail_series(a, b, hu, tailq, f, dfdh);
-                tv += ww[c] * f;
-                tdv += ww[c] * dfdh * (0.5 * sgn);
-            }
-        } else {
-            for (int t = threadIdx.x; t < nwmax; t += blockDim.x) {
-                const double wn = (nwmax + 1 + t) * tw;
-                const double i2 = 1.0 / (wn * wn);
-                const double xv = a * i2 + b * i2 * i2;
-                const double q = xv / (1.0 + hu * xv);
-                tv += ww[c] * (q - xv);
-                tdv += ww[c] * (-0.5 * sgn) * q * q;
-            }
-        }
-    }
-    dv *= -0.5 * sgn;
-    double out[2] = {scale * (v + tv), scale * (dv + tdv)};
+    double out[2];
+    sumrule_block<true>(chiq, cinf, cinf2, w16, tailq, blockIdx.x, nb, jdir, tail, Uv, sgn, T, scale, out[0], out[1]);
     grid_finish<2>(out, r, 0.0);
 }
 
@@ -1149,50 +1047,8 @@ __global__ void __launch_bounds__(kRedThreads)
                    const double *__restrict__ s4, const double *__restrict__ sinfp, const double *__restrict__ ek,
                    const double *__restrict__ w16, int nw0, double mu0, double pmu, double T, int jdir, int tail,
                    Reduce r) {
-    const int NO = nw0 / 2;
-    const double sinf = sinfp[0];
-    double v = 0.0, dv = 0.0;
-    const int blk = blockIdx.x;
-    const int o0 = 4 * blk;
-    double ww[4], e[4], c2[4], c3[4], c4[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        ww[c] = w16[o0 + c];
-        const bool ok = ww[c] != 0.0;
-        e[c] = ok ? ek[o0 + c] : 0.0;
-        c2[c] = ok ? s2[o0 + c] : 0.0;
-        c3[c] = ok ? s3[o0 + c] : 0.0;
-        c4[c] = ok ? s4[o0 + c] : 0.0;
-    }
-    const double pt = 3.141592653589793 * T;
-    const double4 *row = reinterpret_cast<const double4 *>(S + (size_t)blk * 4 * NO);
-    for (int j = threadIdx.x; j < jdir; j += blockDim.x) {
-        const double wn = (2 * j + 1) * pt;
-        const double i1 = 1.0 / wn;
-        const double4 p = ld_stream4(&row[2 * j]), q = ld_stream4(&row[2 * j + 1]);
-        const double2 sv[4] = {make_double2(p.x, p.y), make_double2(p.z, p.w), make_double2(q.x, q.y),
-                               make_double2(q.z, q.w)};
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            if (ww[c] == 0.0) continue;
-            double rS, iS;
-            sigma_full(i1, sinf, c2[c], c3[c], sv[c], rS, iS);
-            trdiff_term(wn, rS, iS, e[c], mu0, pmu, ww[c], v, dv);
-        }
-    }
-    for (int t = threadIdx.x; tail && t <= NO; t += blockDim.x) {
-        const int j = NO + t;
-        const double wn = (2 * j + 1) * pt;
-        const double i1 = 1.0 / wn, i2 = i1 * i1;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            if (ww[c] == 0.0) continue;
-            const double rS = -c2[c] * i2 + c4[c] * i2 * i2;
-            const double iS = -sinf * i1 + c3[c] * i2 * i1;
-            trdiff_term(wn, rS, iS, e[c], mu0, pmu, ww[c], v, dv);
-        }
-    }
-    double out[2] = {v, dv};
+    double out[2];
+    trace_diff_block<true>(S, s2, s3, s4, sinfp, ek, w16, blockIdx.x, nw0, mu0, pmu, T, jdir, tail, out[0], out[1]);
     grid_finish<2>(out, r, 0.0);
 }
 
@@ -1274,37 +1130,6 @@ __global__ void __launch_bounds__(kRedThreads)
     }
     double out[2] = {v.value(), v2.value()};
     grid_finish<2>(out, r, 0.0);
-}
-
-// Tr Sigma G (green::traceSelfG2, src/green.cpp:2929-2976)
-__global__ void __launch_bounds__(kRedThreads)
-    k_trace_self_G2(const double2 *__restrict__ S, const double *__restrict__ s2, const double *__restrict__ s3,
-                    const double *__restrict__ sinfp, const double *__restrict__ ek, const double *__restrict__ w16,
-                    int nw0, double mu, double T, double nk02, Reduce r) {
-    const int blk = blockIdx.x, o0 = 4 * blk, NO = nw0 / 2;
-    const double sinf = sinfp[0];
-    const double pt = 3.141592653589793 * T;
-    KSum v;
-    const double4 *row = reinterpret_cast<const double4 *>(S + (size_t)blk * 4 * NO);
-    for (int j = threadIdx.x; j < NO; j += blockDim.x) {
-        const double wn = (2 * j + 1) * pt;
-        const double i1 = 1.0 / wn;
-        const double4 p = ld_stream4(&row[2 * j]), q = ld_stream4(&row[2 * j + 1]);
-        const double2 sv[4] = {make_double2(p.x, p.y), make_double2(p.z, p.w), make_double2(q.x, q.y),
-                               make_double2(q.z, q.w)};
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const double w8 = 0.5 * w16[o0 + c];
-            if (w8 == 0.0) continue;
-            double rS, iS;
-            sigma_full(i1, sinf, s2[o0 + c], s3[o0 + c], sv[c], rS, iS);
-            const double a = ek[o0 + c] - mu + rS;
-            const double tmp = w8 * T * 2 / (nk02 * ((wn - iS) * (wn - iS) + a * a));
-            v.add(tmp * (iS * wn - iS * iS - (ek[o0 + c] - mu) * rS - rS * rS));
-        }
-    }
-    double out[1] = {v.value()};
-    grid_finish<1>(out, r, 0.0);
 }
 
 // raw and tail parts of chi0::traceChi0 (src/chi0.cpp:1498-1584)
@@ -1875,14 +1700,6 @@ bool supported_grid(int nk0, int nw0) {
     return k_ok && w_ok && nk0 == 2 * (nbk - 1);
 }
 
-cudaError_t launch_density(const GridDev &g, double mu, double n, double T, Reduce r, cudaStream_t st) {
-    const int nb = grid_for(g.n8, 256);
-    k_density<<<nb, 256, 0, st>>>(g.ek, g.n8, g.nbk, mu, T, 4.0 * (g.nbk - 1) * (g.nbk - 1), r.partial);
-    cudaError_t e = launched();
-    if (e != cudaSuccess) return e;
-    return finish<1>(r, nb, -n, st);
-}
-
 cudaError_t launch_gslice(const GridDev &g, double *Grt, double mu0, double T, cudaStream_t st) {
     return dispatch_nbk<RunGslice>(g.nbk, &g, Grt, mu0, T, st);
 }
@@ -2117,13 +1934,6 @@ cudaError_t launch_trace_self_G(const GridDev &g, const double2 *S, const double
                                 const double *sinf, double mu0, double T, Reduce r, cudaStream_t st) {
     const double nk02 = 4.0 * (g.nbk - 1) * (g.nbk - 1);
     k_trace_self_G<<<g.n8p / 4, kRedThreads, 0, st>>>(S, s2, s3, sinf, g.ek, g.w16, g.nw0, mu0, T, nk02, r);
-    return launched();
-}
-
-cudaError_t launch_trace_self_G2(const GridDev &g, const double2 *S, const double *s2, const double *s3,
-                                 const double *sinf, double mu, double T, Reduce r, cudaStream_t st) {
-    const double nk02 = 4.0 * (g.nbk - 1) * (g.nbk - 1);
-    k_trace_self_G2<<<g.n8p / 4, kRedThreads, 0, st>>>(S, s2, s3, sinf, g.ek, g.w16, g.nw0, mu, T, nk02, r);
     return launched();
 }
 

@@ -81,8 +81,6 @@ struct Bp {
 };
 
 // ---- launchers (all asynchronous on `st`) ---------------------------------
-cudaError_t launch_density(const GridDev &g, double mu, double n, double T, Reduce r, cudaStream_t st);
-
 // per-octant (eps - mu0, G0 prefactor) into g.gk
 cudaError_t launch_gk_table(const GridDev &g, double mu0, double T, cudaStream_t st, const Bp &b = Bp{});
 cudaError_t launch_gslice(const GridDev &g, double *Grt, double mu0, double T, cudaStream_t st);
@@ -182,8 +180,6 @@ cudaError_t launch_trace_diff_G(const GridDev &g, const double2 *S, const double
                                 cudaStream_t st, int jdir = -1);
 cudaError_t launch_trace_self_G(const GridDev &g, const double2 *S, const double *s2, const double *s3,
                                 const double *sinf, double mu0, double T, Reduce r, cudaStream_t st);
-cudaError_t launch_trace_self_G2(const GridDev &g, const double2 *S, const double *s2, const double *s3,
-                                 const double *sinf, double mu, double T, Reduce r, cudaStream_t st);
 
 // ---- the Newton form's root searches on the device (tpsc_roots.cu) ----------
 constexpr int kRootMaxBlocks = 1024;
@@ -199,6 +195,15 @@ struct RootScratch {
     // these once it has read a zero error flag after the last launch.
     bool reset_sr = true, reset_mu = true;
 };
+// The reference form's searches (find_zero) on the device: mu0 -> r.result[0..1]
+// (root, success); Usp, Uch -> rs.out as launch_sumrule_roots leaves them; mu
+// and Tr Sigma G at mu -> rs.out as launch_mu_roots leaves them
+cudaError_t launch_mu0_zero(const GridDev &g, double n, double T, Reduce r, cudaStream_t st);
+cudaError_t launch_sumrule_zero(const GridDev &g, const double *chiq, const double *chi0_inf, const double *chi0_inf2,
+                                double T, double n, double nsr, double U, double hi_sp, RootScratch rs,
+                                cudaStream_t st, const double *chi0max = nullptr, double hi_off = 0.0);
+cudaError_t launch_mu_zero(const GridDev &g, const double2 *S, const double *s2, const double *s3, const double *s4,
+                           const double *sinf, double mu0, double T, RootScratch rs, cudaStream_t st);
 // The Newton form's Sigma pass: Tr Sigma G0 (green::traceSelfG) and the
 // find_mu series moments around mu0 over the frequencies n >= jc and the tail
 // -> r.result[0..1] = (trace, asymptotic correction), r.result[2 + 2m],

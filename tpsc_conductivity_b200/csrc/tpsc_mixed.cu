@@ -46,7 +46,6 @@ struct Slice32Plan {
 template <int NBK>
 struct Slice32Smem {
     static constexpr int L = 2 * (NBK - 1);
-    static constexpr int G = FftPlan<L>::G;
     static constexpr int NGRP = Slice32Plan<NBK>::ngrp;
     static constexpr size_t slice_bytes = (size_t)NBK * NBK * sizeof(float);
     static constexpr size_t scr_off = (slice_bytes + 15) & ~(size_t)15;

@@ -18,6 +18,7 @@
 #include <algorithm>
 
 #include "tpsc_device.cuh"
+#include "tpsc_findzero.h"
 
 namespace tpsc {
 
@@ -163,7 +164,10 @@ __device__ void grid_root_sums(const double *part, double &pv, double &pd, doubl
 }
 
 // One safeguarded update with the bracket, bisection fallback and stopping
-// tests of the host routine newton_root (tpsc_engine.cpp).  The step is
+// tests of a safeguarded Newton search ([lo, hi] shrinks to the side that the
+// signs of the value and the derivative leave; converged when |f| is below
+// tol, when the step is below 1e-14 relative, or when it stops shrinking while
+// below 1e-10 relative: f is then at its rounding floor).  The step is
 // Halley's, x - 2 y y' / (2 y'^2 - y y''), while |y y''| <= y'^2 (it is then
 // between 2/3 and 2 Newton steps); else, and with d2y = 0, Newton's.
 __device__ void newton_update(RootCtl &c, double y, double dy, double tol, double d2y = 0.0) {
@@ -866,6 +870,197 @@ __global__ void __launch_bounds__(kRootThreads) k_mu_roots(MuRootArgs a) {
     }
 }
 
+// ---------------------------------------------------------------------------
+// the reference form's root searches (find_zero, tpsc_findzero.h) on the
+// device: every block runs the search on the same function values, one grid
+// barrier per evaluation.  The function is the reference's: every stored
+// frequency and the Matsubara tail, no series over the stored frequencies.
+//
+// What bounded the host-driven search is the round trip of an evaluation (the
+// sum, its gather into mapped memory, the wait: ~20 us, of which the sum
+// itself is 6-8 us up to 64^2 x 1024), 40-60 evaluations a solve; here an
+// evaluation costs the pass and one barrier.  The sums are taken in the order
+// of k_sumrule and k_trace_diff_G -- one partial per column block, added in
+// block order -- so the search sees the same values to the last bit whatever
+// the grid (differences of two roots, as the grid-halving diagnostics form
+// them, keep their digits).
+// ---------------------------------------------------------------------------
+
+// sum over the column blocks of share(blk) over each block's threads, the
+// same in every thread of the grid; part: one value per column block.
+// False: the barrier ran out.
+template <class F>
+__device__ bool grid_total(int nblk, double *part, unsigned *bar, int *err, double &total, const F &share) {
+    __shared__ double red[kRootThreads / 32], s_total;
+    for (int blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
+        double v = share(blk);
+        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double x = 0.0;
+            for (int w = 0; w < kRootThreads / 32; ++w) x += red[w];
+            part[blk] = x;
+        }
+        __syncthreads();
+    }
+    if (gridDim.x > 1 && !grid_sync(bar, err)) return false;
+    if (threadIdx.x < 32) {
+        KSum acc;
+        for (int b = threadIdx.x; b < nblk; b += 32) acc.add(__ldcg(&part[b]));
+        double x = acc.value();
+        for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
+        if (threadIdx.x == 0) s_total = x;
+    }
+    __syncthreads();
+    total = s_total;
+    __syncthreads();
+    return true;
+}
+
+// (not inlined: find_zero evaluates at many places)
+__device__ __noinline__ bool sumrule_total(const SumRootArgs &a, double Uv, double sgn, double *part, double &tr) {
+    return grid_total(a.nblk, part, a.bar, a.err, tr, [&](int blk) {
+        double v, dv;
+        sumrule_block<false>(a.chiq, a.cinf, a.cinf2, a.w16, a.tailq, blk, a.nb, a.nb, 1, Uv, sgn, a.T, a.scale, v,
+                             dv);
+        return v;
+    });
+}
+
+// Usp and Uch (chi::find_Usp_Uch(nq0, nw0, Usc), src/chi.cpp:850-876) -> out
+// as k_sumrule_roots leaves them
+__global__ void __launch_bounds__(kRootThreads, 2) k_sumrule_zero(SumRootArgs a) {
+    const double hi_sp = a.chi0max ? 2.0 / a.chi0max[0] - a.hi_off : a.hi_sp;
+    const double n = a.n, nsr = a.nsr, U = a.U;
+    int parity = 0;
+    double Usp = 0.0;
+#pragma unroll 1
+    for (int phase = 0; phase < 2; ++phase) {
+        const double sgn = phase == 0 ? -1.0 : 1.0;
+        auto f = [&](double Uv, double &y) -> bool {
+            double tr;
+            double *part = a.partial + (size_t)parity * kRootVals * kRootMaxBlocks;
+            parity ^= 1;
+            if (!sumrule_total(a, Uv, sgn, part, tr)) return false;
+            // chi::sum_rule_sp (src/chi.cpp:833-836) and sum_rule_ch (840-843),
+            // rounded as the host's expressions
+            const Rn base = Rn(tr) + Rn(n) - Rn(n) * Rn(n) / Rn(2.0);
+            if (phase == 0)
+                y = (base - Rn(nsr) + Rn(Uv) * Rn(nsr) * Rn(nsr) / (Rn(2.0) * Rn(U))).v;
+            else
+                y = (base - (Rn(nsr) + Rn(Usp) * Rn(nsr) * Rn(nsr) / (Rn(2.0) * Rn(U)) - Rn(nsr) * Rn(nsr))).v;
+            return true;
+        };
+        const double init[3] = {phase == 0 ? U / 2.0 : 0.0, 0.0, phase == 0 ? hi_sp : 1000.0 * U};
+        double root = 0.0;
+        int nev;
+        bool gone;
+        const bool ok = find_zero(f, init, &root, nullptr, &nev, &gone);
+        if (gone) return;
+        if (phase == 0) Usp = root;
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            a.out[phase] = root;
+            a.out[2 + phase] = nev;
+            a.out[4 + phase] = ok;
+        }
+        if (!ok) return;
+    }
+}
+
+__device__ __noinline__ bool trace_diff_total(const MuRootArgs &a, double pmu, double *part, double &tr) {
+    return grid_total(a.nblk, part, a.bar, a.err, tr, [&](int blk) {
+        double v, dv;
+        trace_diff_block<false>(a.S, a.s2, a.s3, a.s4, a.sinf, a.ek, a.w16, blk, a.nw0, a.mu0, pmu, a.T, a.nw0 / 2, 1,
+                                v, dv);
+        return v;
+    });
+}
+
+// find_mu (src/green.cpp:3185-3259), then traceSelfG2 (src/green.cpp:2929-2976)
+// at mu -> out as k_mu_roots leaves them
+__global__ void __launch_bounds__(kRootThreads, 2) k_mu_zero(MuRootArgs a) {
+    int parity = 0;
+    auto buffer = [&]() {
+        parity ^= 1;
+        return a.partial + (size_t)parity * kRootVals * kRootMaxBlocks;
+    };
+    auto f = [&](double pmu, double &y) -> bool { return trace_diff_total(a, pmu, buffer(), y); };
+    const double init[3] = {0.0, -10.0, 10.0}, lims[2] = {-20.0, 20.0};
+    double mu = 0.0;
+    int nev;
+    bool gone;
+    const bool ok = find_zero(f, init, &mu, lims, &nev, &gone);
+    if (gone) return;
+    double tr = 0.0;
+    if (ok && !grid_total(a.nblk, buffer(), a.bar, a.err, tr, [&](int blk) {
+            return trace_self2_block<false>(a.S, a.s2, a.s3, a.sinf, a.ek, a.w16, blk, a.nw0, mu, a.T, a.nk02);
+        }))
+        return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.out[0] = mu;
+        a.out[1] = nev;
+        a.out[2] = ok;
+        a.out[3] = tr;
+    }
+}
+
+// mu0 of the finite lattice (green0::find_mu, src/green0.cpp:182-203, 240-262)
+// in one block -> result[0], result[1] = 1 when the search succeeded
+// The sum is taken in chunks of kMu0Chunk points, each over kMu0Chunk threads (a
+// shuffle tree per warp, then a tree over the warps), then over the chunks.
+constexpr int kMu0Threads = 1024, kMu0Chunk = 256;
+constexpr int kMu0MaxChunks = 64;
+__device__ __noinline__ double density_total(const double *__restrict__ ek, int n8, int nbk, double mu, double T,
+                                             double nk2, double *wsum, double *tot) {
+    const int nchunk = (n8 + kMu0Chunk - 1) / kMu0Chunk, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int WPC = kMu0Chunk / 32;  // warps of a chunk
+    for (int o = threadIdx.x; o < nchunk * kMu0Chunk; o += blockDim.x) {
+        double v = 0.0;
+        if (o < n8) {
+            int l, m;
+            oct_lm(o, l, m);
+            v = 2 * oct_weight(8, l, m, nbk) / ((exp((ek[o] - mu) / T) + 1.0) * nk2);
+        }
+        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+        if (lane == 0) wsum[o >> 5] = v;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        double t = 0.0;
+        for (int c0 = 0; c0 < nchunk; c0 += 32) {
+            double x = 0.0;
+            if (c0 + lane < nchunk) {
+                const double *w = wsum + (c0 + lane) * WPC;
+                x = ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
+            }
+            for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
+            t += x;
+        }
+        if (lane == 0) *tot = t;
+    }
+    __syncthreads();
+    return *tot;
+}
+__global__ void __launch_bounds__(kMu0Threads)
+    k_mu0_zero(const double *__restrict__ ek, int n8, int nbk, double n, double T, double nk2, double *result) {
+    static_assert(kMu0Chunk == 256, "density_total's tree over a chunk's eight warps");
+    __shared__ double wsum[kMu0MaxChunks * kMu0Chunk / 32], tot;
+    auto f = [&](double mu, double &y) -> bool {
+        y = density_total(ek, n8, nbk, mu, T, nk2, wsum, &tot) - n;
+        return true;
+    };
+    const double init[3] = {0.0, -8.0, 8.0};
+    double root = 0.0;
+    int nev;
+    bool gone;
+    const bool ok = find_zero(f, init, &root, nullptr, &nev, &gone);
+    if (threadIdx.x == 0) {
+        result[0] = root;
+        result[1] = ok;
+    }
+}
+
 // The barrier's bound, exercised: block `withhold` never arrives (negative:
 // every block does), so every other block's wait runs out after
 // kBarrierNs and leaves with the error flag set.  words[0..1] the barrier,
@@ -905,6 +1100,89 @@ cudaError_t launch_sigma_moments(const GridDev &g, const double2 *S, const doubl
     cudaError_t e = launched();
     if (e != cudaSuccess) return e;
     return finish<kSigmaMomNV>(r, nb, 0.0, st, b);
+}
+
+// one block per column block, at most the resident grid (or the caller's cap)
+template <typename K>
+static cudaError_t zero_grid(K kernel, int nblk, int *grid, int cap) {
+    cudaError_t e = root_grid(kernel, grid, cap);
+    *grid = std::min(*grid, nblk);
+    return nblk <= kRootVals * kRootMaxBlocks ? e : cudaErrorInvalidValue;
+}
+
+cudaError_t launch_mu0_zero(const GridDev &g, double n, double T, Reduce r, cudaStream_t st) {
+    // (few points: few warps, whose barriers are shorter)
+    const int chunks = (g.n8 + kMu0Chunk - 1) / kMu0Chunk, threads = std::min(kMu0Threads, chunks * kMu0Chunk);
+    if (chunks > kMu0MaxChunks) return cudaErrorInvalidValue;
+    k_mu0_zero<<<1, threads, 0, st>>>(g.ek, g.n8, g.nbk, n, T, 4.0 * (g.nbk - 1) * (g.nbk - 1), r.result);
+    return launched();
+}
+
+cudaError_t launch_mu_zero(const GridDev &g, const double2 *S, const double *s2, const double *s3, const double *s4,
+                           const double *sinf, double mu0, double T, RootScratch rs, cudaStream_t st) {
+    const int nblk = g.n8p / 4;
+    int grid = 0;
+    cudaError_t e = zero_grid(k_mu_zero, nblk, &grid, rs.max_blocks);
+    if (e != cudaSuccess) return e;
+    if (rs.reset_mu && (e = cudaMemsetAsync(rs.bar + 4, 0, 2 * sizeof(unsigned) + sizeof(int), st)) != cudaSuccess)
+        return e;
+    MuRootArgs a{};
+    a.S = S;
+    a.s2 = s2;
+    a.s3 = s3;
+    a.s4 = s4;
+    a.sinf = sinf;
+    a.ek = g.ek;
+    a.w16 = g.w16;
+    a.nw0 = g.nw0;
+    a.nblk = nblk;
+    a.mu0 = mu0;
+    a.T = T;
+    a.nk02 = 4.0 * (g.nbk - 1) * (g.nbk - 1);
+    a.partial = rs.partial;
+    a.bar = rs.bar + 4;
+    a.err = reinterpret_cast<int *>(rs.bar + 6);
+    a.out = rs.out;
+    void *args[] = {&a};
+    e = cudaLaunchCooperativeKernel((const void *)k_mu_zero, dim3(grid), dim3(kRootThreads), args, 0, st);
+    if (e != cudaSuccess) return e;
+    return launched();
+}
+
+cudaError_t launch_sumrule_zero(const GridDev &g, const double *chiq, const double *chi0_inf, const double *chi0_inf2,
+                                double T, double n, double nsr, double U, double hi_sp, RootScratch rs,
+                                cudaStream_t st, const double *chi0max, double hi_off) {
+    const int nblk = g.n8p / 4;
+    int grid = 0;
+    cudaError_t e = zero_grid(k_sumrule_zero, nblk, &grid, rs.max_blocks);
+    if (e != cudaSuccess) return e;
+    if (rs.reset_sr && (e = cudaMemsetAsync(rs.bar, 0, 2 * sizeof(unsigned) + sizeof(int), st)) != cudaSuccess)
+        return e;
+    SumRootArgs a{};
+    a.chiq = reinterpret_cast<const double4 *>(chiq);
+    a.cinf = chi0_inf;
+    a.cinf2 = chi0_inf2;
+    a.w16 = g.w16;
+    a.tailq = g.tailq;
+    a.nb = g.nb;
+    a.nblk = nblk;
+    a.n8 = g.n8;
+    a.T = T;
+    a.scale = T / (4.0 * (g.nbk - 1) * (g.nbk - 1));
+    a.n = n;
+    a.nsr = nsr;
+    a.U = U;
+    a.hi_sp = hi_sp;
+    a.chi0max = chi0max;
+    a.hi_off = hi_off;
+    a.partial = rs.partial;
+    a.bar = rs.bar;
+    a.err = reinterpret_cast<int *>(rs.bar + 2);
+    a.out = rs.out;
+    void *args[] = {&a};
+    e = cudaLaunchCooperativeKernel((const void *)k_sumrule_zero, dim3(grid), dim3(kRootThreads), args, 0, st);
+    if (e != cudaSuccess) return e;
+    return launched();
 }
 
 cudaError_t launch_mu_roots(const GridDev &g, const double2 *S, const double *s2, const double *s3, const double *s4,
