@@ -554,8 +554,8 @@ __device__ __forceinline__ void sigma_full(double i1, double sinf, double c2, do
 constexpr int kTailM = 8;
 constexpr double kTailSeriesMax = 0.004;  // (0.004)^8 < 1e-19: series truncation below rounding
 
-__device__ __forceinline__ void tail_series(double a, double b, double h, const double *__restrict__ Q, double &f,
-                                           double &dfdh) {
+// the power sums S_{m+1} = sum_n chi_n^{m+1}, m = 1..kTailM, of one column
+__device__ __forceinline__ void tail_sums(double a, double b, const double *__restrict__ Q, double (&S)[kTailM]) {
     double ap[kTailM + 2], bp[kTailM + 2];
     ap[0] = bp[0] = 1.0;
 #pragma unroll
@@ -563,9 +563,6 @@ __device__ __forceinline__ void tail_series(double a, double b, double h, const 
         ap[k] = ap[k - 1] * a;
         bp[k] = bp[k - 1] * b;
     }
-    f = 0.0;
-    dfdh = 0.0;
-    double hm = 1.0;  // (-h)^(m-1)
 #pragma unroll
     for (int m = 1; m <= kTailM; ++m) {
         const int p = m + 1;
@@ -575,8 +572,21 @@ __device__ __forceinline__ void tail_series(double a, double b, double h, const 
             Sp += coef * ap[p - i] * bp[i] * __ldg(&Q[p + i]);
             coef = coef * (p - i) / (i + 1);
         }
-        f += (-h) * hm * Sp;           // (-h)^m S_p
-        dfdh += -m * hm * Sp;          // d/dh (-h)^m = -m (-h)^(m-1)
+        S[m - 1] = Sp;
+    }
+}
+
+__device__ __forceinline__ void tail_series(double a, double b, double h, const double *__restrict__ Q, double &f,
+                                           double &dfdh) {
+    double S[kTailM];
+    tail_sums(a, b, Q, S);
+    f = 0.0;
+    dfdh = 0.0;
+    double hm = 1.0;  // (-h)^(m-1)
+#pragma unroll
+    for (int m = 1; m <= kTailM; ++m) {
+        f += (-h) * hm * S[m - 1];     // (-h)^m S_p
+        dfdh += -m * hm * S[m - 1];    // d/dh (-h)^m = -m (-h)^(m-1)
         hm *= -h;
     }
 }
@@ -617,18 +627,14 @@ __device__ __forceinline__ double4 ld_row(const double4 *p) {
 
 // a thread's share of column block blk of the sum-rule trace and of its U
 // derivative (k_sumrule; the reference form's root search takes the same
-// values in the same order)
+// values in the same order): the stored frequencies j < jdir, ww the block's
+// weights, and the tail n = nwmax+1 .. 2 nwmax, S(c, f, dfdh) the series of column c
 template <bool STREAM>
-__device__ __forceinline__ void sumrule_block(const double4 *__restrict__ chiq, const double *__restrict__ cinf,
-                                              const double *__restrict__ cinf2, const double *__restrict__ w16,
-                                              const double *__restrict__ tailq, int blk, int nb, int jdir, int tail,
-                                              double Uv, double sgn, double T, double scale, double &out, double &dout) {
-    const double hu = sgn * Uv / 2.0;
-    double v = 0.0, dv = 0.0, tv = 0.0, tdv = 0.0;
-    const int o0 = 4 * blk;
-    const double4 w = *reinterpret_cast<const double4 *>(w16 + o0);
-    const double ww[4] = {w.x, w.y, w.z, w.w};
+__device__ __forceinline__ void sumrule_stored(const double4 *__restrict__ chiq, const double (&ww)[4], int blk, int nb,
+                                               int jdir, double hu, double &v, double &dv) {
+    v = dv = 0.0;
     const double4 *col = chiq + (size_t)blk * nb;
+#pragma unroll STREAM ? 1 : 4
     for (int j = threadIdx.x; j < jdir; j += blockDim.x) {
         const double4 x = ld_row<STREAM>(&col[j]);
         const double f = j == 0 ? 0.5 : 1.0;
@@ -643,20 +649,25 @@ __device__ __forceinline__ void sumrule_block(const double4 *__restrict__ chiq, 
         v += f * sv;
         dv += f * sd;
     }
-    // tail: n = nwmax+1 .. 2 nwmax
-    const int nwmax = nb - 1;
+}
+template <class Series>
+__device__ __forceinline__ void sumrule_tail(const double *__restrict__ cinf, const double *__restrict__ cinf2,
+                                             const double (&ww)[4], int blk, int nb, double hu, double sgn, double T,
+                                             double &tv, double &tdv, const Series &series) {
+    tv = tdv = 0.0;
+    const int nwmax = nb - 1, o0 = 4 * blk;
     const double tw = 2.0 * 3.141592653589793 * T;
     const double wn1 = (nwmax + 1) * tw;
     const double x1 = 1.0 / (wn1 * wn1);
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-        if (ww[c] == 0.0 || !tail) continue;
+        if (ww[c] == 0.0) continue;
         const double a = cinf[o0 + c], b = cinf2[o0 + c];
         const double cmax = fabs(a) * x1 + fabs(b) * x1 * x1;
         if (fabs(hu) * cmax < kTailSeriesMax) {
             if (threadIdx.x == c) {
                 double f, dfdh;
-                tail_series(a, b, hu, tailq, f, dfdh);
+                series(c, a, b, f, dfdh);
                 tv += ww[c] * f;
                 tdv += ww[c] * dfdh * (0.5 * sgn);
             }
@@ -671,9 +682,6 @@ __device__ __forceinline__ void sumrule_block(const double4 *__restrict__ chiq, 
             }
         }
     }
-    dv *= -0.5 * sgn;
-    out = scale * (v + tv);
-    dout = scale * (dv + tdv);
 }
 
 // a thread's share of column block blk of Tr(G - G0) at pmu and of its

@@ -835,8 +835,18 @@ __global__ void __launch_bounds__(kRedThreads)
     k_sumrule(const double4 *__restrict__ chiq, const double *__restrict__ cinf, const double *__restrict__ cinf2,
               const double *__restrict__ w16, const double *__restrict__ tailq, int nb, int jdir, int tail, double Uv,
               double sgn, double T, double scale, Reduce r) {
-    double out[2];
-    sumrule_block<true>(chiq, cinf, cinf2, w16, tailq, blockIdx.x, nb, jdir, tail, Uv, sgn, T, scale, out[0], out[1]);
+    const int blk = blockIdx.x;
+    const double hu = sgn * Uv / 2.0;
+    const double4 w = *reinterpret_cast<const double4 *>(w16 + 4 * blk);
+    const double ww[4] = {w.x, w.y, w.z, w.w};
+    double v, dv, tv = 0.0, tdv = 0.0;
+    sumrule_stored<true>(chiq, ww, blk, nb, jdir, hu, v, dv);
+    if (tail)
+        sumrule_tail(cinf, cinf2, ww, blk, nb, hu, sgn, T, tv, tdv, [&](int, double a, double b, double &f, double &df) {
+            tail_series(a, b, hu, tailq, f, df);
+        });
+    dv *= -0.5 * sgn;
+    double out[2] = {scale * (v + tv), scale * (dv + tdv)};
     grid_finish<2>(out, r, 0.0);
 }
 

@@ -35,38 +35,53 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
     return t;
 }
 
-// bar[0]: arrivals, bar[1]: generation.  Returns false (and sets *err) when
-// the wait ran out or another block had already failed.  The waiting thread
-// polls the generation word without sleeping: a poll is one L2 round trip,
-// so the barrier opens within about that of the last arrival.
-__device__ bool grid_sync(unsigned *bar, int *err) {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned *gen = bar + 1;
-        const unsigned g0 = *gen;
-        __threadfence();
-        int ok = 1;
-        if (atomicAdd(bar, 1u) == gridDim.x - 1) {
-            atomicExch(bar, 0u);
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-        } else {
-            const unsigned long long t0 = globaltimer_ns();
-            while (*gen == g0) {
-                if (*(volatile int *)err || globaltimer_ns() - t0 > kBarrierNs) {
-                    atomicExch(err, 1);
-                    ok = 0;
-                    break;
+// The grid barrier: bar[0] counts arrivals, bar[1] is the generation (read
+// once: it grows by one per barrier).  sync() returns false (and sets *err)
+// when the wait ran out or another block had already failed.  The arrival is
+// one acq_rel atomic and the waiting thread polls the generation with acquire
+// loads, without sleeping: the barrier opens within about one L2 round trip of
+// the last arrival.  The error word and the clock are looked at only every
+// 64th poll.  (With fences around a plain atomic, the generation and the error
+// word read at every barrier and the clock at every poll, an evaluation of the
+// sum-rule search cost 1.3 us more.)
+struct GridBar {
+    unsigned *bar;
+    int *err;
+    unsigned gen;
+    __device__ GridBar(unsigned *bar_, int *err_) : bar(bar_), err(err_), gen(*(volatile unsigned *)(bar_ + 1)) {}
+    __device__ bool sync() {
+        __shared__ int s_ok;
+        __syncthreads();
+        ++gen;
+        if (threadIdx.x == 0) {
+            int ok = 1;
+            unsigned old;
+            asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(bar) : "memory");
+            if (old == gridDim.x - 1) {
+                asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(bar), "r"(0) : "memory");
+                asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar + 1) : "memory");
+            } else {
+                unsigned long long t0 = 0;
+                for (unsigned i = 1;; ++i) {
+                    unsigned g;
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(g) : "l"(bar + 1) : "memory");
+                    if (g == gen) break;
+                    if (i % 64) continue;
+                    const unsigned long long t = globaltimer_ns();
+                    if (!t0) t0 = t;
+                    if (*(volatile int *)err || t - t0 > kBarrierNs) {
+                        atomicExch(err, 1);
+                        ok = 0;
+                        break;
+                    }
                 }
             }
+            s_ok = ok;
         }
-        __threadfence();
-        s_ok = ok && !*(volatile int *)err;
+        __syncthreads();
+        return s_ok;
     }
-    __syncthreads();
-    return s_ok;
-}
+};
 
 // Grid-stride walk over the items it = blk * nj + j (blk a column block,
 // j < nj a frequency): both indices are stepped by the stride's quotient and
@@ -262,6 +277,7 @@ __global__ void __launch_bounds__(kRootThreads) k_sumrule_roots(SumRootArgs a) {
     const double tw = 2.0 * 3.141592653589793 * a.T;
     double Usp = 0.0;
     int parity = 0;
+    GridBar bar(a.bar, a.err);
 #pragma unroll 1
     for (int phase = 0; phase < 2; ++phase) {
         const double sgn = phase == 0 ? -1.0 : 1.0;
@@ -352,7 +368,7 @@ __global__ void __launch_bounds__(kRootThreads) k_sumrule_roots(SumRootArgs a) {
             }
             double *part = a.partial + (size_t)parity * kRootVals * kRootMaxBlocks;
             block_root_sums(v, dv, d2v, part + kRootVals * blockIdx.x);
-            if (!grid_sync(a.bar, a.err)) return;
+            if (!bar.sync()) return;
             parity ^= 1;
             if (threadIdx.x < 32) {
                 double pv, pd, p2;
@@ -746,6 +762,7 @@ __global__ void __launch_bounds__(kRootThreads) k_mu_roots(MuRootArgs a) {
     const double zmin = a.wc - 2.0 * fabs(sinf) / a.wc;
     const double dmax = zmin > 0.0 ? kMuSeriesMax * zmin : 0.0;
     int parity = 0;
+    GridBar bar(a.bar, a.err);
     if (threadIdx.x == 0) {
         sc.lo = -10.0;
         sc.hi = 10.0;
@@ -793,7 +810,7 @@ __global__ void __launch_bounds__(kRootThreads) k_mu_roots(MuRootArgs a) {
         }
         double *part = a.partial + (size_t)parity * kRootVals * kRootMaxBlocks;
         block_root_sums(v, dv, d2v, part + kRootVals * blockIdx.x);
-        if (!grid_sync(a.bar, a.err)) return;
+        if (!bar.sync()) return;
         parity ^= 1;
         if (threadIdx.x < 32) {
             double pv, pd, p2;
@@ -857,7 +874,7 @@ __global__ void __launch_bounds__(kRootThreads) k_mu_roots(MuRootArgs a) {
     }
     double *part = a.partial + (size_t)parity * kRootVals * kRootMaxBlocks;
     block_root_sums(v, 0.0, 0.0, part + kRootVals * blockIdx.x);
-    if (!grid_sync(a.bar, a.err)) return;
+    if (!bar.sync()) return;
     if (blockIdx.x == 0 && threadIdx.x < 32) {
         double pv, pd, p2;
         grid_root_sums(part, pv, pd, p2);
@@ -890,7 +907,7 @@ __global__ void __launch_bounds__(kRootThreads) k_mu_roots(MuRootArgs a) {
 // same in every thread of the grid; part: one value per column block.
 // False: the barrier ran out.
 template <class F>
-__device__ bool grid_total(int nblk, double *part, unsigned *bar, int *err, double &total, const F &share) {
+__device__ bool grid_total(int nblk, double *part, GridBar &bar, double &total, const F &share) {
     __shared__ double red[kRootThreads / 32], s_total;
     for (int blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
         double v = share(blk);
@@ -904,7 +921,7 @@ __device__ bool grid_total(int nblk, double *part, unsigned *bar, int *err, doub
         }
         __syncthreads();
     }
-    if (gridDim.x > 1 && !grid_sync(bar, err)) return false;
+    if (gridDim.x > 1 && !bar.sync()) return false;
     if (threadIdx.x < 32) {
         KSum acc;
         for (int b = threadIdx.x; b < nblk; b += 32) acc.add(__ldcg(&part[b]));
@@ -918,13 +935,37 @@ __device__ bool grid_total(int nblk, double *part, unsigned *bar, int *err, doub
     return true;
 }
 
+// the tail's power sums of a block's first kZeroTail column blocks, which do
+// not depend on U: formed once per search
+constexpr int kZeroTail = 16;
+struct ZeroTail {
+    double S[kZeroTail][4][kTailM];
+};
+
 // (not inlined: find_zero evaluates at many places)
-__device__ __noinline__ bool sumrule_total(const SumRootArgs &a, double Uv, double sgn, double *part, double &tr) {
-    return grid_total(a.nblk, part, a.bar, a.err, tr, [&](int blk) {
-        double v, dv;
-        sumrule_block<false>(a.chiq, a.cinf, a.cinf2, a.w16, a.tailq, blk, a.nb, a.nb, 1, Uv, sgn, a.T, a.scale, v,
-                             dv);
-        return v;
+__device__ __noinline__ bool sumrule_total(const SumRootArgs &a, const ZeroTail &zt, double Uv, double sgn, double *part,
+                                           GridBar &bar, double &tr) {
+    const double hu = sgn * Uv / 2.0;
+    return grid_total(a.nblk, part, bar, tr, [&](int blk) {
+        const double4 w = reinterpret_cast<const double4 *>(a.w16)[blk];
+        const double ww[4] = {w.x, w.y, w.z, w.w};
+        const int lb = (blk - (int)blockIdx.x) / (int)gridDim.x;
+        double v, dv, tv, tdv;
+        sumrule_stored<false>(a.chiq, ww, blk, a.nb, a.nb, hu, v, dv);
+        sumrule_tail(a.cinf, a.cinf2, ww, blk, a.nb, hu, sgn, a.T, tv, tdv,
+                     [&](int c, double ca, double cb, double &f, double &df) {
+                         if (lb >= kZeroTail) {
+                             tail_series(ca, cb, hu, a.tailq, f, df);
+                             return;
+                         }
+                         f = df = 0.0;
+                         double hm = 1.0;
+                         for (int m = 1; m <= kTailM; ++m) {
+                             f += (-hu) * hm * zt.S[lb][c][m - 1];
+                             hm *= -hu;
+                         }
+                     });
+        return a.scale * (v + tv);
     });
 }
 
@@ -933,6 +974,13 @@ __device__ __noinline__ bool sumrule_total(const SumRootArgs &a, double Uv, doub
 __global__ void __launch_bounds__(kRootThreads, 2) k_sumrule_zero(SumRootArgs a) {
     const double hi_sp = a.chi0max ? 2.0 / a.chi0max[0] - a.hi_off : a.hi_sp;
     const double n = a.n, nsr = a.nsr, U = a.U;
+    __shared__ ZeroTail zt;
+    for (int i = threadIdx.x; i < 4 * kZeroTail; i += blockDim.x) {
+        const int o = 4 * (blockIdx.x + (i >> 2) * gridDim.x) + (i & 3);
+        if (o < a.n8) tail_sums(a.cinf[o], a.cinf2[o], a.tailq, zt.S[i >> 2][i & 3]);
+    }
+    __syncthreads();
+    GridBar bar(a.bar, a.err);
     int parity = 0;
     double Usp = 0.0;
 #pragma unroll 1
@@ -942,7 +990,7 @@ __global__ void __launch_bounds__(kRootThreads, 2) k_sumrule_zero(SumRootArgs a)
             double tr;
             double *part = a.partial + (size_t)parity * kRootVals * kRootMaxBlocks;
             parity ^= 1;
-            if (!sumrule_total(a, Uv, sgn, part, tr)) return false;
+            if (!sumrule_total(a, zt, Uv, sgn, part, bar, tr)) return false;
             // chi::sum_rule_sp (src/chi.cpp:833-836) and sum_rule_ch (840-843),
             // rounded as the host's expressions
             const Rn base = Rn(tr) + Rn(n) - Rn(n) * Rn(n) / Rn(2.0);
@@ -968,8 +1016,8 @@ __global__ void __launch_bounds__(kRootThreads, 2) k_sumrule_zero(SumRootArgs a)
     }
 }
 
-__device__ __noinline__ bool trace_diff_total(const MuRootArgs &a, double pmu, double *part, double &tr) {
-    return grid_total(a.nblk, part, a.bar, a.err, tr, [&](int blk) {
+__device__ __noinline__ bool trace_diff_total(const MuRootArgs &a, double pmu, double *part, GridBar &bar, double &tr) {
+    return grid_total(a.nblk, part, bar, tr, [&](int blk) {
         double v, dv;
         trace_diff_block<false>(a.S, a.s2, a.s3, a.s4, a.sinf, a.ek, a.w16, blk, a.nw0, a.mu0, pmu, a.T, a.nw0 / 2, 1,
                                 v, dv);
@@ -980,12 +1028,13 @@ __device__ __noinline__ bool trace_diff_total(const MuRootArgs &a, double pmu, d
 // find_mu (src/green.cpp:3185-3259), then traceSelfG2 (src/green.cpp:2929-2976)
 // at mu -> out as k_mu_roots leaves them
 __global__ void __launch_bounds__(kRootThreads, 2) k_mu_zero(MuRootArgs a) {
+    GridBar bar(a.bar, a.err);
     int parity = 0;
     auto buffer = [&]() {
         parity ^= 1;
         return a.partial + (size_t)parity * kRootVals * kRootMaxBlocks;
     };
-    auto f = [&](double pmu, double &y) -> bool { return trace_diff_total(a, pmu, buffer(), y); };
+    auto f = [&](double pmu, double &y) -> bool { return trace_diff_total(a, pmu, buffer(), bar, y); };
     const double init[3] = {0.0, -10.0, 10.0}, lims[2] = {-20.0, 20.0};
     double mu = 0.0;
     int nev;
@@ -993,7 +1042,7 @@ __global__ void __launch_bounds__(kRootThreads, 2) k_mu_zero(MuRootArgs a) {
     const bool ok = find_zero(f, init, &mu, lims, &nev, &gone);
     if (gone) return;
     double tr = 0.0;
-    if (ok && !grid_total(a.nblk, buffer(), a.bar, a.err, tr, [&](int blk) {
+    if (ok && !grid_total(a.nblk, buffer(), bar, tr, [&](int blk) {
             return trace_self2_block<false>(a.S, a.s2, a.s3, a.sinf, a.ek, a.w16, blk, a.nw0, mu, a.T, a.nk02);
         }))
         return;
@@ -1068,7 +1117,8 @@ __global__ void __launch_bounds__(kMu0Threads)
 // all zero at launch.
 __global__ void __launch_bounds__(kRootThreads) k_barrier_probe(unsigned *words, int withhold) {
     if ((int)blockIdx.x == withhold) return;
-    const bool ok = grid_sync(words, reinterpret_cast<int *>(words + 2));
+    GridBar bar(words, reinterpret_cast<int *>(words + 2));
+    const bool ok = bar.sync();
     if (threadIdx.x == 0 && !ok) atomicAdd(words + 3, 1u);
 }
 
@@ -1102,12 +1152,15 @@ cudaError_t launch_sigma_moments(const GridDev &g, const double2 *S, const doubl
     return finish<kSigmaMomNV>(r, nb, 0.0, st, b);
 }
 
-// one block per column block, at most the resident grid (or the caller's cap)
+// one block per column block, or per as few of them as the resident grid (or the
+// caller's cap) allows: no more blocks than that many rounds need
 template <typename K>
 static cudaError_t zero_grid(K kernel, int nblk, int *grid, int cap) {
-    cudaError_t e = root_grid(kernel, grid, cap);
-    *grid = std::min(*grid, nblk);
-    return nblk <= kRootVals * kRootMaxBlocks ? e : cudaErrorInvalidValue;
+    const cudaError_t e = root_grid(kernel, grid, cap);
+    if (e != cudaSuccess) return e;
+    const int rounds = (nblk + *grid - 1) / *grid;
+    *grid = (nblk + rounds - 1) / rounds;
+    return nblk <= kRootVals * kRootMaxBlocks ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 cudaError_t launch_mu0_zero(const GridDev &g, double n, double T, Reduce r, cudaStream_t st) {
