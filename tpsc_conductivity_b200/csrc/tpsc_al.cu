@@ -14,7 +14,10 @@
 //      (src/cond_opt.cpp:5158-5248), and their end slopes;
 //    * per column pair: clamped spline of hG over tau, FFT -> hG(q, i q_p)
 //      and its 1/q^2 coefficient (src/cond_opt.cpp:5250-5330);
-//   per grid frequency (launch_al_freq):
+//    * k_al_tables: chi0, hG, the RPA factors and the asymptote at every
+//      frequency, the asymptote in tau and G(k, i k): what every grid
+//      frequency reads;
+//   per batch of grid frequencies (launch_al_freqs):
 //    * k_al_hq: the difference quotient I_n(q, i q_m) of hG against chi0,
 //      times the RPA vertices, minus its closed-form asymptote, FFT to tau,
 //      plus the asymptote's closed form in tau (src/cond_opt.cpp:5351-5622);
@@ -30,6 +33,8 @@
 //      angular bins.
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "tpsc_device.cuh"
 
@@ -208,26 +213,101 @@ __global__ void __launch_bounds__(256, 1)
 }
 
 // ---------------------------------------------------------------------------
-// per grid frequency q_nn
+// what the grid frequencies share, once per call
 // ---------------------------------------------------------------------------
-struct AlHqArgs {
+struct AlTabArgs {
     const double *chiq;            // chi0(q, i q_p), p <= NO, column blocks
     const double *cinf, *cinf2;    // [n8] its 1/q^2, 1/q^4 tail coefficients
     const double *hgq;             // [K4 (NO+1)]
-    const double2 *tw, *ht;        // [N] FFT twiddles, half-step twiddles
-    double2 *HQ, *dHQ;
-    int K4, nbk, nn;
-    double T, Usp, Uch;
+    const double2 *S;              // Sigma as in AlTauArgs
+    const double *s2, *s3, *sinf, *ek;
+    double4 *tab;                  // [K4 (N+1)] (chi0, hG, RPA factor, asymptote) at q_p, p = 0..N
+    double *shape;                 // two-column blocks: the asymptote's closed form at tau_j
+    double2 *dshape;               // [2 K4] its tau-derivatives at 0 and beta
+    double2 *gk;                   // [K4 N] G(k, i k_f), f = 0..N-1
+    int K4, nbk, N;
+    double T, mu, Usp, Uch;
 };
 
-// per-column constants of k_al_hq
-struct HqCol {
-    int o;
-    const double *hq;
-    double ci, ci2, hg2;
-    double2 zsp0, zsp1, dsp0, dsp1;  // spin poles +-i sqrt(Usp ci/2) and their denominators
-    double zch0, zch1, dch0, dch1;   // charge poles +-sqrt(Uch ci/2) and denominators
-    double dt0;                      // d/dtau of the FFT part at 0 (src/cond_opt.cpp:5539-5546)
+// One column c per CTA.  chi0 and hG beyond the stored frequencies by their
+// tails; the RPA factor 3 Usp chisp + Uch chich and the asymptote Hinf(q_p) of
+// the difference quotient's product, Hinf(tau_j) in closed form with its end
+// slopes (src/cond_opt.cpp:5351-5622), and G(k, i k_f)
+// (src/cond_opt.cpp:6253-6290).  They do not depend on the grid frequency: per
+// frequency they cost k_al_hq and k_al_tau 15 divisions, two complex
+// exponentials, two exponentials and two Sigma reads per point.
+__global__ void __launch_bounds__(128) k_al_tables(const AlTabArgs a) {
+    const int c = blockIdx.x, l = c / a.nbk, m = c % a.nbk, o = oct_index(l + 1, m);
+    const int N = a.N, NO = N / 2, NB = NO + 1, NJ = N + 1;
+    const double T = a.T, Usp = a.Usp, Uch = a.Uch, tp = 2.0 * kPi * T;
+    const double *hq = a.hgq + (size_t)c * (NO + 1);
+    const double ci = a.cinf[o], ci2 = a.cinf2[o], hg2 = hq[NO];
+    for (int p = threadIdx.x; p <= N; p += blockDim.x) {
+        const double wn = tp * p, w2 = wn * wn;
+        const double ch = p <= NO ? a.chiq[bidx(p, o, NB)] : ci / w2 + ci2 / (w2 * w2);
+        const double hg = p == 0 ? hq[0] : -hg2 / w2 + hq[p < NO ? p : NO - 1] / (w2 * w2);
+        const double pre = 3 * Usp * (ch / (1.0 - Usp * ch / 2)) + Uch * (ch / (1.0 + Uch * ch / 2));
+        const double hinf =
+            hg2 * (3.0 * Usp * (1.0 / (-w2 + Usp * ci / 2.0)) + Uch * (1.0 / (-w2 - Uch * ci / 2.0)));
+        a.tab[(size_t)c * NJ + p] = make_double4(ch, hg, pre, hinf);
+    }
+    // spin poles +-i sqrt(Usp ci/2), charge poles +-sqrt(Uch ci/2)
+    const double zs = sqrt(Usp * ci / 2.0), zch0 = sqrt(Uch * ci / 2.0), zch1 = -zch0;
+    const double2 zsp0 = make_double2(0.0, zs), zsp1 = make_double2(-0.0, -zs);
+    const double2 one = make_double2(1.0, 0.0);
+    const double2 dsp0 = cmul(csub(cexp2(cscale(zsp0, -1.0 / T)), one), csub(zsp0, zsp1));
+    const double2 dsp1 = cmul(csub(cexp2(cscale(zsp1, -1.0 / T)), one), csub(zsp1, zsp0));
+    const double dch0 = (exp(-zch0 / T) - 1.0) * (zch0 - zch1), dch1 = (1.0 - exp(zch1 / T)) * (zch1 - zch0);
+    for (int j = threadIdx.x; j <= N; j += blockDim.x) {
+        const double t = j / (N * T);
+        // (the two spin poles are conjugate: their sum is real)
+        const double tsp = cadd(cdiv(cexp2(cscale(zsp0, -t)), dsp0), cdiv(cexp2(cscale(zsp1, -t)), dsp1)).x;
+        const double tch = exp(-zch0 * t) / dch0 + exp(zch1 * (1.0 / T - t)) / dch1;
+        a.shape[bidx2(j, c, NJ)] = hg2 * (3.0 * Usp * tsp + Uch * tch);
+    }
+    if (threadIdx.x < 2) {
+        const int side = threadIdx.x;
+        const double2 e0 = side ? cexp2(cscale(zsp0, -1.0 / T)) : one, e1 = side ? cexp2(cscale(zsp1, -1.0 / T)) : one;
+        const double2 tsp = csub(cneg(cdiv(cmul(zsp0, e0), dsp0)), cdiv(cmul(zsp1, e1), dsp1));
+        const double tch = side ? -zch0 * exp(-zch0 / T) / dch0 - zch1 / dch1
+                                : -zch0 / dch0 - zch1 * exp(zch1 / T) / dch1;
+        a.dshape[(size_t)side * a.K4 + c] = crs(hg2, cadd(crs(3.0 * Usp, tsp), make_double2(Uch * tch, 0.0)));
+    }
+    const double e = a.ek[o], sinf = a.sinf[0], C2 = a.s2[o], C3 = a.s3[o];
+    for (int f = threadIdx.x; f < N; f += blockDim.x) {
+        const double kn = (2 * f + 1) * kPi * T;
+        double sr = -C2 / (kn * kn), si = -sinf / kn + C3 / (kn * kn * kn);
+        if (f < NO) {
+            const double2 Sv = a.S[bidx(f, o, NO)];
+            const double k4 = kn * kn * kn * kn;
+            sr += Sv.x / k4;
+            si += Sv.y / k4;
+        }
+        a.gk[(size_t)c * N + f] = cinv(make_double2(-e + a.mu - sr, kn - si));
+    }
+}
+
+// ---------------------------------------------------------------------------
+// per grid frequency q_nn; blockIdx.y (blockIdx.x of the slices' planes) is the
+// frequency's place in the launch's batch
+// ---------------------------------------------------------------------------
+struct AlHqArgs {
+    const double4 *tab;
+    const double *shape;
+    const double2 *dshape;
+    const double2 *tw, *ht;        // [N] FFT twiddles, half-step twiddles
+    const int *ind;                // the batch's frequencies
+    double2 *HQ, *dHQ;
+    int K4, K4p;
+    double T;
+};
+
+// threads of a column pair's CTA: one FFT group
+template <int N>
+struct AlHqPlan {
+    static constexpr int G = FftPlan<N>::G;
+    static constexpr int threads = G < 32 ? 32 : G;
+    static constexpr size_t smem = (size_t)padded_len(N) * sizeof(double2) + 2 * sizeof(TwoLevelTw);
 };
 
 // I_n(q, i q_m) -> H(q, tau) for one column pair per CTA (src/cond_opt.cpp:5351-5622):
@@ -235,124 +315,64 @@ struct HqCol {
 //   I = (3 Usp chisp(p1) + Uch chich(p1)) (hG(p1) - hG(p2)) / (chi0(p1) - chi0(p2)),
 //   with (4 D(m-1) - D(m-2))/3 for the quotient D where p1 = p2 (nn even);
 //   ft_m = T (I - Hinf(q_m)), H(q, tau_j) = FFT_{-}[ft]_j + Hinf(tau_j), closed form.
+// Bound: the FP64 pipe (one division and the FFT per point) and the FFT's
+// exchange.  One FFT group per CTA, so that no thread idles in the transform
+// and six CTAs share an SM; 64^2 x 1024: 150 -> 15 us a frequency against 256
+// threads of which 64 transform and every asymptote formed anew.
 template <int N>
-__global__ void __launch_bounds__(256, 1) k_al_hq(const AlHqArgs a) {
-    constexpr int NO = N / 2, G = FftPlan<N>::G;
+__global__ void __launch_bounds__(AlHqPlan<N>::threads) k_al_hq(const AlHqArgs a) {
+    constexpr int NO = N / 2, G = FftPlan<N>::G, NJ = N + 1, NT = AlHqPlan<N>::threads;
     extern __shared__ __align__(16) double2 X[];
     TwoLevelTw *tw2 = reinterpret_cast<TwoLevelTw *>(X + padded_len(N));
-    __shared__ HqCol col[2];
     __shared__ double sums[2];
-    const int tid = threadIdx.x, NT = blockDim.x;
-    const int c0 = 2 * blockIdx.x;
-    const double T = a.T, Usp = a.Usp, Uch = a.Uch, tp = 2.0 * kPi * T;
-    const int nn = a.nn, nc = nn / 2, NB = NO + 1;
-    tau_tables(tw2, tw2 + 1, a.tw, a.ht, N);  // published by the barrier below
-    if (tid < 2) {
-        const int c = min(c0 + tid, a.K4 - 1);
-        const int l = c / a.nbk, m = c % a.nbk;
-        HqCol &q = col[tid];
-        q.o = oct_index(l + 1, m);
-        q.hq = a.hgq + (size_t)c * (NO + 1);
-        q.ci = a.cinf[q.o];
-        q.ci2 = a.cinf2[q.o];
-        q.hg2 = q.hq[NO];
-        const double s = sqrt(Usp * q.ci / 2.0);
-        q.zsp0 = make_double2(0.0, s);
-        q.zsp1 = make_double2(-0.0, -s);
-        q.dsp0 = cmul(csub(cexp2(cscale(q.zsp0, -1.0 / T)), make_double2(1.0, 0.0)), csub(q.zsp0, q.zsp1));
-        q.dsp1 = cmul(csub(cexp2(cscale(q.zsp1, -1.0 / T)), make_double2(1.0, 0.0)), csub(q.zsp1, q.zsp0));
-        q.zch0 = sqrt(Uch * q.ci / 2.0);
-        q.zch1 = -q.zch0;
-        q.dch0 = (exp(-q.zch0 / T) - 1.0) * (q.zch0 - q.zch1);
-        q.dch1 = (1.0 - exp(q.zch1 / T)) * (q.zch1 - q.zch0);
-    }
-    __syncthreads();
-    auto chi0_at = [&](const HqCol &q, int p) -> double {
-        p = abs(p);
-        if (p <= NO) return a.chiq[bidx(p, q.o, NB)];
-        const double wn = tp * p;
-        return q.ci / (wn * wn) + q.ci2 / (wn * wn * wn * wn);
-    };
-    auto hg_at = [&](const HqCol &q, int p) -> double {
-        p = abs(p);
-        if (p == 0) return q.hq[0];
-        const double wn = tp * p;
-        return -q.hg2 / (wn * wn) + q.hq[p < NO ? p : NO - 1] / (wn * wn * wn * wn);
-    };
-    auto quot = [&](const HqCol &q, int p1, int p2) -> double {
-        return (hg_at(q, p1) - hg_at(q, p2)) / (chi0_at(q, p1) - chi0_at(q, p2));
+    const int tid = threadIdx.x;
+    const int c0 = 2 * blockIdx.x, nn = a.ind[blockIdx.y], nc = nn / 2;
+    const double T = a.T, tp = 2.0 * kPi * T;
+    tau_tables(tw2, tw2 + 1, a.tw, a.ht, N);  // published by block_sum's barrier
+    const double4 *tab[2] = {a.tab + (size_t)c0 * NJ, a.tab + (size_t)min(c0 + 1, a.K4 - 1) * NJ};
+    auto quot = [&](const double4 *t, int p1, int p2) -> double {
+        const double4 u = t[abs(p1)], v = t[abs(p2)];
+        return (u.y - v.y) / (u.x - v.x);
     };
     // ---- the quotient minus its asymptote, packed as Re/Im of one FFT
     double acc[2] = {0.0, 0.0};
     for (int m = tid; m < N; m += NT) {
         const bool first = m < NO - nc;
         const int p1 = first ? m : m - N, p2 = p1 + nn;
-        const double wn = tp * (first ? m : m - N);
+        const double wn = tp * p1;
         double ft[2];
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-            const HqCol &q = col[k];
-            const double ch = chi0_at(q, p1);
-            const double pre = 3 * Usp * (ch / (1.0 - Usp * ch / 2)) + Uch * (ch / (1.0 + Uch * ch / 2));
-            double D;
+            const double4 u = tab[k][abs(p1)], v = tab[k][abs(p2)];
+            double D = (u.y - v.y) / (u.x - v.x);
             if (!first && (nn % 2) == 0 && m - N == -(nn / 2))
-                D = (4 * quot(q, p1 - 1, p2 - 1) - quot(q, p1 - 2, p2 - 2)) / 3.0;
-            else
-                D = quot(q, p1, p2);
-            const double cq = -q.ci;
-            const double hinf =
-                q.hg2 * (3.0 * Usp * (1.0 / (-wn * wn - Usp * cq / 2.0)) + Uch * (1.0 / (-wn * wn + Uch * cq / 2.0)));
-            ft[k] = T * (pre * D - hinf);
+                D = (4 * quot(tab[k], p1 - 1, p2 - 1) - quot(tab[k], p1 - 2, p2 - 2)) / 3.0;
+            ft[k] = T * (u.z * D - u.w);
             acc[k] += wn * ft[k];
         }
         X[pidx(m)] = make_double2(ft[0], ft[1]);
     }
     block_sum<2>(acc, sums);
-    if (tid < 2) col[tid].dt0 = -sums[tid];
     if (tid < G) group_fft<N, -1>(X, tid, (const TwoLevelTw *)tw2, 0);
     __syncthreads();
     // ---- back in tau: the FFT part plus the asymptote's closed form
+    double2 *HQ = a.HQ + (size_t)blockIdx.y * NJ * a.K4p;
+    const double2 *shape = reinterpret_cast<const double2 *>(a.shape) + (size_t)blockIdx.x * NJ;
+    const bool two = c0 + 1 < a.K4;
     for (int j = tid; j <= N; j += NT) {
-        const int k = j % N;
+        const int k = j & (N - 1);
         double2 F[2];
-        split_real(X[pidx(k)], X[pidx((N - k) % N)], F[0], F[1]);
-        const double t = j / (N * T);
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const HqCol &s = col[q];
-            const int c = c0 + q;
-            if (c >= a.K4) continue;
-            double2 tsp;
-            double tch;
-            if (j < N) {
-                tsp = cadd(cdiv(cexp2(cscale(s.zsp0, -t)), s.dsp0), cdiv(cexp2(cscale(s.zsp1, -t)), s.dsp1));
-                tch = exp(-s.zch0 * t) / s.dch0 + exp(s.zch1 * (1.0 / T - t)) / s.dch1;
-            } else {
-                const double2 one = make_double2(1.0, 0.0);
-                tsp = cadd(cinv(cmul(csub(one, cexp2(cscale(s.zsp0, 1.0 / T))), csub(s.zsp0, s.zsp1))),
-                           cinv(cmul(csub(one, cexp2(cscale(s.zsp1, 1.0 / T))), csub(s.zsp1, s.zsp0))));
-                const double e0 = exp(-s.zch0 / T);
-                tch = e0 / ((e0 - 1.0) * (s.zch0 - s.zch1)) + 1.0 / ((1.0 - exp(s.zch1 / T)) * (s.zch1 - s.zch0));
-            }
-            const double2 hinf = crs(s.hg2, cadd(crs(3.0 * Usp, tsp), make_double2(Uch * tch, 0.0)));
-            a.HQ[(size_t)j * a.K4 + c] = cadd(F[q], hinf);
-        }
+        split_real(X[pidx(k)], X[pidx((N - k) & (N - 1))], F[0], F[1]);
+        const double2 hinf = shape[j];
+        double2 *dst = HQ + (size_t)j * a.K4p + c0;
+        dst[0] = make_double2(F[0].x + hinf.x, F[0].y);
+        if (two) dst[1] = make_double2(F[1].x + hinf.y, F[1].y);
     }
-    // the end slopes: i dt0 plus the asymptote's tau-derivative at 0 and beta
-    if (tid < 2 && c0 + tid < a.K4) {
-        const HqCol &s = col[tid];
-        const int c = c0 + tid;
-        const double2 e0 = cexp2(cscale(s.zsp0, -1.0 / T)), e1 = cexp2(cscale(s.zsp1, -1.0 / T));
-        double2 tsp = csub(cneg(cdiv(s.zsp0, s.dsp0)), cdiv(s.zsp1, s.dsp1));
-        const double x1 = exp(s.zch1 / T);
-        double tch = -s.zch0 / s.dch0 - s.zch1 * x1 / s.dch1;
-        double2 dinf = crs(s.hg2, cadd(crs(3.0 * Usp, tsp), make_double2(Uch * tch, 0.0)));
-        a.dHQ[c] = cadd(make_double2(0.0, s.dt0), dinf);
-        tsp = csub(cneg(cdiv(cmul(s.zsp0, e0), s.dsp0)), cdiv(cmul(s.zsp1, e1), s.dsp1));
-        const double x0 = exp(-s.zch0 / T);
-        tch = -s.zch0 * x0 / s.dch0 - s.zch1 / s.dch1;
-        dinf = crs(s.hg2, cadd(crs(3.0 * Usp, tsp), make_double2(Uch * tch, 0.0)));
-        a.dHQ[a.K4 + c] = cadd(make_double2(0.0, s.dt0), dinf);
+    // the end slopes: i dt0 (src/cond_opt.cpp:5539-5546) plus the asymptote's
+    if (tid < 4 && c0 + (tid & 1) < a.K4) {
+        const int q = tid & 1, side = tid >> 1, c = c0 + q;
+        a.dHQ[((size_t)blockIdx.y * 2 + side) * a.K4 + c] =
+            cadd(make_double2(0.0, -sums[q]), a.dshape[(size_t)side * a.K4 + c]);
     }
 }
 
@@ -363,12 +383,13 @@ template <int NBK>
 __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
     k_al_q2r(const double2 *__restrict__ HQ, const double2 *__restrict__ dHQ, const double2 *__restrict__ tw,
              int nw0, double nf, double2 *__restrict__ HR, double2 *__restrict__ dHR) {
-    constexpr int K4 = (NBK - 2) * NBK;
+    constexpr int K4 = (NBK - 2) * NBK, K4p = (K4 + 1) & ~1;
     extern __shared__ __align__(16) double S[];
     const auto *tws = slice_twiddles<NBK>(S, tw);
     const int b = blockIdx.x, NJ = nw0 + 1;
-    const double2 *src = b < NJ ? HQ + (size_t)b * K4 : dHQ + (size_t)(b - NJ) * K4;
-    double *dst = reinterpret_cast<double *>(b < NJ ? HR + (size_t)b * K4 : dHR + (size_t)(b - NJ) * K4);
+    const size_t row = (size_t)blockIdx.y * NJ + b, drow = (size_t)blockIdx.y * 2 + (b - NJ);
+    const double2 *src = b < NJ ? HQ + row * K4p : dHQ + drow * K4;
+    double *dst = reinterpret_cast<double *>(b < NJ ? HR + row * K4p : dHR + drow * K4);
 #pragma unroll 1
     for (int part = 0; part < 2; ++part) {
         for (int c = threadIdx.x; c < K4; c += blockDim.x) S[c] = nf * (part == 0 ? src[c].x : src[c].y);
@@ -391,10 +412,15 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
     k_al_r2k(const double2 *__restrict__ HR, const double2 *__restrict__ dHR, const double *__restrict__ Grt,
              const double *__restrict__ er, const double *__restrict__ dG0p, const double2 *__restrict__ tw, int nw0,
              int n8, double mu0, double2 *__restrict__ HK, double2 *__restrict__ H2K, double2 *__restrict__ dHK) {
-    constexpr int K4 = (NBK - 2) * NBK;
+    constexpr int K4 = (NBK - 2) * NBK, K4p = (K4 + 1) & ~1;
     extern __shared__ __align__(16) double S[];
     const auto *tws = slice_twiddles<NBK>(S, tw);
     const int b = blockIdx.x, NJ = nw0 + 1;
+    HR += (size_t)blockIdx.y * NJ * K4p;
+    dHR += (size_t)blockIdx.y * 2 * K4;
+    HK += (size_t)blockIdx.y * NJ * K4p;
+    H2K += (size_t)blockIdx.y * NJ * K4p;
+    dHK += (size_t)blockIdx.y * 4 * K4;
     const int npass = b < NJ ? 4 : 2;
 #pragma unroll 1
     for (int pass = 0; pass < npass; ++pass) {
@@ -407,14 +433,14 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
             double v;
             if (b < NJ) {
                 const int row = pass < 2 ? b : nw0 - b;
-                v = hr[2 * ((size_t)row * K4 + c) + part] * g_minus(Grt, nw0, n8, b, o);
+                v = hr[2 * ((size_t)row * K4p + c) + part] * g_minus(Grt, nw0, n8, b, o);
             } else {
                 const int k = b - NJ;
                 const int side = k & 1;                                        // 0: tau = 0, 1: beta
                 const int row = (k == 0 || k == 3) ? 0 : nw0;                  // H at 0 / beta
                 const int sl = (k == 0) ? 0 : (k == 1) ? 1 : (k == 2) ? 1 : 0;  // which dH
                 const double sg = k < 2 ? 1.0 : -1.0;
-                v = hr[2 * ((size_t)row * K4 + c) + part] * dg_minus(er, dG0p, mu0, side, o) +
+                v = hr[2 * ((size_t)row * K4p + c) + part] * dg_minus(er, dG0p, mu0, side, o) +
                     sg * dr[2 * ((size_t)sl * K4 + c) + part] * g_minus(Grt, nw0, n8, side == 0 ? 0 : nw0, o);
             }
             S[c] = v;
@@ -435,106 +461,159 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
 
 struct AlTauArgs {
     const double2 *HK, *H2K, *dHK;
-    const double2 *S;
-    const double *s2, *s3, *sinf;
-    const double *ek, *dek;
+    const double2 *gk;   // [K4 N] G(k, i k_f)
+    const double *dek;
     const double *spl;
     const double2 *tw, *ht;
+    const int *ind;
     double *colv;
-    int K4, nbk, nn;
-    double T, mu, U, nf;
+    int K4, K4p, nbk;
+    double T, U, nf;
 };
 
-// shared memory of k_al_tau: the Re/Im columns being splined, the two
-// transforms (H, H2), the twiddle tables
+// shared memory of k_al_tau: the complex columns of H and H2, each splined and
+// transformed in place, and the twiddle tables
 template <int N>
-struct AlTauSmem {
-    static constexpr size_t r_bytes = ((size_t)2 * (N + 1) * sizeof(double) + 15) & ~(size_t)15;
-    static constexpr size_t x_bytes = (size_t)padded_len(N) * sizeof(double2);
-    static constexpr size_t tables_off = r_bytes + 2 * x_bytes;
-    static constexpr size_t bytes = tables_off + 2 * sizeof(TwoLevelTw);
+struct AlTauPlan {
+    static constexpr int G = FftPlan<N>::G;
+    static constexpr int threads = 2 * G < 32 ? 32 : 2 * G;
+    static constexpr int x_len = padded_len(N) + 2;  // N + 1 nodes
+    static constexpr size_t smem = (size_t)2 * x_len * sizeof(double2) + 2 * sizeof(TwoLevelTw);
 };
 
-// One k point per CTA: for H and H2 the Re and Im splines over tau with their
-// end slopes, F_j = sum_l exp(-i pi l/N) 6 (a_l^Re + i a_l^Im) exp(-2 pi i lj/N)
+// spline_second_derivatives for one complex column of N + 1 nodes in the padded
+// layout, by the G threads of a group: both parts of a node by one thread, so
+// that its two chains interleave.  TPC of them sweep, in chunks long enough
+// that the kWarm warm-up rows do not dominate.
+template <int N>
+__device__ void spline_complex(double2 *X, int t, int grp, double h, double2 d0, double2 dN,
+                               const double *__restrict__ invp, const double *__restrict__ cp) {
+    constexpr int G = FftPlan<N>::G, NJ = N + 1;
+    constexpr int TPC = G >= 64 ? G / 2 : G, C = (NJ + TPC - 1) / TPC;
+    const int s = t < TPC ? min(t * C, NJ) : NJ, e = min(s + C, NJ);
+    const double a6 = 6.0 / (h * h), b6 = 6.0 / h, ih = 1.0 / h;
+    const double cpiv = N > kSplinePivotConst ? __ldg(&invp[kSplinePivotConst]) : 0.0;
+    auto piv = [&](int i) -> double { return (i >= kSplinePivotConst && i < N) ? cpiv : __ldg(&invp[i]); };
+    auto sup = [&](int i) -> double { return (i >= kSplinePivotConst && i < N) ? cpiv : __ldg(&cp[i]); };
+    auto rhs1 = [&](int i, double vm, double v0, double vp, double dl, double dr) -> double {
+        if (i == 0) return b6 * ((vp - v0) * ih - dl);
+        if (i == N) return b6 * (dr - (v0 - vm) * ih);
+        return a6 * (vp - 2.0 * v0 + vm);
+    };
+    auto rhs = [&](int i, double2 vm, double2 v0, double2 vp) -> double2 {
+        return make_double2(rhs1(i, vm.x, v0.x, vp.x, d0.x, dN.x), rhs1(i, vm.y, v0.y, vp.y, d0.y, dN.y));
+    };
+    const double2 zero = make_double2(0.0, 0.0);
+    double2 carry = zero, vm_h = zero, vs_h = zero, ve_h = zero;
+    if (s < e) {
+        if (s > 0) {
+            const int i0 = max(0, s - kWarm);
+            double2 vm = i0 > 0 ? X[pidx(i0 - 1)] : zero, v0 = X[pidx(i0)];
+            for (int i = i0; i < s; ++i) {
+                const double2 vp = X[pidx(i + 1)];
+                carry = cscale(csub(rhs(i, vm, v0, vp), carry), piv(i));
+                vm = v0;
+                v0 = vp;
+            }
+            vm_h = X[pidx(s - 1)];
+        }
+        vs_h = X[pidx(s)];
+        if (e < NJ) ve_h = X[pidx(e)];
+    }
+    group_sync<G>(grp);
+    if (s < e) {
+        double2 vm = vm_h, v0 = vs_h;
+        for (int i = s; i < e; ++i) {
+            const double2 vp = (i + 1 < e) ? X[pidx(i + 1)] : ve_h;
+            carry = cscale(csub(rhs(i, vm, v0, vp), carry), piv(i));
+            X[pidx(i)] = carry;
+            vm = v0;
+            v0 = vp;
+        }
+    }
+    group_sync<G>(grp);
+    double2 mm = zero;
+    if (s < e && e < NJ)
+        for (int i = min(N, e - 1 + kWarm); i >= e; --i) mm = csub(X[pidx(i)], cscale(mm, sup(i)));
+    group_sync<G>(grp);
+    if (s < e)
+        for (int i = e - 1; i >= s; --i) {
+            mm = csub(X[pidx(i)], cscale(mm, sup(i)));
+            X[pidx(i)] = mm;
+        }
+    group_sync<G>(grp);
+}
+
+// One k point per CTA, a group of G threads for each of H and H2: the splines of
+// the real and imaginary parts over tau with their end slopes,
+// F_j = sum_l exp(-i pi l/N) 6 (a_l^Re + i a_l^Im) exp(-2 pi i lj/N)
 // (src/cond_opt.cpp:5906-5985, 6187-6251), the fermionic values
 //   H(i w) = -i C1/w - C2/w^2 + i C3/w^3 + (1 - exp(-i (2f+1) pi/N)) F/w^4
 // (H at k_m + q_nn, H2 at k_m), and the term
 //   -i U T nf wt dek sum_m G(k, i k_m) G(k, i k_m + i q_nn) (H - H2) / (2 q_nn)
 // (src/cond_opt.cpp:6253-6398); its real part -> colv[c].
+// Bound: the dependent spline sweeps and the FFTs' exchange.  Both transforms
+// run at once, each in place in its column's buffer (35 KB a CTA at N = 1024
+// instead of 53), so that four CTAs of busy threads share an SM; 64^2 x 1024:
+// 167 -> 46 us a frequency (one after the other in 256 threads, 64 of them in
+// the FFT, with G(k, i k) formed at every point).
 template <int N>
-__global__ void __launch_bounds__(256, 1) k_al_tau(const AlTauArgs a) {
-    constexpr int NJ = N + 1, NO = N / 2, G = FftPlan<N>::G;
-    extern __shared__ __align__(16) double R[];
-    double2 *X1 = reinterpret_cast<double2 *>(reinterpret_cast<char *>(R) + AlTauSmem<N>::r_bytes);
-    double2 *X2 = X1 + padded_len(N);
-    TwoLevelTw *tw2 = reinterpret_cast<TwoLevelTw *>(reinterpret_cast<char *>(R) + AlTauSmem<N>::tables_off);
+__global__ void __launch_bounds__(AlTauPlan<N>::threads, AlTauPlan<N>::threads <= 128 ? 4 : 1)
+    k_al_tau(const AlTauArgs a) {
+    constexpr int NO = N / 2, G = FftPlan<N>::G, NJ = N + 1, NT = AlTauPlan<N>::threads;
+    extern __shared__ __align__(16) double2 X1[];
+    double2 *X2 = X1 + AlTauPlan<N>::x_len;
+    TwoLevelTw *tw2 = reinterpret_cast<TwoLevelTw *>(X2 + AlTauPlan<N>::x_len);
     const TwoLevelTw *ht2 = tw2 + 1;
-    __shared__ double d0s[2], dNs[2];
     __shared__ double2 cw[2], dsum[2], d2sum[2];
-    __shared__ double sums[2];
-    const int tid = threadIdx.x, NT = blockDim.x;
-    const int c = blockIdx.x;
+    __shared__ double sums[1];
+    const int tid = threadIdx.x;
+    const int c = blockIdx.x, nn = a.ind[blockIdx.y], nc = nn / 2;
     const double T = a.T, h = 1.0 / (N * T), ih = 1.0 / h, pT = kPi * T;
     tau_tables(tw2, tw2 + 1, a.tw, a.ht, N);
-#pragma unroll 1
-    for (int which = 0; which < 2; ++which) {
-        const double2 *src = (which == 0 ? a.HK : a.H2K);
-        for (int j = tid; j < NJ; j += NT) {
-            const double2 v = src[bidx2(j, c, NJ)];
-            R[j] = v.x;
-            R[NJ + j] = v.y;
-        }
-        if (tid < 2) {
-            const double2 s0 = a.dHK[(size_t)(2 * which) * a.K4 + c], s1 = a.dHK[(size_t)(2 * which + 1) * a.K4 + c];
-            d0s[tid] = tid == 0 ? s0.x : s0.y;
-            dNs[tid] = tid == 0 ? s1.x : s1.y;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            cw[which] = make_double2(R[0] + R[N], R[NJ] + R[NJ + N]);
-            dsum[which] = make_double2(d0s[0] + dNs[0], d0s[1] + dNs[1]);
-        }
-        spline_second_derivatives<2>(R, NJ, NJ, h, d0s, dNs, a.spl, a.spl + NJ);
-        if (tid == 0) d2sum[which] = make_double2(R[0] + R[N], R[NJ] + R[NJ + N]);
-        double2 *X = which == 0 ? X1 : X2;
-        if (tid < G) {
-            const double *Mr = R, *Mi = R + NJ;
-            auto in = [&](int j) -> double2 {
-                const double2 e = tw_at(ht2, j);
-                return cmul(make_double2(e.x, -e.y), make_double2((Mr[j + 1] - Mr[j]) * ih, (Mi[j + 1] - Mi[j]) * ih));
-            };
-            group_fft_io<N, -1>(X, tid, (const TwoLevelTw *)tw2, 0, in, ScratchIO{X});
-        }
-        __syncthreads();
+    const size_t plane = (size_t)blockIdx.y * NJ * a.K4p;
+    for (int j = tid; j < NJ; j += NT) {
+        X1[pidx(j)] = a.HK[plane + bidx2(j, c, NJ)];
+        X2[pidx(j)] = a.H2K[plane + bidx2(j, c, NJ)];
     }
-    // ---- the sum over k_m
-    const int l = c / a.nbk, m = c % a.nbk;
-    const int o = oct_index(l + 1, m);
-    const int nn = a.nn, nc = nn / 2;
-    const double e = a.ek[o], mu = a.mu, sinf = a.sinf[0], C2 = a.s2[o], C3 = a.s3[o];
-    auto green = [&](int f) -> double2 {
-        const double kn = (2 * f + 1) * pT;
-        double sr = -C2 / (kn * kn), si = -sinf / kn + C3 / (kn * kn * kn);
-        const int n = f >= 0 ? f : -f - 1;
-        if (n < NO) {
-            const double2 Sv = a.S[bidx(n, o, NO)];
-            const double k4 = kn * kn * kn * kn;
-            sr += Sv.x / k4;
-            si += (f >= 0 ? Sv.y : -Sv.y) / k4;
+    __syncthreads();
+    const int which = tid / G;
+    if (which < 2) {
+        const int t = tid % G;
+        double2 *X = which == 0 ? X1 : X2;
+        const double2 *dh = a.dHK + ((size_t)blockIdx.y * 4 + 2 * which) * a.K4 + c;
+        const double2 d0 = dh[0], dN = dh[a.K4];
+        if (t == 0) {
+            cw[which] = cadd(X[0], X[pidx(N)]);
+            dsum[which] = cadd(d0, dN);
         }
-        return cinv(make_double2(-e + mu - sr, kn - si));
+        group_sync<G>(which);
+        spline_complex<N>(X, t, which, h, d0, dN, a.spl, a.spl + NJ);
+        if (t == 0) d2sum[which] = cadd(X[0], X[pidx(N)]);
+        auto in = [&](int j) -> double2 {
+            const double2 e = tw_at(ht2, j);
+            const double2 u = X[pidx(j)], v = X[pidx(j + 1)];
+            return cmul(make_double2(e.x, -e.y), make_double2((v.x - u.x) * ih, (v.y - u.y) * ih));
+        };
+        group_fft_io<N, -1, false, true>(X, t, (const TwoLevelTw *)tw2, which, in, ScratchIO{X});
+    }
+    __syncthreads();
+    // ---- the sum over k_m
+    const double2 *gk = a.gk + (size_t)c * N;
+    auto green = [&](int f) -> double2 {
+        const double2 g = gk[f >= 0 ? f : -f - 1];
+        return f >= 0 ? g : cconj(g);
     };
     auto hval = [&](double2 cwv, double2 ds, double2 d2s, double w, bool has, double2 Fv, int ph) -> double2 {
-        const double w2 = w * w, w3 = w2 * w, w4 = w2 * w2;
-        double2 v = cadd(csub(cmuli(cscale(cwv, -1.0 / w)), cscale(ds, 1.0 / w2)), cmuli(cscale(d2s, 1.0 / w3)));
+        const double i1 = 1.0 / w, i2 = i1 * i1, i3 = i2 * i1, i4 = i2 * i2;
+        double2 v = cadd(csub(cmuli(cscale(cwv, -i1)), cscale(ds, i2)), cmuli(cscale(d2s, i3)));
         if (has) {
             const double2 ex = half_twiddle_conj(ht2, ph, N);
-            v = cadd(v, cscale(cmul(make_double2(1.0 - ex.x, -ex.y), Fv), 1.0 / w4));
+            v = cadd(v, cscale(cmul(make_double2(1.0 - ex.x, -ex.y), Fv), i4));
         }
         return v;
     };
-    double acc[2] = {0.0, 0.0};
+    double acc[1] = {0.0};
     for (int j = tid; j < N; j += NT) {
         const bool first = j < NO - nc;
         const int f1 = first ? j : j - N;
@@ -550,33 +629,32 @@ __global__ void __launch_bounds__(256, 1) k_al_tau(const AlTauArgs a) {
             hval(cw[0], dsum[0], d2sum[0], w1, idx >= 0, idx >= 0 ? X1[pidx(idx)] : make_double2(0, 0), 2 * (j + nn) + 1);
         const double w2 = (2 * f1 + 1) * pT;
         const double2 v2 = hval(cw[1], dsum[1], d2sum[1], w2, true, X2[pidx(j)], 2 * j + 1);
-        const double2 t = cmul(cmul(green(f1), green(f1 + nn)), csub(v1, v2));
-        acc[0] += t.x;
-        acc[1] += t.y;
+        acc[0] += cmul(cmul(green(f1), green(f1 + nn)), csub(v1, v2)).y;
     }
-    block_sum<2>(acc, sums);
+    block_sum<1>(acc, sums);
     if (tid == 0) {
         const double qn = 2.0 * nn * kPi * T;
+        const int m = c % a.nbk;
         const double wt = (m == 0 || m == a.nbk - 1) ? 2.0 : 4.0;
         // Re[-i K acc] = K Im(acc)
-        a.colv[c] = a.U * T * a.nf * wt * a.dek[c] * sums[1] / (2.0 * qn);
+        a.colv[(size_t)blockIdx.y * a.K4 + c] = a.U * T * a.nf * wt * a.dek[c] * sums[0] / (2.0 * qn);
     }
 }
 
 // out[row (1 + nbins) + 0] = sum_c colv[c], then per bin b the sum over the
-// points of bin b; each warp adds one value in a fixed order (lane-strided
-// compensated sums, shuffle tree).
-__global__ void k_al_finish(const double *__restrict__ colv, const int *__restrict__ bin, int K4, int nbins,
-                            double *__restrict__ out) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int v = warp; v <= nbins; v += blockDim.x >> 5) {
-        KSum s;
-        for (int c = lane; c < K4; c += 32)
-            if (v == 0 || (bin ? bin[c] : 0) == v - 1) s.add(colv[c]);
-        double x = s.value();
-        for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
-        if (lane == 0) out[v] = x;
-    }
+// points of bin b; one block per value (x) and frequency (y), in a fixed order
+// (strided compensated sums, shuffle tree, warps in order).
+__global__ void __launch_bounds__(128) k_al_finish(const double *__restrict__ colv, const int *__restrict__ bin, int K4,
+                                                   double *__restrict__ out) {
+    __shared__ double tot[1];
+    const int v = blockIdx.x;
+    colv += (size_t)blockIdx.y * K4;
+    KSum s;
+    for (int c = threadIdx.x; c < K4; c += blockDim.x)
+        if (v == 0 || (bin ? bin[c] : 0) == v - 1) s.add(colv[c]);
+    double x[1] = {s.value()};
+    block_sum<1>(x, tot);
+    if (threadIdx.x == 0) out[(size_t)blockIdx.y * gridDim.x + v] = tot[0];
 }
 
 // ---------------------------------------------------------------------------
@@ -613,98 +691,129 @@ struct RunAlHgTau {
 
 template <int N>
 struct RunAlHq {
-    static cudaError_t run(const AlHqArgs *args, int npairs, cudaStream_t st) {
-        const size_t sm = (size_t)padded_len(N) * sizeof(double2) + 2 * sizeof(TwoLevelTw);
+    static cudaError_t run(const AlHqArgs *args, int npairs, int nf, cudaStream_t st) {
+        const size_t sm = AlHqPlan<N>::smem;
         cudaError_t e = set_smem(k_al_hq<N>, sm);
         if (e != cudaSuccess) return e;
-        k_al_hq<N><<<npairs, 256, sm, st>>>(*args);
+        k_al_hq<N><<<dim3(npairs, nf), AlHqPlan<N>::threads, sm, st>>>(*args);
         return launched();
     }
 };
 
 template <int NBK>
 struct RunAlSlices {
-    static cudaError_t run(const GridDev *g, const AlDev *a, const double *dG0p, double mu0, cudaStream_t st) {
+    static cudaError_t run(const GridDev *g, const AlDev *a, const double *dG0p, double mu0, int nfr, cudaStream_t st) {
         const size_t sm = SliceSmem<NBK>::bytes;
         cudaError_t e = set_smem(k_al_q2r<NBK>, sm);
         if (e != cudaSuccess) return e;
         if ((e = set_smem(k_al_r2k<NBK>, sm)) != cudaSuccess) return e;
         const double nf = 1.0 / ((double)g->nk0 * g->nk0);
-        k_al_q2r<NBK><<<g->nw0 + 3, SlicePlan<NBK>::threads, sm, st>>>(a->HQ, a->dHQ, g->tw_k, g->nw0, nf, a->HR, a->dHR);
+        k_al_q2r<NBK><<<dim3(g->nw0 + 3, nfr), SlicePlan<NBK>::threads, sm, st>>>(a->HQ, a->dHQ, g->tw_k, g->nw0, nf,
+                                                                                  a->HR, a->dHR);
         if ((e = launched()) != cudaSuccess) return e;
-        k_al_r2k<NBK><<<g->nw0 + 5, SlicePlan<NBK>::threads, sm, st>>>(a->HR, a->dHR, a->Grt, g->er, dG0p, g->tw_k, g->nw0,
-                                                              g->n8, mu0, a->HK, a->H2K, a->dHK);
+        // (H(q, tau) is not read any more: G H(k, tau) takes its place)
+        k_al_r2k<NBK><<<dim3(g->nw0 + 5, nfr), SlicePlan<NBK>::threads, sm, st>>>(
+            a->HR, a->dHR, a->Grt, g->er, dG0p, g->tw_k, g->nw0, g->n8, mu0, a->HQ, a->H2K, a->dHK);
         return launched();
     }
 };
 
 template <int N>
 struct RunAlTau {
-    static cudaError_t run(const AlTauArgs *args, cudaStream_t st) {
-        const size_t sm = AlTauSmem<N>::bytes;
+    static cudaError_t run(const AlTauArgs *args, int nf, cudaStream_t st) {
+        const size_t sm = AlTauPlan<N>::smem;
         cudaError_t e = set_smem(k_al_tau<N>, sm);
         if (e != cudaSuccess) return e;
-        k_al_tau<N><<<args->K4, 256, sm, st>>>(*args);
+        k_al_tau<N><<<dim3(args->K4, nf), AlTauPlan<N>::threads, sm, st>>>(*args);
         return launched();
     }
 };
 
 }  // namespace
 
-cudaError_t launch_al_setup(const GridDev &g, const CondDev &c, const AlDev &a, const double *dG0p, double mu0,
-                            double T, cudaStream_t st) {
+int al_batch(const GridDev &g, int K4, int nfreq) {
+    // frequencies per launch: enough CTAs to fill the GPU several times over (the
+    // k kernel has K4 a frequency), so that no half-empty last wave counts, as
+    // long as the three arrays of a batch stay within a GB.  Whole call, 64^2 x
+    // 1024 (96 frequencies): 10 a launch 14.2 ms, 5 15.1, 2 16.4, 1 18.9; 32^2 x
+    // 256 (40): 14 a launch 1.2 ms, 2 2.0, 1 3.2.
+    const size_t bytes = (size_t)3 * (g.nw0 + 1) * ((K4 + 1) & ~1) * sizeof(double2);
+    const int fill = (148 * 64 + K4 - 1) / K4, room = (int)std::max<size_t>(1, ((size_t)1 << 30) / bytes);
+    return std::max(1, std::min({fill, room, nfreq, 40}));
+}
+
+cudaError_t launch_al_setup(const GridDev &g, const CondDev &c, const AlDev &a, const double *dG0p,
+                            const double *chiq, const double *cinf, const double *cinf2, const double2 *S,
+                            const double *s2, const double *s3, const double *sinf, double Usp, double Uch, double mu,
+                            double mu0, double T, cudaStream_t st) {
     cudaError_t e = launch_gslice(g, a.Grt, mu0, T, st);
     if (e != cudaSuccess) return e;
     if ((e = dispatch_nbk<RunAlHg>(g.nbk, &g, &c, &a, dG0p, mu0, T, st)) != cudaSuccess) return e;
-    return dispatch_nw<RunAlHgTau>(g.nw0, &g, &a, T, st);
-}
-
-cudaError_t launch_al_freq(const GridDev &g, const CondDev &c, const AlDev &a, const double *chiq, const double *cinf,
-                           const double *cinf2, const double2 *S, const double *s2, const double *s3,
-                           const double *sinf, const double *dG0p, int nn, int row, double U, double Usp, double Uch,
-                           double mu, double mu0, double T, cudaStream_t st) {
-    AlHqArgs h;
-    h.chiq = chiq;
-    h.cinf = cinf;
-    h.cinf2 = cinf2;
-    h.hgq = a.hgq;
-    h.tw = g.tw_w;
-    h.ht = g.ht_w;
-    h.HQ = a.HQ;
-    h.dHQ = a.dHQ;
-    h.K4 = a.K4;
-    h.nbk = g.nbk;
-    h.nn = nn;
-    h.T = T;
-    h.Usp = Usp;
-    h.Uch = Uch;
-    cudaError_t e = dispatch_nw<RunAlHq>(g.nw0, &h, a.K4p / 2, st);
-    if (e != cudaSuccess) return e;
-    if ((e = dispatch_nbk<RunAlSlices>(g.nbk, &g, &a, dG0p, mu0, st)) != cudaSuccess) return e;
-    AlTauArgs t;
-    t.HK = a.HK;
-    t.H2K = a.H2K;
-    t.dHK = a.dHK;
+    if ((e = dispatch_nw<RunAlHgTau>(g.nw0, &g, &a, T, st)) != cudaSuccess) return e;
+    AlTabArgs t;
+    t.chiq = chiq;
+    t.cinf = cinf;
+    t.cinf2 = cinf2;
+    t.hgq = a.hgq;
     t.S = S;
     t.s2 = s2;
     t.s3 = s3;
     t.sinf = sinf;
     t.ek = g.ek;
+    t.tab = a.tab;
+    t.shape = a.shape;
+    t.dshape = a.dshape;
+    t.gk = a.gk;
+    t.K4 = a.K4;
+    t.nbk = g.nbk;
+    t.N = g.nw0;
+    t.T = T;
+    t.mu = mu;
+    t.Usp = Usp;
+    t.Uch = Uch;
+    k_al_tables<<<a.K4, 128, 0, st>>>(t);
+    return launched();
+}
+
+cudaError_t launch_al_freqs(const GridDev &g, const CondDev &c, const AlDev &a, const double *dG0p, int first, int count,
+                            double U, double mu0, double T, cudaStream_t st) {
+    if (count < 1 || count > a.batch) return cudaErrorInvalidValue;
+    const int *ind = a.ind + first;
+    AlHqArgs h;
+    h.tab = a.tab;
+    h.shape = a.shape;
+    h.dshape = a.dshape;
+    h.tw = g.tw_w;
+    h.ht = g.ht_w;
+    h.ind = ind;
+    h.HQ = a.HQ;
+    h.dHQ = a.dHQ;
+    h.K4 = a.K4;
+    h.K4p = a.K4p;
+    h.T = T;
+    cudaError_t e = dispatch_nw<RunAlHq>(g.nw0, &h, a.K4p / 2, count, st);
+    if (e != cudaSuccess) return e;
+    if ((e = dispatch_nbk<RunAlSlices>(g.nbk, &g, &a, dG0p, mu0, count, st)) != cudaSuccess) return e;
+    AlTauArgs t;
+    t.HK = a.HQ;
+    t.H2K = a.H2K;
+    t.dHK = a.dHK;
+    t.gk = a.gk;
     t.dek = c.dek;
     t.spl = g.spl_full;
     t.tw = g.tw_w;
     t.ht = g.ht_w;
+    t.ind = ind;
     t.colv = a.colv;
     t.K4 = a.K4;
+    t.K4p = a.K4p;
     t.nbk = g.nbk;
-    t.nn = nn;
     t.T = T;
-    t.mu = mu;
     t.U = U;
     t.nf = 1.0 / ((double)g.nk0 * g.nk0);
-    if ((e = dispatch_nw<RunAlTau>(g.nw0, &t, st)) != cudaSuccess) return e;
-    k_al_finish<<<1, 32 * (a.nbins + 1 < 32 ? a.nbins + 1 : 32), 0, st>>>(a.colv, a.nbins > 1 ? c.bin : nullptr, a.K4,
-                                                                          a.nbins, a.out + (size_t)row * (1 + a.nbins));
+    if ((e = dispatch_nw<RunAlTau>(g.nw0, &t, count, st)) != cudaSuccess) return e;
+    k_al_finish<<<dim3(1 + a.nbins, count), 128, 0, st>>>(a.colv, a.nbins > 1 ? c.bin : nullptr, a.K4,
+                                                          a.out + (size_t)first * (1 + a.nbins));
     return launched();
 }
 

@@ -1238,14 +1238,21 @@ int run_al(tpsc_ctx *ctx, int mmin, int nbins) {
         A(dalloc(g, &a.pre, 2 * K4));
         A(dalloc(g, &a.dhG, 2 * K4));
         A(dalloc(g, &a.hgq, K4 * (NO + 1)));
-        A(dalloc(g, &a.HQ, NJ * K4));
-        A(dalloc(g, &a.dHQ, 2 * K4));
-        A(dalloc(g, &a.HR, NJ * K4));
-        A(dalloc(g, &a.dHR, 2 * K4));
-        A(dalloc(g, &a.HK, K4p * NJ));
-        A(dalloc(g, &a.H2K, K4p * NJ));
-        A(dalloc(g, &a.dHK, 4 * K4));
-        A(dalloc(g, &a.colv, K4));
+        // (the frequencies of every mmin, at most Nw0/2: the widest batch)
+        a.batch = al_batch(d, a.K4, d.nw0 / 2);
+        const size_t nf = a.batch;
+        A(dalloc(g, &a.tab, K4 * NJ));
+        A(dalloc(g, &a.shape, K4p * NJ));
+        A(dalloc(g, &a.dshape, 2 * K4));
+        A(dalloc(g, &a.gk, K4 * d.nw0));
+        A(dalloc(g, &a.ind, NO + 2));
+        A(dalloc(g, &a.HQ, nf * NJ * K4p));
+        A(dalloc(g, &a.dHQ, nf * 2 * K4));
+        A(dalloc(g, &a.HR, nf * NJ * K4p));
+        A(dalloc(g, &a.dHR, nf * 2 * K4));
+        A(dalloc(g, &a.H2K, nf * NJ * K4p));
+        A(dalloc(g, &a.dHK, nf * 4 * K4));
+        A(dalloc(g, &a.colv, nf * K4));
 #undef A
         if (e != cudaSuccess) return cuda_fail(ctx, e, "Aslamazov-Larkin allocation");
         g->al_alloc = true;
@@ -1263,10 +1270,17 @@ int run_al(tpsc_ctx *ctx, int mmin, int nbins) {
     CK(cudaMemsetAsync(a.out, 0, need_out * sizeof(double), ctx->st));
     const double mu = ctx->scal[TPSC_S_MU];
     CK(launch_cond_table(d, c, g->mu0, ctx->T, ctx->st));
-    CK(launch_al_setup(d, c, a, g->dG0p, g->mu0, ctx->T, ctx->st));
-    for (int n = 1; n < N; ++n)
-        CK(launch_al_freq(d, c, a, g->chiq, g->cinf, g->cinf2, g->S, g->s2, g->s3, g->sinf, g->dG0p, ind[n], n,
-                          ctx->U, ctx->Usp, ctx->Uch, mu, g->mu0, ctx->T, ctx->st));
+    // (queued before the launches that read it; ind outlives the wait below)
+    CK(cudaMemcpyAsync(a.ind, ind.data(), N * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
+    CK(launch_al_setup(d, c, a, g->dG0p, g->chiq, g->cinf, g->cinf2, g->S, g->s2, g->s3, g->sinf, ctx->Usp, ctx->Uch,
+                       mu, g->mu0, ctx->T, ctx->st));
+    // launches of equal size, so that the last one is not a remainder
+    const int left = N - 1, launches = (left + a.batch - 1) / a.batch;
+    for (int i = 0, n = 1; i < launches; ++i) {
+        const int count = left / launches + (i < left % launches ? 1 : 0);
+        CK(launch_al_freqs(d, c, a, g->dG0p, n, count, ctx->U, g->mu0, ctx->T, ctx->st));
+        n += count;
+    }
     g->al_host.assign(need_out, 0.0);
     CK(cudaMemcpyAsync(g->al_host.data(), a.out, need_out * sizeof(double), cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));

@@ -364,25 +364,32 @@ struct AlDev {
     double *pre = nullptr;      // [2 K4]    h(r, 0), h(r, beta)
     double *dhG = nullptr;      // [2 K4]    d/dtau h G(q) at 0, beta
     double *hgq = nullptr;      // [K4 (NO+1)] h G(q, i q_p), p < NO, then its 1/q^2 coefficient hg2
-    double2 *HQ = nullptr;      // [NJ K4]   H(q, tau_j) of the current frequency
+    double4 *tab = nullptr;     // [K4 NJ]   (chi0, hG, RPA factor, asymptote) at q_p, p = 0..Nw0
+    double *shape = nullptr;    // [K4p NJ]  the asymptote at tau_j, two-column blocks
+    double2 *dshape = nullptr;  // [2 K4]    its tau-derivatives at 0, beta
+    double2 *gk = nullptr;      // [K4 Nw0]  G(k, i k_f), f >= 0
+    int *ind = nullptr;         // [nrows]   the grid frequencies
+    int batch = 0;              // grid frequencies of one launch: planes of the arrays below
+    double2 *HQ = nullptr;      // [NJ K4p]  H(q, tau_j); then G H(k, tau), two-column blocks
     double2 *dHQ = nullptr;     // [2 K4]    d/dtau H(q) at 0, beta
-    double2 *HR = nullptr;      // [NJ K4]   H(r, tau_j)
+    double2 *HR = nullptr;      // [NJ K4p]  H(r, tau_j)
     double2 *dHR = nullptr;     // [2 K4]
-    double2 *HK = nullptr;      // [K4p NJ]  G H(k, tau), two-column blocks
     double2 *H2K = nullptr;     // [K4p NJ]  G H2(k, tau), H2(r, tau) = H(r, beta - tau)
     double2 *dHK = nullptr;     // [4 K4]    end slopes: H at 0, beta; H2 at 0, beta
-    double *colv = nullptr;     // [K4]      per-point term of the current frequency
+    double *colv = nullptr;     // [K4]      per-point terms
     double *out = nullptr;      // [nrows (1 + nbins)] chijj3, then its angular bins
 };
-// once per call: G(r, tau) in FP64, h G(q, tau), its end slopes and h G(q, i q_p)
-// (c.tab, c.dek must be current)
-cudaError_t launch_al_setup(const GridDev &g, const CondDev &c, const AlDev &a, const double *dG0p, double mu0,
-                            double T, cudaStream_t st);
-// one grid frequency q_nn -> row `row` of a.out
-cudaError_t launch_al_freq(const GridDev &g, const CondDev &c, const AlDev &a, const double *chiq, const double *cinf,
-                           const double *cinf2, const double2 *S, const double *s2, const double *s3,
-                           const double *sinf, const double *dG0p, int nn, int row, double U, double Usp, double Uch,
-                           double mu, double mu0, double T, cudaStream_t st);
+// how many grid frequencies one launch takes
+int al_batch(const GridDev &g, int K4, int nfreq);
+// once per call: G(r, tau) in FP64, h G(q, tau), its end slopes and h G(q, i q_p),
+// the tables that every grid frequency reads (c.tab, c.dek must be current)
+cudaError_t launch_al_setup(const GridDev &g, const CondDev &c, const AlDev &a, const double *dG0p,
+                            const double *chiq, const double *cinf, const double *cinf2, const double2 *S,
+                            const double *s2, const double *s3, const double *sinf, double Usp, double Uch, double mu,
+                            double mu0, double T, cudaStream_t st);
+// the grid frequencies a.ind[first .. first + count) -> rows first.. of a.out
+cudaError_t launch_al_freqs(const GridDev &g, const CondDev &c, const AlDev &a, const double *dG0p, int first, int count,
+                            double U, double mu0, double T, cudaStream_t st);
 
 // The root searches' bounded grid barrier on its own, in a cooperative launch
 // of their grid (returned in *blocks): block `withhold` never arrives
