@@ -15,7 +15,7 @@
 //    columns of a pair contiguous along tau) for the tau kernel.
 //  * cond boundary: four CTAs for the tau-derivative end conditions of the
 //    two splines (src/cond_opt.cpp:2744-2887, 2910-3025).
-//  * cond tau: a persistent kernel, one CTA per SM, looping over pairs of K4
+//  * cond tau: a persistent kernel looping over pairs of K4
 //    columns.  Per pair: the two splines + pre-twiddled FFTs give
 //    J(k, ikn) and J0(k, ikn); G(k, ikn) = T/(ikn - eps + mu - Sigma) with
 //    its analytic tail; the two back-transforms to tau; the spline + FFT of
@@ -55,8 +55,19 @@ __device__ __forceinline__ void quad_eval(double2 x, double2 B, double2 C, doubl
 // Roots of z^2 + B z + C: closed form, then Newton polish (tolerance 1e-16 on
 // |p(x)|, at most 10 steps, halving back when a step makes |p| grow), a
 // polished root kept only if it improved |p| (generique::find_roots_2pol,
-// src/generique.cpp:1666-1727, with A = 1).
+// src/generique.cpp:1666-1727, with A = 1).  Real coefficients with two real
+// roots need no polish: the root that adds the magnitudes of -B and the square
+// root is exact to an ulp, the other is C over it (the chain of hypots and
+// complex divisions of ten steps made the tau kernel's column constants 27 us).
 __device__ void roots_2pol(double2 B, double2 C, double2 &r0, double2 &r1) {
+    const double disc = fma(B.x, B.x, -4.0 * C.x);
+    if (B.y == 0.0 && C.y == 0.0 && C.x != 0.0 && disc > 0.0) {
+        const double R = sqrt(disc);
+        const double big = -0.5 * (B.x + (B.x >= 0.0 ? R : -R)), small = C.x / big;
+        r0 = make_double2(B.x >= 0.0 ? big : small, 0.0);
+        r1 = make_double2(B.x >= 0.0 ? small : big, 0.0);
+        return;
+    }
     const double2 R = csqrt2(csub(cmul(B, B), cscale(C, 4.0)));
     double2 root[2] = {cscale(csub(make_double2(-B.x, -B.y), R), 0.5), cscale(cadd(make_double2(-B.x, -B.y), R), 0.5)};
 #pragma unroll 1
@@ -208,275 +219,305 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
 // ---------------------------------------------------------------------------
 // the per-k tau kernel
 // ---------------------------------------------------------------------------
+// What the tau kernel takes per K4 column, from eps, mu and Sigma_inf alone:
+// the roots r1, r2 of z^2 + (mu - eps) z - Sigma_inf, the prefactors of the
+// analytic tails (src/cond_opt.cpp:3421-3467)
+//   G0(tau) = -Re(u1 e1 + u2 e2),  Jinf(tau) = C1 Re(w1 j1 + w2 j2),
+// and the tails' parts of k0, dG/dtau(0+, 0-) and (per C1) dJ/dtau(0, beta).
+struct CondCol {
+    double2 r1, r2, u1, u2, w1, w2;
+    double k0, dGp, dGm, dJ0, dJb;
+    double e, dk, d2, wt;
+    int o, bin;
+};
+constexpr int kCondColWords = sizeof(CondCol) / sizeof(double);
+static_assert(sizeof(CondCol) % sizeof(double) == 0, "copied by double words");
+
+__global__ void __launch_bounds__(64)
+    k_cond_cols(const double *__restrict__ ek, const double *__restrict__ dek, const double *__restrict__ d2ek,
+                const int *__restrict__ bin, const double *__restrict__ sinfp, int K4, int K4p, int nbk, double mu,
+                double T, CondCol *__restrict__ cols) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= K4p) return;
+    const int cc = c < K4 ? c : K4 - 1;
+    const int l = cc / nbk, m = cc % nbk;
+    CondCol q;
+    q.o = oct_index(l + 1, m);
+    q.e = ek[q.o];
+    q.dk = dek[cc];
+    q.d2 = d2ek[cc];
+    q.wt = c < K4 ? ((m == 0 || m == nbk - 1) ? 2.0 : 4.0) : 0.0;
+    q.bin = bin ? bin[cc] : 0;
+    double2 r1, r2;
+    roots_2pol(make_double2(mu - q.e, 0.0), make_double2(-sinfp[0], 0.0), r1, r2);
+    q.r1 = r1;
+    q.r2 = r2;
+    const double2 a1 = cdiv(r1, csub(r1, r2)), a2 = cdiv(r2, csub(r2, r1));
+    const double2 b1 = cdiv(make_double2(1.0, 0.0), csub(r1, r2)), b2 = make_double2(-b1.x, -b1.y);
+    auto branch = [&](double2 r, double2 av, double2 bv, double2 &u, double2 &w, double2 &fp, double2 &fm, double2 &fj,
+                      double2 &fjb) {
+        const bool big = r.x > 0;
+        const double2 ex = big ? cexp2(cscale(r, -1.0 / T)) : cexp2(cscale(r, 1.0 / T));
+        const double2 den = make_double2(ex.x + 1.0, ex.y), rb = cmul(r, bv);
+        const double2 one = cdiv(av, den), exd = cdiv(cmul(av, ex), den);
+        const double2 j1 = cdiv(rb, den), jx = cdiv(cmul(rb, ex), den);
+        fp = big ? one : exd;
+        fm = big ? exd : one;
+        fj = big ? jx : j1;
+        fjb = big ? j1 : jx;
+        u = one;
+        w = cdiv(bv, den);
+    };
+    double2 f1p, f1m, fj1, fj1b, f2p, f2m, fj2, fj2b;
+    branch(r1, a1, b1, q.u1, q.w1, f1p, f1m, fj1, fj1b);
+    branch(r2, a2, b2, q.u2, q.w2, f2p, f2m, fj2, fj2b);
+    q.k0 = f1m.x + f2m.x;
+    q.dGm = cmul(r1, f1m).x + cmul(r2, f2m).x;
+    q.dGp = cmul(r1, f1p).x + cmul(r2, f2p).x;
+    q.dJb = fj1b.x + fj2b.x;
+    q.dJ0 = fj1.x + fj2.x;
+    cols[c] = q;
+}
+
+// Two groups of G = N/16 threads, one per transform in flight, and as many CTAs
+// per SM as leave 128 registers a thread
 template <int N>
-struct CondTauSmem {
-    // one FFT group (N/16 threads) up to N = 2048, so that every thread works
-    // in the FFTs and two CTAs share an SM (the kernel needs ~240 registers
-    // a thread, which holds a 256-thread CTA to one per SM); 256 beyond
-    static constexpr int threads = N >= 4096 ? TauSmem<N>::threads : 128;
-    static constexpr int min_blocks = N >= 4096 ? 1 : 2;
-    static constexpr size_t r_bytes = ((size_t)2 * (N + 1) * sizeof(double) + 15) & ~(size_t)15;
-    static constexpr size_t x_bytes = (size_t)padded_len(N) * sizeof(double2);
-    static constexpr size_t tables_off = r_bytes + 2 * x_bytes;
-    static constexpr size_t bytes = tables_off + 2 * sizeof(TwoLevelTw);
+struct CondTauPlan {
+    static constexpr int G = FftPlan<N>::G;
+    static constexpr int threads = 2 * G < 32 ? 32 : 2 * G;
+    static constexpr int blocks = 512 / threads > 12 ? 12 : 512 / threads;
+    static constexpr int x_len = padded_len(N) + 2;        // N + 1 nodes
+    static constexpr int n_hi = N / 64 + 1, n_lo = 64;     // two-level tails: tau_j, j = 64 hi + lo <= N
+    static constexpr size_t tables_off = (size_t)2 * x_len * sizeof(double2);
+    static constexpr size_t tails_off = tables_off + 2 * sizeof(TwoLevelTw);
+    static constexpr size_t bytes = tails_off + (size_t)4 * (n_hi + n_lo) * sizeof(double);
 };
 
 struct CondTauArgs {
-    const double *hV, *f0V, *dbound;
+    const double2 *hV, *f0V;  // two-column blocks: the two columns of a pair as the parts of one complex
+    const double *dbound;
     const double2 *S;
     const double *s2, *s3, *sinf;
-    const double *ek, *dek, *d2ek;
-    const int *bin;
+    const CondCol *cols;
     const double *spl_full, *spl_half;
     const double2 *tw, *ht;
     double *partial;
-    int K4, K4p, nbk, pw;
+    int K4, K4p, pw;
     double mu, T, nf;
 };
 
-// per-column state of the pair being processed
+// per-column values of the pair being processed
 struct ColState {
-    int o, bin;
-    double e, dk, d2, wt;
-    double2 r1, r2, u1, u2, v1, v2;  // roots; a/den and b/den of each root
-    bool big1, big2;
-    double C1, C2, C3;               // tau moments of the J being built
+    double2 v1, v2;                  // C1 w1, C1 w2
     double q0;                       // Re sum_n G^2 J0 / T, all n
     double k0, dGp, dGm, dJ0, dJb;
     double Gt0, Jt0, Jraw0;
-    double dchi, integ, V0, VN;
+    double dchi, integ;
     double CJ1b, CJ3b;
 };
 
-
-// full Sigma(k, i k_n) at octant o, n >= 0
-__device__ __forceinline__ double2 sigma_at(const CondTauArgs &a, int n, int o, int NO, double ik, double sinf) {
-    const double2 Sv = a.S[bidx(n, o, NO)];
-    double rS, iS;
-    sigma_full(ik, sinf, a.s2[o], a.s3[o], Sv, rS, iS);
-    return make_double2(rS, iS);
-}
-
 // analytic tails at tau: G0(tau) = Re(-u1 e1 - u2 e2), Jinf(tau) = Re(v1 j1 + v2 j2)
 // (src/cond_opt.cpp:3574-3640)
-__device__ __forceinline__ void tails(const ColState &q, double tau, double beta, double &g0, double &jinf) {
-    const double2 e1 = q.big1 ? cexp2(cscale(q.r1, -tau)) : cexp2(cscale(q.r1, beta - tau));
-    const double2 j1 = q.big1 ? cexp2(cscale(q.r1, tau - beta)) : cexp2(cscale(q.r1, tau));
-    const double2 e2 = q.big2 ? cexp2(cscale(q.r2, -tau)) : cexp2(cscale(q.r2, beta - tau));
-    const double2 j2 = q.big2 ? cexp2(cscale(q.r2, tau - beta)) : cexp2(cscale(q.r2, tau));
+__device__ __forceinline__ void tails(const CondCol &q, const ColState &s, double tau, double beta, double &g0,
+                                      double &jinf) {
+    const bool big1 = q.r1.x > 0, big2 = q.r2.x > 0;
+    const double2 e1 = big1 ? cexp2(cscale(q.r1, -tau)) : cexp2(cscale(q.r1, beta - tau));
+    const double2 j1 = big1 ? cexp2(cscale(q.r1, tau - beta)) : cexp2(cscale(q.r1, tau));
+    const double2 e2 = big2 ? cexp2(cscale(q.r2, -tau)) : cexp2(cscale(q.r2, beta - tau));
+    const double2 j2 = big2 ? cexp2(cscale(q.r2, tau - beta)) : cexp2(cscale(q.r2, tau));
     g0 = -cmul(q.u1, e1).x - cmul(q.u2, e2).x;
-    jinf = cmul(q.v1, j1).x + cmul(q.v2, j2).x;
+    jinf = cmul(s.v1, j1).x + cmul(s.v2, j2).x;
 }
 
+__device__ __forceinline__ double part_of(double2 z, int q) { return q == 0 ? z.x : z.y; }
+// T / z by one division
+__device__ __forceinline__ double2 crecip(double T, double x, double y) {
+    const double s = T / (x * x + y * y);
+    return make_double2(x * s, -y * s);
+}
 
+// Persistent over column pairs; the pair's two real columns are the parts of one
+// complex column throughout, in two buffers X1, X2 that two groups of threads
+// spline and transform in place at the same time: f0 V beside h V, G beside J,
+// the bubble beside the Maki-Thompson product.
+// Bound: the FP64 pipe (six N-point FFTs, four splines) and the sweeps' and
+// transforms' latencies at 16 warps per SM.  One transform at a time in 128 or
+// 256 threads at 240 registers (8 warps per SM), with four exponentials, five
+// more divisions per point and the roots' Newton polish in the pair loop took
+// 8290 us at 256^2 x 4096 and 937 at 128^2 x 2048; this takes 3265 and 453.
+// The tails' exponentials exp(-|r| tau_j) are products of two table entries
+// (formed per pair) when the roots are real, as they are for Sigma_inf > 0.
 template <int N>
-__global__ void __launch_bounds__(CondTauSmem<N>::threads, CondTauSmem<N>::min_blocks) k_cond_tau(const CondTauArgs a) {
-    constexpr int NJ = N + 1, NO = N / 2, NJ2 = NO + 1;
-    constexpr int G = FftPlan<N>::G;
-    extern __shared__ __align__(16) double R[];
-    double2 *X1 = reinterpret_cast<double2 *>(reinterpret_cast<char *>(R) + CondTauSmem<N>::r_bytes);
-    double2 *X2 = X1 + padded_len(N);
-    TwoLevelTw *tw2 = reinterpret_cast<TwoLevelTw *>(reinterpret_cast<char *>(R) + CondTauSmem<N>::tables_off);
+__global__ void __launch_bounds__(CondTauPlan<N>::threads, CondTauPlan<N>::blocks) k_cond_tau(const CondTauArgs a) {
+    using P = CondTauPlan<N>;
+    constexpr int NJ = N + 1, NO = N / 2, NJ2 = NO + 1, G = P::G, NT = P::threads;
+    extern __shared__ __align__(16) double2 X1[];
+    double2 *X2 = X1 + P::x_len;
+    TwoLevelTw *tw2 = reinterpret_cast<TwoLevelTw *>(reinterpret_cast<char *>(X1) + P::tables_off);
     const TwoLevelTw *ht2 = tw2 + 1;
+    double *tails_hi = reinterpret_cast<double *>(reinterpret_cast<char *>(X1) + P::tails_off);
+    double *tails_lo = tails_hi + 4 * P::n_hi;
     tau_tables(tw2, tw2 + 1, a.tw, a.ht, N);  // published by the first barrier of the pair loop
+    __shared__ CondCol col[2];
     __shared__ ColState cs[2];
-    __shared__ double d0s[2], dNs[2], sums[8], sV[2], sM[2];
-    const int tid = threadIdx.x, NT = blockDim.x;
+    __shared__ double2 d0s[2], dNs[2];            // end slopes of X1's and X2's columns
+    __shared__ double2 sC1[2], sC2[2], sC3[2];    // tau moments of X1's and X2's columns
+    __shared__ double sums[8], sV[2];
+    const int tid = threadIdx.x, grp = tid / G, t = tid % G;
+    double2 *const X = grp == 0 ? X1 : X2;
     const double T = a.T, h = 1.0 / (N * T), ih = 1.0 / h, beta = 1.0 / T, pT = kPi * T;
     const double sinf = a.sinf[0], mu = a.mu, nf = a.nf;
-    const int PWB = 2 * NJ2;
+    constexpr int PWB = 2 * NJ2;
     double *part = a.partial + (size_t)blockIdx.x * a.pw;
     const int npairs = a.K4p / 2;
-
-    // one spline + pre-twiddled FFT pass: R (two columns, NJ nodes, end slopes
-    // d0s/dNs) -> X1 = FFT_{+}[exp(i pi j/N) 6 a_j] packed; sets C1, C2, C3
-    auto moments_fft = [&]() {
-        if (tid < 2) {
-            ColState &q = cs[tid];
-            q.C1 = -R[tid * NJ] - R[tid * NJ + N];
-            q.C2 = d0s[tid] + dNs[tid];
-        }
-        spline_second_derivatives<2>(R, NJ, NJ, h, d0s, dNs, a.spl_full, a.spl_full + NJ);
-        if (tid < 2) cs[tid].C3 = -(R[tid * NJ] + R[tid * NJ + N]);
-        if (tid < G) {
-            const double *Ma = R, *Mb = R + NJ;
-            auto in = [&](int j) -> double2 {
-                return cmul(tw_at(ht2, j), make_double2((Ma[j + 1] - Ma[j]) * ih, (Mb[j + 1] - Mb[j]) * ih));
-            };
-            group_fft_io<N, +1>(X1, tid, (const TwoLevelTw *)tw2, 0, in, ScratchIO{X1});
-        }
-        __syncthreads();
-    };
-    // J(i k_n), n >= 0, of column q from the split transform F
-    auto jval = [&](const ColState &q, double2 F, double2 f, double ik) -> double2 {
-        const double ik2 = ik * ik;
-        const double2 w = cmul(f, F);
-        return make_double2(-q.C2 * ik2 + w.x * ik2 * ik2, -q.C1 * ik + q.C3 * ik2 * ik + w.y * ik2 * ik2);
-    };
 
 #pragma unroll 1
     for (int p = blockIdx.x; p < npairs; p += gridDim.x) {
         const int c0 = 2 * p;
-        const bool two = c0 + 1 < a.K4;
-        // ---- column constants
-        if (tid < 2) {
-            const int c = c0 + tid;
-            const bool valid = c < a.K4;
-            const int cc = valid ? c : c0;
-            const int l = cc / a.nbk, m = cc % a.nbk;
-            ColState &q = cs[tid];
-            q.o = oct_index(l + 1, m);
-            q.e = a.ek[q.o];
-            q.dk = a.dek[cc];
-            q.d2 = a.d2ek[cc];
-            q.wt = valid ? ((m == 0 || m == a.nbk - 1) ? 2.0 : 4.0) : 0.0;
-            q.bin = a.bin ? a.bin[cc] : 0;
-            roots_2pol(make_double2(mu - q.e, 0.0), make_double2(-sinf, 0.0), q.r1, q.r2);
-            d0s[tid] = valid ? a.dbound[2 * (size_t)a.K4p + c] : 0.0;  // df0V(0)
-            dNs[tid] = valid ? a.dbound[3 * (size_t)a.K4p + c] : 0.0;  // df0V(beta)
+        for (int j = tid; j < NJ; j += NT) {
+            cp_async16(&X1[pidx(j)], a.f0V + (size_t)p * NJ + j);
+            cp_async16(&X2[pidx(j)], a.hV + (size_t)p * NJ + j);
         }
-        // ---- f0 V: J0(i k_n) and sum_n G^2 J0 / T (src/cond_opt.cpp:3236-3308)
-        stage_pair(R, a.f0V + (size_t)p * 2 * NJ, NJ, two);
+        for (int i = tid; i < 2 * kCondColWords; i += NT)
+            reinterpret_cast<double *>(col)[i] = reinterpret_cast<const double *>(a.cols + c0)[i];
+        if (tid < 2) {
+            // f0 V: rows 2, 3 of the end conditions; h V: rows 0, 1
+            const double *b = a.dbound + (size_t)(tid == 0 ? 2 : 0) * a.K4p + c0;
+            const bool two = c0 + 1 < a.K4;
+            d0s[tid] = make_double2(b[0], two ? b[1] : 0.0);
+            dNs[tid] = make_double2(b[a.K4p], two ? b[a.K4p + 1] : 0.0);
+        }
+        cp_async_wait_all();
         __syncthreads();
-        moments_fft();
-        {
-            double acc[2] = {0.0, 0.0};
-            for (int n = tid; n < NO; n += NT) {
-                double2 F[2];
-                split_real(X1[pidx(n)], X1[pidx(N - 1 - n)], F[0], F[1]);
-                // the pre-twiddled split: F_b = (Z_n - conj Z_{N-1-n}) / (2i)
-                const double kn = (2 * n + 1) * pT, ik = 1.0 / kn;
-                const double2 e = tw_at(ht2, 2 * n + 1);
-                const double2 f = make_double2(1.0 - e.x, -e.y);
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const ColState &s = cs[q];
-                    const double2 J0 = jval(s, F[q], f, ik);
-                    const double2 sg = sigma_at(a, n, s.o, NO, ik, sinf);
-                    const double2 Gv = cdiv(make_double2(T, 0.0), make_double2(mu - s.e - sg.x, kn - sg.y));
-                    X2[pidx(q == 0 ? n : N - 1 - n)] = Gv;
-                    acc[q] += cmul(cmul(Gv, Gv), J0).x;
-                }
+        const bool real_roots = col[0].r1.y == 0.0 && col[0].r2.y == 0.0 && col[1].r1.y == 0.0 && col[1].r2.y == 0.0;
+        // exp(-|r| tau_j), column q and root k: row 2 q + k
+        for (int i = tid; i < 4 * (P::n_hi + P::n_lo); i += NT) {
+            const bool hi = i < 4 * P::n_hi;
+            const int ii = hi ? i : i - 4 * P::n_hi, len = hi ? P::n_hi : P::n_lo, row = ii / len, e = ii % len;
+            const CondCol &q = col[row >> 1];
+            const double r = fabs((row & 1) ? q.r2.x : q.r1.x);
+            (hi ? tails_hi : tails_lo)[ii] = exp(-r * ((hi ? 64 * e : e) * h));
+        }
+        // ---- f0 V and h V: splines and F = FFT_{+}[exp(i pi j/N) 6 a_j]
+        // (src/cond_opt.cpp:3204-3308)
+        if (grp < 2) {
+            const double2 d0 = d0s[grp], dN = dNs[grp];
+            if (t == 0) {
+                const double2 v0 = X[0], vN = X[pidx(N)];
+                sC1[grp] = make_double2(-v0.x - vN.x, -v0.y - vN.y);
+                sC2[grp] = cadd(d0, dN);
             }
-            block_sum<2>(acc, sums);
-            if (tid < 2) cs[tid].q0 = 2.0 * sums[tid] / T;
-        }
-        // ---- h V: J(i k_n); G J minus tails; k0, dG/dtau, dJ/dtau sums
-        // (src/cond_opt.cpp:3204-3407)
-        if (tid < 2) {
-            const int c = c0 + tid;
-            const bool valid = c < a.K4;
-            d0s[tid] = valid ? a.dbound[c] : 0.0;                   // dhV(0)
-            dNs[tid] = valid ? a.dbound[(size_t)a.K4p + c] : 0.0;   // dhV(beta)
-        }
-        stage_pair(R, a.hV + (size_t)p * 2 * NJ, NJ, two);
-        __syncthreads();
-        moments_fft();
-        {
-            double acc[6] = {0, 0, 0, 0, 0, 0};
-            for (int n = tid; n < NO; n += NT) {
-                double2 F[2];
-                split_real(X1[pidx(n)], X1[pidx(N - 1 - n)], F[0], F[1]);
-                const double kn = (2 * n + 1) * pT, ik = 1.0 / kn;
-                const double2 e = tw_at(ht2, 2 * n + 1);
-                const double2 f = make_double2(1.0 - e.x, -e.y);
-#pragma unroll
-                for (int q = 0; q < 2; ++q) {
-                    const ColState &s = cs[q];
-                    const int slot = pidx(q == 0 ? n : N - 1 - n);
-                    const double2 J = jval(s, F[q], f, ik);
-                    const double2 Gv = X2[slot];
-                    const double2 Gt = cdiv(make_double2(T, 0.0), make_double2(mu - s.e, kn + sinf * ik));
-                    const double2 Gs = csub(Gv, Gt);
-                    const double2 Js = csub(cmul(Gv, J), cmul(Gt, make_double2(0.0, -s.C1 * ik)));
-                    acc[3 * q] += Gs.x;
-                    acc[3 * q + 1] += kn * Gs.y;
-                    acc[3 * q + 2] -= kn * Js.y;
-                    X2[slot] = Gs;
-                    X1[slot] = Js;
-                }
+            group_sync<G>(grp);
+            spline_complex<N>(X, NJ, t, grp, h, d0, dN, a.spl_full, a.spl_full + NJ);
+            if (t == 0) {
+                const double2 m0 = X[0], mN = X[pidx(N)];
+                sC3[grp] = make_double2(-(m0.x + mN.x), -(m0.y + mN.y));
             }
-            block_sum<6>(acc, sums);
-        }
-        if (tid < 2) {
-            ColState &q = cs[tid];
-            const double k0s = 2.0 * sums[3 * tid], dGs = 2.0 * sums[3 * tid + 1], dJs = 2.0 * sums[3 * tid + 2];
-            const double2 r1 = q.r1, r2 = q.r2;
-            const double2 a1 = cdiv(r1, csub(r1, r2)), a2 = cdiv(r2, csub(r2, r1));
-            const double2 b1 = cdiv(make_double2(q.C1, 0.0), csub(r1, r2)), b2 = make_double2(-b1.x, -b1.y);
-            // src/cond_opt.cpp:3421-3467
-            auto branch = [&](double2 r, double2 av, double2 bv, bool &big, double2 &u, double2 &v, double2 &fp,
-                              double2 &fm, double2 &fj, double2 &fjb) {
-                big = r.x > 0;
-                const double2 ex = big ? cexp2(cscale(r, -1.0 / T)) : cexp2(cscale(r, 1.0 / T));
-                const double2 den = make_double2(ex.x + 1.0, ex.y);
-                const double2 rb = cmul(r, bv);
-                if (big) {
-                    fp = cdiv(av, den);
-                    fm = cdiv(cmul(av, ex), den);
-                    fj = cdiv(cmul(rb, ex), den);
-                    fjb = cdiv(rb, den);
-                } else {
-                    fp = cdiv(cmul(av, ex), den);
-                    fm = cdiv(av, den);
-                    fj = cdiv(rb, den);
-                    fjb = cdiv(cmul(rb, ex), den);
-                }
-                u = cdiv(av, den);
-                v = cdiv(bv, den);
+            auto in = [&](int j) -> double2 {
+                const double2 u = X[pidx(j)], v = X[pidx(j + 1)];
+                return cmul(tw_at(ht2, j), make_double2((v.x - u.x) * ih, (v.y - u.y) * ih));
             };
-            double2 f1p, f1m, fj1, fj1b, f2p, f2m, fj2, fj2b;
-            branch(r1, a1, b1, q.big1, q.u1, q.v1, f1p, f1m, fj1, fj1b);
-            branch(r2, a2, b2, q.big2, q.u2, q.v2, f2p, f2m, fj2, fj2b);
-            q.k0 = k0s + (f1m.x + f2m.x);
-            q.dGm = -dGs + (cmul(r1, f1m).x + cmul(r2, f2m).x);
-            q.dGp = dGs + (cmul(r1, f1p).x + cmul(r2, f2p).x);
-            q.dJb = -dJs + (fj1b.x + fj2b.x);
-            q.dJ0 = dJs + (fj1.x + fj2.x);
+            group_fft_io<N, +1, false, true>(X, t, (const TwoLevelTw *)tw2, grp, in, ScratchIO{X});
         }
         __syncthreads();
+        // ---- J0(i k_n), J(i k_n), G(i k_n); sum_n G^2 J0; G J and G minus tails
+        // in their places; k0, dG/dtau, dJ/dtau sums (src/cond_opt.cpp:3236-3407)
+        {
+            double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            for (int n = tid; n < NO; n += NT) {
+                const int i0 = pidx(n), i1 = pidx(N - 1 - n);
+                // the pre-twiddled split: F_b = (Z_n - conj Z_{N-1-n}) / (2i)
+                double2 F0[2], F[2];
+                split_real(X1[i0], X1[i1], F0[0], F0[1]);
+                split_real(X2[i0], X2[i1], F[0], F[1]);
+                const double kn = (2 * n + 1) * pT, ik = 1.0 / kn, ik2 = ik * ik, ik4 = ik2 * ik2;
+                const double2 e = tw_at(ht2, 2 * n + 1);
+                const double2 f = make_double2(1.0 - e.x, -e.y);
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const CondCol &s = col[q];
+                    // J(i k_n) = -i C1/k_n - C2/k_n^2 + i C3/k_n^3 + f F/k_n^4, n >= 0
+                    const double2 w0 = cmul(f, F0[q]), w = cmul(f, F[q]);
+                    const double2 J0 = make_double2(-part_of(sC2[0], q) * ik2 + w0.x * ik4,
+                                                    -part_of(sC1[0], q) * ik + part_of(sC3[0], q) * ik2 * ik + w0.y * ik4);
+                    const double C1 = part_of(sC1[1], q);
+                    const double2 J = make_double2(-part_of(sC2[1], q) * ik2 + w.x * ik4,
+                                                   -C1 * ik + part_of(sC3[1], q) * ik2 * ik + w.y * ik4);
+                    double rS, iS;
+                    sigma_full(ik, sinf, __ldg(&a.s2[s.o]), __ldg(&a.s3[s.o]), a.S[bidx(n, s.o, NO)], rS, iS);
+                    const double2 Gv = crecip(T, mu - s.e - rS, kn - iS);
+                    const double2 Gt = crecip(T, mu - s.e, kn + sinf * ik);
+                    const double2 Gs = csub(Gv, Gt);
+                    const double2 Js = csub(cmul(Gv, J), cmul(Gt, make_double2(0.0, -C1 * ik)));
+                    acc[4 * q] += cmul(cmul(Gv, Gv), J0).x;
+                    acc[4 * q + 1] += Gs.x;
+                    acc[4 * q + 2] += kn * Gs.y;
+                    acc[4 * q + 3] -= kn * Js.y;
+                    X1[q == 0 ? i0 : i1] = Gs;
+                    X2[q == 0 ? i0 : i1] = Js;
+                }
+            }
+            block_sum<8>(acc, sums);
+        }
+        if (tid < 2) {
+            const CondCol &c = col[tid];
+            ColState &q = cs[tid];
+            const double C1 = part_of(sC1[1], tid), *s = sums + 4 * tid;
+            q.v1 = cscale(c.w1, C1);
+            q.v2 = cscale(c.w2, C1);
+            q.q0 = 2.0 * s[0] / T;
+            q.k0 = 2.0 * s[1] + c.k0;
+            q.dGm = -2.0 * s[2] + c.dGm;
+            q.dGp = 2.0 * s[2] + c.dGp;
+            q.dJb = -2.0 * s[3] + C1 * c.dJb;
+            q.dJ0 = 2.0 * s[3] + C1 * c.dJ0;
+        }
         // ---- back to tau: G(tau) = sum_n G(ikn) e^{-ikn tau}, J(tau) = sum_n J(ikn) e^{+ikn tau}
         // (src/cond_opt.cpp:3545-3620); both real, so the pair packs as Re/Im
-        if (tid < G) {
-            auto inG = [&](int k) -> double2 {
+        if (grp < 2) {
+            auto in = [&](int k) -> double2 {
                 double2 A, B;
                 if (k < NO) {
-                    A = X2[pidx(k)];
-                    B = X2[pidx(N - 1 - k)];
+                    A = X[pidx(k)];
+                    B = X[pidx(N - 1 - k)];
                 } else {
-                    A = cconj(X2[pidx(N - 1 - k)]);
-                    B = cconj(X2[pidx(k)]);
+                    A = cconj(X[pidx(N - 1 - k)]);
+                    B = cconj(X[pidx(k)]);
                 }
                 return make_double2(A.x - B.y, A.y + B.x);
             };
-            group_fft_io<N, -1, false, true>(X2, tid, (const TwoLevelTw *)tw2, 0, inG, ScratchIO{X2});
-            auto inJ = [&](int k) -> double2 {
-                double2 A, B;
-                if (k < NO) {
-                    A = X1[pidx(k)];
-                    B = X1[pidx(N - 1 - k)];
-                } else {
-                    A = cconj(X1[pidx(N - 1 - k)]);
-                    B = cconj(X1[pidx(k)]);
-                }
-                return make_double2(A.x - B.y, A.y + B.x);
-            };
-            group_fft_io<N, +1, false, true>(X1, tid, (const TwoLevelTw *)tw2, 0, inJ, ScratchIO{X1});
+            if (grp == 0)
+                group_fft_io<N, -1, false, true>(X, t, (const TwoLevelTw *)tw2, grp, in, ScratchIO{X});
+            else
+                group_fft_io<N, +1, false, true>(X, t, (const TwoLevelTw *)tw2, grp, in, ScratchIO{X});
         }
         __syncthreads();
-        // ---- G J(tau) into R; G(tau) kept in X2 for the bubble
+        // ---- G(tau) into X1, G J(tau) into X2
         for (int j = tid; j < N; j += NT) {
-            const double tau = j * h;
             const double2 ph = tw_at(ht2, j);
-            const double2 g = cmul(cconj(ph), X2[pidx(j)]);
-            const double2 jr = cmul(ph, X1[pidx(j)]);
-            double g0a, jia, g0b, jib;
-            tails(cs[0], tau, beta, g0a, jia);
-            tails(cs[1], tau, beta, g0b, jib);
-            const double Ga = g.x + g0a, Gb = g.y + g0b, Ja = jr.x + jia, Jb = jr.y + jib;
-            R[j] = Ga * Ja;
-            R[NJ + j] = Gb * Jb;
-            X2[pidx(j)] = make_double2(Ga, Gb);
+            const double2 g = cmul(cconj(ph), X1[pidx(j)]);
+            const double2 jr = cmul(ph, X2[pidx(j)]);
+            double g0[2], ji[2];
+            if (real_roots) {
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const CondCol &c = col[q];
+                    auto E = [&](int k, int jj) -> double {
+                        return tails_hi[(2 * q + k) * P::n_hi + (jj >> 6)] * tails_lo[(2 * q + k) * P::n_lo + (jj & 63)];
+                    };
+                    // r > 0: e = exp(-r tau), j = exp(-r (beta - tau)); r <= 0: the other way round
+                    const double a1 = E(0, j), b1 = E(0, N - j), a2 = E(1, j), b2 = E(1, N - j);
+                    const bool big1 = c.r1.x > 0, big2 = c.r2.x > 0;
+                    g0[q] = -c.u1.x * (big1 ? a1 : b1) - c.u2.x * (big2 ? a2 : b2);
+                    ji[q] = cs[q].v1.x * (big1 ? b1 : a1) + cs[q].v2.x * (big2 ? b2 : a2);
+                }
+            } else {
+                tails(col[0], cs[0], j * h, beta, g0[0], ji[0]);
+                tails(col[1], cs[1], j * h, beta, g0[1], ji[1]);
+            }
+            const double Ga = g.x + g0[0], Gb = g.y + g0[1], Ja = jr.x + ji[0], Jb = jr.y + ji[1];
+            X2[pidx(j)] = make_double2(Ga * Ja, Gb * Jb);
+            X1[pidx(j)] = make_double2(Ga, Gb);
             if (j == 0) {
                 cs[0].Gt0 = Ga;
                 cs[1].Gt0 = Gb;
@@ -487,107 +528,134 @@ __global__ void __launch_bounds__(CondTauSmem<N>::threads, CondTauSmem<N>::min_b
             }
         }
         __syncthreads();
-        if (tid < 2) {
-            ColState &q = cs[tid];
-            double g0b, jinfb;
-            tails(q, beta, beta, g0b, jinfb);
-            const double Jbeta = -q.Jraw0 + jinfb;  // J(beta) = -sum_n J(ikn) + Jinf(beta)
-            R[tid * NJ + N] = (-q.Gt0 - 1.0) * Jbeta;
-            d0s[tid] = q.dGp * q.Jt0 + q.Gt0 * q.dJ0;
-            dNs[tid] = q.dGm * Jbeta - (q.Gt0 + 1.0) * q.dJb;
-            q.CJ1b = R[tid * NJ] - R[tid * NJ + N];
-        }
-        __syncthreads();
-        // ---- Maki-Thompson moment J(iqn) from the G J spline (src/cond_opt.cpp:3622-3660, 3807)
-        spline_second_derivatives<2>(R, NJ, NJ, h, d0s, dNs, a.spl_full, a.spl_full + NJ);
-        if (tid < 2) cs[tid].CJ3b = R[tid * NJ] - R[tid * NJ + N];
-        if (tid < G) {
-            const double *Ma = R, *Mb = R + NJ;
-            auto in = [&](int j) -> double2 {
-                return make_double2((Ma[j + 1] - Ma[j]) * ih, (Mb[j + 1] - Mb[j]) * ih);
-            };
-            group_fft_io<N, -1>(X1, tid, (const TwoLevelTw *)tw2, 0, in, ScratchIO{X1});
-        }
-        __syncthreads();
-        for (int n = 1 + tid; n <= NO; n += NT) {
-            double2 F[2];
-            split_real(X1[pidx(n)], X1[pidx(N - n)], F[0], F[1]);
-            const double wq = 2 * n * pT, iw = 1.0 / wq, iw2 = iw * iw;
-            const double2 e = tw_at(tw2, n);
-            const double2 f = make_double2(1.0 - e.x, -e.y);
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const ColState &s = cs[q];
-                const double imJ = -2.0 * s.CJ1b * iw + 2.0 * s.CJ3b * iw2 * iw + 2.0 * cmul(f, F[q]).y * iw2 * iw2;
-                part[s.bin * PWB + NJ2 + n] -= nf * s.wt * s.dk * imJ * iw;
+        // ---- the bubble -G(tau) G(beta - tau) on [0, beta/2] in X1 (node j reads
+        // nodes j and N - j, and only it does; src/cond_opt.cpp:3662-3700), the
+        // end node and slopes of both splines
+        {
+            KSum va, vb;
+            for (int j = tid; j <= NO; j += NT) {
+                double2 v;
+                if (j == 0) {
+                    v = make_double2(cs[0].Gt0 * (cs[0].Gt0 + 1.0), cs[1].Gt0 * (cs[1].Gt0 + 1.0));
+                } else {
+                    const double2 g = X1[pidx(j)], gm = X1[pidx(N - j)];
+                    v = make_double2(-g.x * gm.x, -g.y * gm.y);
+                }
+                X1[pidx(j)] = v;
+                // trapezoid weights
+                const double w = (j == 0 || j == NO) ? 0.5 : 1.0;
+                va.add(w * v.x);
+                vb.add(w * v.y);
             }
-        }
-        __syncthreads();
-        // ---- bubble -G(tau) G(beta - tau) on [0, beta/2] (src/cond_opt.cpp:3662-3700, 3784-3817)
-        for (int j = tid; j <= NO; j += NT) {
-            const double2 g = X2[pidx(j)];
-            double ga, gb;
-            if (j == 0) {
-                ga = cs[0].Gt0 * (cs[0].Gt0 + 1.0);
-                gb = cs[1].Gt0 * (cs[1].Gt0 + 1.0);
-            } else {
-                const double2 gm = X2[pidx(N - j)];
-                ga = -g.x * gm.x;
-                gb = -g.y * gm.y;
+            if (tid < 2) {
+                ColState &q = cs[tid];
+                double g0b, jinfb;
+                tails(col[tid], q, beta, beta, g0b, jinfb);
+                const double Jbeta = -q.Jraw0 + jinfb;  // J(beta) = -sum_n J(ikn) + Jinf(beta)
+                const double vN = (-q.Gt0 - 1.0) * Jbeta;
+                q.CJ1b = q.Gt0 * q.Jt0 - vN;
+                q.dchi = q.dGp * (q.Gt0 + 1.0) + q.Gt0 * q.dGm;
+                double *xN = reinterpret_cast<double *>(&X2[pidx(N)]);
+                double *s0 = reinterpret_cast<double *>(d0s), *sN = reinterpret_cast<double *>(dNs);
+                xN[tid] = vN;
+                s0[tid] = q.dchi;
+                sN[tid] = 0.0;
+                s0[2 + tid] = q.dGp * q.Jt0 + q.Gt0 * q.dJ0;
+                sN[2 + tid] = q.dGm * Jbeta - (q.Gt0 + 1.0) * q.dJb;
             }
-            R[j] = ga;
-            R[NJ2 + j] = gb;
+            double v2[2] = {va.value(), vb.value()};
+            block_sum<2>(v2, sV);
         }
-        if (tid < 2) {
-            ColState &q = cs[tid];
-            q.dchi = q.dGp * (q.Gt0 + 1.0) + q.Gt0 * q.dGm;
-            d0s[tid] = q.dchi;
-            dNs[tid] = 0.0;
-        }
-        __syncthreads();
-        if (tid < 2) {
-            cs[tid].V0 = R[tid * NJ2];
-            cs[tid].VN = R[tid * NJ2 + NO];
-        }
-        column_sums<2>(R, NJ2, 0, NJ2, sV);
-        spline_second_derivatives<2>(R, NJ2, NJ2, h, d0s, dNs, a.spl_half, a.spl_half + NJ2);
-        column_sums<2>(R, NJ2, 0, NJ2, sM);
-        if (tid < 2) {
-            ColState &q = cs[tid];
-            const double M0 = R[tid * NJ2], MN = R[tid * NJ2 + NO];
-            q.integ = h * (sV[tid] - 0.5 * (q.V0 + q.VN)) - h * h * h / 24.0 * (2.0 * sM[tid] - M0 - MN);
-        }
-        if (tid < G) {
-            const double *Ma = R, *Mb = R + NJ2;
+        // ---- splines and FFT_{-} of both: the bubble's moments from the half
+        // spline (odd about beta/2), the Maki-Thompson moment from the G J
+        // spline (src/cond_opt.cpp:3622-3660, 3784-3817)
+        if (grp == 0) {
+            spline_complex<N>(X1, NJ2, t, 0, h, d0s[0], dNs[0], a.spl_half, a.spl_half + NJ2);
+            KSum ma, mb;
+            for (int j = t; j <= NO; j += G) {
+                const double2 m = X1[pidx(j)];
+                const double w = (j == 0 || j == NO) ? 0.5 : 1.0;
+                ma.add(w * m.x);
+                mb.add(w * m.y);
+            }
+            double2 m = make_double2(ma.value(), mb.value());
+            constexpr int W = G < 32 ? G : 32;
+            const unsigned lanes = G < 32 ? (1u << G) - 1u : 0xffffffffu;
+            for (int off = W / 2; off > 0; off >>= 1) {
+                m.x += __shfl_down_sync(lanes, m.x, off, W);
+                m.y += __shfl_down_sync(lanes, m.y, off, W);
+            }
+            __shared__ double2 red[(G + 31) / 32];
+            if (t % 32 == 0) red[t / 32] = m;
             auto in = [&](int j) -> double2 {
                 const bool lo = j < NO;
                 const int jj = lo ? j : N - 1 - j;
-                const double sg = lo ? 1.0 : -1.0;
-                return make_double2(sg * (Ma[jj + 1] - Ma[jj]) * ih, sg * (Mb[jj + 1] - Mb[jj]) * ih);
+                const double sg = lo ? ih : -ih;
+                const double2 u = X1[pidx(jj)], v = X1[pidx(jj + 1)];
+                return make_double2((v.x - u.x) * sg, (v.y - u.y) * sg);
             };
-            group_fft_io<N, -1>(X1, tid, (const TwoLevelTw *)tw2, 0, in, ScratchIO{X1});
+            group_fft_io<N, -1, false, true>(X1, t, (const TwoLevelTw *)tw2, 0, in, ScratchIO{X1});
+            if (t < 2) {
+                double sM = 0.0;
+                for (int w = 0; w < (G + 31) / 32; ++w) sM += part_of(red[w], t);
+                cs[t].integ = h * sV[t] - h * h * h / 12.0 * sM;
+                if (G == 1) {
+                    sM = red[0].y;
+                    cs[1].integ = h * sV[1] - h * h * h / 12.0 * sM;
+                }
+            }
+        } else if (grp == 1) {
+            spline_complex<N>(X2, NJ, t, 1, h, d0s[1], dNs[1], a.spl_full, a.spl_full + NJ);
+            if (t == 0) {
+                const double2 m0 = X2[0], mN = X2[pidx(N)];
+                cs[0].CJ3b = m0.x - mN.x;
+                cs[1].CJ3b = m0.y - mN.y;
+            }
+            auto in = [&](int j) -> double2 {
+                const double2 u = X2[pidx(j)], v = X2[pidx(j + 1)];
+                return make_double2((v.x - u.x) * ih, (v.y - u.y) * ih);
+            };
+            group_fft_io<N, -1, false, true>(X2, t, (const TwoLevelTw *)tw2, 1, in, ScratchIO{X2});
         }
         __syncthreads();
+        const bool same = col[0].bin == col[1].bin;
         for (int n = 1 + tid; n <= NO; n += NT) {
-            double2 F[2];
-            split_real(X1[pidx(n)], X1[pidx(N - n)], F[0], F[1]);
-            const double wq = 2 * n * pT, iw = 1.0 / wq, iw2 = iw * iw;
+            double2 Fb[2], F[2];
+            split_real(X1[pidx(n)], X1[pidx(N - n)], Fb[0], Fb[1]);
+            split_real(X2[pidx(n)], X2[pidx(N - n)], F[0], F[1]);
+            const double wq = 2 * n * pT, iw = 1.0 / wq, iw2 = iw * iw, iw4 = iw2 * iw2;
             const double2 e = tw_at(tw2, n);
             const double2 f = make_double2(1.0 - e.x, -e.y);
+            double b[2], m[2];
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
+                const CondCol &c = col[q];
                 const ColState &s = cs[q];
-                const double bub = -2.0 * s.dchi * iw2 + cmul(f, F[q]).x * iw2 * iw2;
-                part[s.bin * PWB + n] -= 2.0 * s.wt * nf * s.dk * s.dk * bub;
+                const double imJ = -2.0 * s.CJ1b * iw + 2.0 * s.CJ3b * iw2 * iw + 2.0 * cmul(f, F[q]).y * iw4;
+                const double bub = -2.0 * s.dchi * iw2 + cmul(f, Fb[q]).x * iw4;
+                m[q] = nf * c.wt * c.dk * imJ * iw;
+                b[q] = 2.0 * c.wt * nf * c.dk * c.dk * bub;
+            }
+            double *p0 = part + col[0].bin * PWB + n;
+            if (same) {
+                p0[0] -= b[0] + b[1];
+                p0[NJ2] -= m[0] + m[1];
+            } else {
+                double *p1 = part + col[1].bin * PWB + n;
+                p0[0] -= b[0];
+                p0[NJ2] -= m[0];
+                p1[0] -= b[1];
+                p1[NJ2] -= m[1];
             }
         }
         if (tid == 0) {
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
+                const CondCol &c = col[q];
                 const ColState &s = cs[q];
-                part[s.bin * PWB] -= 2.0 * s.wt * nf * s.dk * s.dk * (2.0 * s.integ);
-                part[s.bin * PWB + NJ2] -= nf * s.wt * s.dk * s.q0;
-                part[a.pw - 1] -= 2.0 * s.wt * nf * s.d2 * s.k0;
+                part[c.bin * PWB] -= 2.0 * c.wt * nf * c.dk * c.dk * (2.0 * s.integ);
+                part[c.bin * PWB + NJ2] -= nf * c.wt * c.dk * s.q0;
+                part[a.pw - 1] -= 2.0 * c.wt * nf * c.d2 * s.k0;
             }
         }
         __syncthreads();
@@ -633,45 +701,50 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// Sum the per-CTA rows in block order: out = [binned (nbins x 2 NB)],
-// [totals chijj1 (NB), chijj2 (NB)], [kx0].  One thread per column of a bin
-// row (i < 2 NB) plus one for kx0 (i = 2 NB).
-__global__ void k_cond_finish(const double *__restrict__ partial, int nblk, int pw, int nbins, int PWB,
-                              const double *__restrict__ lines, int nlines, double *__restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > PWB) return;
-    if (i == PWB) {
+// Sum the per-CTA rows: out = [binned (nbins x 2 NB)], [totals chijj1 (NB),
+// chijj2 (NB)], [kx0].  A block takes 32 columns of a bin row, its warps a
+// segment of the rows each (compensated), added in warp order: deterministic.
+// Block 0 of x = gridDim.x - 1 takes kx0.  One thread per column walked all rows
+// before: 69 us at 256^2 x 4096 with three bins, 19 now.
+constexpr int kCondFinishWarps = 16;
+__global__ void __launch_bounds__(32 * kCondFinishWarps)
+    k_cond_finish(const double *__restrict__ partial, int nblk, int pw, int nbins, int PWB,
+                  const double *__restrict__ lines, int nlines, double *__restrict__ out) {
+    __shared__ double2 seg[kCondFinishWarps][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (blockIdx.x == gridDim.x - 1) {
         KSum s;
-        for (int b = 0; b < nblk; ++b) s.add(partial[(size_t)b * pw + pw - 1]);
-        for (int k = 0; k < nlines; ++k) s.add(lines[k]);
-        out[(size_t)nbins * PWB + PWB] = s.value();
+        for (int b = threadIdx.x; b < nblk + nlines; b += blockDim.x)
+            s.add(b < nblk ? partial[(size_t)b * pw + pw - 1] : lines[b - nblk]);
+        double v[1] = {s.value()};
+        __shared__ double tot[1];
+        block_sum<1>(v, tot);
+        if (threadIdx.x == 0) out[(size_t)nbins * PWB + PWB] = tot[0];
         return;
     }
+    const int i = blockIdx.x * 32 + lane;
+    const int per = (nblk + kCondFinishWarps - 1) / kCondFinishWarps, b0 = warp * per, b1 = min(nblk, b0 + per);
     KSum tot;
     for (int bin = 0; bin < nbins; ++bin) {
-        // eight independent compensated sums over the rows b = r mod 8 (their
-        // loads overlap), added in a fixed order: deterministic
-        constexpr int NS = 8;
-        KSum s8[NS];
-        int b = 0;
-        for (; b + NS <= nblk; b += NS) {
-            double v[NS];
-#pragma unroll
-            for (int r = 0; r < NS; ++r) v[r] = partial[(size_t)(b + r) * pw + bin * PWB + i];
-#pragma unroll
-            for (int r = 0; r < NS; ++r) s8[r].add(v[r]);
-        }
-        for (; b < nblk; ++b) s8[b % NS].add(partial[(size_t)b * pw + bin * PWB + i]);
         KSum s;
-        for (int r = 0; r < NS; ++r) {
-            s.add(s8[r].s);
-            s.add(s8[r].c);
+        if (i < PWB)
+#pragma unroll 4
+            for (int b = b0; b < b1; ++b) s.add(partial[(size_t)b * pw + bin * PWB + i]);
+        seg[warp][lane] = make_double2(s.s, s.c);
+        __syncthreads();
+        if (warp == 0 && i < PWB) {
+            KSum a;
+            for (int w = 0; w < kCondFinishWarps; ++w) {
+                a.add(seg[w][lane].x);
+                a.add(seg[w][lane].y);
+            }
+            const double v = a.value();
+            out[(size_t)bin * PWB + i] = v;
+            tot.add(v);
         }
-        const double v = s.value();
-        out[(size_t)bin * PWB + i] = v;
-        tot.add(v);
+        __syncthreads();
     }
-    out[(size_t)nbins * PWB + i] = tot.value();
+    if (warp == 0 && i < PWB) out[(size_t)nbins * PWB + i] = tot.value();
 }
 
 // ---------------------------------------------------------------------------
@@ -746,21 +819,22 @@ template <int N>
 struct RunCondTau {
     static cudaError_t run(const GridDev *g, const CondDev *c, const double2 *S, const double *s2, const double *s3,
                            const double *sinf, double mu, double T, cudaStream_t st) {
-        const size_t sm = CondTauSmem<N>::bytes;
+        const size_t sm = CondTauPlan<N>::bytes;
         cudaError_t e = set_smem(k_cond_tau<N>, sm);
         if (e != cudaSuccess) return e;
+        CondCol *cols = reinterpret_cast<CondCol *>(c->cols);
+        k_cond_cols<<<(c->K4p + 63) / 64, 64, 0, st>>>(g->ek, c->dek, c->d2ek, c->nbins > 1 ? c->bin : nullptr, sinf,
+                                                       c->K4, c->K4p, g->nbk, mu, T, cols);
+        if ((e = launched()) != cudaSuccess) return e;
         CondTauArgs a;
-        a.hV = c->hV;
-        a.f0V = c->f0V;
+        a.hV = reinterpret_cast<const double2 *>(c->hV);
+        a.f0V = reinterpret_cast<const double2 *>(c->f0V);
         a.dbound = c->dbound;
         a.S = S;
         a.s2 = s2;
         a.s3 = s3;
         a.sinf = sinf;
-        a.ek = g->ek;
-        a.dek = c->dek;
-        a.d2ek = c->d2ek;
-        a.bin = c->nbins > 1 ? c->bin : nullptr;
+        a.cols = cols;
         a.spl_full = g->spl_full;
         a.spl_half = g->spl_half;
         a.tw = g->tw_w;
@@ -768,14 +842,13 @@ struct RunCondTau {
         a.partial = c->partial;
         a.K4 = c->K4;
         a.K4p = c->K4p;
-        a.nbk = g->nbk;
         a.pw = c->pw;
         a.mu = mu;
         a.T = T;
         a.nf = 1.0 / ((double)g->nk0 * g->nk0);
         const size_t pbytes = (size_t)c->nblk * c->pw * sizeof(double);
         if ((e = cudaMemsetAsync(c->partial, 0, pbytes, st)) != cudaSuccess) return e;
-        k_cond_tau<N><<<c->nblk, CondTauSmem<N>::threads, sm, st>>>(a);
+        k_cond_tau<N><<<c->nblk, CondTauPlan<N>::threads, sm, st>>>(a);
         return launched();
     }
 };
@@ -783,13 +856,13 @@ struct RunCondTau {
 template <int N>
 struct CondBlocks {
     static cudaError_t run(int *blocks) {
-        cudaError_t e = set_smem(k_cond_tau<N>, CondTauSmem<N>::bytes);
+        cudaError_t e = set_smem(k_cond_tau<N>, CondTauPlan<N>::bytes);
         if (e != cudaSuccess) return e;
         int dev = 0, sms = 0, per = 0;
         if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
         if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cond_tau<N>, CondTauSmem<N>::threads,
-                                                          CondTauSmem<N>::bytes);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cond_tau<N>, CondTauPlan<N>::threads,
+                                                          CondTauPlan<N>::bytes);
         if (e != cudaSuccess) return e;
         *blocks = sms * (per > 0 ? per : 1);
         return cudaSuccess;
@@ -797,6 +870,8 @@ struct CondBlocks {
 };
 
 }  // namespace
+
+size_t cond_col_words() { return kCondColWords; }
 
 cudaError_t cond_blocks(const GridDev &g, int *blocks) { return dispatch_nw<CondBlocks>(g.nw0, blocks); }
 
@@ -843,7 +918,7 @@ cudaError_t launch_cond_finish(const GridDev &g, const CondDev &c, const double2
     cudaError_t e = launched();
     if (e != cudaSuccess) return e;
     const int PWB = 2 * (g.nw0 / 2 + 1);
-    k_cond_finish<<<(PWB + 1 + 255) / 256, 256, 0, st>>>(c.partial, c.nblk, c.pw, c.nbins, PWB, c.lines, 2 * g.nbk,
+    k_cond_finish<<<(PWB + 31) / 32 + 1, 32 * kCondFinishWarps, 0, st>>>(c.partial, c.nblk, c.pw, c.nbins, PWB, c.lines, 2 * g.nbk,
                                                           c.out);
     return launched();
 }

@@ -845,6 +845,70 @@ __device__ __forceinline__ void stage_pair(double *R, const double *g, int NJ, b
     cp_async_wait_all();
 }
 
+// spline_second_derivatives for one complex column (or two real ones as its
+// parts) of NJ <= N + 1 nodes in the padded layout, by the G threads of a group
+// of the N-point FFT: both parts of a node by one thread, so that its two
+// chains interleave.  TPC of them sweep, in chunks long enough
+// that the kWarm warm-up rows do not dominate.
+template <int N>
+__device__ void spline_complex(double2 *X, int NJ, int t, int grp, double h, double2 d0, double2 dN,
+                               const double *__restrict__ invp, const double *__restrict__ cp) {
+    constexpr int G = FftPlan<N>::G, TPC = G >= 64 ? G / 2 : G;
+    const int C = (NJ + TPC - 1) / TPC, last = NJ - 1;
+    const int s = t < TPC ? min(t * C, NJ) : NJ, e = min(s + C, NJ);
+    const double a6 = 6.0 / (h * h), b6 = 6.0 / h, ih = 1.0 / h;
+    const double cpiv = last > kSplinePivotConst ? __ldg(&invp[kSplinePivotConst]) : 0.0;
+    auto piv = [&](int i) -> double { return (i >= kSplinePivotConst && i < last) ? cpiv : __ldg(&invp[i]); };
+    auto sup = [&](int i) -> double { return (i >= kSplinePivotConst && i < last) ? cpiv : __ldg(&cp[i]); };
+    auto rhs1 = [&](int i, double vm, double v0, double vp, double dl, double dr) -> double {
+        if (i == 0) return b6 * ((vp - v0) * ih - dl);
+        if (i == last) return b6 * (dr - (v0 - vm) * ih);
+        return a6 * (vp - 2.0 * v0 + vm);
+    };
+    auto rhs = [&](int i, double2 vm, double2 v0, double2 vp) -> double2 {
+        return make_double2(rhs1(i, vm.x, v0.x, vp.x, d0.x, dN.x), rhs1(i, vm.y, v0.y, vp.y, d0.y, dN.y));
+    };
+    const double2 zero = make_double2(0.0, 0.0);
+    double2 carry = zero, vm_h = zero, vs_h = zero, ve_h = zero;
+    if (s < e) {
+        if (s > 0) {
+            const int i0 = max(0, s - kWarm);
+            double2 vm = i0 > 0 ? X[pidx(i0 - 1)] : zero, v0 = X[pidx(i0)];
+            for (int i = i0; i < s; ++i) {
+                const double2 vp = X[pidx(i + 1)];
+                carry = cscale(csub(rhs(i, vm, v0, vp), carry), piv(i));
+                vm = v0;
+                v0 = vp;
+            }
+            vm_h = X[pidx(s - 1)];
+        }
+        vs_h = X[pidx(s)];
+        if (e < NJ) ve_h = X[pidx(e)];
+    }
+    group_sync<G>(grp);
+    if (s < e) {
+        double2 vm = vm_h, v0 = vs_h;
+        for (int i = s; i < e; ++i) {
+            const double2 vp = (i + 1 < e) ? X[pidx(i + 1)] : ve_h;
+            carry = cscale(csub(rhs(i, vm, v0, vp), carry), piv(i));
+            X[pidx(i)] = carry;
+            vm = v0;
+            v0 = vp;
+        }
+    }
+    group_sync<G>(grp);
+    double2 mm = zero;
+    if (s < e && e < NJ)
+        for (int i = min(last, e - 1 + kWarm); i >= e; --i) mm = csub(X[pidx(i)], cscale(mm, sup(i)));
+    group_sync<G>(grp);
+    if (s < e)
+        for (int i = e - 1; i >= s; --i) {
+            mm = csub(X[pidx(i)], cscale(mm, sup(i)));
+            X[pidx(i)] = mm;
+        }
+    group_sync<G>(grp);
+}
+
 // ---------------------------------------------------------------------------
 // dispatch over the compiled sizes
 // ---------------------------------------------------------------------------

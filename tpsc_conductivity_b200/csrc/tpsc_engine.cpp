@@ -1103,6 +1103,7 @@ int ensure_cond(tpsc_ctx *ctx, Grid *g, int nbins) {
         A(dalloc(g, &c.f0V, K4p * NJ));
         A(dalloc(g, &c.pre, 4 * K4p));
         A(dalloc(g, &c.dbound, 4 * K4p));
+        A(dalloc(g, &c.cols, cond_col_words() * K4p));
         A(dalloc(g, &c.lines, (size_t)2 * nbk));
 #undef A
         if (e != cudaSuccess) return cuda_fail(ctx, e, "conductivity allocation");

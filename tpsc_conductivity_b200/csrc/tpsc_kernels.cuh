@@ -255,11 +255,13 @@ struct CondDev {
     double *f0V = nullptr;     // [K4p (Nw0+1)] f0 V(r, tau), two-column blocks
     double *pre = nullptr;     // [4 K4p] transformed h, f0 at tau = 0, beta
     double *dbound = nullptr;  // [4 K4p] dhV(0), dhV(beta), df0V(0), df0V(beta)
+    double *cols = nullptr;    // [K4p cond_col_words()] per-column constants of the tau kernel
     double *partial = nullptr; // [nblk pw] per-CTA sums
     double *lines = nullptr;   // [2 nbk] kx0 terms of the kx = 0, pi lines
     double *out = nullptr;     // [nbins 2 NB] binned, [2 NB] totals, kx0 (NB = Nw0/2+1)
 };
 
+size_t cond_col_words();
 cudaError_t cond_blocks(const GridDev &g, int *blocks);
 // the (eps - mu0, A, B) table of the h and f0 slices into c.tab
 cudaError_t launch_cond_table(const GridDev &g, const CondDev &c, double mu0, double T, cudaStream_t st);
