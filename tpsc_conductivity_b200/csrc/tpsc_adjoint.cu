@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
                         double *__restrict__ part) {
     constexpr int K4 = (NBK - 2) * NBK;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK, SlicePlan<NBK>::wide>(S, tw);
+    const auto *tws = slice_twiddles<NBK, SliceGroups<NBK>::wide>(S, tw);
     const int kind = blockIdx.x;
     const double sg = kind ? -1.0 : 1.0, beta = 1.0 / T, tE = kind ? beta : 0.0;
     const int nb = nw0 / 2 + 1;
@@ -719,7 +719,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
                      double *__restrict__ tmpU, double *__restrict__ vcond, double *__restrict__ part) {
     constexpr int K4 = (NBK - 2) * NBK;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = plan_twiddles<NBK>(S, tw);
     const int jv = blockIdx.x, nb = nw0 / 2 + 1;
     const double beta = 1.0 / T;
     double *u = tmpU + (size_t)jv * K4p;
@@ -733,7 +733,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
         // u = T^T hVb(j)
         for (int c = threadIdx.x; c < K4; c += blockDim.x) S[c] = hVb[bidx2(j, c, nw0 + 1)] / edge_w(c % NBK, NBK);
         __syncthreads();
-        dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+        plan_dst_dct<NBK>(S, tws);
         for (int c = threadIdx.x; c < K4; c += blockDim.x) u[c] = S[c] * edge_w(c % NBK, NBK);
         __syncthreads();
         // h_j = T (A E(t))
@@ -742,7 +742,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
             S[c] = xa.y * h_E(xa.x, t, beta);
         }
         __syncthreads();
-        dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+        plan_dst_dct<NBK>(S, tws);
         for (int c = threadIdx.x; c < K4; c += blockDim.x) {
             const int l = c / NBK, m = c % NBK;
             const double uc = u[c];
@@ -754,7 +754,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
             S[c] = hb / edge_w(m, NBK);
         }
         __syncthreads();
-        dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+        plan_dst_dct<NBK>(S, tws);
         for (int c = threadIdx.x; c < K4; c += blockDim.x) {
             const double s = S[c] * edge_w(c % NBK, NBK);
             const double *tc = htab + 8 * (size_t)c;
@@ -928,7 +928,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
     constexpr int n8 = NBK * (NBK + 1) / 2;
     constexpr int NR = (n8 + SlicePlan<NBK>::threads - 1) / SlicePlan<NBK>::threads;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = plan_twiddles<NBK>(S, tw);
     const int jv = blockIdx.x, nb = nw0 / 2 + 1;
     double vacc[NR];
 #pragma unroll
@@ -944,7 +944,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
             put_sym<NBK>(S, l, m, stb[bidx(j, o, nw0 + 1)] / oct_tw(l, m, NBK));
         }
         __syncthreads();
-        dct2_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+        plan_dct2<NBK>(S, tws);
         int k = 0;
         const size_t rj = (size_t)j * n8;
         for (int o = threadIdx.x; o < n8; o += blockDim.x, ++k) {
@@ -1004,7 +1004,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
     constexpr int n8 = NBK * (NBK + 1) / 2;
     constexpr int NR = (n8 + kSliceThreads - 1) / kSliceThreads;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK, SlicePlan<NBK>::wide>(S, tw);
+    const auto *tws = slice_twiddles<NBK, SliceGroups<NBK>::wide>(S, tw);
     const int nb = nw0 / 2 + 1;
     double u[2][NR];
 #pragma unroll 1
@@ -1134,7 +1134,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
                    double U, double Usp, double Uch, double *__restrict__ part) {
     constexpr int n8 = NBK * (NBK + 1) / 2;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = plan_twiddles<NBK>(S, tw);
     const int n = blockIdx.x;
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
@@ -1142,7 +1142,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
         put_sym<NBK>(S, l, m, Vb[bidx(n, o, nb)] / oct_tw(l, m, NBK));
     }
     __syncthreads();
-    dct2_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+    plan_dct2<NBK>(S, tws);
     const double nU = normFact * U;
     double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // th1, th2, Usp, Uch, U
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
@@ -1208,7 +1208,7 @@ template <int NBK>
 struct RunCondSliceBwd {
     static cudaError_t run(const GridDev *g, const CondDev *c, const AdjDev *a, const double *V,
                            const double *dchirt0, double mu0, double T, double fact4, double dmu0_2, cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes, smw = SliceSmem<NBK, SlicePlan<NBK>::wide>::bytes;
+        const size_t sm = SlicePlan<NBK>::bytes, smw = SliceSmem<NBK, SliceGroups<NBK>::wide>::bytes;
         cudaError_t e = set_smem(k_cond_boundary_bwd<NBK>, smw);
         if (e != cudaSuccess) return e;
         if ((e = set_smem(k_cond_slice_bwd<NBK>, sm)) != cudaSuccess) return e;
@@ -1240,7 +1240,7 @@ struct RunSigmaSliceBwd {
     static cudaError_t run(const GridDev *g, const CondDev *c, const AdjDev *a, const double *Grt, const double *V,
                            const double *dchirt0, const double *dG0p, double mu0, double fact8, double dmu0_2,
                            cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes, smw = SliceSmem<NBK, SlicePlan<NBK>::wide>::bytes;
+        const size_t sm = SlicePlan<NBK>::bytes, smw = SliceSmem<NBK, SliceGroups<NBK>::wide>::bytes;
         cudaError_t e = set_smem(k_sigma_slice_bwd<NBK>, sm);
         if (e != cudaSuccess) return e;
         if ((e = set_smem(k_sigma_boundary_bwd<NBK>, smw)) != cudaSuccess) return e;
@@ -1271,7 +1271,7 @@ template <int NBK>
 struct RunVertexQBwd {
     static cudaError_t run(const GridDev *g, const AdjDev *a, const double *chiq, double U, double Usp, double Uch,
                            double T, cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes;
+        const size_t sm = SlicePlan<NBK>::bytes;
         cudaError_t e = set_smem(k_vertex_q_bwd<NBK>, sm);
         if (e != cudaSuccess) return e;
         const double normFact = T / ((double)g->nk0 * g->nk0);

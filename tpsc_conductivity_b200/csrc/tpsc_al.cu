@@ -81,7 +81,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
                   int nw0, int n8, double T, double *__restrict__ hGt, double *__restrict__ pre) {
     constexpr int K4 = (NBK - 2) * NBK;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = plan_twiddles<NBK>(S, tw);
     const int j = blockIdx.x;
     const double t = j / (nw0 * T);
     const double bt = 1.0 / T - t;
@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
         S[c] = xa.y * exp(xa.x > 0 ? -xa.x * t : xa.x * bt);
     }
     __syncthreads();
-    dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+    plan_dst_dct<NBK>(S, tws);
     for (int c = threadIdx.x; c < K4; c += blockDim.x) {
         const int l = c / NBK, m = c % NBK;
         const double v = S[c];
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
         S[c] = v * g_minus(Grt, nw0, n8, j, oct_index(l + 1, m));
     }
     __syncthreads();
-    dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+    plan_dst_dct<NBK>(S, tws);
     for (int c = threadIdx.x; c < K4; c += blockDim.x) hGt[bidx2(j, c, nw0 + 1)] = S[c];
 }
 
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
                   double *__restrict__ dhG) {
     constexpr int K4 = (NBK - 2) * NBK;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK, SlicePlan<NBK>::wide>(S, tw);
+    const auto *tws = slice_twiddles<NBK, SliceGroups<NBK>::wide>(S, tw);
     const int kind = blockIdx.x;
     for (int c = threadIdx.x; c < K4; c += blockDim.x) {
         const int l = c / NBK, m = c % NBK;
@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
              int nw0, double nf, double2 *__restrict__ HR, double2 *__restrict__ dHR) {
     constexpr int K4 = (NBK - 2) * NBK, K4p = (K4 + 1) & ~1;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = plan_twiddles<NBK>(S, tw);
     const int b = blockIdx.x, NJ = nw0 + 1;
     const size_t row = (size_t)blockIdx.y * NJ + b, drow = (size_t)blockIdx.y * 2 + (b - NJ);
     const double2 *src = b < NJ ? HQ + row * K4p : dHQ + drow * K4;
@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
     for (int part = 0; part < 2; ++part) {
         for (int c = threadIdx.x; c < K4; c += blockDim.x) S[c] = nf * (part == 0 ? src[c].x : src[c].y);
         __syncthreads();
-        dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+        plan_dst_dct<NBK>(S, tws);
         for (int c = threadIdx.x; c < K4; c += blockDim.x) dst[2 * c + part] = S[c];
         __syncthreads();
     }
@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
              int n8, double mu0, double2 *__restrict__ HK, double2 *__restrict__ H2K, double2 *__restrict__ dHK) {
     constexpr int K4 = (NBK - 2) * NBK, K4p = (K4 + 1) & ~1;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = plan_twiddles<NBK>(S, tw);
     const int b = blockIdx.x, NJ = nw0 + 1;
     HR += (size_t)blockIdx.y * NJ * K4p;
     dHR += (size_t)blockIdx.y * 2 * K4;
@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
             S[c] = v;
         }
         __syncthreads();
-        dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+        plan_dst_dct<NBK>(S, tws);
         for (int c = threadIdx.x; c < K4; c += blockDim.x) {
             double *dst;
             if (b < NJ)
@@ -601,7 +601,7 @@ template <int NBK>
 struct RunAlHg {
     static cudaError_t run(const GridDev *g, const CondDev *c, const AlDev *a, const double *dG0p, double mu0,
                            double T, cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes, smw = SliceSmem<NBK, SlicePlan<NBK>::wide>::bytes;
+        const size_t sm = SlicePlan<NBK>::bytes, smw = SliceSmem<NBK, SliceGroups<NBK>::wide>::bytes;
         cudaError_t e = set_smem(k_al_hg_slice<NBK>, sm);
         if (e != cudaSuccess) return e;
         if ((e = set_smem(k_al_hg_bound<NBK>, smw)) != cudaSuccess) return e;
@@ -640,7 +640,7 @@ struct RunAlHq {
 template <int NBK>
 struct RunAlSlices {
     static cudaError_t run(const GridDev *g, const AlDev *a, const double *dG0p, double mu0, int nfr, cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes;
+        const size_t sm = SlicePlan<NBK>::bytes;
         cudaError_t e = set_smem(k_al_q2r<NBK>, sm);
         if (e != cudaSuccess) return e;
         if ((e = set_smem(k_al_r2k<NBK>, sm)) != cudaSuccess) return e;

@@ -135,30 +135,35 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
                  double *__restrict__ pre) {
     constexpr int K4 = (NBK - 2) * NBK;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = plan_twiddles<NBK>(S, tw);
     const int j = blockIdx.x, y = blockIdx.y;
     const int nb = nw0 / 2 + 1;
     const double t = j / (nw0 * T);
     const double bt = 1.0 / T - t;
-    for (int c = threadIdx.x; c < K4; c += blockDim.x) {
-        const double2 xa = *reinterpret_cast<const double2 *>(tab + 4 * c);
-        const double b = tab[4 * c + 2];
-        const double E = exp(xa.x > 0 ? -xa.x * t : xa.x * bt);
-        S[c] = (y == 0) ? xa.y * E : (xa.y * t + b) * E;  // row l, column m: c = l NBK + m
-    }
+    batched<4>(
+        K4,
+        [&](int c) -> double3 {
+            const double2 xa = *reinterpret_cast<const double2 *>(tab + 4 * c);
+            return make_double3(xa.x, xa.y, y == 0 ? 0.0 : tab[4 * c + 2]);
+        },
+        [&](int c, double3 v) {
+            const double E = exp(v.x > 0 ? -v.x * t : v.x * bt);
+            S[c] = (y == 0) ? v.y * E : (v.y * t + v.z) * E;  // row l, column m: c = l NBK + m
+        });
     __syncthreads();
-    dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+    plan_dst_dct<NBK>(S, tws);
     const int jv = j < nb ? j : nw0 - j;
     const bool edge = (j == 0 || j == nw0);
     double *pe = pre + (size_t)(2 * y + (j == nw0 ? 1 : 0)) * K4p;
-    for (int c = threadIdx.x; c < K4; c += blockDim.x) {
-        const int l = c / NBK, m = c % NBK;
-        const double v = S[c];
-        if (edge) pe[c] = v;
-        S[c] = v * (2.0 * V[bidx(jv, oct_index(l + 1, m), nb)]);
-    }
+    batched<8>(
+        K4, [&](int c) -> double { return V[bidx(jv, oct_index(c / NBK + 1, c % NBK), nb)]; },
+        [&](int c, double w) {
+            const double v = S[c];
+            if (edge) pe[c] = v;
+            S[c] = v * (2.0 * w);
+        });
     __syncthreads();
-    dst_dct_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+    plan_dst_dct<NBK>(S, tws);
     double *out = (y == 0) ? hV : f0V;
     for (int c = threadIdx.x; c < K4; c += blockDim.x) out[bidx2(j, c, nw0 + 1)] = S[c];
 }
@@ -175,7 +180,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
                     int nw0, int K4p, double mu0, double T, double nf, double fact, double *__restrict__ dbound) {
     constexpr int K4 = (NBK - 2) * NBK;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK, SlicePlan<NBK>::wide>(S, tw);
+    const auto *tws = slice_twiddles<NBK, SliceGroups<NBK>::wide>(S, tw);
     const int kind = blockIdx.x;
     const int nb = nw0 / 2 + 1;
     for (int c = threadIdx.x; c < K4; c += blockDim.x) {
@@ -795,7 +800,7 @@ struct RunCondSlices {
     // ny = 2: the h and f0 slices and all four end conditions; ny = 1: h only
     static cudaError_t run(const GridDev *g, const CondDev *c, const double *V, const double *dchirt0, double mu0,
                            double T, double fact, int ny, bool f32, cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes, smw = SliceSmem<NBK, SlicePlan<NBK>::wide>::bytes;
+        const size_t sm = SlicePlan<NBK>::bytes, smw = SliceSmem<NBK, SliceGroups<NBK>::wide>::bytes;
         cudaError_t e = set_smem(k_cond_slice<NBK>, sm);
         if (e != cudaSuccess) return e;
         if ((e = set_smem(k_cond_boundary<NBK>, smw)) != cudaSuccess) return e;

@@ -145,29 +145,21 @@ cudaError_t finish(Reduce r, int nblocks, double offset0, cudaStream_t st, const
 // ---------------------------------------------------------------------------
 // slice kernels: shared-memory plan of one nbk x nbk slice + FFT scratch
 // ---------------------------------------------------------------------------
-// Threads, FFT groups and CTAs per SM of an FP64 slice kernel.  A pass
+// FFT groups of an FP64 slice kernel whose lines go through the plain FFT.  A pass
 // transforms (NBK + 1)/2 line pairs, one per group of G threads, and the
 // groups' scratch is most of the shared memory, so a block holds the groups
-// that a pass can use and no more: 129 lines take 22 groups (65 pairs in 3
-// rounds, one CTA per SM), smaller slices one group per pair and as many
-// CTAs as the registers allow.  A fixed 352 threads left 25% (65 lines) to
+// that a pass can use and no more: a fixed 352 threads left 25% (65 lines) to
 // 95% (9 lines) of a block idle in the transforms at one CTA per SM.
-// 128^2 x 2048, G slices (2049 per SM-filling launch): 121 -> 100 us, cond
-// slices with both transforms 236 -> 184; 64^2 x 1024, r -> k slices of the
-// Aslamazov-Larkin term 85 -> 60 us.  65 lines in 2 rounds of 17 groups at
-// three CTAs took 104 us, in 3 rounds of 11 groups 119.
 template <int NBK>
-struct SlicePlan {
+struct SliceGroups {
     static constexpr int G = FftPlan<2 * (NBK - 1)>::G;
     static constexpr int ngrp = NBK >= 129 ? kSliceThreads / G : (NBK + 1) / 2;
-    static constexpr int threads = NBK >= 129 ? kSliceThreads : NBK == 17 ? 64 : (ngrp * G + 31) / 32 * 32;
-    static constexpr int blocks = NBK >= 129 ? 1 : NBK == 65 ? 2 : NBK == 33 ? 4 : 8;
     // groups of a kSliceThreads block: the one- to four-CTA boundary kernels,
     // whose single slice should be done as soon as possible
     static constexpr int wide = kSliceThreads / G;
 };
 
-template <int NBK, int NG = SlicePlan<NBK>::ngrp>
+template <int NBK, int NG = SliceGroups<NBK>::ngrp>
 struct SliceSmem {
     static constexpr int L = 2 * (NBK - 1);
     static constexpr int G = FftPlan<L>::G;
@@ -191,7 +183,7 @@ __device__ __forceinline__ double2 *slice_scratch(double *S) {
 // FFT scratch -- the full table, or where that does not fit the two-level
 // table (entry m = hi[m >> 6] lo[m & 63]); the first __syncthreads of the
 // kernel publishes it.
-template <int NBK, int NG = SlicePlan<NBK>::ngrp>
+template <int NBK, int NG = SliceGroups<NBK>::ngrp>
 __device__ __forceinline__ auto slice_twiddles(double *S, const double2 *__restrict__ tw) {
     constexpr int L = SliceSmem<NBK>::L;
     char *base = reinterpret_cast<char *>(S) + SliceSmem<NBK, NG>::tw_off;
@@ -207,6 +199,63 @@ __device__ __forceinline__ auto slice_twiddles(double *S, const double2 *__restr
         }
         return (const TwoLevelTw *)t;
     }
+}
+
+// Threads, shared memory and CTAs per SM of an FP64 slice kernel, and how its
+// lines are transformed: by the symmetric FFT (sym_lines) from 33 lines on, which
+// takes 0.6 of the plain one's arithmetic and shared-memory traffic and fits 33
+// groups where 22 did (129 lines: 2 rounds of line pairs instead of 3); below, one
+// radix-16 pass is all of the transform and symmetry saves nothing.  KEEP: G and
+// chi0 up to 65 lines stay on the plain FFT -- the reference's diagnostics
+// |Usp - Usp(half grid)| / Usp are ~1e-9, so a rounding of chi0 that differs in
+// the last bit moves them by 1e-8 of themselves.
+// Plain -> symmetric, one launch: correlator slices (two transforms) 256^2 x 4096
+// 3390 -> 2940 us, 128^2 x 2048 184 -> 156; G 256^2 778 -> 687, Sigma 724 -> 630;
+// Aslamazov-Larkin q -> r 64^2 x 1024 18.0 -> 14.2 us a frequency.
+template <int NBK, bool KEEP = false>
+struct SlicePlan {
+    static constexpr bool sym = NBK >= (KEEP ? 129 : 33);
+    static constexpr int warps = NBK >= 129 ? 11 : NBK == 65 ? 6 : 2;  // of symmetric groups
+    static constexpr int G = FftPlan<2 * (NBK - 1)>::G;
+    static constexpr int threads = sym ? 32 * warps : NBK == 17 ? 64 : (SliceGroups<NBK>::ngrp * G + 31) / 32 * 32;
+    static constexpr int blocks = NBK >= 129 ? 1 : NBK == 65 ? 2 : NBK == 33 ? (sym ? 8 : 4) : 8;
+    static constexpr size_t scr_off = SliceSmem<NBK>::scr_off;
+    static constexpr size_t sym_scr() {
+        using F = SymFft<2 * (NBK - 1) >= 64 ? 2 * (NBK - 1) : 64>;
+        return (size_t)warps * F::per_warp * F::len * sizeof(double2);
+    }
+    static constexpr size_t sym_tw() { return SymFft<2 * (NBK - 1) >= 64 ? 2 * (NBK - 1) : 64>::ntw * sizeof(double2); }
+    static constexpr size_t tw_off = sym ? scr_off + sym_scr() : SliceSmem<NBK>::tw_off;
+    static constexpr size_t bytes = sym ? tw_off + sym_tw() : SliceSmem<NBK>::bytes;
+    static_assert(bytes <= 232448, "slice does not fit in shared memory");
+};
+
+// the twiddles of the plan's transform in shared memory (the first
+// __syncthreads of the kernel publishes them)
+template <int NBK, bool KEEP = false>
+__device__ __forceinline__ auto plan_twiddles(double *S, const double2 *__restrict__ tw) {
+    if constexpr (SlicePlan<NBK, KEEP>::sym) {
+        using F = SymFft<2 * (NBK - 1)>;
+        double2 *t = reinterpret_cast<double2 *>(reinterpret_cast<char *>(S) + SlicePlan<NBK, KEEP>::tw_off);
+        for (int i = threadIdx.x; i < F::ntw; i += blockDim.x) t[i] = __ldg(&tw[(i / F::G + 1) * (i % F::G)]);
+        return (const double2 *)t;
+    } else {
+        return slice_twiddles<NBK>(S, tw);
+    }
+}
+template <int NBK, bool KEEP = false, class TW>
+__device__ __forceinline__ void plan_dct2(double *S, const TW *tws) {
+    if constexpr (SlicePlan<NBK, KEEP>::sym)
+        sym_dct2_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+    else
+        dct2_slice<NBK, SliceGroups<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+}
+template <int NBK, class TW>
+__device__ __forceinline__ void plan_dst_dct(double *S, const TW *tws) {
+    if constexpr (SlicePlan<NBK>::sym)
+        sym_dst_dct_slice<NBK>(S, slice_scratch<NBK>(S), tws);
+    else
+        dst_dct_slice<NBK, SliceGroups<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
 }
 
 // L2 prefetch by the CTA of [p, p + bytes), one request per 128-byte line,
@@ -275,6 +324,27 @@ __device__ __forceinline__ void fill_octant(T *S, int n8, const Value &value) {
                 S[l * NBK + m] = v[b];
                 S[m * NBK + l] = v[b];
             }
+        }
+    }
+}
+
+// use(i, load(i)) for the block's i < n, KB points of a thread loaded before the
+// first of them is used: a loop of one load and one use each waits a memory
+// latency per point (with one CTA per SM half the time of the correlator's 129-
+// line slices)
+template <int KB, class Load, class Use>
+__device__ __forceinline__ void batched(int n, const Load &load, const Use &use) {
+    for (int base = threadIdx.x; base < n; base += KB * blockDim.x) {
+        decltype(load(0)) v[KB];
+#pragma unroll
+        for (int b = 0; b < KB; ++b) {
+            const int i = base + b * blockDim.x;
+            if (i < n) v[b] = load(i);
+        }
+#pragma unroll
+        for (int b = 0; b < KB; ++b) {
+            const int i = base + b * blockDim.x;
+            if (i < n) use(i, v[b]);
         }
     }
 }

@@ -268,16 +268,7 @@ __device__ __forceinline__ void stockham_pass(C *x, int t, int Ns, const TW *__r
         if (Ns > 1) {
             // twiddle exp(SIGN 2 pi i k q / (Ns R)) = tw[k q N/(Ns R)] (conjugated for SIGN>0)
             const int step = k * (N / (Ns * R));
-            if constexpr (N == 256 && R == 16 && !FIRST && sizeof(C) == sizeof(float2)) {
-                // the FP32 256-point transform's second pass (Ns = 16, step = k):
-                // its twiddles tw[k q], q = 1..15, are read from the transposed
-                // copy behind the table, entry 256 + (q - 1) 16 + k, so that the
-                // 16 threads of a group read 16 consecutive entries (no bank
-                // conflicts; strided reads tw[k q] are up to 16-way for even q)
-#pragma unroll
-                for (int q = 1; q < R; ++q)
-                    v[u * R + q] = twiddle<SIGN, SMEM_TW>(v[u * R + q], tw, 256 + (q - 1) * 16 + k);
-            } else if constexpr (R == 16 && sizeof(C) == sizeof(double2)) {
+            if constexpr (R == 16 && sizeof(C) == sizeof(double2)) {
                 twiddle16_powers<N, SIGN, SMEM_TW>(&v[u * R], tw, step);
             } else {
 #pragma unroll
@@ -365,6 +356,165 @@ template <int N, int SIGN, bool SMEM_TW = false, class C, class TW>
 __device__ __forceinline__ void group_fft(C *x, int t, const TW *__restrict__ tw, int grp) {
     const ScratchIOT<C> io{x};
     group_fft_io<N, SIGN, SMEM_TW, true>(x, t, tw, grp, io, io);
+}
+
+// ---------------------------------------------------------------------------
+// L-point FFT (sign -1) of a sequence with z_{L-j} = SIG z_j (SIG = 1 even,
+// -1 odd), L = 16 B, whose outputs have the same symmetry: of the B radix-16
+// butterflies of the first pass and the 16 radix-B ones of the second only
+// B/2 + 1 and 9 are formed, the others follow:
+//   A_b(r) = sum_q z_{b + B q} w_16^{q r},  T_b(r) = w_L^{b r} A_b(r),
+//   T_{B-b}(r) = SIG T_b(-r),
+//   Z_{r + 16 m} = sum_b w_B^{b m} T_b(r),  Z_{L-k} = SIG Z_k.
+// A group of B/2 + 1 threads makes one transform (9, 5 and 3 threads for L =
+// 256, 128 and 64 instead of 16, 8 and 4), with one exchange of 17 (B/2 + 1)
+// points through its scratch x instead of L: 0.6 of the arithmetic and of the
+// shared-memory traffic.  T_b(r) is stored for r = -8..8 (both signs of 8: the
+// twiddle is that of the signed r).
+// ---------------------------------------------------------------------------
+template <int L>
+struct SymFft {
+    static constexpr int B = L / 16;
+    static constexpr int G = B / 2 + 1;           // threads
+    static constexpr int per_warp = 32 / G;       // groups of a warp
+    static constexpr int len = 17 * G;            // scratch, complex
+    static constexpr int R = (9 + G - 1) / G;     // second-pass butterflies per thread
+    static constexpr int ntw = 8 * G;             // twiddles w_L^{b m}, entry (m - 1) G + b
+};
+// v[1..15] -> T_b(signed r) into x[8 + r]; tw as ntw describes
+template <int L>
+__device__ __forceinline__ void sym_store(const double2 (&v)[16], double2 *x, int b, const double2 *__restrict__ tw) {
+    constexpr int G = SymFft<L>::G;
+    const double2 w1 = tw[b], w2 = tw[G + b], w4 = tw[3 * G + b], w8 = tw[7 * G + b];
+    const double2 w3 = cmul(w2, w1), w5 = cmul(w4, w1), w6 = cmul(w4, w2), w7 = cmul(w4, w3);
+    const double2 w[9] = {w1, w1, w2, w3, w4, w5, w6, w7, w8};
+    x[8] = v[0];
+#pragma unroll
+    for (int r = 1; r <= 8; ++r) {
+        x[8 + r] = cmul(v[r], w[r]);
+        x[8 - r] = cmul(v[(16 - r) & 15], cconj(w[r]));
+    }
+}
+template <int L>
+__device__ __forceinline__ void sym_store(const float2 (&v)[16], float2 *x, int b, const float4 *__restrict__ tw) {
+    constexpr int G = SymFft<L>::G;
+    x[8] = v[0];
+#pragma unroll
+    for (int r = 1; r <= 8; ++r) {
+        const int e = (r - 1) * G + b;
+        x[8 + r] = twiddle<-1, true>(v[r], tw, e);
+        x[8 - r] = twiddle<+1, true>(v[(16 - r) & 15], tw, e);
+    }
+}
+// The transforms of lines [0, nline) in packed pairs, a group of the block's
+// warps per pair and round; in(p, j) is z_j of pair p (any j < L), out(p, k, Z_k)
+// takes the outputs k <= L/2.  All threads of the block must call.
+template <int L, int SIG, class C, class TW, class In, class Out>
+__device__ __forceinline__ void sym_lines(C *scr, const TW *__restrict__ tw, int npair, const In &in, const Out &out) {
+    using P = SymFft<L>;
+    constexpr int B = P::B, G = P::G, N = L / 2;
+    const int lane = threadIdx.x & 31, g = lane / G, t = lane % G;
+    const int ngrp = (blockDim.x >> 5) * P::per_warp, grp = (threadIdx.x >> 5) * P::per_warp + g;
+    C *x = scr + grp * P::len;
+#pragma unroll 1
+    for (int p0 = 0; p0 < npair; p0 += ngrp) {
+        const int p = p0 + grp;
+        const bool on = g < P::per_warp && p < npair;
+        if (on) {
+            C v[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) v[q] = in(p, t + B * q);
+            dft<-1, 16>(v);
+            sym_store<L>(v, x + 17 * t, t, tw);
+        }
+        __syncwarp();
+        if (on) {
+#pragma unroll
+            for (int i = 0; i < P::R; ++i) {
+                const int r = t + G * i;
+                if (P::R * G > 9 && r > 8) break;
+                C u[B];
+#pragma unroll
+                for (int b = 0; b < B; ++b) {
+                    if (b <= B / 2) {
+                        u[b] = x[17 * b + 8 + r];
+                    } else {
+                        u[b] = x[17 * (B - b) + 8 - r];
+                        if (SIG < 0) u[b] = C{-u[b].x, -u[b].y};
+                    }
+                }
+                dft<-1, B>(u);
+#pragma unroll
+                for (int m = 0; m < B; ++m) {
+                    const int k = r + 16 * m;
+                    if (k <= N) {
+                        out(p, k, u[m]);
+                    } else if (r != 0 && r != 8) {
+                        out(p, L - k, SIG < 0 ? C{-u[m].x, -u[m].y} : u[m]);
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// dct2_slice and dst_dct_slice (below) by symmetric transforms: scr holds
+// SymFft<L>::len complex per group of every warp, tw SymFft<L>::ntw twiddles.
+template <int NBK, class T, class C, class TW>
+__device__ void sym_dct2_slice(T *S, C *scr, const TW *tw) {
+    constexpr int L = 2 * (NBK - 1);
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+        const int es = pass == 0 ? 1 : NBK, ls = pass == 0 ? NBK : 1;
+        auto in = [&](int p, int j) -> C {
+            const int c = (j < NBK ? j : L - j) * es;
+            const T *a = S + 2 * p * ls;
+            return C{a[c], 2 * p + 1 < NBK ? a[ls + c] : (T)0};
+        };
+        auto out = [&](int p, int k, C z) {
+            T *a = S + 2 * p * ls + k * es;
+            a[0] = z.x;
+            if (2 * p + 1 < NBK) a[ls] = z.y;
+        };
+        sym_lines<L, 1>(scr, tw, (NBK + 1) / 2, in, out);
+        __syncthreads();
+    }
+}
+template <int NBK, class T, class C, class TW>
+__device__ void sym_dst_dct_slice(T *S, C *scr, const TW *tw) {
+    constexpr int L = 2 * (NBK - 1), NR = NBK - 2;
+    {
+        auto in = [&](int p, int j) -> C {
+            const T *a = S + 2 * p * NBK + (j < NBK ? j : L - j);
+            return C{a[0], 2 * p + 1 < NR ? a[NBK] : (T)0};
+        };
+        auto out = [&](int p, int k, C z) {
+            T *a = S + 2 * p * NBK + k;
+            a[0] = z.x;
+            if (2 * p + 1 < NR) a[NBK] = z.y;
+        };
+        sym_lines<L, 1>(scr, tw, (NR + 1) / 2, in, out);
+    }
+    __syncthreads();
+    {
+        // z = [0, X, 0, -reverse(X)]: its transform is -i Y_a + Y_b
+        auto in = [&](int p, int j) -> C {
+            if (j == 0 || j == NR + 1) return C{(T)0, (T)0};
+            const bool lo = j <= NR;
+            const T *a = S + 2 * p + (lo ? j - 1 : L - j - 1) * NBK;
+            const T x = a[0], y = 2 * p + 1 < NBK ? a[1] : (T)0;
+            return lo ? C{x, y} : C{-x, -y};
+        };
+        auto out = [&](int p, int k, C z) {
+            if (k < 1 || k > NR) return;
+            T *a = S + 2 * p + (k - 1) * NBK;
+            a[0] = -z.y;
+            if (2 * p + 1 < NBK) a[1] = z.x;
+        };
+        sym_lines<L, -1>(scr, tw, (NBK + 1) / 2, in, out);
+    }
+    __syncthreads();
 }
 
 // 2D DCT-I (REDFT00 x REDFT00) in place on a symmetric NBK x NBK slice S

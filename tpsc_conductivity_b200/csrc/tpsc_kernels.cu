@@ -97,11 +97,11 @@ __global__ void k_gk_table(const double *__restrict__ ek, int n8, double mu0, do
 // -G(r, beta - tau), so one table serves both stages.  Plain layout
 // Grt[j * n8 + o].
 template <int NBK>
-__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
+__global__ void __launch_bounds__(SlicePlan<NBK, true>::threads, SlicePlan<NBK, true>::blocks)
     k_gslice(const double2 *__restrict__ gk, const double2 *__restrict__ tw,
              int n8, int nw0, double T, double *__restrict__ Grt) {
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = plan_twiddles<NBK, true>(S, tw);
     const int j = blockIdx.x;
     const double t = j / (nw0 * T);
     const double bt = 1.0 / T - t;
@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
         return c.y * exp((c.x > 0 ? -t : bt) * c.x);
     });
     __syncthreads();
-    dct2_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+    plan_dct2<NBK, true>(S, tws);
     double *out = Grt + (size_t)j * n8;
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
@@ -123,22 +123,22 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
 // j = 0..Nw0/2 (src/chi0.cpp:393-418, 497-517, 545-558).  tau = 0 uses
 // G(r,0-) = G(r,0+) + delta_r0, tau = beta/2 uses 2 G^2.
 template <int NBK>
-__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
+__global__ void __launch_bounds__(SlicePlan<NBK, true>::threads, SlicePlan<NBK, true>::blocks)
     k_chi0_slice(const double *__restrict__ Grt, const double2 *__restrict__ tw,
                  int n8, int nw0, double *__restrict__ chirt, double *__restrict__ chiq) {
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = plan_twiddles<NBK, true>(S, tw);
     const int j = blockIdx.x;
     const int nb = nw0 / 2 + 1;
     // G(r, tau_j) and G(r, beta - tau_j) staged in the slice / scratch area
-    static_assert(2 * StageRows<NBK>::drow_bytes <= SliceSmem<NBK>::tw_off, "inputs must fit");
+    static_assert(2 * StageRows<NBK>::drow_bytes <= SlicePlan<NBK, true>::tw_off, "inputs must fit");
     double *gp = S;
     double *gm = S + StageRows<NBK>::drow_bytes / sizeof(double);
     stage_drow<NBK>(gp, Grt + (size_t)j * n8);
     stage_drow<NBK>(gm, Grt + (size_t)(nw0 - j) * n8);
     cp_async_wait_all();
     __syncthreads();
-    fill_from_staged<NBK, SlicePlan<NBK>::threads>(S, [&](int o) -> double {
+    fill_from_staged<NBK, SlicePlan<NBK, true>::threads>(S, [&](int o) -> double {
         const double a = gp[o];
         double c;
         if (j == 0)
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
         return c;
     });
     __syncthreads();
-    dct2_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+    plan_dct2<NBK, true>(S, tws);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
         oct_lm(o, l, m);
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
                     double nk02, double *__restrict__ dG0p, double *__restrict__ dtau_chirt0,
                     double *__restrict__ dtau_chiqt0, Bp b) {
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK, SlicePlan<NBK>::wide>(S, tw);
+    const auto *tws = slice_twiddles<NBK, SliceGroups<NBK>::wide>(S, tw);
     ek = at(ek, b.arena);
     er = at(er, b.arena);
     Grt = at(Grt, b.arena);
@@ -226,11 +226,11 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
     k_vertex_q(const double *__restrict__ chiq, const double2 *__restrict__ tw,
                int n8, int nb, double normFact, double U, const double *__restrict__ Usc, double *__restrict__ Vr) {
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = plan_twiddles<NBK>(S, tw);
     const int j = blockIdx.x;
     const double Usp = Usc[0], Uch = Usc[1];
     // chi0(q, iq_j) staged in the slice / scratch area
-    static_assert(StageRows<NBK>::blockrow_bytes <= SliceSmem<NBK>::tw_off, "inputs must fit");
+    static_assert(StageRows<NBK>::blockrow_bytes <= SlicePlan<NBK>::tw_off, "inputs must fit");
     double *cs = S;
     stage_blockrow<NBK>(cs, chiq, j, nb);
     cp_async_wait_all();
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
         return normFact * U * (3.0 * Usp * (sp - c0) + Uch * (ch - c0)) / 8.0;
     });
     __syncthreads();
-    dct2_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+    plan_dct2<NBK>(S, tws);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
         oct_lm(o, l, m);
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
                      const double *__restrict__ dG0p, int n8, int nw0, int n8p, double mu0, double U,
                      const double *__restrict__ Usc, double *__restrict__ dS, Bp b) {
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK, SlicePlan<NBK>::wide>(S, tw);
+    const auto *tws = slice_twiddles<NBK, SliceGroups<NBK>::wide>(S, tw);
     er = at(er, b.arena);
     Grt = at(Grt, b.arena);
     V = at(V, b.arena);
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
     k_sigma_slice(const double *__restrict__ Grt, const double *__restrict__ V,
                   const double2 *__restrict__ tw, int n8, int nw0, int ahead, double *__restrict__ sigt) {
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = plan_twiddles<NBK>(S, tw);
     const int j = blockIdx.x;
     const int nb = nw0 / 2 + 1;
     const int jv = j < nb ? j : nw0 - j;
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
         prefetch_l2_blockrow(V, jn < nb ? jn : nw0 - jn, nb, (n8 + 3) / 4);
     }
     // V(r, tau_j) and G(r, tau_j) staged in the slice / scratch area
-    static_assert(StageRows<NBK>::blockrow_bytes + StageRows<NBK>::drow_bytes <= SliceSmem<NBK>::tw_off,
+    static_assert(StageRows<NBK>::blockrow_bytes + StageRows<NBK>::drow_bytes <= SlicePlan<NBK>::tw_off,
                   "inputs must fit");
     double *vs = S;
     double *gs = S + StageRows<NBK>::blockrow_bytes / sizeof(double);
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
     __syncthreads();
     fill_from_staged<NBK, SlicePlan<NBK>::threads>(S, [&](int o) -> double { return gs[o] * vs[o]; });
     __syncthreads();
-    dct2_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+    plan_dct2<NBK>(S, tws);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
         oct_lm(o, l, m);
@@ -1511,13 +1511,13 @@ __global__ void k_store(StoreVals s, double *__restrict__ dst) {
 template <int NBK>
 struct RunGslice {
     static cudaError_t run(const GridDev *g, double *Grt, double mu0, double T, cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes;
+        const size_t sm = SlicePlan<NBK, true>::bytes;
         cudaError_t e = set_smem(k_gslice<NBK>, sm);
         if (e != cudaSuccess) return e;
         const double nk02 = (double)g->nk0 * g->nk0;
         k_gk_table<<<(g->n8 + 255) / 256, 256, 0, st>>>(g->ek, g->n8, mu0, T, nk02, g->gk, Bp{});
         if ((e = launched()) != cudaSuccess) return e;
-        k_gslice<NBK><<<g->nw0 + 1, SlicePlan<NBK>::threads, sm, st>>>(g->gk, g->tw_k, g->n8, g->nw0, T, Grt);
+        k_gslice<NBK><<<g->nw0 + 1, SlicePlan<NBK, true>::threads, sm, st>>>(g->gk, g->tw_k, g->n8, g->nw0, T, Grt);
         return launched();
     }
 };
@@ -1526,7 +1526,7 @@ struct RunChi0Boundary {
     template <class GT>
     static cudaError_t run(const GridDev *g, const GT *Grt, double mu0, double T, double *dG0p, double *dchirt0,
                            double *dchiqt0, const Bp *b, cudaStream_t st) {
-        const size_t smw = SliceSmem<NBK, SlicePlan<NBK>::wide>::bytes;
+        const size_t smw = SliceSmem<NBK, SliceGroups<NBK>::wide>::bytes;
         cudaError_t e = set_smem(k_chi0_boundary<NBK, GT>, smw);
         if (e != cudaSuccess) return e;
         const double nk02 = (double)g->nk0 * g->nk0;
@@ -1538,10 +1538,10 @@ struct RunChi0Boundary {
 template <int NBK>
 struct RunChi0Slice {
     static cudaError_t run(const GridDev *g, const double *Grt, double *chirt, double *chiq, cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes;
+        const size_t sm = SlicePlan<NBK, true>::bytes;
         cudaError_t e = set_smem(k_chi0_slice<NBK>, sm);
         if (e != cudaSuccess) return e;
-        k_chi0_slice<NBK><<<g->nb, SlicePlan<NBK>::threads, sm, st>>>(Grt, g->tw_k, g->n8, g->nw0, chirt, chiq);
+        k_chi0_slice<NBK><<<g->nb, SlicePlan<NBK, true>::threads, sm, st>>>(Grt, g->tw_k, g->n8, g->nw0, chirt, chiq);
         return launched();
     }
 };
@@ -1549,7 +1549,7 @@ template <int NBK>
 struct RunVertexQ {
     static cudaError_t run(const GridDev *g, const double *chiq, double *Vr, double U, const double *Usc, double T,
                            cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes;
+        const size_t sm = SlicePlan<NBK>::bytes;
         cudaError_t e = set_smem(k_vertex_q<NBK>, sm);
         if (e != cudaSuccess) return e;
         const double normFact = T / ((double)g->nk0 * g->nk0);
@@ -1563,7 +1563,7 @@ struct RunSigmaBoundary {
     static cudaError_t run(const GridDev *g, const GT *Grt, const double *V, const double *dchirt0,
                            const double *dG0p, double mu0, double U, const double *Usc, double *dS, const Bp *b,
                            cudaStream_t st) {
-        const size_t smw = SliceSmem<NBK, SlicePlan<NBK>::wide>::bytes;
+        const size_t smw = SliceSmem<NBK, SliceGroups<NBK>::wide>::bytes;
         cudaError_t e = set_smem(k_sigma_boundary<NBK, GT>, smw);
         if (e != cudaSuccess) return e;
         k_sigma_boundary<NBK, GT><<<dim3(2, 1, b->P), kSliceThreads, smw, st>>>(g->er, g->tw_k, Grt, V, dchirt0, dG0p,
@@ -1575,7 +1575,7 @@ struct RunSigmaBoundary {
 template <int NBK>
 struct RunSigmaSlice {
     static cudaError_t run(const GridDev *g, const double *Grt, const double *V, double *sigt, cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes;
+        const size_t sm = SlicePlan<NBK>::bytes;
         cudaError_t e = set_smem(k_sigma_slice<NBK>, sm);
         if (e != cudaSuccess) return e;
         const int ahead = resident_ctas(k_sigma_slice<NBK>, SlicePlan<NBK>::threads, sm);

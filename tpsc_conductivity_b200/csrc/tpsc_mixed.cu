@@ -18,8 +18,8 @@
 // the near field contributes sum_a w_a cos(pi a k1/(nbk-1)) u_a(k2) at
 // (k1, k2), kNear + 1 FMAs per output point.
 //
-// Each FP32 slice needs ~105 KB of shared memory (the 129 x 129 float slice,
-// 16 groups' float2 FFT scratch and the hi/lo twiddles), so two CTAs run on
+// Each FP32 slice needs ~100 KB of shared memory (the 129 x 129 float slice, its
+// line pairs' float2 FFT scratch and the hi/lo twiddles), so two CTAs run on
 // an SM where the FP64 slice kernels fit one.
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -30,31 +30,34 @@ namespace tpsc {
 
 namespace {
 
-constexpr int kSlice32Threads = 256;
-
-// Threads, FFT groups and CTAs per SM of an FP32 slice kernel (see SlicePlan):
-// 65 lines in 2 rounds of 17 groups at three CTAs per SM (128^2 x 2048, all
-// five slice kernels: 606 us with 256 threads, 527 so, 554 in one round of 33)
+// Threads, shared memory and CTAs per SM of an FP32 slice kernel, and its
+// transform (see SlicePlan): symmetric from 33 lines on, where 129 lines take 2
+// rounds of 33 line pairs in 352 threads (5 rounds of 16 in 256 with the plain
+// FFT).  Plain -> symmetric, one launch: 256^2 x 4096 G 505 -> 432 us, Sigma
+// 521 -> 481, chi0 258 -> 228, V 246 -> 223 (three rounds of 24 pairs: 470, 482,
+// 239, 225); 128^2 x 2048 correlator slices 268 -> 205, G 77 -> 57 (three CTAs
+// of 192 threads 223 and 63).  The transforms' arithmetic is hidden behind their
+// shared-memory exchange; without any transform G takes 229 us, Sigma 294, chi0
+// 119: reading, forming and writing the slices is now the larger part.
 template <int NBK>
 struct Slice32Plan {
-    static constexpr int G = FftPlan<2 * (NBK - 1)>::G;
-    static constexpr int ngrp = NBK >= 129 ? kSlice32Threads / G : NBK == 65 ? 17 : (NBK + 1) / 2;
-    static constexpr int threads = NBK >= 129 ? kSlice32Threads : NBK == 17 ? 64 : (ngrp * G + 31) / 32 * 32;
-    static constexpr int blocks = NBK >= 129 ? 2 : NBK == 65 ? 3 : NBK == 33 ? 5 : 8;
-};
-
-template <int NBK>
-struct Slice32Smem {
     static constexpr int L = 2 * (NBK - 1);
-    static constexpr int NGRP = Slice32Plan<NBK>::ngrp;
+    static constexpr bool sym = NBK >= 33;
+    using F = SymFft<L >= 64 ? L : 64>;
+    static constexpr int G = FftPlan<L>::G, ngrp = (NBK + 1) / 2;
+    static constexpr int warps = NBK >= 129 ? 11 : NBK == 65 ? 6 : 2;
+    static constexpr int threads = sym ? 32 * warps : NBK == 17 ? 64 : (ngrp * G + 31) / 32 * 32;
+    static constexpr int blocks = NBK >= 129 ? 2 : NBK == 65 ? 4 : 8;
     static constexpr size_t slice_bytes = (size_t)NBK * NBK * sizeof(float);
     static constexpr size_t scr_off = (slice_bytes + 15) & ~(size_t)15;
-    // (the float4 twiddles behind an odd number of 17-point scratch areas)
-    static constexpr size_t tw_off = (scr_off + (size_t)NGRP * padded_len(L) * sizeof(float2) + 15) & ~(size_t)15;
-    // the L twiddles, and for L = 256 the second pass's twiddles transposed
-    // behind them (15 x 16, see stockham_pass)
-    static constexpr int NTW = L + (L == 256 ? 15 * 16 : 0);
-    static constexpr size_t bytes = tw_off + (size_t)NTW * sizeof(float4);
+    static constexpr size_t scr_bytes =
+        (sym ? (size_t)warps * F::per_warp * F::len : (size_t)ngrp * padded_len(L)) * sizeof(float2);
+    // the staged inputs (a row of doubles and one of floats) overlap the slice and the scratch
+    static constexpr size_t stage_bytes =
+        StageRows<NBK>::blockrow_bytes + (((size_t)StageRows<NBK>::N8 * sizeof(float) + 15) & ~(size_t)15);
+    static constexpr size_t work_bytes = scr_off + scr_bytes > stage_bytes ? scr_off + scr_bytes : stage_bytes;
+    static constexpr size_t tw_off = (work_bytes + 15) & ~(size_t)15;
+    static constexpr size_t bytes = tw_off + (size_t)(sym ? F::ntw : L) * sizeof(float4);
 };
 
 // Input staging (see stage_blockrow / fill_from_staged): the FP32 slices'
@@ -64,8 +67,8 @@ struct Stage32 {
     static constexpr int N8 = NBK * (NBK + 1) / 2;
     static constexpr size_t blockrow_bytes = StageRows<NBK>::blockrow_bytes;
     static constexpr size_t frow_bytes = ((size_t)N8 * sizeof(float) + 15) & ~(size_t)15;  // one FP32 G row
-    static_assert(blockrow_bytes + frow_bytes <= Slice32Smem<NBK>::tw_off, "inputs must fit before the twiddles");
-    static_assert(2 * frow_bytes <= Slice32Smem<NBK>::tw_off, "inputs must fit before the twiddles");
+    static_assert(blockrow_bytes + frow_bytes <= Slice32Plan<NBK>::tw_off, "inputs must fit before the twiddles");
+    static_assert(2 * frow_bytes <= Slice32Plan<NBK>::tw_off, "inputs must fit before the twiddles");
 };
 
 // n8 floats from src -> dst (4-byte copies: the FP32 G rows are not 16-byte aligned)
@@ -76,20 +79,32 @@ __device__ __forceinline__ void stage_frow(float *dst, const float *__restrict__
 
 template <int NBK>
 __device__ __forceinline__ float2 *scratch32(float *S) {
-    return reinterpret_cast<float2 *>(reinterpret_cast<char *>(S) + Slice32Smem<NBK>::scr_off);
+    return reinterpret_cast<float2 *>(reinterpret_cast<char *>(S) + Slice32Plan<NBK>::scr_off);
 }
 
-// the hi/lo twiddles in shared memory, and for L = 256 entry 256 + (q-1) 16 + k
-// = tw[k q] (q = 1..15, k < 16); the kernel's first barrier publishes them
+// the hi/lo twiddles of the plan's transform in shared memory; the kernel's
+// first barrier publishes them
 template <int NBK>
 __device__ __forceinline__ const float4 *twiddles32(float *S, const float4 *__restrict__ tw) {
-    constexpr int L = Slice32Smem<NBK>::L;
-    float4 *t = reinterpret_cast<float4 *>(reinterpret_cast<char *>(S) + Slice32Smem<NBK>::tw_off);
-    for (int i = threadIdx.x; i < Slice32Smem<NBK>::NTW; i += blockDim.x) {
-        const int m = i < L ? i : (((i - L) & 15) * ((i - L) / 16 + 1)) & (L - 1);
-        t[i] = __ldg(&tw[m]);
-    }
+    using P = Slice32Plan<NBK>;
+    float4 *t = reinterpret_cast<float4 *>(reinterpret_cast<char *>(S) + P::tw_off);
+    for (int i = threadIdx.x; i < (P::sym ? P::F::ntw : P::L); i += blockDim.x)
+        t[i] = __ldg(&tw[P::sym ? (i / P::F::G + 1) * (i % P::F::G) : i]);
     return t;
+}
+template <int NBK>
+__device__ __forceinline__ void dct2_slice32(float *S, const float4 *tws) {
+    if constexpr (Slice32Plan<NBK>::sym)
+        sym_dct2_slice<NBK>(S, scratch32<NBK>(S), tws);
+    else
+        dct2_slice<NBK, Slice32Plan<NBK>::ngrp>(S, scratch32<NBK>(S), tws);
+}
+template <int NBK>
+__device__ __forceinline__ void dst_dct_slice32(float *S, const float4 *tws) {
+    if constexpr (Slice32Plan<NBK>::sym)
+        sym_dst_dct_slice<NBK>(S, scratch32<NBK>(S), tws);
+    else
+        dst_dct_slice<NBK, Slice32Plan<NBK>::ngrp>(S, scratch32<NBK>(S), tws);
 }
 
 // G(r, tau_j) = DCT-I[ G0(k, tau_j) / L^2 ] in FP32 (the FP64 k_gslice's
@@ -112,7 +127,7 @@ __global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::b
         return (float)(c.y * exp((c.x > 0 ? -t : bt) * c.x));
     });
     __syncthreads();
-    dct2_slice<NBK, Slice32Plan<NBK>::ngrp>(S32, scratch32<NBK>(S32), tws);
+    dct2_slice32<NBK>(S32, tws);
     float *out = Grt + (size_t)j * n8;
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
@@ -160,7 +175,7 @@ __global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::b
         return (float)c;
     });
     __syncthreads();
-    dct2_slice<NBK, Slice32Plan<NBK>::ngrp>(S32, scratch32<NBK>(S32), tws);
+    dct2_slice32<NBK>(S32, tws);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
         oct_lm(o, l, m);
@@ -200,7 +215,7 @@ __global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::b
         return (float)(0.125 * normFact * U * c0 * c0 * num / (ds * dc));
     });
     __syncthreads();
-    dct2_slice<NBK, Slice32Plan<NBK>::ngrp>(S32, scratch32<NBK>(S32), tws);
+    dct2_slice32<NBK>(S32, tws);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
         oct_lm(o, l, m);
@@ -220,7 +235,7 @@ template <int NBK>
 struct SigmaSlice32Smem {
     static constexpr int R = kNear < NBK - 1 ? kNear : NBK - 2;
     static constexpr int NOCT = (R + 1) * (R + 2) / 2;
-    static constexpr size_t near_off = (Slice32Smem<NBK>::bytes + 15) & ~(size_t)15;
+    static constexpr size_t near_off = (Slice32Plan<NBK>::bytes + 15) & ~(size_t)15;
     static constexpr size_t u_off = near_off + (size_t)NOCT * sizeof(double);
     static constexpr size_t bytes = u_off + (size_t)(R + 1) * NBK * sizeof(double);
 };
@@ -284,7 +299,7 @@ __global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::b
         u[i] = acc;
     }
     // (the transform's barriers publish u)
-    dct2_slice<NBK, Slice32Plan<NBK>::ngrp>(S32, scratch32<NBK>(S32), tws);
+    dct2_slice32<NBK>(S32, tws);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
         oct_lm(o, l, m);
@@ -315,25 +330,30 @@ __global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::b
     const int nb = nw0 / 2 + 1;
     const double t = j / (nw0 * T);
     const double bt = 1.0 / T - t;
-    for (int c = threadIdx.x; c < K4; c += blockDim.x) {
-        const double2 xa = *reinterpret_cast<const double2 *>(tab + 4 * c);
-        const double b = tab[4 * c + 2];
-        const double E = exp(xa.x > 0 ? -xa.x * t : xa.x * bt);
-        S32[c] = (float)((y == 0) ? xa.y * E : (xa.y * t + b) * E);
-    }
+    batched<4>(
+        K4,
+        [&](int c) -> double3 {
+            const double2 xa = *reinterpret_cast<const double2 *>(tab + 4 * c);
+            return make_double3(xa.x, xa.y, y == 0 ? 0.0 : tab[4 * c + 2]);
+        },
+        [&](int c, double3 v) {
+            const double E = exp(v.x > 0 ? -v.x * t : v.x * bt);
+            S32[c] = (float)((y == 0) ? v.y * E : (v.y * t + v.z) * E);
+        });
     __syncthreads();
-    dst_dct_slice<NBK, Slice32Plan<NBK>::ngrp>(S32, scratch32<NBK>(S32), tws);
+    dst_dct_slice32<NBK>(S32, tws);
     const int jv = j < nb ? j : nw0 - j;
     const bool edge = (j == 0 || j == nw0);
     double *pe = pre + (size_t)(2 * y + (j == nw0 ? 1 : 0)) * K4p;
-    for (int c = threadIdx.x; c < K4; c += blockDim.x) {
-        const int l = c / NBK, m = c % NBK;
-        const double v = S32[c];
-        if (edge) pe[c] = v;
-        S32[c] = (float)(v * (2.0 * V[bidx(jv, oct_index(l + 1, m), nb)]));
-    }
+    batched<8>(
+        K4, [&](int c) -> double { return V[bidx(jv, oct_index(c / NBK + 1, c % NBK), nb)]; },
+        [&](int c, double w) {
+            const double v = S32[c];
+            if (edge) pe[c] = v;
+            S32[c] = (float)(v * (2.0 * w));
+        });
     __syncthreads();
-    dst_dct_slice<NBK, Slice32Plan<NBK>::ngrp>(S32, scratch32<NBK>(S32), tws);
+    dst_dct_slice32<NBK>(S32, tws);
     double *out = (y == 0) ? hV : f0V;
     for (int c = threadIdx.x; c < K4; c += blockDim.x) out[bidx2(j, c, nw0 + 1)] = S32[c];
 }
@@ -341,7 +361,7 @@ __global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::b
 template <int NBK>
 struct RunCondSlice32 {
     static cudaError_t run(const GridDev *g, const CondDev *c, const double *V, double T, int ny, cudaStream_t st) {
-        const size_t sm = Slice32Smem<NBK>::bytes;
+        const size_t sm = Slice32Plan<NBK>::bytes;
         cudaError_t e = set_smem(k_cond_slice32<NBK>, sm);
         if (e != cudaSuccess) return e;
         k_cond_slice32<NBK><<<dim3(g->nw0 + 1, ny), Slice32Plan<NBK>::threads, sm, st>>>(c->tab, V, g->tw_k32, g->nw0, T,
@@ -357,7 +377,7 @@ struct RunGslice32 {
     static cudaError_t run(const GridDev *g, float *Grt, double mu0, double T, const Bp *b, cudaStream_t st) {
         const int plan = slice_plan(kSliceG, NBK);
         if (plan == kSliceDirect && g->dct32) return launch_gslice_dct(*g, Grt, mu0, T, st, *b);
-        const size_t sm = Slice32Smem<NBK>::bytes;
+        const size_t sm = Slice32Plan<NBK>::bytes;
         cudaError_t e = set_smem(k_gslice32<NBK>, sm);
         if (e != cudaSuccess) return e;
         if ((e = launch_gk_table(*g, mu0, T, st, *b)) != cudaSuccess) return e;
@@ -372,7 +392,7 @@ struct RunChi0Slice32 {
                            cudaStream_t st) {
         const int plan = slice_plan(kSliceChi0, NBK);
         if (plan == kSliceDirect && g->dct32) return launch_chi0_slice_dct(*g, Grt, chirt, chiq, st, *b);
-        const size_t sm = Slice32Smem<NBK>::bytes;
+        const size_t sm = Slice32Plan<NBK>::bytes;
         cudaError_t e = set_smem(k_chi0_slice32<NBK>, sm);
         if (e != cudaSuccess) return e;
         const int ahead = b->P > 1 ? 0 : resident_ctas(k_chi0_slice32<NBK>, Slice32Plan<NBK>::threads, sm);
@@ -388,7 +408,7 @@ struct RunVertexQ32 {
         const int plan = slice_plan(kSliceVertex, NBK);
         if (plan == kSliceTensor && g->dct_tc) return launch_vertex_q_tc(*g, chiq, Vr, U, Usc, T, st, *b);
         if (plan == kSliceDirect && g->dct32) return launch_vertex_q_dct(*g, chiq, Vr, U, Usc, T, st, *b);
-        const size_t sm = Slice32Smem<NBK>::bytes;
+        const size_t sm = Slice32Plan<NBK>::bytes;
         cudaError_t e = set_smem(k_vertex_q32<NBK>, sm);
         if (e != cudaSuccess) return e;
         const double normFact = T / ((double)g->nk0 * g->nk0);

@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
     k_gslice_tan(const double2 *__restrict__ gk, const double2 *__restrict__ fd, const double2 *__restrict__ tw,
                  int n8, int nw0, double T, double *__restrict__ dGrt) {
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = plan_twiddles<NBK>(S, tw);
     const int j = blockIdx.x;
     const double t = j / (nw0 * T);
     const double bt = 1.0 / T - t;
@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
         return c.y * exp((c.x > 0 ? -t : bt) * c.x) * (q.x - t) * q.y;
     });
     __syncthreads();
-    dct2_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+    plan_dct2<NBK>(S, tws);
     double *out = dGrt + (size_t)j * n8;
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
     k_chi0_slice_tan(const double *__restrict__ Grt, const double *__restrict__ dGrt,
                      const double2 *__restrict__ tw, int n8, int nw0, double *__restrict__ dchiq) {
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK>(S, tw);
+    const auto *tws = plan_twiddles<NBK>(S, tw);
     const int j = blockIdx.x;
     const int nb = nw0 / 2 + 1;
     const double *gp = Grt + (size_t)j * n8, *dgp = dGrt + (size_t)j * n8;
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
         return 2.0 * (dgm[o] * a + gm[o] * da);
     });
     __syncthreads();
-    dct2_slice<NBK, SlicePlan<NBK>::ngrp>(S, slice_scratch<NBK>(S), tws);
+    plan_dct2<NBK>(S, tws);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
         oct_lm(o, l, m);
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
                         double dmu0, double T, double nk02, double *__restrict__ d_dtau_chiqt0,
                         double *__restrict__ out_ddG0p, double *__restrict__ out_ddchir) {
     extern __shared__ __align__(16) double S[];
-    const auto *tws = slice_twiddles<NBK, SlicePlan<NBK>::wide>(S, tw);
+    const auto *tws = slice_twiddles<NBK, SliceGroups<NBK>::wide>(S, tw);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
         int l, m;
         oct_lm(o, l, m);
@@ -132,7 +132,7 @@ template <int NBK>
 struct RunChi0Tan {
     static cudaError_t run(const GridDev *g, const TangentBufs *t, double mu0, double dmu0, double T,
                            cudaStream_t st) {
-        const size_t sm = SliceSmem<NBK>::bytes, smw = SliceSmem<NBK, SlicePlan<NBK>::wide>::bytes;
+        const size_t sm = SlicePlan<NBK>::bytes, smw = SliceSmem<NBK, SliceGroups<NBK>::wide>::bytes;
         cudaError_t e;
         if ((e = set_smem(k_gslice_tan<NBK>, sm)) != cudaSuccess) return e;
         if ((e = set_smem(k_chi0_slice_tan<NBK>, sm)) != cudaSuccess) return e;
