@@ -643,7 +643,7 @@ int run_chi0(tpsc_ctx *ctx, bool read = true) {
     }
     if ((rc = join_side(ctx, 0))) return rc;
     g->g_mixed = mixed(ctx);
-    CK(launch_chi0_tau(d, g->chiq, g->dchiqt0, g->cinf, g->cinf2, ctx->T, ctx->st));
+    CK(launch_chi0_tau(d, g->chiq, g->dchiqt0, g->cinf, g->cinf2, ctx->T, ctx->st, !mixed(ctx)));
     CK(launch_chi0max(d, g->chiq, ctx->red, ctx->st));
     g->have_chi0 = true;
     g->have_V = g->have_S = g->have_mom = g->have_U = false;
@@ -1591,7 +1591,7 @@ int tpsc_sumrule_tangents(tpsc_ctx *ctx, double out[9]) {
         tb.ddG0p = g->adj.ddG0p[p - 1];
         tb.ddchir = g->adj.ddchir[p - 1];
         CK(launch_chi0_tangent(d, tb, mu0, dmu0, T, ctx->st));
-        CK(launch_chi0_tau(d, dchiq, g->t_ddq0, g->t_dcinf, g->t_dcinf2, T, ctx->st));
+        CK(launch_chi0_tau(d, dchiq, g->t_ddq0, g->t_dcinf, g->t_dcinf2, T, ctx->st, false));
         CK(launch_sumrule_tan(d, g->chiq, dchiq, g->cinf, g->cinf2, g->t_dcinf, g->t_dcinf2, Usp, -1.0, T,
                               ctx->red, ctx->st));
         if ((rc = read_result(ctx, 1, &dRsp[p]))) return rc;
@@ -1994,7 +1994,7 @@ int group_queue(tpsc_ctx *ctx, Group *q, int P, cudaStream_t st, int root_cap) {
     CK(launch_gslice32(d, q->Grt32, 0.0, 0.0, st, b));
     CK(launch_chi0_boundary(d, (const float *)q->Grt32, 0.0, 0.0, q->dG0p, q->dchirt0, q->dchiqt0, st, b));
     CK(launch_chi0_slice32(d, q->Grt32, q->chirt, q->chiq, st, b));
-    CK(launch_chi0_tau(d, q->chiq, q->dchiqt0, q->cinf, q->cinf2, 0.0, st, b));
+    CK(launch_chi0_tau(d, q->chiq, q->dchiqt0, q->cinf, q->cinf2, 0.0, st, false, b));
     CK(launch_chi0max(d, q->chiq, q->red, st, b));
     CK(launch_chi0_moments(d, q->chiq, q->mom, q->cmax, st, b));
     CK(launch_tail_moments(d, q->cinf, q->cinf2, 0.0, q->redm, st, b));
@@ -2335,7 +2335,7 @@ int tpsc_tune_tau_tiles(tpsc_ctx *ctx, int reps, double ms[6]) {
         for (int tile = 0; tile < 2; ++tile) {
             set_tau_tile(kind, d.nw0, tile);
             auto run = [&]() -> cudaError_t {
-                if (kind == kTauChi0) return launch_chi0_tau(d, g->chiq, g->dchiqt0, g->cinf, g->cinf2, ctx->T, ctx->st);
+                if (kind == kTauChi0) return launch_chi0_tau(d, g->chiq, g->dchiqt0, g->cinf, g->cinf2, ctx->T, ctx->st, !mixed(ctx));
                 if (kind == kTauVertex) return launch_vertex_tau(d, g->V, g->chirt, ctx->U, ctx->dres, ctx->st);
                 return launch_sigma_tau(d, g->sigt, g->dS, g->S, g->s2, g->s3, g->s4, g->sinf, ctx->T, ctx->st);
             };
@@ -2383,7 +2383,7 @@ int tpsc_tune_tau_plans(tpsc_ctx *ctx, int reps, double ms[9]) {
             if (plan >= nplans) continue;
             set_tau_tile(kind, d.nw0, plan);
             auto run = [&]() -> cudaError_t {
-                if (kind == kTauChi0) return launch_chi0_tau(d, g->chiq, g->dchiqt0, g->cinf, g->cinf2, ctx->T, ctx->st);
+                if (kind == kTauChi0) return launch_chi0_tau(d, g->chiq, g->dchiqt0, g->cinf, g->cinf2, ctx->T, ctx->st, !mixed(ctx));
                 if (kind == kTauVertex) return launch_vertex_tau(d, g->V, g->chirt, ctx->U, ctx->dres, ctx->st);
                 return launch_sigma_tau(d, g->sigt, g->dS, g->S, g->s2, g->s3, g->s4, g->sinf, ctx->T, ctx->st);
             };
@@ -3106,7 +3106,7 @@ int tpsc_run_kernel(tpsc_ctx *ctx, int which) {
             else
                 CK(launch_chi0_slice(d, g->Grt, g->chirt, g->chiq, ctx->st));
             break;
-        case 2: CK(launch_chi0_tau(d, g->chiq, g->dchiqt0, g->cinf, g->cinf2, ctx->T, ctx->st)); break;
+        case 2: CK(launch_chi0_tau(d, g->chiq, g->dchiqt0, g->cinf, g->cinf2, ctx->T, ctx->st, !mixed(ctx))); break;
         case 3:
             if (g->g_mixed)
                 CK(launch_vertex_q32(d, g->chiq, g->V, ctx->U, ctx->dres, ctx->T, ctx->st));
@@ -3136,7 +3136,7 @@ int tpsc_run_kernel(tpsc_ctx *ctx, int which) {
                 CK(launch_chi0_slice32(d, g->Grt32, g->chirt, g->chiq, ctx->st));
             else
                 CK(launch_chi0_slice(d, g->Grt, g->chirt, g->chiq, ctx->st));
-            CK(launch_chi0_tau(d, g->chiq, g->dchiqt0, g->cinf, g->cinf2, ctx->T, ctx->st));
+            CK(launch_chi0_tau(d, g->chiq, g->dchiqt0, g->cinf, g->cinf2, ctx->T, ctx->st, !mixed(ctx)));
             break;
         case 10: {
             // one Newton-form sum-rule evaluation at Usp: low frequencies, series above

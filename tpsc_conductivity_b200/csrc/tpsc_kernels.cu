@@ -771,6 +771,249 @@ __global__ void __launch_bounds__(256, 2)
 }
 
 // ---------------------------------------------------------------------------
+// tau transforms by groups: a pair of columns is one complex column in a buffer
+// of its own, splined (spline_complex) and transformed in place by one FFT group
+// of G = N/16 threads; a CTA of 128 threads takes 128/G pairs, so that every
+// thread transforms whatever N is, and its barriers are the groups' own.  Pair kernels of 256 threads (k_*_tau2) left all but N/16
+// of them idle in the transform and swept columns of 65 nodes in chunks of one
+// row with 30 warm-up rows.  64 points of the parameter sweep, one launch: chi0 at
+// Nw0 = 256 189 -> 39 us, Sigma 183 -> 39, at 1024 256 -> 115 and 253 -> 132;
+// 128^2 x 2048: chi0 58 -> 45, Sigma 65 -> 55, V 30 -> 26.  At Nw0 = 4096, where
+// the pair kernels' 256 threads all transform, they stay: Sigma 380 us against
+// 399, chi0 306 against 316, V 182 against 189 (half the threads sweep here).
+// ---------------------------------------------------------------------------
+constexpr int kTau3Max = 2048;
+template <int N>
+struct Tau3Plan {
+    static constexpr int G = FftPlan<N>::G;
+    static constexpr int threads = 128;
+    static constexpr int pairs = threads / G;  // of a CTA
+    static constexpr int blocks = 4;           // of an SM
+    static_assert(G <= threads, "one pair needs at most the block");
+    static constexpr int x_len = padded_len(N) + 2;        // N + 1 nodes
+    static constexpr size_t tables_off = (size_t)pairs * x_len * sizeof(double2);
+    static constexpr size_t bytes = tables_off + 2 * sizeof(TwoLevelTw);
+};
+template <int N>
+struct Tau3Group {
+    double2 *X;
+    TwoLevelTw *tw2;  // FFT twiddles, then the half-step ones
+    int grp, t, pair;
+    __device__ explicit Tau3Group(double2 *smem) {
+        using P = Tau3Plan<N>;
+        grp = threadIdx.x / P::G;
+        t = threadIdx.x % P::G;
+        pair = blockIdx.x * P::pairs + grp;
+        X = smem + grp * P::x_len;
+        tw2 = reinterpret_cast<TwoLevelTw *>(reinterpret_cast<char *>(smem) + P::tables_off);
+    }
+    // the pair's two columns (NJ rows) of their four-column block; columns from n8 on as zeros
+    __device__ void load(const double *a, int NJ, int n8) {
+        const double *src = a + (size_t)(pair >> 1) * 4 * NJ + 2 * (pair & 1);
+        for (int j = t; j < NJ; j += Tau3Plan<N>::G) cp_async16(&X[pidx(j)], src + 4 * (size_t)j);
+        cp_async_wait_all();
+        if (2 * pair + 1 >= n8)
+            for (int j = t; j < NJ; j += Tau3Plan<N>::G) {
+                const double2 v = X[pidx(j)];
+                X[pidx(j)] = make_double2(2 * pair < n8 ? v.x : 0.0, 0.0);
+            }
+    }
+    __device__ void sync() { group_sync<Tau3Plan<N>::G>(grp); }
+    // sum of v over the group's threads, in its thread 0; red: one entry per warp of the block
+    __device__ double2 sum(double2 v, double2 *red) {
+        constexpr int G = Tau3Plan<N>::G, W = G < 32 ? G : 32;
+        const unsigned lanes = G < 32 ? ((1u << W) - 1u) << ((threadIdx.x & 31) / W * W) : 0xffffffffu;
+        for (int off = W / 2; off > 0; off >>= 1) {
+            v.x += __shfl_down_sync(lanes, v.x, off, W);
+            v.y += __shfl_down_sync(lanes, v.y, off, W);
+        }
+        if constexpr (G > 32) {
+            if (t % 32 == 0) red[threadIdx.x / 32] = v;
+            sync();
+            if (t == 0)
+                for (int w = 1; w < G / 32; ++w) v = cadd(v, red[threadIdx.x / 32 + w]);
+            sync();
+        }
+        return v;
+    }
+};
+// the two columns of a packed transform at bins n and its partner
+__device__ __forceinline__ void store_pair(double *g, double a, double b) {
+    *reinterpret_cast<double2 *>(g) = make_double2(a, b);
+}
+
+// k_sigma_tau by groups
+template <int N>
+__global__ void __launch_bounds__(Tau3Plan<N>::threads, Tau3Plan<N>::blocks)
+    k_sigma_tau3(const double *__restrict__ sigt, const double *__restrict__ dS, double2 *__restrict__ Sout,
+                 double *__restrict__ s2, double *__restrict__ s3, double *__restrict__ s4, double *__restrict__ sinf,
+                 const double *__restrict__ spl, const double2 *__restrict__ tw, const double2 *__restrict__ ht,
+                 double T, int n8, int n8p, Bp b) {
+    constexpr int NJ = N + 1, NO = N / 2, G = Tau3Plan<N>::G;
+    sigt = at(sigt, b.arena);
+    dS = at(dS, b.arena);
+    Sout = at(Sout, b.arena);
+    s2 = at(s2, b.arena);
+    s3 = at(s3, b.arena);
+    s4 = at(s4, b.arena);
+    sinf = at(sinf, b.arena);
+    T = bpar(b, kPpT, T);
+    extern __shared__ __align__(16) double2 smem3[];
+    Tau3Group<N> q(smem3);
+    tau_tables(q.tw2, q.tw2 + 1, tw, ht, N);
+    __syncthreads();
+    const int o0 = 2 * q.pair;
+    if (o0 >= n8p) return;
+    const TwoLevelTw *ht2 = q.tw2 + 1;
+    double2 *X = q.X;
+    const double2 d0 = make_double2(dS[o0], dS[o0 + 1]), dN = make_double2(dS[n8p + o0], dS[n8p + o0 + 1]);
+    q.load(sigt, NJ, n8);
+    q.sync();
+    if (q.t == 0) {
+        const double2 v0 = X[0], vN = X[pidx(N)];
+        if (o0 == 0) sinf[0] = -(v0.x + vN.x);
+        if (o0 < n8) s2[o0] = d0.x + dN.x;
+        if (o0 + 1 < n8) s2[o0 + 1] = d0.y + dN.y;
+    }
+    q.sync();
+    const double h = 1.0 / (N * T), ih = 1.0 / h;
+    spline_complex<N>(X, NJ, q.t, q.grp, h, d0, dN, spl, spl + NJ);
+    if (q.t == 0) {
+        const double2 m0 = X[0], mN = X[pidx(N)];
+        if (o0 < n8) s3[o0] = -(m0.x + mN.x);
+        if (o0 + 1 < n8) s3[o0 + 1] = -(m0.y + mN.y);
+    }
+    auto in = [&](int j) -> double2 {
+        const double2 u = X[pidx(j)], v = X[pidx(j + 1)];
+        return cmul(tw_at(ht2, j), make_double2((v.x - u.x) * ih, (v.y - u.y) * ih));
+    };
+    group_fft_io<N, +1, false, true>(X, q.t, (const TwoLevelTw *)q.tw2, q.grp, in, ScratchIO{X});
+    q.sync();
+    for (int n = q.t; n < NO; n += G) {
+        double2 Fa, Fb;
+        split_real(X[pidx(n)], X[pidx(N - 1 - n)], Fa, Fb);
+        const double2 e = tw_at(ht2, 2 * n + 1);
+        const double2 f = make_double2(1.0 - e.x, -e.y);
+        const double2 Sa = cmul(f, Fa), Sb = cmul(f, Fb);
+        Sout[bidx(n, o0, NO)] = Sa;
+        Sout[bidx(n, o0 + 1, NO)] = Sb;
+        if (n == NO - 1) {
+            if (o0 < n8) s4[o0] = Sa.x;
+            if (o0 + 1 < n8) s4[o0 + 1] = Sb.x;
+        }
+    }
+}
+
+// k_chi0_tau by groups (the mixed form's: its sums are taken in another order
+// than k_chi0_tau2's, see launch_chi0_tau)
+template <int N>
+__global__ void __launch_bounds__(Tau3Plan<N>::threads, Tau3Plan<N>::blocks)
+    k_chi0_tau3(double *__restrict__ chiq, const double *__restrict__ dtau_chiqt0, double *__restrict__ chi0_inf,
+                double *__restrict__ chi0_inf2, const double *__restrict__ spl, const double2 *__restrict__ tw,
+                double T, int n8, int n8p, Bp b) {
+    constexpr int NO = N / 2, NJ = NO + 1, G = Tau3Plan<N>::G;
+    chiq = at(chiq, b.arena);
+    dtau_chiqt0 = at(dtau_chiqt0, b.arena);
+    chi0_inf = at(chi0_inf, b.arena);
+    chi0_inf2 = at(chi0_inf2, b.arena);
+    T = bpar(b, kPpT, T);
+    extern __shared__ __align__(16) double2 smem3[];
+    __shared__ double2 red[Tau3Plan<N>::threads / 32];
+    Tau3Group<N> q(smem3);
+    tau_tables(q.tw2, q.tw2 + 1, tw, tw, N);
+    __syncthreads();
+    const int o0 = 2 * q.pair;
+    if (o0 >= n8p) return;
+    double2 *X = q.X;
+    const double2 d0 =
+        make_double2(o0 < n8 ? dtau_chiqt0[o0] : 0.0, o0 + 1 < n8 ? dtau_chiqt0[o0 + 1] : 0.0);
+    const double2 zero = make_double2(0.0, 0.0);
+    q.load(chiq, NJ, n8);
+    q.sync();
+    // trapezoid sums of the nodes and of the second derivatives
+    auto trapezoid = [&]() -> double2 {
+        KSum a, c;
+        for (int j = q.t; j < NJ; j += G) {
+            const double2 v = X[pidx(j)];
+            const double w = (j == 0 || j == NO) ? 0.5 : 1.0;
+            a.add(w * v.x);
+            c.add(w * v.y);
+        }
+        return q.sum(make_double2(a.value(), c.value()), red);
+    };
+    const double h = 1.0 / (N * T), ih = 1.0 / h;
+    const double2 sV = trapezoid();
+    q.sync();
+    spline_complex<N>(X, NJ, q.t, q.grp, h, d0, zero, spl, spl + NJ);
+    const double2 sM = trapezoid();
+    q.sync();
+    auto in = [&](int j) -> double2 {
+        const bool lo = j < NO;
+        const int jj = lo ? j : N - 1 - j;
+        const double sg = lo ? ih : -ih;
+        const double2 u = X[pidx(jj)], v = X[pidx(jj + 1)];
+        return make_double2((v.x - u.x) * sg, (v.y - u.y) * sg);
+    };
+    group_fft_io<N, +1, false, true>(X, q.t, (const TwoLevelTw *)q.tw2, q.grp, in, ScratchIO{X});
+    q.sync();
+    double *g = chiq + (size_t)(q.pair >> 1) * 4 * NJ + 2 * (q.pair & 1);
+    for (int n = q.t + 1; n < NJ; n += G) {
+        double2 Fa, Fb;
+        split_real(X[pidx(n)], X[pidx(N - n)], Fa, Fb);
+        const double wn = 2 * n * kPi * T, iw = 1.0 / wn, i2 = iw * iw;
+        const double2 w = tw_at(q.tw2, n);
+        const double cth = w.x, sth = -w.y;
+        const double va = (-2.0 * d0.x + ((1.0 - cth) * Fa.x + sth * Fa.y) * i2) * i2;
+        const double vb = (-2.0 * d0.y + ((1.0 - cth) * Fb.x + sth * Fb.y) * i2) * i2;
+        store_pair(g + 4 * n, o0 == 0 ? 0.0 : va, vb);
+        if (n == NJ - 1) {
+            if (o0 < n8) chi0_inf2[o0] = o0 == 0 ? 0.0 : 2.0 * Fa.x;
+            if (o0 + 1 < n8) chi0_inf2[o0 + 1] = 2.0 * Fb.x;
+        }
+    }
+    if (q.t == 0) {
+        const double h3 = h * h * h / 12.0;
+        store_pair(g, 2.0 * (h * sV.x - h3 * sM.x), 2.0 * (h * sV.y - h3 * sM.y));
+        if (o0 < n8) chi0_inf[o0] = o0 == 0 ? 0.0 : -2.0 * d0.x;
+        if (o0 + 1 < n8) chi0_inf[o0 + 1] = -2.0 * d0.y;
+    }
+}
+
+// k_vertex_tau by groups
+template <int N>
+__global__ void __launch_bounds__(Tau3Plan<N>::threads, Tau3Plan<N>::blocks)
+    k_vertex_tau3(double *__restrict__ Vr, const double *__restrict__ chirt, const double2 *__restrict__ tw, double U,
+                  const double *__restrict__ Usc, int n8, int n8p, Bp b) {
+    constexpr int NJ = N / 2 + 1, G = Tau3Plan<N>::G;
+    Vr = at(Vr, b.arena);
+    chirt = at(chirt, b.arena);
+    Usc = at(Usc, b.arena);
+    U = bpar(b, kPpU, U);
+    const double fact = vertex_fact(U, Usc);
+    extern __shared__ __align__(16) double2 smem3[];
+    Tau3Group<N> q(smem3);
+    tau_tables(q.tw2, q.tw2 + 1, tw, tw, N);
+    __syncthreads();
+    const int o0 = 2 * q.pair;
+    if (o0 >= n8p) return;
+    double2 *X = q.X;
+    q.load(Vr, NJ, n8);
+    q.sync();
+    // even extension of the two columns: a DCT-I each, packed as Re/Im
+    auto in = [&](int j) -> double2 { return X[pidx(j < NJ ? j : N - j)]; };
+    group_fft_io<N, -1, false, true>(X, q.t, (const TwoLevelTw *)q.tw2, q.grp, in, ScratchIO{X});
+    q.sync();
+    const size_t off = (size_t)(q.pair >> 1) * 4 * NJ + 2 * (q.pair & 1);
+    double *g = Vr + off;
+    const double2 *cr = reinterpret_cast<const double2 *>(chirt + off);
+    for (int n = q.t; n < NJ; n += G) {
+        const double2 Z = X[pidx(n)];
+        const double2 c = __ldcs(&cr[2 * n]);
+        store_pair(g + 4 * n, o0 < n8 ? Z.x + fact * c.x : 0.0, o0 + 1 < n8 ? Z.y + fact * c.y : 0.0);
+    }
+}
+
+// ---------------------------------------------------------------------------
 // sum rules and traces
 // ---------------------------------------------------------------------------
 
@@ -1585,12 +1828,25 @@ struct RunSigmaSlice {
 };
 
 template <int N>
+dim3 tau3_grid(const GridDev &g, const Bp &b) {
+    return dim3((g.n8p / 2 + Tau3Plan<N>::pairs - 1) / Tau3Plan<N>::pairs, 1, b.P);
+}
+template <int N>
 struct RunChi0Tau {
     // (a batched launch, b->pp set, always takes the pair-per-CTA kernel)
     static cudaError_t run(const GridDev *g, double *chiq, const double *dchiqt0, double *cinf, double *cinf2,
-                           double T, const Bp *b, cudaStream_t st) {
+                           double T, bool keep, const Bp *b, cudaStream_t st) {
         cudaError_t e;
         const int tile = tau_tile(kTauChi0, N);
+        if constexpr (N <= kTau3Max) {
+            if (!keep && (tile == 0 || (tile == 1 && b->pp))) {
+                const size_t sm = Tau3Plan<N>::bytes;
+                if ((e = set_smem(k_chi0_tau3<N>, sm)) != cudaSuccess) return e;
+                k_chi0_tau3<N><<<tau3_grid<N>(*g, *b), Tau3Plan<N>::threads, sm, st>>>(
+                    chiq, dchiqt0, cinf, cinf2, g->spl_half, g->tw_w, T, g->n8, g->n8p, *b);
+                return launched();
+            }
+        }
         if constexpr (N / 8 <= 256) {
             if (tile == 2) {
                 const size_t sm = Tau2Smem<N>::bytes;
@@ -1632,13 +1888,19 @@ struct RunVertexTau {
                 return launched();
             }
         }
-        if constexpr (N / 16 <= 256) {
+        if constexpr (N <= kTau3Max) {
             if (tile != 1 || b->pp) {
-                const size_t sm = Tau2Smem<N>::bytes;
-                if ((e = set_smem(k_vertex_tau2<N>, sm)) != cudaSuccess) return e;
-                k_vertex_tau2<N><<<dim3(g->n8p / 2, 1, b->P), 256, sm, st>>>(Vr, chirt, g->tw_w, U, Usc, g->n8, *b);
+                const size_t sm = Tau3Plan<N>::bytes;
+                if ((e = set_smem(k_vertex_tau3<N>, sm)) != cudaSuccess) return e;
+                k_vertex_tau3<N><<<tau3_grid<N>(*g, *b), Tau3Plan<N>::threads, sm, st>>>(Vr, chirt, g->tw_w, U, Usc, g->n8,
+                                                                                          g->n8p, *b);
                 return launched();
             }
+        } else if (tile != 1 || b->pp) {
+            const size_t sm = Tau2Smem<N>::bytes;
+            if ((e = set_smem(k_vertex_tau2<N>, sm)) != cudaSuccess) return e;
+            k_vertex_tau2<N><<<dim3(g->n8p / 2, 1, b->P), 256, sm, st>>>(Vr, chirt, g->tw_w, U, Usc, g->n8, *b);
+            return launched();
         }
         const size_t sm = TauSmem<N>::bytes(N / 2 + 1);
         e = set_smem(k_vertex_tau<N>, sm);
@@ -1662,15 +1924,19 @@ struct RunSigmaTau {
                 return launched();
             }
         }
-        if constexpr (N / 16 <= 256) {
+        if constexpr (N <= kTau3Max) {
             if (tile != 1 || b->pp) {
-                // one pair per CTA, two CTAs per SM
-                const size_t sm = Tau2Smem<N>::bytes;
-                if ((e = set_smem(k_sigma_tau2<N>, sm)) != cudaSuccess) return e;
-                k_sigma_tau2<N><<<dim3(g->n8p / 2, 1, b->P), 256, sm, st>>>(sigt, dS, S, s2, s3, s4, sinf, g->spl_full,
-                                                                           g->tw_w, g->ht_w, T, g->n8, g->n8p, *b);
+                const size_t sm = Tau3Plan<N>::bytes;
+                if ((e = set_smem(k_sigma_tau3<N>, sm)) != cudaSuccess) return e;
+                k_sigma_tau3<N><<<tau3_grid<N>(*g, *b), Tau3Plan<N>::threads, sm, st>>>(
+                    sigt, dS, S, s2, s3, s4, sinf, g->spl_full, g->tw_w, g->ht_w, T, g->n8, g->n8p, *b);
                 return launched();
             }
+        } else if (tile != 1 || b->pp) {
+            const size_t sm = Tau2Smem<N>::bytes;
+            if ((e = set_smem(k_sigma_tau2<N>, sm)) != cudaSuccess) return e;
+            k_sigma_tau2<N><<<dim3(g->n8p / 2, 1, b->P), 256, sm, st>>>(sigt, dS, S, s2, s3, s4, sinf, g->spl_full, g->tw_w, g->ht_w, T, g->n8, g->n8p, *b);
+            return launched();
         }
         const size_t sm = TauSmem<N>::bytes(N + 1);
         if ((e = set_smem(k_sigma_tau<N>, sm)) != cudaSuccess) return e;
@@ -1734,8 +2000,8 @@ cudaError_t launch_chi0_slice(const GridDev &g, const double *Grt, double *chirt
 }
 
 cudaError_t launch_chi0_tau(const GridDev &g, double *chiq, const double *dtau_chiqt0, double *chi0_inf,
-                            double *chi0_inf2, double T, cudaStream_t st, const Bp &b) {
-    return dispatch_nw<RunChi0Tau>(g.nw0, &g, chiq, dtau_chiqt0, chi0_inf, chi0_inf2, T, &b, st);
+                            double *chi0_inf2, double T, cudaStream_t st, bool keep, const Bp &b) {
+    return dispatch_nw<RunChi0Tau>(g.nw0, &g, chiq, dtau_chiqt0, chi0_inf, chi0_inf2, T, keep, &b, st);
 }
 
 cudaError_t launch_sumrule(const GridDev &g, const double *chiq, const double *chi0_inf, const double *chi0_inf2,

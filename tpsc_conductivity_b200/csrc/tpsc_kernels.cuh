@@ -47,7 +47,7 @@ constexpr int kSplinePivotConst = 32;
 
 constexpr int kMaxBlocks = 4096;
 constexpr int kTailP = 41;  // P_p for p < kTailP: the find_mu tail series uses p <= kMuMomP + 28
-constexpr int kTailQ = 20;  // Q_k for k < kTailQ (the series uses k <= 18)  // >= column blocks of the largest grid (2097)
+constexpr int kTailQ = 28;  // Q_k for k < kTailQ (the moments use k <= 2 kMomP + 2, the tail series k <= 18)
 struct Reduce {
     double *partial = nullptr;   // [4 * kMaxBlocks]
     double *result = nullptr;    // [8]
@@ -97,8 +97,11 @@ cudaError_t launch_chi0_slice32(const GridDev &g, const float *Grt, double *chir
 cudaError_t launch_vertex_q32(const GridDev &g, const double *chiq, double *Vr, double U, const double *Usc, double T,
                               cudaStream_t st, const Bp &b = Bp{});
 cudaError_t launch_chi0_slice(const GridDev &g, const double *Grt, double *chirt, double *chiq, cudaStream_t st);
+// keep: the pair-per-CTA kernel's order of sums, to the last bit (the FP64 forms:
+// their diagnostics difRel are differences of roots that agree to ~1e-9, and
+// resolve the last bits of chi0); else the grouped kernel
 cudaError_t launch_chi0_tau(const GridDev &g, double *chiq, const double *dtau_chiqt0, double *chi0_inf,
-                            double *chi0_inf2, double T, cudaStream_t st, const Bp &b = Bp{});
+                            double *chi0_inf2, double T, cudaStream_t st, bool keep = true, const Bp &b = Bp{});
 
 // mu0 by safeguarded Newton in one block -> r.result[0] (iterations in r.result[1])
 cudaError_t launch_mu0_newton(const GridDev &g, double n, double T, Reduce r, cudaStream_t st, const Bp &b = Bp{});
@@ -115,8 +118,10 @@ cudaError_t launch_sumrule(const GridDev &g, const double *chiq, const double *c
 cudaError_t launch_tail_moments(const GridDev &g, const double *chi0_inf, const double *chi0_inf2, double T,
                                 Reduce r, cudaStream_t st, const Bp &b = Bp{});
 // per-frequency moments sum_q w f chi^(k+2), k < kMomP -> mom [nb][kMomP]; max_q |chi| -> cmax [nb]
-constexpr int kMomP = 8;
-constexpr double kMomSeriesMax = 0.004;  // |h chi| bound of the series terms: 0.004^8 < 1e-19
+// Twelve moments against eight with |h chi| < 0.004 move the series' first
+// frequency down by sqrt(0.026 / 0.004) = 2.5: an evaluation sums that much less
+constexpr int kMomP = 12;
+constexpr double kMomSeriesMax = 0.026;  // |h chi| bound of the series terms: 0.026^12 < 1e-19
 constexpr double kMomMuRange = 0.35;     // |mu - mu0| the find_mu series is built to cover
 constexpr int kMuMomP = 12;              // terms of the find_mu series
 constexpr double kMuSeriesMax = 0.03;    // |mu - mu0| / |z| bound of its terms: 0.03^12 < 1e-18
