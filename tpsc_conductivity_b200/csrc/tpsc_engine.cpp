@@ -1637,41 +1637,11 @@ int tpsc_sumrule_vjp(tpsc_ctx *ctx, const double cot[3], double grad[3]) {
 // spin correlation length: host post-processing of chi0(q, 0) and Usp
 // ---------------------------------------------------------------------------
 
-// green0::find_FS(nk) (src/green0.cpp:626-676): on each line kx - ky = kx0,
-// kx0 = j pi/(nk - 1), the root kx in [kx0, pi] of eps(kx, kx - kx0) - mu0 by
-// the bounded find_zero from {(kx0 + pi)/2, kx0, pi}; the first line without
-// a root ends the search and the later points stay (-1, -1).
-void find_fs(const tpsc_ctx *ctx, double mu0, int nk, std::vector<double> &fs) {
-    fs.assign(2 * (size_t)nk, -1.0);
-    for (int j = 0; j < nk; ++j) {
-        const double kx0 = j * PI / (nk - 1);
-        const double init[3] = {0.5 * (kx0 + PI), kx0, PI}, lims[2] = {kx0, PI};
-        auto f = [&](double kx, double &y) -> bool {
-            y = dispk(kx, kx - kx0, ctx->tp, ctx->tpp, ctx->t3) - mu0;
-            return true;
-        };
-        double root = 0.0;
-        int nev;
-        bool derr;
-        if (!find_zero(f, init, &root, lims, &nev, &derr)) break;
-        fs[2 * (size_t)j] = root;
-        fs[2 * (size_t)j + 1] = root - kx0;
-    }
-}
-
-// chi::vF_hot_spots (src/chi.cpp:420-447): the first pair of consecutive
-// Fermi-surface points across kx + ky = pi (or the last pair), |grad eps| at
-// their midpoint (hamiltonien::grad_ek, src/hamiltonien.cpp:125-131).
-double vf_hot_spots(const tpsc_ctx *ctx, const std::vector<double> &fs, int nk) {
-    double kx1 = fs[0], ky1 = fs[1], kx2 = fs[2], ky2 = fs[3];
-    int j = 1;
-    while ((kx1 + ky1 - PI) * (kx2 + ky2 - PI) > 0 && j < nk - 1) {
-        ++j;
-        kx1 = kx2;
-        ky1 = ky2;
-        kx2 = fs[2 * (size_t)j];
-        ky2 = fs[2 * (size_t)j + 1];
-    }
+// |grad eps| (hamiltonien::grad_ek, src/hamiltonien.cpp:125-131) at the midpoint of
+// the two Fermi-surface points of the hot spot (chi::vF_hot_spots,
+// src/chi.cpp:420-447), p = (kx, ky) of both
+double vf_hot_spots(const tpsc_ctx *ctx, const double p[4]) {
+    const double kx1 = p[0], ky1 = p[1], kx2 = p[2], ky2 = p[3];
     const double kx = (kx1 + kx2) / 2, ky = (ky1 + ky2) / 2;
     const double tp = ctx->tp, tpp = ctx->tpp, t3 = ctx->t3;
     const double gx = 2.0 * std::sin(kx) + 4.0 * tp * std::sin(kx) * std::cos(ky) + 4.0 * tpp * std::sin(2 * kx) +
@@ -1697,15 +1667,18 @@ int tpsc_sp_corr_length_fs(tpsc_ctx *ctx, double mu_fs, double out[7]) {
     cudaSetDevice(ctx->device);
     const GridDev &d = g->d;
     const int nbq = d.nbk;
+    // the hot spot on find_FS's 10001 lines, searched on the device beside the copy of chi0
+    const int nkfs = 10001;
+    if ((rc = ensure_stage(ctx, (nkfs + 4) * sizeof(double)))) return rc;
+    double *fs = static_cast<double *>(ctx->stage);
+    CK(launch_hot_pair(nkfs, mu_fs, ctx->tp, ctx->tpp, ctx->t3, fs + 4, fs, ctx->st));
+    if ((rc = queue_read_back(ctx, {{fs, 4 * sizeof(double), 0}}))) return rc;
     // chi0(q, 0): row j = 0 of the column-block layout, 4 columns per block
     std::vector<double> a((size_t)d.n8p);
     CK(cudaMemcpy2DAsync(a.data(), 4 * sizeof(double), g->chiq, (size_t)d.nb * 4 * sizeof(double),
                          4 * sizeof(double), d.n8p / 4, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
-    const int nkfs = 10001;
-    std::vector<double> fs;
-    find_fs(ctx, mu_fs, nkfs, fs);
-    const double vF = vf_hot_spots(ctx, fs, nkfs);
+    const double vF = vf_hot_spots(ctx, ctx->h_res);
     // chi::sp_corr_length (src/chi.cpp:450-718): half maximum of
     // chi_sp(q, 0) = chi0/(1 - Usp chi0/2) around qmax along y and x, and the
     // asymptotic (Ornstein-Zernike) lengths from the second difference of chi0

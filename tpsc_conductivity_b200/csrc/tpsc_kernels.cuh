@@ -204,6 +204,10 @@ struct RootScratch {
 // (root, success); Usp, Uch -> rs.out as launch_sumrule_roots leaves them; mu
 // and Tr Sigma G at mu -> rs.out as launch_mu_roots leaves them
 cudaError_t launch_mu0_zero(const GridDev &g, double n, double T, Reduce r, cudaStream_t st);
+// the two Fermi-surface points (kx, ky) around the hot spot on nk lines ->
+// out [4]; scratch [nk]
+cudaError_t launch_hot_pair(int nk, double mu, double tp, double tpp, double t3, double *scratch, double *out,
+                            cudaStream_t st);
 cudaError_t launch_sumrule_zero(const GridDev &g, const double *chiq, const double *chi0_inf, const double *chi0_inf2,
                                 double T, double n, double nsr, double U, double hi_sp, RootScratch rs,
                                 cudaStream_t st, const double *chi0max = nullptr, double hi_off = 0.0);

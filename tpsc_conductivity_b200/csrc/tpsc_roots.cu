@@ -1110,6 +1110,69 @@ __global__ void __launch_bounds__(kMu0Threads)
     }
 }
 
+// ---------------------------------------------------------------------------
+// the non-interacting Fermi surface's hot spot (green0::find_FS(nk),
+// src/green0.cpp:626-676; chi::vF_hot_spots, src/chi.cpp:420-447)
+// ---------------------------------------------------------------------------
+// eps_k of hamiltonien::dispk (src/hamiltonien.cpp:428-431), rounded as the host rounds it
+__device__ double dispk_dev(double kx, double ky, double tp, double tpp, double t3) {
+    const Rn cx(cos(kx)), cy(cos(ky));
+    Rn e = Rn(-2.0) * (cx + cy) - Rn(4.0) * Rn(tp) * cx * cy;
+    if (tpp != 0.0 || t3 != 0.0) {
+        const Rn c2x(cos(2 * kx)), c2y(cos(2 * ky));
+        e = e - Rn(2.0) * Rn(tpp) * (c2x + c2y) - Rn(4.0) * Rn(t3) * (c2x * cy + c2y * cx);
+    }
+    return e.v;
+}
+// On line j, kx - ky = kx0 = j pi/(nk - 1): the root kx in [kx0, pi] of
+// eps(kx, kx - kx0) - mu by the bounded find_zero from {(kx0 + pi)/2, kx0, pi} ->
+// kx[j], or NaN where there is none.  10001 lines of ~10 evaluations, bound by a host
+// thread's latency, took 5 to 10 ms; one thread each, 15 us, and the pair's search
+// below 9 us (a scan of 15 temperatures on a 64 x 64 grid: 17.5 -> 4.1 ms).
+__global__ void __launch_bounds__(128) k_fermi_lines(int nk, double mu, double tp, double tpp, double t3,
+                                                     double *__restrict__ kx) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= nk) return;
+    const double kx0 = j * kPi / (nk - 1);
+    const double init[3] = {0.5 * (kx0 + kPi), kx0, kPi}, lims[2] = {kx0, kPi};
+    auto f = [&](double k, double &y) -> bool {
+        y = dispk_dev(k, k - kx0, tp, tpp, t3) - mu;
+        return true;
+    };
+    double root = 0.0;
+    int nev;
+    bool gone;
+    const bool ok = find_zero(f, init, &root, lims, &nev, &gone);
+    kx[j] = ok ? root : nan("");
+}
+// The first pair of consecutive points across kx + ky = pi (or the last pair) ->
+// out = (kx, ky) of both; from the first line without a root on every point is
+// (-1, -1).  One block.
+__global__ void __launch_bounds__(1024) k_hot_pair(const double *__restrict__ kx, int nk, double *__restrict__ out) {
+    __shared__ int s_end, s_hit;
+    if (threadIdx.x == 0) {
+        s_end = nk;
+        s_hit = nk - 1;
+    }
+    __syncthreads();
+    for (int j = threadIdx.x; j < nk; j += blockDim.x)
+        if (isnan(kx[j])) atomicMin(&s_end, j);
+    __syncthreads();
+    const int end = s_end;
+    auto point = [&](int j, double &x, double &y) {
+        x = j < end ? kx[j] : -1.0;
+        y = j < end ? x - j * kPi / (nk - 1) : -1.0;
+    };
+    for (int j = threadIdx.x + 1; j < nk - 1; j += blockDim.x) {
+        double x1, y1, x2, y2;
+        point(j - 1, x1, y1);
+        point(j, x2, y2);
+        if (!((x1 + y1 - kPi) * (x2 + y2 - kPi) > 0)) atomicMin(&s_hit, j);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) point(s_hit - 1 + threadIdx.x, out[2 * threadIdx.x], out[2 * threadIdx.x + 1]);
+}
+
 // The barrier's bound, exercised: block `withhold` never arrives (negative:
 // every block does), so every other block's wait runs out after
 // kBarrierNs and leaves with the error flag set.  words[0..1] the barrier,
@@ -1161,6 +1224,15 @@ static cudaError_t zero_grid(K kernel, int nblk, int *grid, int cap) {
     const int rounds = (nblk + *grid - 1) / *grid;
     *grid = (nblk + rounds - 1) / rounds;
     return nblk <= kRootVals * kRootMaxBlocks ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+cudaError_t launch_hot_pair(int nk, double mu, double tp, double tpp, double t3, double *scratch, double *out,
+                            cudaStream_t st) {
+    k_fermi_lines<<<(nk + 127) / 128, 128, 0, st>>>(nk, mu, tp, tpp, t3, scratch);
+    cudaError_t e = launched();
+    if (e != cudaSuccess) return e;
+    k_hot_pair<<<1, 1024, 0, st>>>(scratch, nk, out);
+    return launched();
 }
 
 cudaError_t launch_mu0_zero(const GridDev &g, double n, double T, Reduce r, cudaStream_t st) {
