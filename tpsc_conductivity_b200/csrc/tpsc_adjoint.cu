@@ -44,13 +44,6 @@ __device__ __forceinline__ double fermi_fn(double r, double T) {
     }
     return 1.0 / (exp(r / T) + 1.0);
 }
-// e^{-tau r} (1 - f(r)) and e^{r tau} f(r) without overflow
-__device__ __forceinline__ double tail_g(double r, double tau, double beta) {
-    return r > 0 ? exp(-tau * r) / (1.0 + exp(-beta * r)) : exp((beta - tau) * r) / (exp(beta * r) + 1.0);
-}
-__device__ __forceinline__ double tail_j(double r, double tau, double beta) {
-    return r > 0 ? exp(r * (tau - beta)) / (exp(-beta * r) + 1.0) : exp(r * tau) / (exp(beta * r) + 1.0);
-}
 // the two real roots of z^2 + B z - sinf (sinf > 0), smaller first
 __device__ __forceinline__ void real_roots(double B, double sinf, double &r1, double &r2) {
     const double disc = sqrt(B * B + 4.0 * sinf);
@@ -84,430 +77,481 @@ __device__ __forceinline__ void tp_dirs(int l1, int m, int nbk, double &de, doub
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// the per-k tau kernel of chi_jj, backward: one K4 column per CTA iteration
+// the per-k tau kernel of chi_jj, backward: one pair of K4 columns per CTA
+// iteration
 // ---------------------------------------------------------------------------
+// One FFT group (N/16 threads, a warp at least) and one complex buffer of N + 1
+// nodes per CTA, and as many CTAs per SM as leave 128 registers a thread
 template <int N>
-struct CondBwdSmem {
-    static constexpr int NJ = N + 1;
-    static constexpr size_t x_bytes = (size_t)padded_len(N) * sizeof(double2);
-    static constexpr size_t r_bytes = ((size_t)NJ * sizeof(double) + 15) & ~(size_t)15;
-    static constexpr size_t gt_off = x_bytes;
-    static constexpr size_t jt_off = gt_off + r_bytes;
-    static constexpr size_t r_off = jt_off + r_bytes;
-    static constexpr size_t q_off = r_off + r_bytes;
-    static constexpr size_t tw_off = q_off + r_bytes;
-    static constexpr size_t bytes = tw_off + 2 * sizeof(TwoLevelTw);
-    static_assert(bytes <= 232448, "cond backward column does not fit");
-    static_assert(x_bytes >= (size_t)(2 * N + 2) * sizeof(double), "X must hold the two spline adjoints");
+struct CondBwdPlan {
+    static constexpr int G = FftPlan<N>::G;
+    static constexpr int threads = G < 32 ? 32 : G;
+    static constexpr int blocks = 512 / threads > 12 ? 12 : 512 / threads;
+    static constexpr int x_len = padded_len(N) + 2;        // N + 1 nodes
+    static constexpr int n_hi = N / 64 + 1, n_lo = 64;     // two-level tails: tau_j, j = 64 hi + lo <= N
+    static constexpr size_t tables_off = (size_t)x_len * sizeof(double2);
+    static constexpr size_t tails_off = tables_off + 2 * sizeof(TwoLevelTw);
+    static constexpr size_t bytes = tails_off + (size_t)4 * (n_hi + n_lo) * sizeof(double);
+    static_assert(bytes + 1024 <= 233472 / blocks, "the CTAs of an SM share its memory");
 };
 
 struct CondBwdCol {
     int o, l, m;
     double e, dk, d2, wt;
     double C1, C2, C3;
-    double k0s, dGs, dJs;
-    double r[2], f[2], a[2], b[2];
+    double r[2], f[2], omf[2], u[2], a[2], b[2];  // u: the tails' 1 / (1 + exp(-|r| beta)), omf = 1 - f
     double k0, dGp, dGm, dJb, dJ0;
-    double Gt0, Jt0, Jraw0, Jbeta, dchi, CJ1b, CJ3b;
+    double Gt0, Jt0, Jbeta, dchi, CJ1b, CJ3b;
     // adjoints
     double dkb, dchib, CJ1bb, CJ3bb, d0b2, dNb2;
-    double Gt0bs, Jt0bs, dGpb, dGmb, dJ0b, dJbb, Jbetab;
-    double k0sb, dGsb, dJsb, C1bs, mub, eb, sinfb;
+    double dGpb, dGmb, dJ0b, dJbb, Jbetab;
+    double k0sb, dGsb, dJsb, mub, eb, sinfb;
+    double C1b, C2b, C3b;
 };
 
-// threads of the backward tau kernel: one FFT group (N/16) from N = 2048 on,
-// so that every thread works in the FFTs and two CTAs share an SM up to 2048
+// Persistent over column pairs.  h V of the pair and, at the end, its cotangent are
+// the parts of one complex column: one spline and one FFT each for two columns.
+// In between the columns come one after the other; everything of a column is one
+// complex column in place in X: G and J, then (G J, G G) with the bubble extended
+// evenly about beta/2 (its half spline is the full one with slopes d, -d), then the
+// cotangents of both.  What has to outlive X (G, J in frequency and tau, the first
+// column's cotangent) goes through the block's workspace, which stays in L2; node j
+// and N - j, or bin n and N - 1 - n, belong to one thread throughout.
+// Bound: the FP64 pipe and the sweeps' and transforms' latencies at 16 warps per SM.
+// One column per CTA, real splines and separate G, J, G J, G G buffers (100 KB, 8
+// warps per SM), six transforms and eight exponentials a point took 1596 us at
+// 128^2 x 2048; five transforms a column and tails from tables of exp(-|r| tau)
+// take 869 (4096: 3263 -> 1524).
 template <int N>
-constexpr int cond_bwd_threads() {
-    return N >= 4096 ? 256 : 128;
-}
-
-template <int N>
-__global__ void __launch_bounds__(cond_bwd_threads<N>(), N >= 4096 ? 1 : 2) k_cond_tau_bwd(const CondBwdArgs a) {
-    constexpr int NJ = N + 1, NO = N / 2, NJ2 = NO + 1;
-    constexpr int G = FftPlan<N>::G;
-    using SM = CondBwdSmem<N>;
-    extern __shared__ __align__(16) double smem[];
-    char *base = reinterpret_cast<char *>(smem);
-    double2 *X = reinterpret_cast<double2 *>(smem);
-    double *Xd = smem;
-    double *Gt = reinterpret_cast<double *>(base + SM::gt_off);
-    double *Jt = reinterpret_cast<double *>(base + SM::jt_off);
-    double *R = reinterpret_cast<double *>(base + SM::r_off);
-    double *Q = reinterpret_cast<double *>(base + SM::q_off);
-    TwoLevelTw *tw2 = reinterpret_cast<TwoLevelTw *>(base + SM::tw_off);
+__global__ void __launch_bounds__(CondBwdPlan<N>::threads, CondBwdPlan<N>::blocks) k_cond_tau_bwd(const CondBwdArgs a) {
+    using P = CondBwdPlan<N>;
+    constexpr int NJ = N + 1, NO = N / 2, G = P::G, NT = P::threads;
+    extern __shared__ __align__(16) double2 X[];
+    TwoLevelTw *tw2 = reinterpret_cast<TwoLevelTw *>(reinterpret_cast<char *>(X) + P::tables_off);
     const TwoLevelTw *ht2 = tw2 + 1;
-    tau_tables(tw2, tw2 + 1, a.tw, a.ht, N);
-    __shared__ CondBwdCol cs;
-    __shared__ double sums[8], d0s[1], dNs[1], e0s[1], eNs[1];
-    const int tid = threadIdx.x, NT = blockDim.x;
+    double *tails_hi = reinterpret_cast<double *>(reinterpret_cast<char *>(X) + P::tails_off);
+    double *tails_lo = tails_hi + 4 * P::n_hi;
+    tau_tables(tw2, tw2 + 1, a.tw, a.ht, N);  // published by the first barrier of the pair loop
+    __shared__ CondBwdCol col[2];
+    __shared__ double sums[8];
+    __shared__ double2 sd0, sdN;
+    const int tid = threadIdx.x;
     const double T = a.T, h = 1.0 / (N * T), ih = 1.0 / h, beta = 1.0 / T, pT = kPi * T;
     const double a6 = 6.0 / (h * h), b6 = 6.0 / h;
     const double sinf = a.sinf[0], mu = a.mu, nf = a.nf;
-    double2 *wsG = a.ws + (size_t)blockIdx.x * 2 * NO, *wsJ = wsG + NO;
+    // per block: G, J of the two columns (i k_n), and (G, J)(tau) or its cotangent
+    double2 *const wsG = a.ws + (size_t)blockIdx.x * kCondBwdWs * NO, *const wsJ = wsG + NO, *const wsT = wsJ + 2 * NO;
     double acc_mu = 0.0, acc_sinf = 0.0, acc_tp = 0.0;  // thread 0
+    const int npairs = (a.K4 + 1) / 2;
 
 #pragma unroll 1
-    for (int c = blockIdx.x; c < a.K4; c += gridDim.x) {
-        // ---- column constants and the h V column
-        if (tid == 0) {
-            cs.l = c / a.nbk;
-            cs.m = c % a.nbk;
-            cs.o = oct_index(cs.l + 1, cs.m);
-            cs.e = a.ek[cs.o];
-            cs.dk = a.dek[c];
-            cs.d2 = a.d2ek[c];
-            cs.wt = (cs.m == 0 || cs.m == a.nbk - 1) ? 2.0 : 4.0;
-            d0s[0] = a.dbound[c];
-            dNs[0] = a.dbound[(size_t)a.K4p + c];
-        }
-        for (int j = tid; j < NJ; j += NT) R[j] = a.hV[bidx2(j, c, NJ)];
-        __syncthreads();
-        if (tid == 0) {
-            cs.C1 = -R[0] - R[N];
-            cs.C2 = d0s[0] + dNs[0];
-        }
-        spline_second_derivatives<1>(R, NJ, NJ, h, d0s, dNs, a.spl_full, a.spl_full + NJ);
-        if (tid == 0) cs.C3 = -(R[0] + R[N]);
-        if (tid < G) {
-            auto in = [&](int j) -> double2 { return cscale(tw_at(ht2, j), (R[j + 1] - R[j]) * ih); };
-            group_fft_io<N, +1>(X, tid, (const TwoLevelTw *)tw2, 0, in, ScratchIO{X});
-        }
-        __syncthreads();
-        // ---- J(i k_n), G(i k_n), the tail-subtracted G and G J; packed for the tau transform
-        {
-            double acc[3] = {0.0, 0.0, 0.0};
-            const double e = cs.e, C1 = cs.C1, C2 = cs.C2, C3 = cs.C3;
-            const double s2 = a.s2[cs.o], s3 = a.s3[cs.o];
-            for (int n = tid; n < NO; n += NT) {
-                const double kn = (2 * n + 1) * pT, ik = 1.0 / kn, ik2 = ik * ik;
-                const double2 ee = tw_at(ht2, 2 * n + 1);
-                const double2 f = make_double2(1.0 - ee.x, -ee.y);
-                const double2 fF = cmul(f, X[pidx(n)]);
-                const double2 J =
-                    make_double2(-C2 * ik2 + fF.x * ik2 * ik2, -C1 * ik + C3 * ik2 * ik + fF.y * ik2 * ik2);
-                double rS, iS;
-                sigma_full(ik, sinf, s2, s3, a.S[bidx(n, cs.o, NO)], rS, iS);
-                const double2 Gv = cdiv(make_double2(T, 0.0), make_double2(mu - e - rS, kn - iS));
-                const double2 Gl = cdiv(make_double2(T, 0.0), make_double2(mu - e, kn + sinf * ik));
-                const double2 Gs = csub(Gv, Gl);
-                const double2 Js = csub(cmul(Gv, J), cmul(Gl, make_double2(0.0, -C1 * ik)));
-                wsG[n] = Gv;
-                wsJ[n] = J;
-                // Gs + i conj(Js) at n, conj(Gs) + i Js at N - 1 - n
-                X[pidx(n)] = make_double2(Gs.x + Js.y, Gs.y + Js.x);
-                X[pidx(N - 1 - n)] = make_double2(Gs.x - Js.y, -Gs.y + Js.x);
-                acc[0] += Gs.x;
-                acc[1] += kn * Gs.y;
-                acc[2] -= kn * Js.y;
-            }
-            block_sum<3>(acc, sums);
-        }
-        if (tid == 0) {
-            cs.k0s = 2.0 * sums[0];
-            cs.dGs = 2.0 * sums[1];
-            cs.dJs = 2.0 * sums[2];
-            real_roots(mu - cs.e, sinf, cs.r[0], cs.r[1]);
-            const double d = cs.r[0] - cs.r[1];
-            cs.a[0] = cs.r[0] / d;
-            cs.a[1] = -cs.r[1] / d;
-            cs.b[0] = cs.C1 / d;
-            cs.b[1] = -cs.C1 / d;
-            double k0 = cs.k0s, dGm = -cs.dGs, dGp = cs.dGs, dJb = -cs.dJs, dJ0 = cs.dJs;
+    for (int p = blockIdx.x; p < npairs; p += gridDim.x) {
+        const int c0 = 2 * p, ncol = c0 + 1 < a.K4 ? 2 : 1;
+        // ---- the pair's h V, and what its columns have from eps, mu and Sigma_inf alone
+        for (int j = tid; j < NJ; j += NT) cp_async16(&X[pidx(j)], reinterpret_cast<const double2 *>(a.hV) + (size_t)p * NJ + j);
+        if (tid < 2) {
+            CondBwdCol &q = col[tid];
+            const int c = min(c0 + tid, a.K4 - 1);
+            q.l = c / a.nbk;
+            q.m = c % a.nbk;
+            q.o = oct_index(q.l + 1, q.m);
+            q.e = a.ek[q.o];
+            q.dk = a.dek[c];
+            q.d2 = a.d2ek[c];
+            q.wt = (q.m == 0 || q.m == a.nbk - 1) ? 2.0 : 4.0;
+            real_roots(mu - q.e, sinf, q.r[0], q.r[1]);
+            const double d = q.r[0] - q.r[1];
+            q.a[0] = q.r[0] / d;
+            q.a[1] = -q.r[1] / d;
+            double k0 = 0.0, dGm = 0.0, dGp = 0.0;
             for (int i = 0; i < 2; ++i) {
-                const double f = fermi_fn(cs.r[i], T);
-                cs.f[i] = f;
-                k0 += cs.a[i] * f;
-                dGm += cs.r[i] * cs.a[i] * f;
-                dGp += cs.r[i] * cs.a[i] * (1.0 - f);
-                dJb += cs.r[i] * cs.b[i] * (1.0 - f);
-                dJ0 += cs.r[i] * cs.b[i] * f;
+                const double r = q.r[i], ex = exp(-fabs(r) * beta), u = 1.0 / (1.0 + ex);
+                q.u[i] = u;
+                q.f[i] = r > 0 ? ex * u : u;
+                q.omf[i] = r > 0 ? u : ex * u;
+                k0 += q.a[i] * q.f[i];
+                dGm += r * q.a[i] * q.f[i];
+                dGp += r * q.a[i] * q.omf[i];
             }
-            cs.k0 = k0;
-            cs.dGm = dGm;
-            cs.dGp = dGp;
-            cs.dJb = dJb;
-            cs.dJ0 = dJ0;
+            q.k0 = k0;
+            q.dGm = dGm;
+            q.dGp = dGp;
         }
+        cp_async_wait_all();
         __syncthreads();
-        // ---- back to tau: G(tau) + i J(tau) = conj(ht) FFT_-[Gs + i conj Js] plus the analytic tails
-        if (tid < G) group_fft_io<N, -1, false, true>(X, tid, (const TwoLevelTw *)tw2, 0, ScratchIO{X}, ScratchIO{X});
-        __syncthreads();
-        for (int j = tid; j < N; j += NT) {
-            const double tau = j * h;
-            const double2 Z = cmul(cconj(tw_at(ht2, j)), X[pidx(j)]);
-            const double g0t = -cs.a[0] * tail_g(cs.r[0], tau, beta) - cs.a[1] * tail_g(cs.r[1], tau, beta);
-            const double jin = cs.b[0] * tail_j(cs.r[0], tau, beta) + cs.b[1] * tail_j(cs.r[1], tau, beta);
-            Gt[j] = Z.x + g0t;
-            Jt[j] = Z.y + jin;
-            if (j == 0) cs.Jraw0 = Z.y;
+        // exp(-|r| tau_j), column q and root i: row 2 q + i
+        for (int i = tid; i < 4 * (P::n_hi + P::n_lo); i += NT) {
+            const bool hi = i < 4 * P::n_hi;
+            const int ii = hi ? i : i - 4 * P::n_hi, len = hi ? P::n_hi : P::n_lo, row = ii / len, e = ii % len;
+            (hi ? tails_hi : tails_lo)[ii] = exp(-fabs(col[row >> 1].r[row & 1]) * ((hi ? 64 * e : e) * h));
         }
-        __syncthreads();
-        if (tid == 0) {
-            cs.Gt0 = Gt[0];
-            cs.Jt0 = Jt[0];
-            cs.Jbeta = -cs.Jraw0 + cs.b[0] * tail_j(cs.r[0], beta, beta) + cs.b[1] * tail_j(cs.r[1], beta, beta);
-            d0s[0] = cs.dGp * cs.Jt0 + cs.Gt0 * cs.dJ0;
-            dNs[0] = cs.dGm * cs.Jbeta - (cs.Gt0 + 1.0) * cs.dJb;
-            cs.dchi = cs.dGp * (cs.Gt0 + 1.0) + cs.Gt0 * cs.dGm;
-            e0s[0] = cs.dchi;
-            eNs[0] = 0.0;
-            cs.CJ1b = cs.Gt0 * cs.Jt0 + (cs.Gt0 + 1.0) * cs.Jbeta;
-            R[N] = (-cs.Gt0 - 1.0) * cs.Jbeta;
-            Q[0] = cs.Gt0 * (cs.Gt0 + 1.0);
-        }
-        for (int j = tid; j < N; j += NT) R[j] = Gt[j] * Jt[j];
-        for (int j = 1 + tid; j <= NO; j += NT) Q[j] = -Gt[j] * Gt[N - j];
-        __syncthreads();
-        spline_second_derivatives<1>(R, NJ, NJ, h, d0s, dNs, a.spl_full, a.spl_full + NJ);
-        spline_second_derivatives<1>(Q, NJ2, NJ2, h, e0s, eNs, a.spl_half, a.spl_half + NJ2);
-        if (tid == 0) cs.CJ3b = R[0] - R[N];
-        // ---- the Maki-Thompson moment and the bubble: FFT_-[y2 + i fb]
         if (tid < G) {
-            auto in = [&](int j) -> double2 {
-                const double y2 = (R[j + 1] - R[j]) * ih;
-                const double fb = j < NO ? (Q[j + 1] - Q[j]) * ih : -(Q[N - j] - Q[N - 1 - j]) * ih;
-                return make_double2(y2, fb);
-            };
-            group_fft_io<N, -1>(X, tid, (const TwoLevelTw *)tw2, 0, in, ScratchIO{X});
-        }
-        __syncthreads();
-        // ---- backward seeds at n = 1..NO; the cotangents of J0f and Fb parked in R, Q
-        {
-            double acc[4] = {0.0, 0.0, 0.0, 0.0};
-            const double wt = cs.wt, dk = cs.dk;
-            for (int n = 1 + tid; n <= NO; n += NT) {
-                double2 J0f, Fb;
-                split_real(X[pidx(n)], X[pidx(N - n)], J0f, Fb);
-                const double wq = 2 * n * pT, iw = 1.0 / wq, iw2 = iw * iw, iw4 = iw2 * iw2;
-                const double2 w = tw_at(tw2, n);
-                const double2 zq = make_double2(1.0 - w.x, -w.y);
-                const double imJ = -2.0 * cs.CJ1b * iw + 2.0 * cs.CJ3b * iw2 * iw + 2.0 * cmul(zq, J0f).y * iw4;
-                const double bub = -2.0 * cs.dchi * iw2 + cmul(zq, Fb).x * iw4;
-                const double cwn = a.cw[n];
-                const double bubb = cwn * (-2.0 * wt * nf * dk * dk);
-                const double imJb = cwn * (-nf * wt * dk * iw);
-                acc[0] += cwn * (-4.0 * wt * nf * dk * bub) + cwn * (-nf * wt * imJ * iw);
-                acc[1] += bubb * (-2.0 * iw2);
-                acc[2] += imJb * (-2.0 * iw);
-                acc[3] += imJb * (2.0 * iw2 * iw);
-                // Fb_bar = bubb conj(zq) / wq^4, J0f_bar = imJb (2 / wq^4) i conj(zq)
-                reinterpret_cast<double2 *>(Q)[n - 1] = cscale(cconj(zq), bubb * iw4);
-                reinterpret_cast<double2 *>(R)[n - 1] = cscale(make_double2(zq.y, zq.x), 2.0 * imJb * iw4);
-            }
-            block_sum<4>(acc, sums);
-        }
-        if (tid == 0) {
-            cs.dkb = sums[0];
-            cs.dchib = sums[1];
-            cs.CJ1bb = sums[2];
-            cs.CJ3bb = sums[3];
-        }
-        // Hermitian parts, packed: P_k = Jh_k + i Fh_k
-        for (int k = tid; k < N; k += NT) {
-            double2 jh = make_double2(0.0, 0.0), fh = jh;
-            const double2 *Jb = reinterpret_cast<const double2 *>(R);
-            const double2 *Fbb = reinterpret_cast<const double2 *>(Q);
-            if (k >= 1 && k < NO) {
-                jh = cscale(Jb[k - 1], 0.5);
-                fh = cscale(Fbb[k - 1], 0.5);
-            } else if (k == NO) {
-                jh = make_double2(Jb[NO - 1].x, 0.0);
-                fh = make_double2(Fbb[NO - 1].x, 0.0);
-            } else if (k > NO) {
-                jh = cscale(cconj(Jb[N - k - 1]), 0.5);
-                fh = cscale(cconj(Fbb[N - k - 1]), 0.5);
-            }
-            X[pidx(k)] = make_double2(jh.x - fh.y, jh.y + fh.x);
-        }
-        __syncthreads();
-        if (tid < G) group_fft_io<N, +1, false, true>(X, tid, (const TwoLevelTw *)tw2, 0, ScratchIO{X}, ScratchIO{X});
-        __syncthreads();
-        // M_bar of the G J spline (R, NJ) and of the bubble spline (Q, NJ2)
-        for (int i = tid; i <= N; i += NT) {
-            const double ym = i >= 1 ? X[pidx(i - 1)].x : 0.0;
-            const double y0 = i < N ? X[pidx(i)].x : 0.0;
-            double v = ih * (ym - y0);
-            if (i == 0) v += cs.CJ3bb;
-            if (i == N) v -= cs.CJ3bb;
-            R[i] = v;
-        }
-        for (int i = tid; i <= NO; i += NT) {
-            auto y3 = [&](int k) -> double {
-                if (k < 0 || k >= NO) return 0.0;
-                return X[pidx(k)].y - X[pidx(N - 1 - k)].y;
-            };
-            Q[i] = ih * (y3(i - 1) - y3(i));
-        }
-        __syncthreads();
-        spline_second_derivatives<1, true>(R, NJ, NJ, h, nullptr, nullptr, a.spl_full, a.spl_full + NJ);
-        spline_second_derivatives<1, true>(Q, NJ2, NJ2, h, nullptr, nullptr, a.spl_half, a.spl_half + NJ2);
-        // d L / d gj into Xd[0..N], d L / d GG into Xd[N+1 .. N+1+NO]
-        for (int i = tid; i <= N; i += NT) {
-            double v = spline_rT(R, i, N, a6);
-            if (i == 0) v += cs.CJ1bb;
-            if (i == N) v -= cs.CJ1bb;
-            Xd[i] = v;
-        }
-        for (int i = tid; i <= NO; i += NT) Xd[N + 1 + i] = spline_rT(Q, i, NO, a6);
-        __syncthreads();
-        if (tid == 0) {
-            cs.d0b2 = -b6 * R[0];
-            cs.dNb2 = b6 * R[N];
-            cs.dchib += -b6 * Q[0];
-            const double gjbN = Xd[N], GGb0 = Xd[N + 1];
-            const double dchib = cs.dchib, d0b = cs.d0b2, dNb = cs.dNb2;
-            cs.Gt0bs = dchib * (cs.dGp + cs.dGm) + d0b * cs.dJ0 - dNb * cs.dJb - gjbN * cs.Jbeta +
-                       GGb0 * (2.0 * cs.Gt0 + 1.0);
-            cs.Jt0bs = d0b * cs.dGp;
-            cs.dGpb = dchib * (cs.Gt0 + 1.0) + d0b * cs.Jt0;
-            cs.dGmb = dchib * cs.Gt0 + dNb * cs.Jbeta;
-            cs.dJ0b = d0b * cs.Gt0;
-            cs.dJbb = -dNb * (cs.Gt0 + 1.0);
-            cs.Jbetab = gjbN * (-cs.Gt0 - 1.0) + dNb * cs.dGm;
-        }
-        __syncthreads();
-        // ---- d L / d G(tau), d L / d J(tau) (into R, Q) and the tails' parameters
-        {
-            double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // a1, a2, b1, b2, r1, r2
-            for (int j = tid; j < N; j += NT) {
-                const double gjb = Xd[j];
-                double gtb = gjb * Jt[j], jtb = gjb * Gt[j];
-                if (j >= 1) {
-                    const double ggs = (j <= NO ? Xd[N + 1 + j] : 0.0) + (j >= NO ? Xd[N + 1 + N - j] : 0.0);
-                    gtb -= ggs * Gt[N - j];
-                } else {
-                    gtb += cs.Gt0bs;
-                    jtb += cs.Jt0bs;
-                }
-                R[j] = gtb;
-                Q[j] = jtb;
-                const double tau = j * h;
-#pragma unroll
+            const double *db = a.dbound + c0;
+            const double2 d0 = make_double2(db[0], ncol == 2 ? db[1] : 0.0);
+            const double2 dN = make_double2(db[a.K4p], ncol == 2 ? db[a.K4p + 1] : 0.0);
+            for (int k = tid; k < 2; k += G) {
+                CondBwdCol &q = col[k];
+                const double v0 = reinterpret_cast<const double *>(&X[0])[k];
+                const double vN = reinterpret_cast<const double *>(&X[pidx(N)])[k];
+                const double d = q.r[0] - q.r[1];
+                q.C1 = -v0 - vN;
+                q.C2 = k == 0 ? d0.x + dN.x : d0.y + dN.y;
+                q.b[0] = q.C1 / d;
+                q.b[1] = -q.C1 / d;
+                double dJb = 0.0, dJ0 = 0.0;
                 for (int i = 0; i < 2; ++i) {
-                    const double g = tail_g(cs.r[i], tau, beta), jj = tail_j(cs.r[i], tau, beta);
-                    acc[i] -= gtb * g;
-                    acc[4 + i] += gtb * (-cs.a[i]) * g * (cs.f[i] / T - tau);
-                    acc[2 + i] += jtb * jj;
-                    acc[4 + i] += jtb * cs.b[i] * jj * (tau - (1.0 - cs.f[i]) / T);
+                    dJb += q.r[i] * q.b[i] * q.omf[i];
+                    dJ0 += q.r[i] * q.b[i] * q.f[i];
+                }
+                q.dJb = dJb;
+                q.dJ0 = dJ0;
+            }
+            group_sync<G>(0);
+            spline_complex<N>(X, NJ, tid, 0, h, d0, dN, a.spl_full, a.spl_full + NJ);
+            for (int k = tid; k < 2; k += G)
+                col[k].C3 = -(reinterpret_cast<const double *>(&X[0])[k] +
+                              reinterpret_cast<const double *>(&X[pidx(N)])[k]);
+            auto in = [&](int j) -> double2 {
+                const double2 u = X[pidx(j)], v = X[pidx(j + 1)];
+                return cmul(tw_at(ht2, j), make_double2((v.x - u.x) * ih, (v.y - u.y) * ih));
+            };
+            group_fft_io<N, +1, false, true>(X, tid, (const TwoLevelTw *)tw2, 0, in, ScratchIO{X});
+        }
+        __syncthreads();
+        // ---- J(i k_n) of both columns
+        for (int n = tid; n < NO; n += NT) {
+            double2 F[2];
+            split_real(X[pidx(n)], X[pidx(N - 1 - n)], F[0], F[1]);
+            const double kn = (2 * n + 1) * pT, ik = 1.0 / kn, ik2 = ik * ik, ik4 = ik2 * ik2;
+            const double2 ee = tw_at(ht2, 2 * n + 1);
+            const double2 f = make_double2(1.0 - ee.x, -ee.y);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const double2 w = cmul(f, F[q]);
+                wsJ[q * NO + n] = make_double2(-col[q].C2 * ik2 + w.x * ik4,
+                                               -col[q].C1 * ik + col[q].C3 * ik2 * ik + w.y * ik4);
+            }
+        }
+#pragma unroll 1
+        for (int q = 0; q < ncol; ++q) {
+            CondBwdCol &cs = col[q];
+            double2 *const wJ = wsJ + q * NO;
+            const double e = cs.e, C1 = cs.C1;
+            // ---- G(i k_n), the tail-subtracted G and G J, packed for the tau transform
+            {
+                double acc[3] = {0.0, 0.0, 0.0};
+                const double s2 = a.s2[cs.o], s3 = a.s3[cs.o];
+                for (int n = tid; n < NO; n += NT) {
+                    const double kn = (2 * n + 1) * pT, ik = 1.0 / kn;
+                    const double2 J = wJ[n];
+                    double rS, iS;
+                    sigma_full(ik, sinf, s2, s3, a.S[bidx(n, cs.o, NO)], rS, iS);
+                    const double2 Gv = crecip(T, mu - e - rS, kn - iS);
+                    const double2 Gl = crecip(T, mu - e, kn + sinf * ik);
+                    const double2 Gs = csub(Gv, Gl);
+                    const double2 Js = csub(cmul(Gv, J), cmul(Gl, make_double2(0.0, -C1 * ik)));
+                    wsG[n] = Gv;
+                    // Gs + i conj(Js) at n, conj(Gs) + i Js at N - 1 - n
+                    X[pidx(n)] = make_double2(Gs.x + Js.y, Gs.y + Js.x);
+                    X[pidx(N - 1 - n)] = make_double2(Gs.x - Js.y, -Gs.y + Js.x);
+                    acc[0] += Gs.x;
+                    acc[1] += kn * Gs.y;
+                    acc[2] -= kn * Js.y;
+                }
+                block_sum<3>(acc, sums);
+            }
+            // ---- back to tau: G(tau) + i J(tau) = conj(ht) FFT_-[Gs + i conj Js] plus the analytic tails
+            if (tid < G)
+                group_fft_io<N, -1, false, true>(X, tid, (const TwoLevelTw *)tw2, 0, ScratchIO{X}, ScratchIO{X});
+            __syncthreads();
+            const bool big0 = cs.r[0] > 0, big1 = cs.r[1] > 0;
+            const double *hi0 = tails_hi + 2 * q * P::n_hi, *hi1 = hi0 + P::n_hi;
+            const double *lo0 = tails_lo + 2 * q * P::n_lo, *lo1 = lo0 + P::n_lo;
+            // the tails of tau_j: g_i = e^{-tau r_i} (1 - f_i), j_i = e^{tau r_i} f_i
+            auto tail = [&](int j, double &g0, double &g1, double &j0, double &j1) {
+                const int jm = N - j;
+                const double x0 = cs.u[0] * (hi0[j >> 6] * lo0[j & 63]), y0 = cs.u[0] * (hi0[jm >> 6] * lo0[jm & 63]);
+                const double x1 = cs.u[1] * (hi1[j >> 6] * lo1[j & 63]), y1 = cs.u[1] * (hi1[jm >> 6] * lo1[jm & 63]);
+                g0 = big0 ? x0 : y0;
+                j0 = big0 ? y0 : x0;
+                g1 = big1 ? x1 : y1;
+                j1 = big1 ? y1 : x1;
+            };
+            for (int j = tid; j <= NO; j += NT) {
+                double g0, g1, j0, j1;
+                tail(j, g0, g1, j0, j1);
+                const double2 Z = cmul(cconj(tw_at(ht2, j)), X[pidx(j)]);
+                const double Gt = Z.x - cs.a[0] * g0 - cs.a[1] * g1, Jt = Z.y + cs.b[0] * j0 + cs.b[1] * j1;
+                wsT[j] = make_double2(Gt, Jt);
+                if (j == 0) {
+                    // the ends: values, slopes and moments of both products
+                    const double k0 = cs.k0 + 2.0 * sums[0], dGm = cs.dGm - 2.0 * sums[1], dGp = cs.dGp + 2.0 * sums[1];
+                    const double dJb = cs.dJb - 2.0 * sums[2], dJ0 = cs.dJ0 + 2.0 * sums[2];
+                    const double Jbeta = -Z.y + cs.b[0] * cs.omf[0] + cs.b[1] * cs.omf[1];
+                    const double dchi = dGp * (Gt + 1.0) + Gt * dGm;
+                    cs.k0 = k0;
+                    cs.dGm = dGm;
+                    cs.dGp = dGp;
+                    cs.dJb = dJb;
+                    cs.dJ0 = dJ0;
+                    cs.Gt0 = Gt;
+                    cs.Jt0 = Jt;
+                    cs.Jbeta = Jbeta;
+                    cs.dchi = dchi;
+                    cs.CJ1b = Gt * Jt + (Gt + 1.0) * Jbeta;
+                    sd0 = make_double2(dGp * Jt + Gt * dJ0, dchi);
+                    sdN = make_double2(dGm * Jbeta - (Gt + 1.0) * dJb, -dchi);
+                    X[0] = make_double2(Gt * Jt, Gt * (Gt + 1.0));
+                    X[pidx(N)] = make_double2((-Gt - 1.0) * Jbeta, Gt * (Gt + 1.0));
+                } else {
+                    double Gm = Gt, Jm = Jt;
+                    if (j < NO) {
+                        tail(N - j, g0, g1, j0, j1);
+                        const double2 Zm = cmul(cconj(tw_at(ht2, N - j)), X[pidx(N - j)]);
+                        Gm = Zm.x - cs.a[0] * g0 - cs.a[1] * g1;
+                        Jm = Zm.y + cs.b[0] * j0 + cs.b[1] * j1;
+                        wsT[N - j] = make_double2(Gm, Jm);
+                        X[pidx(N - j)] = make_double2(Gm * Jm, -Gt * Gm);
+                    }
+                    X[pidx(j)] = make_double2(Gt * Jt, -Gt * Gm);
                 }
             }
-            block_sum<6>(acc, sums);
-        }
-        if (tid == 0) {
-            double ab[2] = {sums[0], sums[1]}, bb[2] = {sums[2], sums[3]}, rb[2] = {sums[4], sums[5]};
-            const double k0b = a.kx0b * (-2.0 * cs.wt * nf * cs.d2);
-            for (int i = 0; i < 2; ++i) {
-                const double r = cs.r[i], f = cs.f[i], av = cs.a[i], bv = cs.b[i];
-                const double jb = tail_j(r, beta, beta);
-                bb[i] += cs.Jbetab * jb;
-                rb[i] += cs.Jbetab * bv * jb * (beta - (1.0 - f) / T);
-                const double fp = -f * (1.0 - f) / T;
-                ab[i] += k0b * f + cs.dGmb * r * f + cs.dGpb * r * (1.0 - f);
-                bb[i] += cs.dJbb * r * (1.0 - f) + cs.dJ0b * r * f;
-                rb[i] += k0b * av * fp + cs.dGmb * av * (f + r * fp) + cs.dGpb * av * ((1.0 - f) - r * fp) +
-                         cs.dJbb * bv * ((1.0 - f) - r * fp) + cs.dJ0b * bv * (f + r * fp);
+            __syncthreads();
+            // ---- the Maki-Thompson moment and the bubble: FFT_-[y2 + i fb]
+            if (tid < G) {
+                spline_complex<N>(X, NJ, tid, 0, h, sd0, sdN, a.spl_full, a.spl_full + NJ);
+                if (tid == 0) cs.CJ3b = X[0].x - X[pidx(N)].x;
+                auto in = [&](int j) -> double2 {
+                    const double2 u = X[pidx(j)], v = X[pidx(j + 1)];
+                    return make_double2((v.x - u.x) * ih, (v.y - u.y) * ih);
+                };
+                group_fft_io<N, -1, false, true>(X, tid, (const TwoLevelTw *)tw2, 0, in, ScratchIO{X});
             }
-            const double r1 = cs.r[0], r2 = cs.r[1], d = r1 - r2, d2i = 1.0 / (d * d);
-            rb[0] += ab[0] * (-r2 * d2i) + ab[1] * (r2 * d2i);
-            rb[1] += ab[0] * (r1 * d2i) + ab[1] * (-r1 * d2i);
-            cs.C1bs = (bb[0] - bb[1]) / d;
-            const double db = -(bb[0] - bb[1]) * cs.C1 * d2i;
-            rb[0] += db;
-            rb[1] -= db;
-            const double B = mu - cs.e;
-            double Bb = 0.0, Cb = 0.0;
-            for (int i = 0; i < 2; ++i) {
-                Bb += rb[i] * (-cs.r[i] / (2.0 * cs.r[i] + B));
-                Cb += rb[i] * (-1.0 / (2.0 * cs.r[i] + B));
+            __syncthreads();
+            // ---- backward seeds at n = 1..NO; the cotangents of both transforms,
+            // Hermitian parts, packed in their places: P_k = Jh_k + i Fh_k
+            {
+                double acc[4] = {0.0, 0.0, 0.0, 0.0};
+                const double wt = cs.wt, dk = cs.dk, CJ1b = cs.CJ1b, CJ3b = cs.CJ3b, dchi = cs.dchi;
+                for (int n = 1 + tid; n <= NO; n += NT) {
+                    double2 J0f, Fb;
+                    split_real(X[pidx(n)], X[pidx(N - n)], J0f, Fb);
+                    const double wq = 2 * n * pT, iw = 1.0 / wq, iw2 = iw * iw, iw4 = iw2 * iw2;
+                    const double2 w = tw_at(tw2, n);
+                    const double2 zq = make_double2(1.0 - w.x, -w.y);
+                    const double imJ = -2.0 * CJ1b * iw + 2.0 * CJ3b * iw2 * iw + 2.0 * cmul(zq, J0f).y * iw4;
+                    const double bub = -2.0 * dchi * iw2 + cmul(zq, Fb).x * iw4;
+                    const double cwn = a.cw[n];
+                    const double bubb = cwn * (-2.0 * wt * nf * dk * dk);
+                    const double imJb = cwn * (-nf * wt * dk * iw);
+                    acc[0] += cwn * (-4.0 * wt * nf * dk * bub) + cwn * (-nf * wt * imJ * iw);
+                    acc[1] += bubb * (-2.0 * iw2);
+                    acc[2] += imJb * (-2.0 * iw);
+                    acc[3] += imJb * (2.0 * iw2 * iw);
+                    // Fb_bar = bubb conj(zq) / wq^4, J0f_bar = imJb (2 / wq^4) i conj(zq)
+                    double2 fh = cscale(cconj(zq), bubb * iw4);
+                    double2 jh = cscale(make_double2(zq.y, zq.x), 2.0 * imJb * iw4);
+                    if (n == NO) {
+                        X[pidx(NO)] = make_double2(jh.x, fh.x);
+                    } else {
+                        fh = cscale(fh, 0.5);
+                        jh = cscale(jh, 0.5);
+                        X[pidx(n)] = make_double2(jh.x - fh.y, jh.y + fh.x);
+                        X[pidx(N - n)] = make_double2(jh.x + fh.y, -jh.y + fh.x);
+                    }
+                }
+                if (tid == 0) X[0] = make_double2(0.0, 0.0);
+                block_sum<4>(acc, sums);
             }
-            cs.mub = Bb;
-            cs.eb = -Bb;
-            cs.sinfb = -Cb;
-            cs.k0sb = k0b;
-            cs.dGsb = cs.dGpb - cs.dGmb;
-            cs.dJsb = cs.dJ0b - cs.dJbb;
+            if (tid < G) {
+                group_fft_io<N, +1, false, true>(X, tid, (const TwoLevelTw *)tw2, 0, ScratchIO{X}, ScratchIO{X});
+                if constexpr (FftPlan<N>::NPASS == 1) group_sync<G>(0);
+                // M_bar of both splines, and the adjoint solve
+                const double C3 = sums[3];
+                spline_sweeps<N>(X, NJ, tid, 0, a.spl_full, a.spl_full + NJ,
+                                 [&](int i, double2 vm, double2 v0, double2) -> double2 {
+                                     if (i == 0) return make_double2(-ih * v0.x + C3, -ih * v0.y);
+                                     if (i == N) return make_double2(ih * vm.x - C3, ih * vm.y);
+                                     return make_double2(ih * (vm.x - v0.x), ih * (vm.y - v0.y));
+                                 });
+            }
+            __syncthreads();
+            // ---- d L / d G(tau), d L / d J(tau) in the places of G, J (tau), and the tails' parameters
+            {
+                double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // a1, a2, b1, b2, r1, r2
+                auto put = [&](int j, double gtb, double jtb) {
+                    double g0, g1, j0, j1;
+                    tail(j, g0, g1, j0, j1);
+                    const double tau = j * h;
+                    wsT[j] = make_double2(gtb, jtb);
+                    acc[0] -= gtb * g0;
+                    acc[1] -= gtb * g1;
+                    acc[2] += jtb * j0;
+                    acc[3] += jtb * j1;
+                    acc[4] += -gtb * cs.a[0] * g0 * (cs.f[0] * beta - tau) + jtb * cs.b[0] * j0 * (tau - cs.omf[0] * beta);
+                    acc[5] += -gtb * cs.a[1] * g1 * (cs.f[1] * beta - tau) + jtb * cs.b[1] * j1 * (tau - cs.omf[1] * beta);
+                };
+                // R^T of the adjoint solution, interior rows
+                auto vr = [&](int i) -> double2 {
+                    const double2 u = X[pidx(i - 1)], v = X[pidx(i)], w = X[pidx(i + 1)];
+                    return make_double2(a6 * (u.x - 2.0 * v.x + w.x), a6 * (u.y - 2.0 * v.y + w.y));
+                };
+                for (int j = tid; j <= NO; j += NT) {
+                    const double2 gj = wsT[j];  // G, J
+                    if (j == 0) {
+                        const double2 x0 = X[0], x1 = X[pidx(1)], xm = X[pidx(N - 1)], xN = X[pidx(N)];
+                        const double gjb0 = a6 * (x1.x - x0.x) + sums[2], gjbN = a6 * (xm.x - xN.x) - sums[2];
+                        const double GGb0 = a6 * ((x1.y - x0.y) + (xm.y - xN.y));
+                        const double d0b = -b6 * x0.x, dNb = b6 * xN.x;
+                        const double dchib = sums[1] - b6 * (x0.y + xN.y);
+                        cs.dkb = sums[0];
+                        cs.dGpb = dchib * (cs.Gt0 + 1.0) + d0b * cs.Jt0;
+                        cs.dGmb = dchib * cs.Gt0 + dNb * cs.Jbeta;
+                        cs.dJ0b = d0b * cs.Gt0;
+                        cs.dJbb = -dNb * (cs.Gt0 + 1.0);
+                        cs.Jbetab = gjbN * (-cs.Gt0 - 1.0) + dNb * cs.dGm;
+                        const double Gt0b = dchib * (cs.dGp + cs.dGm) + d0b * cs.dJ0 - dNb * cs.dJb - gjbN * cs.Jbeta +
+                                            GGb0 * (2.0 * cs.Gt0 + 1.0);
+                        put(0, gjb0 * gj.y + Gt0b, gjb0 * gj.x + d0b * cs.dGp);
+                    } else {
+                        const int jm = N - j;
+                        const double2 gm = wsT[jm], v = vr(j), vm = vr(jm);
+                        const double ggs = v.y + vm.y;
+                        put(j, v.x * gj.y - ggs * gm.x, v.x * gj.x);
+                        if (jm != j) put(jm, vm.x * gm.y - ggs * gj.x, vm.x * gm.x);
+                    }
+                }
+                block_sum<6>(acc, sums);
+            }
+            if (tid == 0) {
+                double ab[2] = {sums[0], sums[1]}, bb[2] = {sums[2], sums[3]}, rb[2] = {sums[4], sums[5]};
+                const double k0b = a.kx0b * (-2.0 * cs.wt * nf * cs.d2);
+                for (int i = 0; i < 2; ++i) {
+                    const double r = cs.r[i], f = cs.f[i], om = cs.omf[i], av = cs.a[i], bv = cs.b[i];
+                    const double jb = om;  // the tail of J at beta
+                    bb[i] += cs.Jbetab * jb;
+                    rb[i] += cs.Jbetab * bv * jb * (beta - om / T);
+                    const double fp = -f * om / T;
+                    ab[i] += k0b * f + cs.dGmb * r * f + cs.dGpb * r * om;
+                    bb[i] += cs.dJbb * r * om + cs.dJ0b * r * f;
+                    rb[i] += k0b * av * fp + cs.dGmb * av * (f + r * fp) + cs.dGpb * av * (om - r * fp) +
+                             cs.dJbb * bv * (om - r * fp) + cs.dJ0b * bv * (f + r * fp);
+                }
+                const double r1 = cs.r[0], r2 = cs.r[1], d = r1 - r2, d2i = 1.0 / (d * d);
+                rb[0] += ab[0] * (-r2 * d2i) + ab[1] * (r2 * d2i);
+                rb[1] += ab[0] * (r1 * d2i) + ab[1] * (-r1 * d2i);
+                cs.C1b = (bb[0] - bb[1]) / d;
+                const double db = -(bb[0] - bb[1]) * cs.C1 * d2i;
+                rb[0] += db;
+                rb[1] -= db;
+                const double B = mu - cs.e;
+                double Bb = 0.0, Cb = 0.0;
+                for (int i = 0; i < 2; ++i) {
+                    Bb += rb[i] * (-cs.r[i] / (2.0 * cs.r[i] + B));
+                    Cb += rb[i] * (-1.0 / (2.0 * cs.r[i] + B));
+                }
+                cs.mub = Bb;
+                cs.eb = -Bb;
+                cs.sinfb = -Cb;
+                cs.k0sb = k0b;
+                cs.dGsb = cs.dGpb - cs.dGmb;
+                cs.dJsb = cs.dJ0b - cs.dJbb;
+            }
+            // ---- to frequency: FFT_+[ht (Gt_bar + i Jt_bar)]
+            if (tid < G) {
+                auto in = [&](int j) -> double2 { return cmul(tw_at(ht2, j), wsT[j]); };
+                group_fft_io<N, +1>(X, tid, (const TwoLevelTw *)tw2, 0, in, ScratchIO{X});
+            }
+            __syncthreads();
+            {
+                double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // C1, C2, C3, mu, eps, sinf
+                double2 *const sigc = a.sigc + (size_t)(c0 + q) * NO;
+                const double k0sb = cs.k0sb, dGsb = cs.dGsb, dJsb = cs.dJsb, Jbetab = cs.Jbetab;
+                for (int n = tid; n < NO; n += NT) {
+                    const double kn = (2 * n + 1) * pT, ik = 1.0 / kn, ik2 = ik * ik;
+                    double2 A, B;
+                    split_real(X[pidx(n)], X[pidx(N - 1 - n)], A, B);
+                    const double2 Gsb = make_double2(2.0 * A.x + 2.0 * k0sb, 2.0 * A.y + 2.0 * kn * dGsb);
+                    const double2 Jsb = make_double2(2.0 * B.x - 2.0 * Jbetab, -2.0 * B.y - 2.0 * kn * dJsb);
+                    const double2 Gv = wsG[n], J = wJ[n];
+                    const double2 Gl = crecip(T, mu - e, kn + sinf * ik);
+                    const double2 Gvb = cadd(Gsb, cmul(Jsb, cconj(J)));
+                    const double2 Jb = cmul(Jsb, cconj(Gv));
+                    const double2 Glb = csub(make_double2(-Gsb.x, -Gsb.y), cmul(Jsb, make_double2(0.0, C1 * ik)));
+                    const double2 iGl = cmul(make_double2(0.0, ik), Gl);
+                    acc[0] += cmul(cconj(iGl), Jsb).x;
+                    acc[0] += -Jb.y * ik;
+                    acc[1] += -Jb.x * ik2;
+                    acc[2] += Jb.y * ik2 * ik;
+                    const double2 ee = tw_at(ht2, 2 * n + 1);
+                    const double2 f = make_double2(1.0 - ee.x, -ee.y);
+                    const double2 Fbar = cscale(cmul(cconj(f), Jb), 0.5 * ik2 * ik2);
+                    const double2 gg = cscale(cmul(Gv, Gv), 1.0 / T);
+                    const double2 sg = cmul(Gvb, cconj(gg));
+                    sigc[n] = sg;
+                    acc[3] -= sg.x;
+                    acc[4] += sg.x;
+                    const double2 qq = cscale(cmul(Gl, Gl), -1.0 / T);
+                    const double rq = cmul(Glb, cconj(qq)).x;
+                    acc[3] += rq;
+                    acc[4] -= rq;
+                    acc[5] += cmul(Glb, cconj(cmul(qq, make_double2(0.0, ik)))).x;
+                    // half of F_bar, extended to a Hermitian sequence: a real transform;
+                    // the first column's waits in the place of its J
+                    if (q + 1 < ncol) {
+                        wJ[n] = Fbar;
+                    } else {
+                        const double2 A0 = q == 0 ? Fbar : wsJ[n], B0 = q == 0 ? make_double2(0.0, 0.0) : Fbar;
+                        X[pidx(n)] = make_double2(A0.x - B0.y, A0.y + B0.x);
+                        X[pidx(N - 1 - n)] = make_double2(A0.x + B0.y, -A0.y + B0.x);
+                    }
+                }
+                block_sum<6>(acc, sums);
+            }
+            if (tid == 0) {
+                cs.C1b += sums[0];
+                cs.C2b = sums[1];
+                cs.C3b = sums[2];
+                acc_mu += cs.mub + sums[3];
+                acc_sinf += cs.sinfb + sums[5];
+                double de, ddek, dd2;
+                tp_dirs(cs.l + 1, cs.m, a.nbk, de, ddek, dd2);
+                const double d2b = a.kx0b * (-2.0 * cs.wt * nf * cs.k0);
+                acc_tp += (cs.eb + sums[4]) * de + cs.dkb * ddek + d2b * dd2;
+            }
         }
         __syncthreads();
-        // ---- to frequency: FFT_+[ht (Gt_bar + i Jt_bar)]
+        // ---- the cotangent of h V
         if (tid < G) {
-            auto in = [&](int j) -> double2 { return cmul(tw_at(ht2, j), make_double2(R[j], Q[j])); };
-            group_fft_io<N, +1>(X, tid, (const TwoLevelTw *)tw2, 0, in, ScratchIO{X});
+            group_fft_io<N, -1, false, true>(
+                X, tid, (const TwoLevelTw *)tw2, 0, ScratchIO{X},
+                [&](int j, double2 z) { X[pidx(j)] = cmul(cconj(tw_at(ht2, j)), z); });
+            if constexpr (FftPlan<N>::NPASS == 1) group_sync<G>(0);
+            const double2 C3 = make_double2(col[0].C3b, ncol == 2 ? col[1].C3b : 0.0);
+            spline_sweeps<N>(X, NJ, tid, 0, a.spl_full, a.spl_full + NJ,
+                             [&](int i, double2 vm, double2 v0, double2) -> double2 {
+                                 if (i == 0) return make_double2(-ih * v0.x - C3.x, -ih * v0.y - C3.y);
+                                 if (i == N) return make_double2(ih * vm.x - C3.x, ih * vm.y - C3.y);
+                                 return make_double2(ih * (vm.x - v0.x), ih * (vm.y - v0.y));
+                             });
         }
         __syncthreads();
         {
-            double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // C1, C2, C3, mu, eps, sinf
-            const double e = cs.e, C1 = cs.C1;
-            double2 *Fbar = reinterpret_cast<double2 *>(R);
-            double2 *sigc = a.sigc + (size_t)c * NO;
-            for (int n = tid; n < NO; n += NT) {
-                const double kn = (2 * n + 1) * pT, ik = 1.0 / kn, ik2 = ik * ik;
-                double2 A, B;
-                split_real(X[pidx(n)], X[pidx(N - 1 - n)], A, B);
-                const double2 Gsb = make_double2(2.0 * A.x + 2.0 * cs.k0sb, 2.0 * A.y + 2.0 * kn * cs.dGsb);
-                const double2 Jsb = make_double2(2.0 * B.x - 2.0 * cs.Jbetab, -2.0 * B.y - 2.0 * kn * cs.dJsb);
-                const double2 Gv = wsG[n], J = wsJ[n];
-                const double2 Gl = cdiv(make_double2(T, 0.0), make_double2(mu - e, kn + sinf * ik));
-                const double2 Gvb = cadd(Gsb, cmul(Jsb, cconj(J)));
-                const double2 Jb = cmul(Jsb, cconj(Gv));
-                const double2 Glb = csub(make_double2(-Gsb.x, -Gsb.y), cmul(Jsb, make_double2(0.0, C1 * ik)));
-                const double2 iGl = cmul(make_double2(0.0, ik), Gl);
-                acc[0] += cmul(cconj(iGl), Jsb).x;
-                acc[0] += -Jb.y * ik;
-                acc[1] += -Jb.x * ik2;
-                acc[2] += Jb.y * ik2 * ik;
-                const double2 ee = tw_at(ht2, 2 * n + 1);
-                const double2 f = make_double2(1.0 - ee.x, -ee.y);
-                Fbar[n] = cscale(cmul(cconj(f), Jb), ik2 * ik2);
-                const double2 gg = cscale(cmul(Gv, Gv), 1.0 / T);
-                sigc[n] = cmul(Gvb, cconj(gg));
-                const double rg = cmul(Gvb, cconj(gg)).x;
-                acc[3] -= rg;
-                acc[4] += rg;
-                const double2 q = cscale(cmul(Gl, Gl), -1.0 / T);
-                const double rq = cmul(Glb, cconj(q)).x;
-                acc[3] += rq;
-                acc[4] -= rq;
-                acc[5] += cmul(Glb, cconj(cmul(q, make_double2(0.0, ik)))).x;
-            }
-            block_sum<6>(acc, sums);
-        }
-        for (int k = tid; k < N; k += NT)
-            X[pidx(k)] = k < NO ? reinterpret_cast<const double2 *>(R)[k] : make_double2(0.0, 0.0);
-        __syncthreads();
-        if (tid < G) group_fft_io<N, -1, false, true>(X, tid, (const TwoLevelTw *)tw2, 0, ScratchIO{X}, ScratchIO{X});
-        __syncthreads();
-        {
-            const double C3b = sums[2];
+            const double2 C1b = make_double2(col[0].C1b, ncol == 2 ? col[1].C1b : 0.0);
+            double2 *const out = reinterpret_cast<double2 *>(a.hVb) + (size_t)p * NJ;
             for (int i = tid; i <= N; i += NT) {
-                const double ym = i >= 1 ? cmul(cconj(tw_at(ht2, i - 1)), X[pidx(i - 1)]).x : 0.0;
-                const double y0 = i < N ? cmul(cconj(tw_at(ht2, i)), X[pidx(i)]).x : 0.0;
-                double v = ih * (ym - y0);
-                if (i == 0) v -= C3b;
-                if (i == N) v -= C3b;
-                R[i] = v;
+                const double2 v = X[pidx(i)];
+                const double2 u = i > 0 ? X[pidx(i - 1)] : v, w = i < N ? X[pidx(i + 1)] : v;
+                double2 r = make_double2(a6 * ((u.x - v.x) + (w.x - v.x)), a6 * ((u.y - v.y) + (w.y - v.y)));
+                if (i == 0 || i == N) r = csub(r, C1b);
+                out[i] = r;
             }
         }
-        __syncthreads();
-        spline_second_derivatives<1, true>(R, NJ, NJ, h, nullptr, nullptr, a.spl_full, a.spl_full + NJ);
-        {
-            const double C1b = sums[0] + cs.C1bs;
-            for (int i = tid; i <= N; i += NT) {
-                double v = spline_rT(R, i, N, a6);
-                if (i == 0 || i == N) v -= C1b;
-                a.hVb[bidx2(i, c, NJ)] = v;
-            }
-        }
-        if (tid == 0) {
-            const double C2b = sums[1];
-            a.dbb[c] = -b6 * R[0] + C2b;
-            a.dbb[(size_t)a.K4p + c] = b6 * R[N] + C2b;
-            acc_mu += cs.mub + sums[3];
-            acc_sinf += cs.sinfb + sums[5];
-            double de, ddek, dd2;
-            tp_dirs(cs.l + 1, cs.m, a.nbk, de, ddek, dd2);
-            const double d2b = a.kx0b * (-2.0 * cs.wt * nf * cs.k0);
-            acc_tp += (cs.eb + sums[4]) * de + cs.dkb * ddek + d2b * dd2;
+        if (tid < ncol) {
+            const double r0 = reinterpret_cast<const double *>(&X[0])[tid];
+            const double rN = reinterpret_cast<const double *>(&X[pidx(N)])[tid];
+            a.dbb[c0 + tid] = -b6 * r0 + col[tid].C2b;
+            a.dbb[(size_t)a.K4p + c0 + tid] = b6 * rN + col[tid].C2b;
         }
         __syncthreads();
     }
@@ -1181,23 +1225,23 @@ namespace {
 template <int N>
 struct RunCondTauBwd {
     static cudaError_t run(const CondBwdArgs *a, int nblk, cudaStream_t st) {
-        const size_t sm = CondBwdSmem<N>::bytes;
+        const size_t sm = CondBwdPlan<N>::bytes;
         cudaError_t e = set_smem(k_cond_tau_bwd<N>, sm);
         if (e != cudaSuccess) return e;
-        k_cond_tau_bwd<N><<<nblk, cond_bwd_threads<N>(), sm, st>>>(*a);
+        k_cond_tau_bwd<N><<<nblk, CondBwdPlan<N>::threads, sm, st>>>(*a);
         return launched();
     }
 };
 template <int N>
 struct CondBwdBlocks {
     static cudaError_t run(int *blocks) {
-        const size_t sm = CondBwdSmem<N>::bytes;
+        const size_t sm = CondBwdPlan<N>::bytes;
         cudaError_t e = set_smem(k_cond_tau_bwd<N>, sm);
         if (e != cudaSuccess) return e;
         int dev = 0, sms = 0, per = 0;
         if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
         if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cond_tau_bwd<N>, cond_bwd_threads<N>(), sm)) !=
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cond_tau_bwd<N>, CondBwdPlan<N>::threads, sm)) !=
             cudaSuccess)
             return e;
         *blocks = sms * (per > 0 ? per : 1);

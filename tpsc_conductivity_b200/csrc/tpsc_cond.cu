@@ -335,12 +335,6 @@ __device__ __forceinline__ void tails(const CondCol &q, const ColState &s, doubl
 }
 
 __device__ __forceinline__ double part_of(double2 z, int q) { return q == 0 ? z.x : z.y; }
-// T / z by one division
-__device__ __forceinline__ double2 crecip(double T, double x, double y) {
-    const double s = T / (x * x + y * y);
-    return make_double2(x * s, -y * s);
-}
-
 // Persistent over column pairs; the pair's two real columns are the parts of one
 // complex column throughout, in two buffers X1, X2 that two groups of threads
 // spline and transform in place at the same time: f0 V beside h V, G beside J,

@@ -874,6 +874,12 @@ __device__ __forceinline__ double2 cexp2(double2 z) {
 
 __device__ __forceinline__ double2 cscale(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
 
+// T / z by one division
+__device__ __forceinline__ double2 crecip(double T, double x, double y) {
+    const double s = T / (x * x + y * y);
+    return make_double2(x * s, -y * s);
+}
+
 // block-wide sum of NV values per thread -> out[0..NV) (all threads must call;
 // out visible to every thread on return)
 template <int NV>
@@ -915,29 +921,21 @@ __device__ __forceinline__ void stage_pair(double *R, const double *g, int NJ, b
     cp_async_wait_all();
 }
 
-// spline_second_derivatives for one complex column (or two real ones as its
-// parts) of NJ <= N + 1 nodes in the padded layout, by the G threads of a group
-// of the N-point FFT: both parts of a node by one thread, so that its two
-// chains interleave.  TPC of them sweep, in chunks long enough
-// that the kWarm warm-up rows do not dominate.
-template <int N>
-__device__ void spline_complex(double2 *X, int NJ, int t, int grp, double h, double2 d0, double2 dN,
-                               const double *__restrict__ invp, const double *__restrict__ cp) {
+// The clamped spline's sweeps for one complex column (or two real ones as its
+// parts) of NJ <= N + 1 nodes in the padded layout, in place, by the G threads of
+// a group of the N-point FFT: both parts of a node by one thread, so that its two
+// chains interleave.  TPC of them sweep, in chunks long enough that the kWarm
+// warm-up rows do not dominate.  rhs(i, X[i-1], X[i], X[i+1]) is row i of the
+// right-hand side (the neighbour beyond an end is not to be used).
+template <int N, class Rhs>
+__device__ void spline_sweeps(double2 *X, int NJ, int t, int grp, const double *__restrict__ invp,
+                              const double *__restrict__ cp, const Rhs &rhs) {
     constexpr int G = FftPlan<N>::G, TPC = G >= 64 ? G / 2 : G;
     const int C = (NJ + TPC - 1) / TPC, last = NJ - 1;
     const int s = t < TPC ? min(t * C, NJ) : NJ, e = min(s + C, NJ);
-    const double a6 = 6.0 / (h * h), b6 = 6.0 / h, ih = 1.0 / h;
     const double cpiv = last > kSplinePivotConst ? __ldg(&invp[kSplinePivotConst]) : 0.0;
     auto piv = [&](int i) -> double { return (i >= kSplinePivotConst && i < last) ? cpiv : __ldg(&invp[i]); };
     auto sup = [&](int i) -> double { return (i >= kSplinePivotConst && i < last) ? cpiv : __ldg(&cp[i]); };
-    auto rhs1 = [&](int i, double vm, double v0, double vp, double dl, double dr) -> double {
-        if (i == 0) return b6 * ((vp - v0) * ih - dl);
-        if (i == last) return b6 * (dr - (v0 - vm) * ih);
-        return a6 * (vp - 2.0 * v0 + vm);
-    };
-    auto rhs = [&](int i, double2 vm, double2 v0, double2 vp) -> double2 {
-        return make_double2(rhs1(i, vm.x, v0.x, vp.x, d0.x, dN.x), rhs1(i, vm.y, v0.y, vp.y, d0.y, dN.y));
-    };
     const double2 zero = make_double2(0.0, 0.0);
     double2 carry = zero, vm_h = zero, vs_h = zero, ve_h = zero;
     if (s < e) {
@@ -977,6 +975,23 @@ __device__ void spline_complex(double2 *X, int NJ, int t, int grp, double h, dou
             X[pidx(i)] = mm;
         }
     group_sync<G>(grp);
+}
+
+// spline_second_derivatives for such a column: the node values in X become the
+// node second derivatives
+template <int N>
+__device__ void spline_complex(double2 *X, int NJ, int t, int grp, double h, double2 d0, double2 dN,
+                               const double *__restrict__ invp, const double *__restrict__ cp) {
+    const int last = NJ - 1;
+    const double a6 = 6.0 / (h * h), b6 = 6.0 / h, ih = 1.0 / h;
+    auto rhs1 = [&](int i, double vm, double v0, double vp, double dl, double dr) -> double {
+        if (i == 0) return b6 * ((vp - v0) * ih - dl);
+        if (i == last) return b6 * (dr - (v0 - vm) * ih);
+        return a6 * (vp - 2.0 * v0 + vm);
+    };
+    spline_sweeps<N>(X, NJ, t, grp, invp, cp, [&](int i, double2 vm, double2 v0, double2 vp) -> double2 {
+        return make_double2(rhs1(i, vm.x, v0.x, vp.x, d0.x, dN.x), rhs1(i, vm.y, v0.y, vp.y, d0.y, dN.y));
+    });
 }
 
 // ---------------------------------------------------------------------------

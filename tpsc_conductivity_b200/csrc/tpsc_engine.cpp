@@ -2824,7 +2824,7 @@ int ensure_adj(tpsc_ctx *ctx, Grid *g) {
     AdjDev &a = g->adj;
     int nblk = 0;
     CK(cond_bwd_blocks(d, &nblk));
-    a.nblk = std::max(1, std::min(nblk, c.K4));
+    a.nblk = std::max(1, std::min(nblk, (c.K4 + 1) / 2));
     const size_t NO = d.nw0 / 2, NJ = d.nw0 + 1, nb = d.nb, K4 = c.K4, K4p = c.K4p, n8 = d.n8, n8p = d.n8p;
     a.row_ct = 0;
     a.row_cl = a.row_ct + a.nblk;
@@ -2842,7 +2842,7 @@ int ensure_adj(tpsc_ctx *ctx, Grid *g) {
         e = (x);            \
     }
     A(dalloc(g, &a.cw, NO + 1));
-    A(dalloc(g, &a.ws, (size_t)a.nblk * 2 * NO));
+    A(dalloc(g, &a.ws, (size_t)a.nblk * kCondBwdWs * NO));
     A(dalloc(g, &a.hVb, K4p * NJ));
     A(dalloc(g, &a.dbb, 2 * K4p));
     A(dalloc(g, &a.sigc, K4 * NO));
@@ -2931,7 +2931,6 @@ int tpsc_sigma_iqn_bwd(tpsc_ctx *ctx, int nq, const double *cot, double grad[3],
     ca.dek = c.dek;
     ca.d2ek = c.d2ek;
     ca.spl_full = d.spl_full;
-    ca.spl_half = d.spl_half;
     ca.tw = d.tw_w;
     ca.ht = d.ht_w;
     ca.cw = a.cw;

@@ -327,16 +327,17 @@ struct AdjDev {
     int row_ct = 0, row_cl = 0, row_cb = 0, row_cs = 0, row_sg = 0, row_ss = 0, row_sb = 0, row_vt = 0, row_vq = 0;
     int rows = 0;
 };
+constexpr int kCondBwdWs = 5;
 struct CondBwdArgs {
-    const double *hV = nullptr, *dbound = nullptr;
+    const double *hV = nullptr, *dbound = nullptr;  // hV: two-column blocks
     const double2 *S = nullptr;
     const double *s2 = nullptr, *s3 = nullptr, *sinf = nullptr;
     const double *ek = nullptr, *dek = nullptr, *d2ek = nullptr;
-    const double *spl_full = nullptr, *spl_half = nullptr;
+    const double *spl_full = nullptr;
     const double2 *tw = nullptr, *ht = nullptr;
     const double *cw = nullptr;
     double kx0b = 0.0;
-    double2 *ws = nullptr;
+    double2 *ws = nullptr;  // kCondBwdWs nw0/2 per block
     double *hVb = nullptr, *dbb = nullptr;
     double2 *sigc = nullptr;
     double *part = nullptr;
