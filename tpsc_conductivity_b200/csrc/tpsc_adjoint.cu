@@ -1218,6 +1218,19 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
     }
 }
 
+// The partial rows summed per slot, one block a slot: compensated strided sums, then
+// the tree and the warps in order.  Reading 6000 rows back for a host loop took the
+// host 0.2 ms of a gradient.
+__global__ void __launch_bounds__(256) k_adj_sums(const double *__restrict__ part, int nrows, double *__restrict__ out) {
+    const int slot = blockIdx.x;
+    KSum acc;
+    for (int r = threadIdx.x; r < nrows; r += blockDim.x) acc.add(part[(size_t)r * kAdjW + slot]);
+    double v[1] = {acc.value()};
+    __shared__ double tot[1];
+    block_sum<1>(v, tot);
+    if (threadIdx.x == 0) out[slot] = tot[0];
+}
+
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
@@ -1328,6 +1341,10 @@ struct RunVertexQBwd {
 
 cudaError_t cond_bwd_blocks(const GridDev &g, int *blocks) { return dispatch_nw<CondBwdBlocks>(g.nw0, blocks); }
 
+cudaError_t launch_adj_sums(const AdjDev &a, int r0, int r1, double *out, cudaStream_t st) {
+    k_adj_sums<<<kAdjW, 256, 0, st>>>(a.part + (size_t)r0 * kAdjW, r1 - r0, out);
+    return launched();
+}
 cudaError_t launch_cond_tau_bwd(const GridDev &g, const CondBwdArgs &a, int nblk, cudaStream_t st) {
     return dispatch_nw<RunCondTauBwd>(g.nw0, &a, nblk, st);
 }

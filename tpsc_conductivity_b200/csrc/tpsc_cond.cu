@@ -100,6 +100,30 @@ __device__ void roots_2pol(double2 B, double2 C, double2 &r0, double2 &r1) {
 //   x <= 0: A = dek/L^2 / (e^{x/T} + 1),   B = -dek/L^2 / (T (e^{x/T} + 1)^2)
 // tab[4c..4c+2] = (x, A, B)
 // ---------------------------------------------------------------------------
+// d eps/d kx and d2 eps/d kx2 (hamiltonien::grad_ek direction 0 and Hessian_ek
+// (0, 0), src/hamiltonien.cpp:134-155) on k = (l+1, m) pi/(nbk-1)
+// (src/cond_opt.cpp:2588-2611), and the second on the kx = 0, pi lines, from the
+// grid's table of sines and cosines.  Ten host sines and cosines a point took 0.3 ms at
+// 128 x 128 and 1.2 ms at 256 x 256 of every call.
+__global__ void __launch_bounds__(256)
+    k_cond_model(const double *__restrict__ ktab, int nbk, int K4, double tp, double tpp, double t3,
+                 double *__restrict__ dek, double *__restrict__ d2ek, double *__restrict__ d2line) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= K4 + 2 * nbk) return;
+    const int line = i - K4;  // >= 0: the points of the two lines
+    const int l = line < 0 ? i / nbk + 1 : (line < nbk ? 0 : nbk - 1), m = (line < 0 ? i : line) % nbk;
+    const double *c1 = ktab, *s1 = ktab + nbk, *c2 = ktab + 2 * nbk, *s2 = ktab + 3 * nbk;
+    const double h = 2.0 * c1[l] + 4.0 * tp * c1[l] * c1[m] + 8.0 * tpp * c2[l] +
+                     4.0 * t3 * (4.0 * c2[l] * c1[m] + c2[m] * c1[l]);
+    if (line >= 0) {
+        d2line[line] = h;
+        return;
+    }
+    d2ek[i] = h;
+    dek[i] = 2.0 * s1[l] + 4.0 * tp * s1[l] * c1[m] + 4.0 * tpp * s2[l] +
+             4.0 * t3 * (2.0 * s2[l] * c1[m] + c2[m] * s1[l]);
+}
+
 __global__ void k_cond_table(const double *__restrict__ ek, const double *__restrict__ dek, int K4, int nbk,
                              double mu0, double T, double nf, double *__restrict__ tab) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -873,6 +897,12 @@ struct CondBlocks {
 size_t cond_col_words() { return kCondColWords; }
 
 cudaError_t cond_blocks(const GridDev &g, int *blocks) { return dispatch_nw<CondBlocks>(g.nw0, blocks); }
+
+cudaError_t launch_cond_model(const GridDev &g, const CondDev &c, double tp, double tpp, double t3, cudaStream_t st) {
+    const int n = c.K4 + 2 * g.nbk;
+    k_cond_model<<<(n + 255) / 256, 256, 0, st>>>(g.ktab, g.nbk, c.K4, tp, tpp, t3, c.dek, c.d2ek, c.d2line);
+    return launched();
+}
 
 cudaError_t launch_cond_table(const GridDev &g, const CondDev &c, double mu0, double T, cudaStream_t st) {
     const double nf = 1.0 / ((double)g.nk0 * g.nk0);

@@ -47,10 +47,43 @@ struct SolveKey {
     }
 };
 
+// The tail power sums of a frequency axis without their powers of T (long double):
+// q[k] = sum_{n = Nw0/2+1}^{Nw0} n^(-2k) of the sum-rule tail series (smallest terms
+// first; q[0] is not used and 0), and p[k] = sum_{t=0}^{Nw0/2} (Nw0 + 2t + 1)^-k, the
+// fermionic tail of the find_mu moments (largest t first)
+struct TailSums {
+    long double q[kTailQ], p[kTailP];
+    void build(int nw0) {
+        for (long double &v : q) v = 0.0L;
+        for (long double &v : p) v = 0.0L;
+        const int NO = nw0 / 2;
+        for (int j = nw0; j > NO; --j) {
+            const long double x = 1.0L / ((long double)j * j);
+            long double xp = x;
+            for (int k = 1; k < kTailQ; ++k, xp *= x) q[k] += xp;
+        }
+        for (int t = NO; t >= 0; --t) {
+            const long double x = 1.0L / (2.0L * (NO + t) + 1.0L);
+            long double xp = 1.0L;
+            for (int k = 0; k < kTailP; ++k, xp *= x) p[k] += xp;
+        }
+    }
+    // Q_k = sum qn^(-2k), qn = 2 pi n T, and P_k = sum w^-k, w = (Nw0 + 2t + 1) pi T
+    void at(double T, double tailq[kTailQ], double tailP[kTailP]) const {
+        const long double x = 1.0L / (3.141592653589793238462643383279502884L * (long double)T), x2 = x * x / 4.0L;
+        long double xp = 1.0L;
+        for (int k = 0; k < kTailQ; ++k, xp *= x2) tailq[k] = (double)(q[k] * xp);
+        xp = 1.0L;
+        for (int k = 0; k < kTailP; ++k, xp *= x) tailP[k] = (double)(p[k] * xp);
+    }
+};
+
 struct Grid {
     GridDev d;
     cudaStream_t st = nullptr;    // the owning context's stream: every fill and upload is ordered on it
-    std::vector<double> ek_host;  // [nbk * nbk], ek[m + l*nbk]
+    std::vector<double> ktab;     // [4 nbk] cos k, sin k, cos 2k, sin 2k on k = l pi/(nbk - 1)
+    double hop[3] = {0, 0, 0};    // t', t'', t3 of the grid's eps_k
+    TailSums tails;
     double mu0 = 0.0;
     double *Grt = nullptr;        // [(Nw0+1) * n8]      G(r, tau_j)
     float *Grt32 = nullptr;       // [(Nw0+1) * n8]      G(r, tau_j) in FP32 (mixed form; allocated on first use)
@@ -86,9 +119,6 @@ struct Grid {
     // the reverse pass of sigma(iq_n) (tpsc_sigma_iqn_bwd; allocated on first use)
     AdjDev adj;
     bool adj_alloc = false;
-    double tailq_T = -1.0;         // temperature the tail power sums were built for
-    double tailq_host[kTailQ] = {0};
-    double tailP_host[kTailP] = {0};
     std::vector<void *> allocs;
     unsigned warm_forms = 0;  // bit f: a direct (uncaptured) Newton solve in form f ran on this grid
     // the solve on this grid as an executable CUDA graph, the key
@@ -103,6 +133,7 @@ struct Grid {
     size_t cond_part_cap = 0, cond_out_cap = 0;  // doubles in cond.partial, cond.out
     std::vector<double> cond_host;
     int cond_bins = 0;                            // n_theta of cond_host (0: none yet)
+    int bins_made = 1;                            // n_theta of the device's angle bins (zeros at first)
     // Aslamazov-Larkin correction: device state (allocated on first use) and
     // the last result, [N (1 + n_theta)] on the grid al_ind
     AlDev al;
@@ -122,9 +153,10 @@ struct Grid {
 struct Group {
     int nk0 = 0, nw0 = 0, cap = 0;  // cap: points the arenas are allocated for
     GridDev d;                      // the shape's tables; ek, er, gk, tailq, tailP of point 0
+    const Grid *grid = nullptr;     // the grid of the shape (the context keeps every grid)
     char *base = nullptr;           // cap * arena bytes
     long long arena = 0;
-    size_t in_bytes = 0;            // the per-point inputs at arena offset 0: ek, er, tailq, tailP, scalars
+    size_t in_off = 0, in_bytes = 0;  // the per-point inputs in the arena: tailq, tailP, scalars
     size_t res_off = 0;             // the results block: kGroupRes doubles
     double *pp = nullptr;           // point 0's scalars [kPP]
     float *Grt32 = nullptr;
@@ -252,22 +284,13 @@ void free_grid(Grid *g) {
 }
 
 // eps_k = -2(cx + cy) - 4 t' cx cy - 2 t''(c2x + c2y) - 4 t3 (c2x cy + c2y cx) on
-// k = l pi/(nbk-1) (hamiltonien::calc_ek / dispk, src/hamiltonien.cpp:358-375, 428-431)
-double dispk(double kx, double ky, double tp, double tpp, double t3) {
-    return -2.0 * (std::cos(kx) + std::cos(ky)) - 4.0 * tp * std::cos(kx) * std::cos(ky) -
-           2.0 * tpp * (std::cos(2 * kx) + std::cos(2 * ky)) -
-           4 * t3 * (std::cos(2 * kx) * std::cos(ky) + std::cos(2 * ky) * std::cos(kx));
-}
-
-// d eps/d kx and d2 eps/d kx2 (hamiltonien::grad_ek direction 0 and
-// Hessian_ek (0, 0), src/hamiltonien.cpp:134-155)
-double grad_ek_x(double kx, double ky, double tp, double tpp, double t3) {
-    return 2.0 * std::sin(kx) + 4.0 * tp * std::sin(kx) * std::cos(ky) + 4.0 * tpp * std::sin(2 * kx) +
-           4 * t3 * (2.0 * std::sin(2 * kx) * std::cos(ky) + std::cos(2 * ky) * std::sin(kx));
-}
-double hessian_ek_xx(double kx, double ky, double tp, double tpp, double t3) {
-    return 2.0 * std::cos(kx) + 4.0 * tp * std::cos(kx) * std::cos(ky) + 8.0 * tpp * std::cos(2 * kx) +
-           4 * t3 * (4.0 * std::cos(2 * kx) * std::cos(ky) + std::cos(2 * ky) * std::cos(kx));
+// k = l pi/(nbk-1) (hamiltonien::calc_ek / dispk, src/hamiltonien.cpp:358-375, 428-431):
+// eps of lattice point (l, m) of grid g's quadrant
+double grid_eps(const Grid *g, int l, int m) {
+    const double *c1 = g->ktab.data(), *c2 = c1 + 2 * g->d.nbk;
+    const double tp = g->hop[0], tpp = g->hop[1], t3 = g->hop[2];
+    return -2.0 * (c1[l] + c1[m]) - 4.0 * tp * c1[l] * c1[m] - 2.0 * tpp * (c2[l] + c2[m]) -
+           4 * t3 * (c2[l] * c1[m] + c2[m] * c1[l]);
 }
 
 // Thomas-algorithm tables of the clamped-spline system with NJ nodes:
@@ -355,6 +378,15 @@ int build_grid(tpsc_ctx *ctx, int nk0, int nw0, Grid **out) {
             if (m == l) w /= 2;
             w16[m + l * (l + 1) / 2] = w;
         }
+    g->ktab.resize((size_t)4 * d.nbk);
+    for (int l = 0; l < d.nbk; ++l) {
+        const double k = l * PI / (d.nbk - 1);
+        g->ktab[l] = std::cos(k);
+        g->ktab[d.nbk + l] = std::sin(k);
+        g->ktab[2 * d.nbk + l] = std::cos(2 * k);
+        g->ktab[3 * d.nbk + l] = std::sin(2 * k);
+    }
+    g->tails.build(nw0);
     std::vector<double2> twk, tww, htw;
     std::vector<float4> twk32;
     twiddles32(nk0, twk32);
@@ -373,6 +405,7 @@ int build_grid(tpsc_ctx *ctx, int nk0, int nw0, Grid **out) {
         e = (x);                                   \
     }
     A(upload(g, &d.w16, w16));
+    A(upload(g, &d.ktab, g->ktab));
     A(upload(g, &d.tw_k, twk));
     A(upload(g, &d.tw_k32, twk32));
     std::vector<float> dct;
@@ -459,68 +492,14 @@ int read_result(tpsc_ctx *ctx, int count, double *out, const double *src = nullp
 
 // eps_k tables of the grid for the current model, then mu0 by the density
 // root of green0::find_mu (src/green0.cpp:240-262)
-// power sums Q_k = sum_{n = Nw0/2+1}^{Nw0} qn^(-2k), qn = 2 pi n T, for the
-// sum-rule tail series (smallest terms first, long double), and
-// P_p = sum_{t=0}^{Nw0/2} w^-p, w = (Nw0 + 2t + 1) pi T: the fermionic tail of
-// the find_mu moments (largest t first, long double)
-void tail_power_sums(int nw0, double T, double tailq[kTailQ], double tailP[kTailP]) {
-    std::vector<long double> acc(kTailQ, 0.0L);
-    const int nwmax = nw0 / 2;
-    for (int j = 2 * nwmax; j > nwmax; --j) {
-        const long double wn = 2.0L * 3.141592653589793238462643383279502884L * j * (long double)T;
-        const long double x = 1.0L / (wn * wn);
-        long double xp = x;
-        for (int k = 1; k < kTailQ; ++k, xp *= x) acc[k] += xp;
-    }
-    for (int k = 0; k < kTailQ; ++k) tailq[k] = (double)acc[k];
-    std::vector<long double> pw(kTailP, 0.0L);
-    const int NO = nw0 / 2;
-    for (int t = NO; t >= 0; --t) {
-        const long double x =
-            1.0L / ((2.0L * (NO + t) + 1.0L) * 3.141592653589793238462643383279502884L * (long double)T);
-        long double xp = 1.0L;
-        for (int k = 0; k < kTailP; ++k, xp *= x) pw[k] += xp;
-    }
-    for (int k = 0; k < kTailP; ++k) tailP[k] = (double)pw[k];
-}
-
-// eps_k on the octant of the nbk x nbk quadrant (dispk from tables of cos(k)
-// and cos(2k): the same values and expression as the reference's, one pair
-// of cosines per index instead of ten per point); full = the quadrant, or null
-void octant_eps(int nbk, double tp, double tpp, double t3, double *eo, std::vector<double> *full) {
-    std::vector<double> c1(nbk), c2(nbk);
-    for (int l = 0; l < nbk; ++l) {
-        const double k = l * PI / (nbk - 1);
-        c1[l] = std::cos(k);
-        c2[l] = std::cos(2 * k);
-    }
-    if (full) full->assign((size_t)nbk * nbk, 0.0);
-    for (int l = 0; l < nbk; ++l)
-        for (int m = 0; m < nbk; ++m) {
-            const double e = -2.0 * (c1[l] + c1[m]) - 4.0 * tp * c1[l] * c1[m] - 2.0 * tpp * (c2[l] + c2[m]) -
-                             4 * t3 * (c2[l] * c1[m] + c2[m] * c1[l]);
-            if (full) (*full)[m + (size_t)l * nbk] = e;
-            if (m <= l) eo[m + (size_t)l * (l + 1) / 2] = e;
-        }
-}
-
 int grid_set_model(tpsc_ctx *ctx, Grid *g) {
     GridDev &d = g->d;
-    std::vector<double> eo(d.n8), er(d.n8, 0.0);
-    octant_eps(d.nbk, ctx->tp, ctx->tpp, ctx->t3, eo.data(), &g->ek_host);
-    er[1] = -1;
-    er[2] = -ctx->tp;
-    er[3] = -ctx->tpp;
-    er[4] = -ctx->t3;
-    CK(cudaMemcpyAsync(d.ek, eo.data(), d.n8 * sizeof(double), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemcpyAsync(d.er, er.data(), d.n8 * sizeof(double), cudaMemcpyHostToDevice, ctx->st));
-    if (g->tailq_T != ctx->T) {
-        tail_power_sums(d.nw0, ctx->T, g->tailq_host, g->tailP_host);
-        CK(cudaMemcpyAsync(d.tailq, g->tailq_host, kTailQ * sizeof(double), cudaMemcpyHostToDevice, ctx->st));
-        CK(cudaMemcpyAsync(d.tailP, g->tailP_host, kTailP * sizeof(double), cudaMemcpyHostToDevice, ctx->st));
-        g->tailq_T = ctx->T;
-    }
-    CK(cudaStreamSynchronize(ctx->st));
+    ModelTables m;
+    m.tp = g->hop[0] = ctx->tp;
+    m.tpp = g->hop[1] = ctx->tpp;
+    m.t3 = g->hop[2] = ctx->t3;
+    g->tails.at(ctx->T, m.tailq, m.tailP);
+    CK(launch_model_tables(d, m, ctx->st));
     g->have_chi0 = g->have_V = g->have_S = false;
     if (ctx->n == 1.0 && ctx->tp == 0 && ctx->tpp == 0) {
         g->mu0 = 0.0 + ctx->mu_shift;
@@ -1127,36 +1106,25 @@ int ensure_cond(tpsc_ctx *ctx, Grid *g, int nbins) {
         CK(cudaMalloc(&c.out, need_out * sizeof(double)));
         g->cond_out_cap = need_out;
     }
-    // tables on k = (l+1, m) pi/(nbk-1) (src/cond_opt.cpp:2588-2611) and on
-    // the kx = 0, pi lines; the angle bin theta_k = atan((L/2 - m)/(L/2 - l - 1)),
-    // floor(theta_k / (pi / (2 n_theta))) (src/cond_opt.cpp:3174, 3790-3793)
-    std::vector<double> dek(c.K4), d2(c.K4), d2l(2 * nbk);
-    std::vector<int> bins(c.K4, 0);
-    const int nk0 = d.nk0;
-    const double Dtheta = PI / (2.0 * nbins);
-    for (int l = 0; l < nbk - 2; ++l) {
-        const double kx = (l + 1) * PI / (nbk - 1);
-        for (int m = 0; m < nbk; ++m) {
-            const double ky = m * PI / (nbk - 1);
-            dek[m + l * nbk] = grad_ek_x(kx, ky, ctx->tp, ctx->tpp, ctx->t3);
-            d2[m + l * nbk] = hessian_ek_xx(kx, ky, ctx->tp, ctx->tpp, ctx->t3);
-            if (nbins > 1) {
-                const double th = std::atan((1.0 * (nk0 / 2 - m)) / (nk0 / 2 - l - 1));
-                bins[m + l * nbk] = std::min(nbins - 1, std::max(0, (int)std::floor(th / Dtheta)));
-            }
-        }
+    CK(launch_cond_model(d, c, ctx->tp, ctx->tpp, ctx->t3, ctx->st));
+    // the angle bin theta_k = atan((L/2 - m)/(L/2 - l - 1)), floor(theta_k /
+    // (pi / (2 n_theta))) (src/cond_opt.cpp:3174, 3790-3793), of the grid and n_theta alone
+    if (nbins != g->bins_made) {
+        std::vector<int> bins(c.K4, 0);
+        const int nk0 = d.nk0;
+        const double Dtheta = PI / (2.0 * nbins);
+        if (nbins > 1)
+            for (int l = 0; l < nbk - 2; ++l)
+                for (int m = 0; m < nbk; ++m) {
+                    const double th = std::atan((1.0 * (nk0 / 2 - m)) / (nk0 / 2 - l - 1));
+                    bins[m + l * nbk] = std::min(nbins - 1, std::max(0, (int)std::floor(th / Dtheta)));
+                }
+        g->bins_made = 0;
+        CK(cudaMemcpyAsync(c.bin, bins.data(), c.K4 * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
+        // the host vector is released when this block ends
+        CK(cudaStreamSynchronize(ctx->st));
+        g->bins_made = nbins;
     }
-    for (int side = 0; side < 2; ++side) {
-        const double kx = side == 0 ? 0.0 : (nbk - 1) * PI / (nbk - 1);
-        for (int m = 0; m < nbk; ++m)
-            d2l[side * nbk + m] = hessian_ek_xx(kx, m * PI / (nbk - 1), ctx->tp, ctx->tpp, ctx->t3);
-    }
-    CK(cudaMemcpyAsync(c.dek, dek.data(), c.K4 * sizeof(double), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemcpyAsync(c.d2ek, d2.data(), c.K4 * sizeof(double), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemcpyAsync(c.d2line, d2l.data(), 2 * nbk * sizeof(double), cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaMemcpyAsync(c.bin, bins.data(), c.K4 * sizeof(int), cudaMemcpyHostToDevice, ctx->st));
-    // the host vectors are released when this function returns
-    CK(cudaStreamSynchronize(ctx->st));
     return TPSC_OK;
 }
 
@@ -1541,12 +1509,11 @@ int tpsc_sumrule_tangents(tpsc_ctx *ctx, double out[9]) {
     for (int l = 0; l < nbk; ++l)
         for (int m = 0; m <= l; ++m) {
             const size_t o = m + (size_t)l * (l + 1) / 2;
-            const double kx = l * PI / (nbk - 1), ky = m * PI / (nbk - 1);
-            xi[o] = g->ek_host[m + (size_t)l * nbk] - mu0;
+            xi[o] = grid_eps(g, l, m) - mu0;
             const double z = xi[o] / T;
-            const double f = z > 0 ? std::exp(-z) / (1.0 + std::exp(-z)) : 1.0 / (1.0 + std::exp(z));
+            const double ez = std::exp(-std::fabs(z)), f = z > 0 ? ez / (1.0 + ez) : 1.0 / (1.0 + ez);
             bf[o] = beta * f;
-            deps[o] = -4.0 * std::cos(kx) * std::cos(ky);
+            deps[o] = -4.0 * g->ktab[l] * g->ktab[m];
             // the density's weight (k_density) times df/dxi = -beta f (1 - f)
             double w = 8;
             if (l == 0 || l == nbk - 1) w /= 2;
@@ -1594,10 +1561,15 @@ int tpsc_sumrule_tangents(tpsc_ctx *ctx, double out[9]) {
         CK(launch_chi0_tau(d, dchiq, g->t_ddq0, g->t_dcinf, g->t_dcinf2, T, ctx->st, false));
         CK(launch_sumrule_tan(d, g->chiq, dchiq, g->cinf, g->cinf2, g->t_dcinf, g->t_dcinf2, Usp, -1.0, T,
                               ctx->red, ctx->st));
-        if ((rc = read_result(ctx, 1, &dRsp[p]))) return rc;
+        if ((rc = queue_read_back(ctx, {{ctx->red.result, sizeof(double), 2 * p}}))) return rc;
         CK(launch_sumrule_tan(d, g->chiq, dchiq, g->cinf, g->cinf2, g->t_dcinf, g->t_dcinf2, Uch, 1.0, T,
                               ctx->red, ctx->st));
-        if ((rc = read_result(ctx, 1, &dRch[p]))) return rc;
+        if ((rc = queue_read_back(ctx, {{ctx->red.result, sizeof(double), 2 * p + 1}}))) return rc;
+    }
+    CK(cudaStreamSynchronize(ctx->st));
+    for (int p = 1; p < 3; ++p) {
+        dRsp[p] = ctx->h_res[2 * p];
+        dRch[p] = ctx->h_res[2 * p + 1];
     }
     // the roots' own derivatives (the Newton derivative of each sum rule)
     double tr, dtr_sp, dtr_ch;
@@ -1840,6 +1812,7 @@ int group_alloc(tpsc_ctx *ctx, int nk0, int nw0, int P, Group **out) {
     q->nk0 = nk0;
     q->nw0 = nw0;
     q->cap = P;
+    q->grid = g;
     q->d = g->d;
     const GridDev &d = q->d;
     const size_t n8 = d.n8, n8p = d.n8p, nb = d.nb, nw = nw0, NO = nw0 / 2;
@@ -1851,7 +1824,8 @@ int group_alloc(tpsc_ctx *ctx, int nk0, int nw0, int P, Group **out) {
     };
     const size_t o_ek = take(n8 * 8), o_er = take(n8 * 8), o_tq = take(kTailQ * 8), o_tp = take(kTailP * 8),
                  o_pp = take(kPP * 8);
-    q->in_bytes = off;
+    q->in_off = o_tq;
+    q->in_bytes = off - o_tq;
     q->res_off = take(kGroupRes * 8);
     const size_t o_gk = take(n8 * 16), o_grt = take((nw + 1) * n8 * 4), o_chirt = take(nb * n8p * 8),
                  o_chiq = take(nb * n8p * 8), o_V = take(nb * n8p * 8), o_dG0p = take(n8 * 8),
@@ -1918,10 +1892,9 @@ int group_alloc(tpsc_ctx *ctx, int nk0, int nw0, int P, Group **out) {
     return TPSC_OK;
 }
 
-// the input block of one point (params row nk0, Nw0, n, T, t', t'', t3, U):
-// eps_k on the octant, the hopping table, the tail power sums, the scalars
+// the input block of one point (params row nk0, Nw0, n, T, t', t'', t3, U): the tail
+// power sums and the scalars
 void group_point_inputs(const Group *q, const double *p, char *dst) {
-    const GridDev &d = q->d;
     const double n = p[2], T = p[3], tp = p[4], tpp = p[5], t3 = p[6], U = p[7];
     size_t off = 0;
     auto next = [&](size_t bytes) {
@@ -1929,15 +1902,8 @@ void group_point_inputs(const Group *q, const double *p, char *dst) {
         off += (bytes + 255) & ~(size_t)255;
         return r;
     };
-    double *ek = next((size_t)d.n8 * 8), *er = next((size_t)d.n8 * 8), *tq = next(kTailQ * 8),
-           *tpw = next(kTailP * 8), *pp = next(kPP * 8);
-    octant_eps(d.nbk, tp, tpp, t3, ek, nullptr);
-    std::fill(er, er + d.n8, 0.0);
-    er[1] = -1;
-    er[2] = -tp;
-    er[3] = -tpp;
-    er[4] = -t3;
-    tail_power_sums(q->nw0, T, tq, tpw);
+    double *tq = next(kTailQ * 8), *tpw = next(kTailP * 8), *pp = next(kPP * 8);
+    q->grid->tails.at(T, tq, tpw);
     std::fill(pp, pp + kPP, 0.0);
     pp[kPpT] = T;
     pp[kPpU] = U;
@@ -1951,6 +1917,9 @@ void group_point_inputs(const Group *q, const double *p, char *dst) {
     pp[kPpWc] = wc;
     // the reference's shortcut for mu0 (green0::find_mu): half filling without t', t''
     pp[kPpMu0Fixed] = (n == 1.0 && tp == 0 && tpp == 0) ? 1.0 : 0.0;
+    pp[kPpTp] = tp;
+    pp[kPpTpp] = tpp;
+    pp[kPpT3] = t3;
 }
 
 // the Newton-form mixed solve of the group's first P points, queued on
@@ -1961,8 +1930,9 @@ int group_queue(tpsc_ctx *ctx, Group *q, int P, cudaStream_t st, int root_cap) {
     b.P = P;
     b.arena = q->arena;
     b.pp = q->pp;
-    CK(cudaMemcpy2DAsync(q->base, (size_t)q->arena, q->h_in, q->in_bytes, q->in_bytes, P, cudaMemcpyHostToDevice,
-                         st));
+    CK(cudaMemcpy2DAsync(q->base + q->in_off, (size_t)q->arena, q->h_in, q->in_bytes, q->in_bytes, P,
+                         cudaMemcpyHostToDevice, st));
+    CK(launch_model_tables(d, ModelTables{}, st, b));
     CK(launch_mu0_newton(d, 0.0, 0.0, q->mu0r, st, b));
     CK(launch_gslice32(d, q->Grt32, 0.0, 0.0, st, b));
     CK(launch_chi0_boundary(d, (const float *)q->Grt32, 0.0, 0.0, q->dG0p, q->dchirt0, q->dchiqt0, st, b));
@@ -2213,7 +2183,9 @@ int tpsc_get_dims(tpsc_ctx *ctx, int dims[4]) {
 int tpsc_get_ek(tpsc_ctx *ctx, double *ek) {
     int rc = need_model(ctx);
     if (rc) return rc;
-    std::memcpy(ek, ctx->cur->ek_host.data(), ctx->cur->ek_host.size() * sizeof(double));
+    const Grid *g = ctx->cur;
+    for (int l = 0; l < g->d.nbk; ++l)
+        for (int m = 0; m < g->d.nbk; ++m) ek[m + (size_t)l * g->d.nbk] = grid_eps(g, l, m);
     return TPSC_OK;
 }
 
@@ -2866,23 +2838,10 @@ int ensure_adj(tpsc_ctx *ctx, Grid *g) {
     g->adj_alloc = true;
     return TPSC_OK;
 }
-
-// sums of the partial-row slots over rows [r0, r1) of the reverse pass, in row order
-int adj_rows(tpsc_ctx *ctx, const AdjDev &a, int r0, int r1, std::vector<double> &rows) {
-    rows.assign((size_t)(r1 - r0) * kAdjW, 0.0);
-    CK(cudaMemcpyAsync(rows.data(), a.part + (size_t)r0 * kAdjW, rows.size() * sizeof(double),
-                       cudaMemcpyDeviceToHost, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    return TPSC_OK;
-}
-double adj_slot(const std::vector<double> &rows, int slot) {
-    double s = 0.0, c = 0.0;  // compensated, in row order
-    for (size_t i = slot; i < rows.size(); i += kAdjW) {
-        const double y = rows[i] - c, t = s + y;
-        c = (t - s) - y;
-        s = t;
-    }
-    return s;
+// the partial rows [r0, r1) summed per slot -> s[kAdjW]
+int adj_sums(tpsc_ctx *ctx, const AdjDev &a, int r0, int r1, double *s) {
+    CK(launch_adj_sums(a, r0, r1, ctx->redm.result, ctx->st));
+    return read_result(ctx, kAdjW, s, ctx->redm.result);
 }
 
 int tpsc_sigma_iqn_bwd(tpsc_ctx *ctx, int nq, const double *cot, double grad[3], double dD[3]) {
@@ -2950,30 +2909,29 @@ int tpsc_sigma_iqn_bwd(tpsc_ctx *ctx, int nq, const double *cot, double grad[3],
     CK(launch_cond_lines_bwd(d, c, a, g->S, g->s2, g->s3, g->sinf, mu, T, kx0b, ctx->st));
     // mu is the root of traceDiffG: its cotangent moves to Sigma, eps and mu0
     // through lam = -(d L / d mu) / (d traceDiffG / d mu)
-    std::vector<double> rows;
-    if ((rc = adj_rows(ctx, a, a.row_ct, a.row_cb, rows))) return rc;
-    const double mub = adj_slot(rows, kAdjMu);
-    const double sinfb_c = adj_slot(rows, kAdjSinf);
+    double s[kAdjW], fr[2];
     CK(launch_trace_diff_G(d, g->S, g->s2, g->s3, g->s4, g->sinf, mu0, mu, T, ctx->red, ctx->st));
-    double fr[2];
-    if ((rc = read_result(ctx, 2, fr))) return rc;
+    CK(launch_adj_sums(a, a.row_ct, a.row_cb, ctx->redm.result, ctx->st));
+    if ((rc = read_back(ctx, {{ctx->red.result, sizeof(fr), 0}, {ctx->redm.result, sizeof(s), 2}}))) return rc;
+    std::memcpy(fr, ctx->h_res, sizeof(fr));
+    const double mub = ctx->h_res[2 + kAdjMu], sinfb_c = ctx->h_res[2 + kAdjSinf];
     if (!(fr[1] != 0.0) || !std::isfinite(fr[1])) return fail(ctx, TPSC_ERR_NONFINITE, "d traceDiffG / d mu is zero");
     const double lam = -mub / fr[1];
     CK(launch_cond_slices_bwd(d, c, a, g->V, g->dchirt0, mu0, T, fact4, dmu0_2, ctx->st));
     CK(launch_sigbar(d, c, a, g->S, g->s2, g->s3, g->s4, g->sinf, mu0, mu, lam, T, dmu0_2, ctx->st));
-    if ((rc = adj_rows(ctx, a, a.row_sg, a.row_sg + d.n8, rows))) return rc;
-    const double sinfb = sinfb_c + adj_slot(rows, kAdjSinf);
+    if ((rc = adj_sums(ctx, a, a.row_sg, a.row_sg + d.n8, s))) return rc;
+    const double sinfb = sinfb_c + s[kAdjSinf];
     CK(launch_sigma_tau_bwd(d, a, sinfb, T, ctx->st));
     CK(launch_sigma_slices_bwd(d, c, a, g->Grt, g->V, g->dchirt0, g->dG0p, mu0, fact8, dmu0_2, ctx->st));
     CK(launch_vertex_bwd(d, a, g->chirt, g->chiq, g->Grt, U, Usp, Uch, T, ctx->st));
-    if ((rc = adj_rows(ctx, a, 0, a.rows, rows))) return rc;
+    if ((rc = adj_sums(ctx, a, 0, a.rows, s))) return rc;
     // assembly: the mu0-shift and t' directions from the contractions; U, and
     // the roots' sensitivities d{Usp, Uch}/d theta (J) for every direction
-    const double f4b = adj_slot(rows, kAdjFact4), f8b = adj_slot(rows, kAdjFact8);
-    const double Uspb = adj_slot(rows, kAdjUsp) + f4b * 3.0 * U / 4.0 + f8b * 3.0 * U / 8.0;
-    const double Uchb = adj_slot(rows, kAdjUch) + f4b * U / 4.0 + f8b * U / 8.0;
-    const double Ub = adj_slot(rows, kAdjU) + f4b * (3.0 * Usp + Uch) / 4.0 + f8b * (3.0 * Usp + Uch) / 8.0;
-    const double th[3] = {Ub, adj_slot(rows, kAdjTh1), adj_slot(rows, kAdjTh2)};
+    const double f4b = s[kAdjFact4], f8b = s[kAdjFact8];
+    const double Uspb = s[kAdjUsp] + f4b * 3.0 * U / 4.0 + f8b * 3.0 * U / 8.0;
+    const double Uchb = s[kAdjUch] + f4b * U / 4.0 + f8b * U / 8.0;
+    const double Ub = s[kAdjU] + f4b * (3.0 * Usp + Uch) / 4.0 + f8b * (3.0 * Usp + Uch) / 8.0;
+    const double th[3] = {Ub, s[kAdjTh1], s[kAdjTh2]};
     for (int p = 0; p < 3; ++p) {
         grad[p] = th[p] + Uspb * J[3 * p] + Uchb * J[3 * p + 1];
         if (dD) dD[p] = J[3 * p + 2];

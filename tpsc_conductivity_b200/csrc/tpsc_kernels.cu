@@ -24,6 +24,7 @@
 #include <utility>
 
 #include "tpsc_device.cuh"
+#include "tpsc_findzero.h"
 
 namespace tpsc {
 
@@ -1988,6 +1989,35 @@ cudaError_t launch_chi0_boundary(const GridDev &g, const double *Grt, double mu0
 cudaError_t launch_chi0_boundary(const GridDev &g, const float *Grt, double mu0, double T, double *dG0p,
                                  double *dtau_chirt0, double *dtau_chiqt0, cudaStream_t st, const Bp &b) {
     return dispatch_nbk<RunChi0Boundary>(g.nbk, &g, Grt, mu0, T, dG0p, dtau_chirt0, dtau_chiqt0, &b, st);
+}
+
+// eps_k on the octant (hamiltonien::calc_ek, src/hamiltonien.cpp:358-375), rounded
+// operation by operation as the host expression is, the hopping table and the tail
+// power sums.  The host's loops and copies of these tables cost 15 to 60 us a model,
+// and a batch's 64 points were tabulated one by one before their group could start.
+__global__ void __launch_bounds__(256)
+    k_model_tables(const double *__restrict__ ktab, int nbk, int n8, const ModelTables m, double *__restrict__ ek,
+                   double *__restrict__ er, double *__restrict__ tailq, double *__restrict__ tailP, Bp b) {
+    ek = at(ek, b.arena);
+    er = at(er, b.arena);
+    const double tp = bpar(b, kPpTp, m.tp), tpp = bpar(b, kPpTpp, m.tpp), t3 = bpar(b, kPpT3, m.t3);
+    const int o = blockIdx.x * blockDim.x + threadIdx.x;
+    if (!b.pp) {
+        if (o < kTailQ) tailq[o] = m.tailq[o];
+        if (o < kTailP) tailP[o] = m.tailP[o];
+    }
+    if (o >= n8) return;
+    int l, q;
+    oct_lm(o, l, q);
+    const Rn cl(ktab[l]), cm(ktab[q]), dl(ktab[2 * nbk + l]), dm(ktab[2 * nbk + q]);
+    ek[o] = (Rn(-2.0) * (cl + cm) - Rn(4.0) * Rn(tp) * cl * cm - Rn(2.0) * Rn(tpp) * (dl + dm) -
+             Rn(4.0) * Rn(t3) * (dl * cm + dm * cl)).v;
+    er[o] = o == 1 ? -1.0 : o == 2 ? -tp : o == 3 ? -tpp : o == 4 ? -t3 : 0.0;
+}
+cudaError_t launch_model_tables(const GridDev &g, const ModelTables &m, cudaStream_t st, const Bp &b) {
+    k_model_tables<<<dim3((g.n8 + 255) / 256, 1, b.P), 256, 0, st>>>(g.ktab, g.nbk, g.n8, m, g.ek, g.er, g.tailq,
+                                                                      g.tailP, b);
+    return launched();
 }
 
 cudaError_t launch_gk_table(const GridDev &g, double mu0, double T, cudaStream_t st, const Bp &b) {

@@ -21,6 +21,7 @@ struct GridDev {
     double *er = nullptr;          // [n8] real-space hopping table
     double *w16 = nullptr;         // [n8p] octant weight: 16 halved on edges and diagonal, 0 on padding
     double *tailq = nullptr;       // [kTailQ] sum-rule tail power sums Q_k = sum_n qn^-2k (T dependent)
+    double *ktab = nullptr;        // [4 nbk] cos k, sin k, cos 2k, sin 2k on k = l pi/(nbk - 1), from the host
     double *tailP = nullptr;       // [kTailP] P_p = sum over the fermionic tail n = Nw0/2..Nw0 of w_n^-p
     double2 *tw_k = nullptr;       // [L]   exp(-2 pi i m / L)
     float4 *tw_k32 = nullptr;      // [L]   the same as (cos, sin) rounded to float, then the float remainders
@@ -73,6 +74,9 @@ enum PpSlot {
     kPpJc,          // first frequency of the find_mu series
     kPpWc,          // w_jc
     kPpMu0Fixed,    // 1: mu0 = 0 (half filling with t' = t'' = 0), no root search
+    kPpTp = 12,     // t', t'', t3 (slots 10, 11: the density root's result)
+    kPpTpp,
+    kPpT3,
 };
 struct Bp {
     int P = 1;
@@ -81,6 +85,13 @@ struct Bp {
 };
 
 // ---- launchers (all asynchronous on `st`) ---------------------------------
+// the model's tables from g.ktab: eps_k and the hopping table, and (plain launch:
+// a batch has them in its inputs) the tail power sums of m
+struct ModelTables {
+    double tp = 0.0, tpp = 0.0, t3 = 0.0;
+    double tailq[kTailQ] = {}, tailP[kTailP] = {};
+};
+cudaError_t launch_model_tables(const GridDev &g, const ModelTables &m, cudaStream_t st, const Bp &b = Bp{});
 // per-octant (eps - mu0, G0 prefactor) into g.gk
 cudaError_t launch_gk_table(const GridDev &g, double mu0, double T, cudaStream_t st, const Bp &b = Bp{});
 cudaError_t launch_gslice(const GridDev &g, double *Grt, double mu0, double T, cudaStream_t st);
@@ -273,6 +284,8 @@ struct CondDev {
 size_t cond_col_words();
 cudaError_t cond_blocks(const GridDev &g, int *blocks);
 // the (eps - mu0, A, B) table of the h and f0 slices into c.tab
+// d eps/d kx, d2 eps/d kx2 on the K4 points, the second on the kx = 0, pi lines
+cudaError_t launch_cond_model(const GridDev &g, const CondDev &c, double tp, double tpp, double t3, cudaStream_t st);
 cudaError_t launch_cond_table(const GridDev &g, const CondDev &c, double mu0, double T, cudaStream_t st);
 // table + h V, f0 V slices + end conditions (fact = U (3 Usp + Uch)/4)
 cudaError_t launch_cond_slices(const GridDev &g, const CondDev &c, const double *V, const double *dtau_chirt0,
@@ -353,6 +366,8 @@ cudaError_t launch_cond_lines_bwd(const GridDev &g, const CondDev &c, const AdjD
 cudaError_t launch_cond_slices_bwd(const GridDev &g, const CondDev &c, const AdjDev &a, const double *V,
                                    const double *dchirt0, double mu0, double T, double fact4, double dmu0_2,
                                    cudaStream_t st);
+// the sums over rows [r0, r1) of a.part -> out[kAdjW], in a fixed order
+cudaError_t launch_adj_sums(const AdjDev &a, int r0, int r1, double *out, cudaStream_t st);
 // lam = -(d L / d mu) / (d traceDiffG / d mu)
 cudaError_t launch_sigbar(const GridDev &g, const CondDev &c, const AdjDev &a, const double2 *S, const double *s2,
                           const double *s3, const double *s4, const double *sinf, double mu0, double mu, double lam,
