@@ -369,7 +369,7 @@ int tpsc_pade_batch(tpsc_ctx *ctx, int nf, int Nn, const double *x, const double
  * be NULL): host wall time of the solves, device idle at both ends.  The
  * context's own model and grids are not changed. */
 int tpsc_solve_points(tpsc_ctx *ctx, int npts, const double *params, double *results, int *status, double *ms);
-/* Streams tpsc_solve_points spreads its groups over (1..4, default 2), the
+/* Streams tpsc_solve_points spreads its groups over (1..4, default 4), the
  * largest first onto the least loaded; each group's cooperative root searches
  * then take 2 blocks per SM / n. */
 int tpsc_set_group_streams(tpsc_ctx *ctx, int n);

@@ -226,7 +226,9 @@ struct tpsc_ctx {
     long long graph_kernels = 0;  // in the graph of the last captured or replayed solve
     long long graph_replays = 0, graph_captures = 0;
     std::map<std::pair<int, int>, Group *> groups;  // tpsc_solve_points' shape groups
-    int group_streams = 2;                          // streams the groups are spread over (1..4)
+    // streams the groups are spread over (1..4); 64 points of a sweep, 18 shapes, on 1, 2, 3, 4 of
+    // them: 11.4, 10.3, 8.8, 7.9 ms (a group of few small points leaves most of the GPU idle)
+    int group_streams = 4;
     cudaStream_t gst[2] = {nullptr, nullptr};       // the third and fourth (st, st2 are the first two)
     std::string err;
 };
@@ -2093,9 +2095,9 @@ int tpsc_solve_points(tpsc_ctx *ctx, int npts, const double *params, double *res
     const auto t0 = std::chrono::steady_clock::now();
     std::string first_msg;
     // every group queued without a wait (the host builds the next group's
-    // tables while the device runs the previous ones), largest first, on two
-    // streams by least queued work (a group's root searches then take half
-    // of the resident grid, so that both streams' fit on the GPU together); a
+    // tables while the device runs the previous ones), largest first, on
+    // group_streams streams by least queued work (a group's root searches then take that
+    // part of the resident grid, so that all streams' fit on the GPU together); a
     // shape with more than kGroupMax points waits for its previous chunk
     // before its staging buffers are refilled
     struct Chunk {

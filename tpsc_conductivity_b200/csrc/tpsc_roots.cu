@@ -442,29 +442,31 @@ __global__ void __launch_bounds__(kRootThreads) k_sumrule_roots(SumRootArgs a) {
 // point constants live in shared memory and Tr Sigma G0, its Hartree part and
 // G0 share one reciprocal per (k, n), so that two CTAs fit on an SM.
 //
-// Blocks 0 .. nblk-1 take one column block each over the stored frequencies;
-// the four columns of a row are formed without a branch (a padding column
-// has weight 0 and finite stand-in values), so that their chains interleave.
-// Blocks nblk .. nblk + ceil(nblk / 2) - 1 take the tail, one warp per
-// column, away from the Sigma stream.  Per-block partials (block_store).
+// Blocks 0 .. take per_s column blocks each over the stored frequencies, their rows
+// as one sequence; the four columns of a row are formed without a branch (a padding
+// column has weight 0 and finite stand-in values), so that their chains interleave.
+// The blocks after them take the tail, half a warp per column and per_t columns one
+// after the other, away from the Sigma stream.  Per-block partials (block_store).
+// The reduction of a block's kSigmaMomNV sums and, below 256 frequencies, the threads
+// without a row were most of a small-cutoff point's time at one column block per block
+// and one tail column per warp: at 64 points of a sweep (129 lines, 64 to 1024
+// frequencies) 1731 us for its 18 groups, against 960 (256^2 x 4096: 170 -> 149).
 constexpr int kMuMomF64 = 4;
 constexpr int kTailR = 28;           // terms of the tail power series (needs kMuMomP + kTailR < kTailP)
 constexpr double kTailRatio = 0.05;  // series when rho / w_NO < this: terms below 0.05^28 (~1e-36) relative
 static_assert(kMuMomP + kTailR < kTailP, "tail power sums too short");
 constexpr int kMomThreads = 256;
-constexpr int kMomTailCols = kMomThreads / 32;  // columns of a tail block
-
-__host__ __device__ constexpr int sigma_moment_tail_blocks(int nblk) {
-    return (4 * nblk + kMomTailCols - 1) / kMomTailCols;
-}
+constexpr int kMomTailCols = kMomThreads / 16;  // columns of a tail block at a time
+constexpr int kMomPerMax = 32;                  // column blocks of a block
+constexpr int kMomRows = 8;                     // rows of a thread (32 terms, as the FP32 sums allow)
 
 __global__ void __launch_bounds__(kMomThreads, 2)
     k_sigma_moments(const double2 *__restrict__ S, const double *__restrict__ s2, const double *__restrict__ s3,
                     const double *__restrict__ s4, const double *__restrict__ sinfp, const double *__restrict__ ek,
                     const double *__restrict__ w16, const double *__restrict__ tailP, int nw0, double mu0,
-                    double T, double nk02, int jc, int nblk, double *partial, Bp b) {
+                    double T, double nk02, int jc, int nblk, int per_s, int per_t, double *partial, Bp b) {
     constexpr int NV = kSigmaMomNV, P64 = kMuMomF64, P32 = kMuMomP - kMuMomF64;
-    __shared__ double cw[4], cx[4], c2[4], c3[4];
+    __shared__ double cw[4 * kMomPerMax], cx[4 * kMomPerMax], c2[4 * kMomPerMax], c3[4 * kMomPerMax];
     __shared__ __align__(16) double2 s_row[2][kMomThreads][4];  // two stages of 64-byte Sigma rows
     S = at(S, b.arena);
     s2 = at(s2, b.arena);
@@ -477,7 +479,7 @@ __global__ void __launch_bounds__(kMomThreads, 2)
     mu0 = bpar(b, kPpMu0, mu0);
     T = bpar(b, kPpT, T);
     jc = (int)bpar(b, kPpJc, (double)jc);
-    const int blk = blockIdx.x, NO = nw0 / 2;
+    const int NO = nw0 / 2, nsb = (nblk + per_s - 1) / per_s;  // blocks of the stored frequencies
     const double sinf = sinfp[0];
     const double pt = 3.141592653589793 * T;
     double tsg = 0.0, har = 0.0, g0 = 0.0;
@@ -513,10 +515,10 @@ __global__ void __launch_bounds__(kMomThreads, 2)
         const double zx = -x - rS, zy = wn - iS;
         moments_rr(zx, zy, 1.0 / (zx * zx + zy * zy), x, w, inv);
     };
-    double fermi = 0.0;  // traceSelfG's Fermi-function term, threads 0..3 of a stored-frequency block
-    if (blk < nblk) {
-        const int o0 = 4 * blk;
-        if (threadIdx.x < 4) {
+    double fermi = 0.0;  // traceSelfG's Fermi-function term of a stored-frequency block's columns
+    if ((int)blockIdx.x < nsb) {
+        const int blk0 = blockIdx.x * per_s, o0 = 4 * blk0, ncb = min(per_s, nblk - blk0), ncol = 4 * ncb;
+        if ((int)threadIdx.x < ncol) {
             // a padding column: weight 0, x = 1 and Sigma's coefficients 0,
             // so that |z| and w_n^2 + x^2 stay away from 0 and its terms are 0
             const int c = threadIdx.x;
@@ -528,20 +530,22 @@ __global__ void __launch_bounds__(kMomThreads, 2)
             c3[c] = ok ? s3[o0 + c] : 0.0;
         }
         __syncthreads();
-        // this thread's Sigma rows j = tid + 256 i through two shared-memory
-        // stages: row i + 1 is copied (cp.async, 4 x 16 bytes) while row i is
-        // formed; each thread reads back only its own copies
-        const double2 *row = S + (size_t)blk * 4 * NO;
+        // this thread's Sigma rows tid + 256 i of the block's column blocks through
+        // two shared-memory stages: row i + 1 is copied (cp.async, 4 x 16 bytes)
+        // while row i is formed; each thread reads back only its own copies
+        const double2 *row = S + (size_t)blk0 * 4 * NO;
+        const int nrow = ncb * NO, lno = 31 - __clz(NO);  // NO is a power of two
         auto issue = [&](int jj, int st) {
 #pragma unroll
             for (int c = 0; c < 4; ++c) cp_async16(&s_row[st][threadIdx.x][c], row + 4 * (size_t)jj + c);
             asm volatile("cp.async.commit_group;\n" ::: "memory");
         };
-        if ((int)threadIdx.x < NO) issue(threadIdx.x, 0);
-        for (int j = threadIdx.x, st = 0; j < NO; j += blockDim.x, st ^= 1) {
+        if ((int)threadIdx.x < nrow) issue(threadIdx.x, 0);
+        for (int i = threadIdx.x, st = 0; i < nrow; i += blockDim.x, st ^= 1) {
+            const int j = i & (NO - 1), cb = 4 * (i >> lno);
             const double wn = (2 * j + 1) * pt, i1 = 1.0 / wn;
-            if (j + (int)blockDim.x < NO) {
-                issue(j + blockDim.x, st ^ 1);
+            if (i + (int)blockDim.x < nrow) {
+                issue(i + blockDim.x, st ^ 1);
                 asm volatile("cp.async.wait_group 1;\n" ::: "memory");
             } else {
                 asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -551,10 +555,10 @@ __global__ void __launch_bounds__(kMomThreads, 2)
             if (j >= jc) {
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    const double w = cw[c], x = cx[c];
+                    const double w = cw[cb + c], x = cx[cb + c];
                     const double2 s = w != 0.0 ? sv[c] : make_double2(0.0, 0.0);
                     double rS, iS;
-                    sigma_full(i1, sinf, c2[c], c3[c], s, rS, iS);
+                    sigma_full(i1, sinf, c2[cb + c], c3[cb + c], s, rS, iS);
                     // one reciprocal for 1/(w_n^2 + x^2) and 1/|z|^2
                     const double b = wn * wn + x * x;
                     const double zx = -x - rS, zy = wn - iS, a = zx * zx + zy * zy;
@@ -566,10 +570,10 @@ __global__ void __launch_bounds__(kMomThreads, 2)
             } else {
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
-                    const double w = cw[c], x = cx[c];
+                    const double w = cw[cb + c], x = cx[cb + c];
                     const double2 s = w != 0.0 ? sv[c] : make_double2(0.0, 0.0);
                     double rS, iS;
-                    sigma_full(i1, sinf, c2[c], c3[c], s, rS, iS);
+                    sigma_full(i1, sinf, c2[cb + c], c3[cb + c], s, rS, iS);
                     const double inv = 1.0 / (wn * wn + x * x);
                     tsg += w * inv * (rS * (-x) + iS * wn);
                     har += w * inv;
@@ -577,7 +581,7 @@ __global__ void __launch_bounds__(kMomThreads, 2)
             }
         }
         // traceSelfG's Fermi-function term per octant point
-        if (threadIdx.x < 4) {
+        if ((int)threadIdx.x < ncol) {
             const int c = threadIdx.x;
             const double w8 = 0.5 * cw[c];
             if (w8 != 0.0) {
@@ -591,7 +595,7 @@ __global__ void __launch_bounds__(kMomThreads, 2)
             }
         }
     } else {
-        // The tail n = NO .. 2 NO (asymptotic Sigma), warp `warp` for column o:
+        // The tail n = NO .. 2 NO (asymptotic Sigma), half a warp for column o:
         // with u = 1/(i w_n), z^-1 = u / (1 - q(u)), q(u) = x u + Sinf u^2 +
         // C2 u^3 + C3 u^4 + C4 u^5 (real coefficients), and h^(p) the
         // coefficients of (1 - q)^-p,
@@ -599,76 +603,99 @@ __global__ void __launch_bounds__(kMomThreads, 2)
         //   sum_tail Re 1/(i w_n - x) = -x sum_k (-x^2)^k P_(2k+2),
         // P_p = sum_tail w_n^-p (tailP).  (1 - q)^-p obeys H' (1 - q) = p q' H,
         // so R h_R = sum_{s=1..5} q_s h_(R-s) (R - s + p s),   h_0 = 1:
-        // lane p - 1 runs the recurrence of moment m = p - 1 in registers.  The
-        // terms fall like (rho / w_NO)^r, rho a bound on q's root radius; above
-        // kTailRatio the warp sums term by term.
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int o = (blk - nblk) * kMomTailCols + warp;
-        const double w = o < 4 * nblk ? __ldg(&w16[o]) : 0.0;
-        if (w != 0.0) {
-            const double x = __ldg(&ek[o]) - mu0;
-            const double q1 = x, q2 = sinf, q3 = __ldg(&s2[o]), q4 = __ldg(&s3[o]), q5 = __ldg(&s4[o]);
-            const double rho = fabs(x) + sqrt(fabs(sinf)) + cbrt(fabs(q3)) + sqrt(sqrt(fabs(q4))) + pow(fabs(q5), 0.2);
-            const double w_no = (2 * NO + 1) * pt;
-            if (rho < kTailRatio * w_no) {
-                double re = 0.0, im = 0.0;
-                if (lane < kMuMomP) {
-                    const double p = lane + 1;
-                    // h_(R-1) .. h_(R-5) in a register window
-                    double h1 = 1.0, h2 = 0.0, h3 = 0.0, h4 = 0.0, h5 = 0.0;
-                    // r = 0 term: (-i)^p P_p
-                    auto add = [&](int k, double h) {
-                        const double t = h * __ldg(&tailP[k]);
-                        switch (k & 3) {
-                            case 0: re += t; break;
-                            case 1: im -= t; break;
-                            case 2: re -= t; break;
-                            default: im += t; break;
-                        }
-                    };
-                    add(lane + 1, 1.0);
-                    // unrolled: 1 / R is a constant of each step
+        // lane p - 1 of the half runs the recurrence of moment m = p - 1 in registers
+        // and keeps the sum over its columns.  The terms fall like (rho / w_NO)^r, rho
+        // a bound on q's root radius; above kTailRatio the warp sums term by term.
+        static_assert(kMuMomP < 16, "the moments and G0 of a column in half a warp");
+        const int lane = threadIdx.x & 31, sub = lane & 15, half = threadIdx.x >> 4;
+        const double w_no = (2 * NO + 1) * pt;
+        double sre = 0.0, sim = 0.0;  // lanes sub < kMuMomP: w C_sub, sub = kMuMomP: w G0
+        for (int r = 0; r < per_t; ++r) {
+            const int o = ((blockIdx.x - nsb) * per_t + r) * kMomTailCols + half;
+            const double w = o < 4 * nblk ? __ldg(&w16[o]) : 0.0;
+            double x = 0.0, q3 = 0.0, q4 = 0.0, q5 = 0.0;
+            const double q2 = sinf;
+            bool series = true;
+            if (w != 0.0) {
+                x = __ldg(&ek[o]) - mu0;
+                q3 = __ldg(&s2[o]);
+                q4 = __ldg(&s3[o]);
+                q5 = __ldg(&s4[o]);
+                const double rho =
+                    fabs(x) + sqrt(fabs(sinf)) + cbrt(fabs(q3)) + sqrt(sqrt(fabs(q4))) + pow(fabs(q5), 0.2);
+                series = rho < kTailRatio * w_no;
+                if (series) {
+                    double re = 0.0, im = 0.0;
+                    if (sub < kMuMomP) {
+                        const double p = sub + 1;
+                        // h_(R-1) .. h_(R-5) in a register window
+                        double h1 = 1.0, h2 = 0.0, h3 = 0.0, h4 = 0.0, h5 = 0.0;
+                        // r = 0 term: (-i)^p P_p
+                        auto add = [&](int k, double h) {
+                            const double t = h * __ldg(&tailP[k]);
+                            switch (k & 3) {
+                                case 0: re += t; break;
+                                case 1: im -= t; break;
+                                case 2: re -= t; break;
+                                default: im += t; break;
+                            }
+                        };
+                        add(sub + 1, 1.0);
+                        // unrolled: 1 / R is a constant of each step
 #pragma unroll
-                    for (int R = 1; R <= kTailR; ++R) {
-                        const double hR = (q1 * h1 * (R - 1 + p) + q2 * h2 * (R - 2 + 2 * p) +
-                                           q3 * h3 * (R - 3 + 3 * p) + q4 * h4 * (R - 4 + 4 * p) +
-                                           q5 * h5 * (R - 5 + 5 * p)) *
-                                          (1.0 / R);
-                        add(lane + 1 + R, hR);
-                        h5 = h4;
-                        h4 = h3;
-                        h3 = h2;
-                        h2 = h1;
-                        h1 = hR;
-                    }
-                } else if (lane == kMuMomP) {
-                    // G0: -x sum_k (-x^2)^k P_(2k+2)
-                    double xp = 1.0;
-                    for (int k = 0; 2 * k + 2 < kTailP; ++k, xp *= -x * x) re += xp * __ldg(&tailP[2 * k + 2]);
-                    re *= -x;
-                }
-#pragma unroll
-                for (int m = 0; m < kMuMomP; ++m) {
-                    const double rm = __shfl_sync(0xffffffffu, re, m), imm = __shfl_sync(0xffffffffu, im, m);
-                    if (lane == 0) {
-                        if (m < P64) {
-                            m64[2 * m] += w * rm;
-                            m64[2 * m + 1] += w * imm;
-                        } else {
-                            m32[2 * (m - P64)] += (float)(w * rm);
-                            m32[2 * (m - P64) + 1] += (float)(w * imm);
+                        for (int R = 1; R <= kTailR; ++R) {
+                            const double hR = (x * h1 * (R - 1 + p) + q2 * h2 * (R - 2 + 2 * p) +
+                                               q3 * h3 * (R - 3 + 3 * p) + q4 * h4 * (R - 4 + 4 * p) +
+                                               q5 * h5 * (R - 5 + 5 * p)) *
+                                              (1.0 / R);
+                            add(sub + 1 + R, hR);
+                            h5 = h4;
+                            h4 = h3;
+                            h3 = h2;
+                            h2 = h1;
+                            h1 = hR;
                         }
+                    } else if (sub == kMuMomP) {
+                        // G0: -x sum_k (-x^2)^k P_(2k+2)
+                        double xp = 1.0;
+                        for (int k = 0; 2 * k + 2 < kTailP; ++k, xp *= -x * x) re += xp * __ldg(&tailP[2 * k + 2]);
+                        re *= -x;
+                    }
+                    sre += w * re;
+                    sim += w * im;
+                }
+            }
+            // the columns of the warp that the series does not hold for
+            const unsigned slow = __ballot_sync(0xffffffffu, !series);
+            for (int hf = 0; hf < 2; ++hf)
+                if (slow >> (16 * hf) & 1u) {
+                    const double wc = __shfl_sync(0xffffffffu, w, 16 * hf), xc = __shfl_sync(0xffffffffu, x, 16 * hf);
+                    const double a3 = __shfl_sync(0xffffffffu, q3, 16 * hf), a4 = __shfl_sync(0xffffffffu, q4, 16 * hf),
+                                 a5 = __shfl_sync(0xffffffffu, q5, 16 * hf);
+                    for (int t = lane; t <= NO; t += 32) {
+                        const double wn = (2 * (NO + t) + 1) * pt, i1 = 1.0 / wn, i2 = i1 * i1;
+                        moments(wn, -a3 * i2 + a5 * i2 * i2, -sinf * i1 + a4 * i2 * i1, xc, wc,
+                                1.0 / (wn * wn + xc * xc));
                     }
                 }
-                const double gt = __shfl_sync(0xffffffffu, re, kMuMomP);
-                if (lane == 0) g0 += w * gt;
-            } else {
-                for (int t = lane; t <= NO; t += 32) {
-                    const double wn = (2 * (NO + t) + 1) * pt, i1 = 1.0 / wn, i2 = i1 * i1;
-                    moments(wn, -q3 * i2 + q5 * i2 * i2, -sinf * i1 + q4 * i2 * i1, x, w, 1.0 / (wn * wn + x * x));
+        }
+        sre += __shfl_down_sync(0xffffffffu, sre, 16);
+        sim += __shfl_down_sync(0xffffffffu, sim, 16);
+#pragma unroll
+        for (int m = 0; m < kMuMomP; ++m) {
+            const double rm = __shfl_sync(0xffffffffu, sre, m), imm = __shfl_sync(0xffffffffu, sim, m);
+            if (lane == 0) {
+                if (m < P64) {
+                    m64[2 * m] += rm;
+                    m64[2 * m + 1] += imm;
+                } else {
+                    m32[2 * (m - P64)] += (float)rm;
+                    m32[2 * (m - P64) + 1] += (float)imm;
                 }
             }
         }
+        const double gt = __shfl_sync(0xffffffffu, sre, kMuMomP);
+        if (lane == 0) g0 += gt;
     }
     double acc[NV];
     acc[0] = tsg * T / nk02;
@@ -1205,11 +1232,24 @@ cudaError_t root_grid(K kernel, int *grid, int cap) {
 cudaError_t launch_sigma_moments(const GridDev &g, const double2 *S, const double *s2, const double *s3,
                                  const double *s4, const double *sinf, double mu0, double T, int jc, Reduce r,
                                  cudaStream_t st, const Bp &b) {
-    const int nblk = g.n8p / 4, nb = nblk + sigma_moment_tail_blocks(nblk);
+    // as many column blocks (8 rows a thread at most) and tail columns per block as
+    // leave four blocks per SM: fewer reductions and, at small cutoffs, full blocks;
+    // at 129 lines and more than 1024 frequencies, or one point of 65 lines and
+    // less, one each, as a grid without its last blocks would be slower
+    const int nblk = g.n8p / 4, fill = 4 * 148;
+    auto per = [&](int units, int most) {
+        int k = 1;
+        while (2 * k <= most && (long long)units * b.P >= 2LL * k * fill) k *= 2;
+        return k;
+    };
+    const int ncols = (4 * nblk + kMomTailCols - 1) / kMomTailCols;  // tail columns, in blocks of kMomTailCols
+    const int per_s = per(nblk, std::min(kMomPerMax, std::max(1, kMomRows * kMomThreads / (g.nw0 / 2))));
+    const int per_t = per(ncols, 8);
+    const int nb = (nblk + per_s - 1) / per_s + (ncols + per_t - 1) / per_t;
     if (nb > kMaxBlocks) return cudaErrorInvalidValue;
     const double nk02 = 4.0 * (g.nbk - 1) * (g.nbk - 1);
     k_sigma_moments<<<dim3(nb, 1, b.P), kMomThreads, 0, st>>>(S, s2, s3, s4, sinf, g.ek, g.w16, g.tailP, g.nw0, mu0,
-                                                               T, nk02, jc, nblk, r.partial, b);
+                                                               T, nk02, jc, nblk, per_s, per_t, r.partial, b);
     cudaError_t e = launched();
     if (e != cudaSuccess) return e;
     return finish<kSigmaMomNV>(r, nb, 0.0, st, b);
