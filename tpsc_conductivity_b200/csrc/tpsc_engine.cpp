@@ -1322,7 +1322,7 @@ tpsc_ctx *tpsc_create(int device, int *status) {
                                                  sizeof(double))) != cudaSuccess)
         return bad(e);
     if ((e = cudaMalloc(&ctx->redm.result, 32 * sizeof(double))) != cudaSuccess) return bad(e);
-    if ((e = cudaMalloc(&ctx->roots.partial, 2 * kRootVals * kRootMaxBlocks * sizeof(double))) != cudaSuccess)
+    if ((e = cudaMalloc(&ctx->roots.partial, kRootPartial * sizeof(double))) != cudaSuccess)
         return bad(e);
     if ((e = cudaMalloc(&ctx->roots.bar, 8 * sizeof(unsigned))) != cudaSuccess) return bad(e);
     if ((e = cudaMemsetAsync(ctx->roots.bar, 0, 8 * sizeof(unsigned), ctx->st)) != cudaSuccess) return bad(e);

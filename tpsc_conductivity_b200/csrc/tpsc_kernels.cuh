@@ -200,8 +200,10 @@ cudaError_t launch_trace_self_G(const GridDev &g, const double2 *S, const double
 // ---- the Newton form's root searches on the device (tpsc_roots.cu) ----------
 constexpr int kRootMaxBlocks = 1024;
 constexpr int kRootVals = 3;  // per-block partials of an evaluation: value and two derivatives
+constexpr int kRootPartial = 3 * kRootVals * kRootMaxBlocks;
 struct RootScratch {
-    double *partial = nullptr;  // [2 kRootVals kRootMaxBlocks]: two parities
+    double *partial = nullptr;  // [kRootPartial]: two parities of (value, two derivatives) per block, or three
+                                // sets of one value per column block
     unsigned *bar = nullptr;    // [8]: arrivals, generation, error flag of the sum-rule search (0..2)
                                 //      and of the mu search (4..6)
     double *out = nullptr;      // [8] results

@@ -52,9 +52,16 @@ struct GridBar {
     __device__ bool sync() {
         __shared__ int s_ok;
         __syncthreads();
+        const int ok = sync_warp0();
+        if (threadIdx.x == 0) s_ok = ok;
+        __syncthreads();
+        return s_ok;
+    }
+    // by a block's first warp alone, for what its lane 0 has written: the result in lane 0
+    __device__ int sync_warp0() {
+        int ok = 1;
         ++gen;
         if (threadIdx.x == 0) {
-            int ok = 1;
             unsigned old;
             asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(bar) : "memory");
             if (old == gridDim.x - 1) {
@@ -76,10 +83,8 @@ struct GridBar {
                     }
                 }
             }
-            s_ok = ok;
         }
-        __syncthreads();
-        return s_ok;
+        return ok;
     }
 };
 
@@ -132,6 +137,7 @@ struct SumRootArgs {
     int *err;         // zero at launch
     double *out;      // Usp, Uch, evals_sp, evals_ch, ok_sp, ok_ch
     Bp b;             // batched launch: point blockIdx.z, blocks blockIdx.x of gridDim.x per point
+    int cached;  // (k_sumrule_zero) column blocks of a block whose rows are kept in its shared memory
 };
 
 // the value and its derivatives, each summed in a fixed order, into
@@ -719,6 +725,7 @@ struct MuRootArgs {
     int *err;
     double *out;  // mu, evals, ok, Tr Sigma G at mu
     Bp b;         // batched launch: point blockIdx.z
+    int cached;  // (k_mu_zero) as above, Sigma
 };
 
 // the four octant points of column block blk at frequency j of
@@ -1081,6 +1088,359 @@ __global__ void __launch_bounds__(kRootThreads, 2) k_mu_zero(MuRootArgs a) {
     }
 }
 
+// Up to kSlotBlocks column blocks: a column block's value goes to every block
+// through a slot that a warp of every block polls: one store and one load, where a
+// barrier and then a read take an atomic, a store and two loads, behind fences.  A slot
+// is two 64-bit words, each half of the value and the number of the evaluation: a word
+// is stored and loaded whole, so that no order between words or slots matters and the
+// accesses are relaxed (with an empty-slot value instead of the number the stores had to
+// release and the loads to acquire, and every kernel's L1 was emptied: 5% slower).  Two sets of slots in turn: a block
+// stores evaluation e + 2 after it has read all of e + 1, which every block stored
+// after it had read e.  kSlotCopies copies of a set, each for as many readers, as one
+// would be polled by every SM at once.  With more column blocks every block would
+// poll (and wait for) hundreds of slots: there the kernels above are faster
+// (537 column blocks: 348 and 324 us a search, with slots 373 and 355).
+constexpr int kSlotBlocks = 148, kSlotCopies = 8, kSlotStride = 160;
+static_assert(2 * 2 * kSlotCopies * kSlotStride <= kRootPartial && kSlotStride >= kSlotBlocks, "slots do not fit");
+__device__ __forceinline__ void slot_store(ulonglong2 *p, double x, unsigned n) {
+    const unsigned long long b = __double_as_longlong(x), t = (unsigned long long)n << 32;
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(t | (b >> 32)), "l"(t | (b & 0xffffffffu))
+                 : "memory");
+}
+// true when the slot holds evaluation n: x
+__device__ __forceinline__ bool slot_load(const ulonglong2 *p, unsigned n, double &x) {
+    unsigned long long h, l;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(h), "=l"(l) : "l"(p) : "memory");
+    x = __longlong_as_double((long long)(h << 32 | (l & 0xffffffffu)));
+    return (unsigned)(h >> 32) == n && (unsigned)(l >> 32) == n;
+}
+struct ZeroSlots {
+    ulonglong2 *base;  // [2][kSlotCopies][kSlotStride]
+    int nblk;
+    unsigned n;  // the evaluation, from 1
+    // (the first warp) all slots of evaluation 0, seen by every block
+    __device__ bool begin(double *base_, int nblk_, GridBar &bar) {
+        base = reinterpret_cast<ulonglong2 *>(base_);
+        nblk = nblk_;
+        n = 1;
+        if (threadIdx.x == 0)
+            for (int blk = blockIdx.x; blk < nblk; blk += gridDim.x)
+                for (int k = 0; k < 2 * kSlotCopies; ++k) slot_store(base + k * kSlotStride + blk, 0.0, 0);
+        return __shfl_sync(0xffffffffu, bar.sync_warp0(), 0);
+    }
+    __device__ ulonglong2 *slot(int copy, int blk) const {
+        return base + ((n & 1) * kSlotCopies + copy) * kSlotStride + blk;
+    }
+};
+
+// What the first warp asks of a block's threads: an evaluation of kind op at x, or the
+// end of the search.  Only that warp runs find_zero; with the search in every thread
+// its spilled state, 400 bytes a thread, moved at every evaluation.  The searches for
+// Usp and Uch and for mu: 180 and 118 us through barriers at 16^2 x 128, now 119 and
+// 78; at 32^2 x 512 224 and 138, now 147 and 61; at 64^2 x 1024 262 and 172, now 210
+// and 161 (an evaluation is then 3500 cycles of values, 5700 until the last of 141
+// blocks is read, 1400 of find_zero).
+struct ZeroCmd {
+    double x;
+    int op;
+};
+constexpr int kZeroDone = -1;
+
+// a block's share of the sum: share(blk) over its threads, in thread order, for each of
+// its column blocks -> the slots (the first warp)
+template <class F>
+__device__ __forceinline__ void block_values(int nblk, const ZeroSlots *zs, const F &share) {
+    __shared__ double red[kRootThreads / 32];
+    for (int blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
+        double v = share(blk);
+        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+        __syncthreads();
+        if (threadIdx.x < kSlotCopies) {
+            double x = 0.0;
+            for (int w = 0; w < kRootThreads / 32; ++w) x += red[w];
+            slot_store(zs->slot(threadIdx.x, blk), x, zs->n);
+        }
+        if (blk + (int)gridDim.x < nblk) __syncthreads();
+    }
+}
+
+// (the first warp, after block_values) the sum over the column blocks in block order,
+// the same in every block of the grid.  False: a wait ran out (bounded as the barrier's).
+__device__ __noinline__ bool slot_total(ZeroSlots &zs, GridBar &bar, double &total) {
+    const int nblk = zs.nblk, lane = threadIdx.x & 31;
+    const ulonglong2 *mine = zs.slot(blockIdx.x % kSlotCopies, 0);
+    constexpr int U = (kSlotBlocks + 31) / 32;
+    KSum acc;
+    bool ok = true, have[U];
+    double v[U];
+    unsigned long long t0 = 0;
+#pragma unroll
+    for (int u = 0; u < U; ++u) have[u] = lane + 32 * u >= nblk || slot_load(mine + lane + 32 * u, zs.n, v[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        if (lane + 32 * u >= nblk) continue;
+        for (unsigned i = 1; ok && !have[u]; ++i) {
+            have[u] = slot_load(mine + lane + 32 * u, zs.n, v[u]);
+            if (i % 64) continue;
+            const unsigned long long t = globaltimer_ns();
+            if (!t0) t0 = t;
+            if (*(volatile int *)bar.err || t - t0 > kBarrierNs) {
+                atomicExch(bar.err, 1);
+                ok = false;
+            }
+        }
+        acc.add(v[u]);
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    ++zs.n;
+    double x = acc.value();
+    for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
+    total = __shfl_sync(0xffffffffu, x, 0);
+    return ok;
+}
+
+// What a block keeps of its column blocks through a search: the chi0 rows (dynamic
+// shared memory, of the first a.cached) and, of its first kZeroTail column
+// blocks, the weights and the tail's power sums, which do not depend on U, with the
+// bound that decides for the series.  The polls' acquire loads empty L1, so that rows
+// read from there cost an L2 trip per evaluation.
+struct SlotTail {
+    double S[kZeroTail][4][kTailM], w[kZeroTail][4], cmax[kZeroTail][4];
+};
+
+__device__ __noinline__ void sumrule_values(const SumRootArgs &a, const SlotTail &zt, const double4 *rows, double Uv,
+                                            double sgn, const ZeroSlots *zs) {
+    const double hu = sgn * Uv / 2.0;
+    block_values(a.nblk, zs, [&](int blk) {
+        const int lb = (blk - (int)blockIdx.x) / (int)gridDim.x;
+        double ww[4];
+        bool kept = lb < kZeroTail;
+        if (kept) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) ww[c] = zt.w[lb][c];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (ww[c] != 0.0 && !(fabs(hu) * zt.cmax[lb][c] < kTailSeriesMax)) kept = false;
+        } else {
+            const double4 w = reinterpret_cast<const double4 *>(a.w16)[blk];
+            ww[0] = w.x;
+            ww[1] = w.y;
+            ww[2] = w.z;
+            ww[3] = w.w;
+        }
+        double v, dv, tv, tdv;
+        const double4 *col = lb < a.cached ? rows + (size_t)lb * a.nb : a.chiq + (size_t)blk * a.nb;
+        sumrule_stored<false>(col, ww, 0, a.nb, a.nb, hu, v, dv);
+        auto series = [&](int c, double ca, double cb, double &f, double &df) {
+            if (lb >= kZeroTail) {
+                tail_series(ca, cb, hu, a.tailq, f, df);
+                return;
+            }
+            f = df = 0.0;
+            double hm = 1.0;
+            for (int m = 1; m <= kTailM; ++m) {
+                f += (-hu) * hm * zt.S[lb][c][m - 1];
+                hm *= -hu;
+            }
+        };
+        if (kept) {
+            // every column by its series, thread c column c
+            tv = 0.0;
+            if (threadIdx.x < 4 && zt.w[lb][threadIdx.x] != 0.0) {
+                double f, df;
+                series(threadIdx.x, 0.0, 0.0, f, df);
+                tv += zt.w[lb][threadIdx.x] * f;
+            }
+        } else {
+            sumrule_tail(a.cinf, a.cinf2, ww, blk, a.nb, hu, sgn, a.T, tv, tdv, series);
+        }
+        return a.scale * (v + tv);
+    });
+}
+
+// Usp and Uch as k_sumrule_zero, through slots
+__global__ void __launch_bounds__(kRootThreads, 2) k_sumrule_slots(SumRootArgs a) {
+    const double hi_sp = a.chi0max ? 2.0 / a.chi0max[0] - a.hi_off : a.hi_sp;
+    const double n = a.n, nsr = a.nsr, U = a.U;
+    __shared__ SlotTail zt;
+    extern __shared__ __align__(16) double4 zrows[];
+    const double tw = 2.0 * 3.141592653589793 * a.T, wn1 = a.nb * tw, x1 = 1.0 / (wn1 * wn1);
+    for (int i = threadIdx.x; i < 4 * kZeroTail; i += blockDim.x) {
+        const int o = 4 * (blockIdx.x + (i >> 2) * gridDim.x) + (i & 3);
+        if (o >= 4 * a.nblk) continue;
+        const double w = a.w16[o];
+        zt.w[i >> 2][i & 3] = w;
+        if (o >= a.n8) continue;
+        const double ca = a.cinf[o], cb = a.cinf2[o];
+        zt.cmax[i >> 2][i & 3] = fabs(ca) * x1 + fabs(cb) * x1 * x1;
+        tail_sums(ca, cb, a.tailq, zt.S[i >> 2][i & 3]);
+    }
+    for (int blk = blockIdx.x, lb = 0; blk < a.nblk && lb < a.cached; blk += gridDim.x, ++lb)
+        for (int j = threadIdx.x; j < a.nb; j += blockDim.x)
+            zrows[(size_t)lb * a.nb + j] = a.chiq[(size_t)blk * a.nb + j];
+    __syncthreads();
+    __shared__ ZeroCmd cmd;
+    if (threadIdx.x >= 32) {
+        for (;;) {
+            __syncthreads();
+            if (cmd.op == kZeroDone) return;
+            sumrule_values(a, zt, zrows, cmd.x, cmd.op == 0 ? -1.0 : 1.0, nullptr);
+        }
+    }
+    auto ask = [&](int op, double x) {
+        if (threadIdx.x == 0) {
+            cmd.op = op;
+            cmd.x = x;
+        }
+        __syncthreads();
+    };
+    GridBar bar(a.bar, a.err);
+    ZeroSlots zs;
+    bool ok = zs.begin(a.partial, a.nblk, bar);
+    double Usp = 0.0;
+#pragma unroll 1
+    for (int phase = 0; ok && phase < 2; ++phase) {
+        auto f = [&](double Uv, double &y) -> bool {
+            double tr;
+            ask(phase, Uv);
+            sumrule_values(a, zt, zrows, Uv, phase == 0 ? -1.0 : 1.0, &zs);
+            if (!slot_total(zs, bar, tr)) return false;
+            // chi::sum_rule_sp (src/chi.cpp:833-836) and sum_rule_ch (840-843),
+            // rounded as the host's expressions
+            const Rn base = Rn(tr) + Rn(n) - Rn(n) * Rn(n) / Rn(2.0);
+            if (phase == 0)
+                y = (base - Rn(nsr) + Rn(Uv) * Rn(nsr) * Rn(nsr) / (Rn(2.0) * Rn(U))).v;
+            else
+                y = (base - (Rn(nsr) + Rn(Usp) * Rn(nsr) * Rn(nsr) / (Rn(2.0) * Rn(U)) - Rn(nsr) * Rn(nsr))).v;
+            return true;
+        };
+        const double init[3] = {phase == 0 ? U / 2.0 : 0.0, 0.0, phase == 0 ? hi_sp : 1000.0 * U};
+        double root = 0.0;
+        int nev;
+        bool gone;
+        ok = find_zero(f, init, &root, nullptr, &nev, &gone);
+        if (phase == 0) Usp = root;
+        if (!gone && blockIdx.x == 0 && threadIdx.x == 0) {
+            a.out[phase] = root;
+            a.out[2 + phase] = nev;
+            a.out[4 + phase] = ok;
+        }
+        ok = ok && !gone;
+    }
+    ask(kZeroDone, 0.0);
+}
+
+// zrow: Sigma of the block's column blocks at every frequency of the trace, [lb][4][nw0 + 1]
+// (stored ones and the asymptotic tail), of those kept in shared memory
+__device__ __noinline__ void trace_diff_values(const MuRootArgs &a, const double2 *zrow, double pmu,
+                                               const ZeroSlots *zs) {
+    block_values(a.nblk, zs, [&](int blk) {
+        double v = 0.0, dv = 0.0;
+        const int lb = (blk - (int)blockIdx.x) / (int)gridDim.x;
+        if (lb >= a.cached) {
+            trace_diff_block<false>(a.S, a.s2, a.s3, a.s4, a.sinf, a.ek, a.w16, blk, a.nw0, a.mu0, pmu, a.T, a.nw0 / 2,
+                                    1, v, dv);
+            return v;
+        }
+        // trace_diff_block's terms in its order
+        const int NO = a.nw0 / 2, R = a.nw0 + 1;
+        const double2 *z = zrow + (size_t)lb * 4 * R;
+        const double pt = 3.141592653589793 * a.T;
+        double ww[4], e[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            ww[c] = a.w16[4 * blk + c];
+            e[c] = ww[c] != 0.0 ? a.ek[4 * blk + c] : 0.0;
+        }
+        auto row = [&](int j) {
+            const double wn = (2 * j + 1) * pt;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                if (ww[c] == 0.0) continue;
+                const double2 q = z[c * R + j];
+                trdiff_term(wn, q.x, q.y, e[c], a.mu0, pmu, ww[c], v, dv);
+            }
+        };
+        for (int j = threadIdx.x; j < NO; j += blockDim.x) row(j);
+        for (int t = threadIdx.x; t <= NO; t += blockDim.x) row(NO + t);
+        return v;
+    });
+}
+
+// mu and Tr Sigma G as k_mu_zero, through slots
+__global__ void __launch_bounds__(kRootThreads, 2) k_mu_slots(MuRootArgs a) {
+    extern __shared__ __align__(16) double2 zself[];
+    if (a.cached) {
+        const int NO = a.nw0 / 2, R = a.nw0 + 1;
+        const double sinf = a.sinf[0], pt = 3.141592653589793 * a.T;
+        for (int blk = blockIdx.x, lb = 0; blk < a.nblk && lb < a.cached; blk += gridDim.x, ++lb)
+            for (int i = threadIdx.x; i < 4 * R; i += blockDim.x) {
+                const int j = i >> 2, c = i & 3, o = 4 * blk + c;
+                double rS = 0.0, iS = 0.0;
+                if (a.w16[o] != 0.0) {
+                    const double wn = (2 * j + 1) * pt, i1 = 1.0 / wn, i2 = i1 * i1;
+                    if (j < NO) {
+                        sigma_full(i1, sinf, a.s2[o], a.s3[o], a.S[((size_t)blk * NO + j) * 4 + c], rS, iS);
+                    } else {
+                        rS = -a.s2[o] * i2 + a.s4[o] * i2 * i2;
+                        iS = -sinf * i1 + a.s3[o] * i2 * i1;
+                    }
+                }
+                zself[((size_t)lb * 4 + c) * R + j] = make_double2(rS, iS);
+            }
+        __syncthreads();
+    }
+    __shared__ ZeroCmd cmd;
+    auto values = [&](int op, double x, const ZeroSlots *zs) {
+        if (op == 0) {
+            trace_diff_values(a, zself, x, zs);
+            return;
+        }
+        block_values(a.nblk, zs, [&](int blk) {
+            return trace_self2_block<false>(a.S, a.s2, a.s3, a.sinf, a.ek, a.w16, blk, a.nw0, x, a.T, a.nk02);
+        });
+    };
+    if (threadIdx.x >= 32) {
+        for (;;) {
+            __syncthreads();
+            if (cmd.op == kZeroDone) return;
+            values(cmd.op, cmd.x, nullptr);
+        }
+    }
+    auto ask = [&](int op, double x) {
+        if (threadIdx.x == 0) {
+            cmd.op = op;
+            cmd.x = x;
+        }
+        __syncthreads();
+    };
+    GridBar bar(a.bar, a.err);
+    ZeroSlots zs;
+    bool ok = zs.begin(a.partial, a.nblk, bar), gone = !ok;
+    auto f = [&](double pmu, double &y) -> bool {
+        ask(0, pmu);
+        trace_diff_values(a, zself, pmu, &zs);
+        return slot_total(zs, bar, y);
+    };
+    const double init[3] = {0.0, -10.0, 10.0}, lims[2] = {-20.0, 20.0};
+    double mu = 0.0, tr = 0.0;
+    int nev = 0;
+    if (ok) ok = find_zero(f, init, &mu, lims, &nev, &gone);
+    if (ok && !gone) {
+        ask(1, mu);
+        values(1, mu, &zs);
+        gone = !slot_total(zs, bar, tr);
+    }
+    if (!gone && blockIdx.x == 0 && threadIdx.x == 0) {
+        a.out[0] = mu;
+        a.out[1] = nev;
+        a.out[2] = ok;
+        a.out[3] = tr;
+    }
+    ask(kZeroDone, 0.0);
+}
+
 // mu0 of the finite lattice (green0::find_mu, src/green0.cpp:182-203, 240-262)
 // in one block -> result[0], result[1] = 1 when the search succeeded
 // The sum is taken in chunks of kMu0Chunk points, each over kMu0Chunk threads (a
@@ -1255,15 +1615,23 @@ cudaError_t launch_sigma_moments(const GridDev &g, const double2 *S, const doubl
     return finish<kSigmaMomNV>(r, nb, 0.0, st, b);
 }
 
-// one block per column block, or per as few of them as the resident grid (or the
-// caller's cap) allows: no more blocks than that many rounds need
+// One block per column block, or per as few of them as the resident grid (or the
+// caller's cap) allows: no more blocks than that many rounds need.  *slots: the grid
+// exchanges values through slots (few enough column blocks); *cached: those of a
+// block's column blocks, col_bytes each, that it then keeps in shared memory with two
+// blocks on an SM (100 KB each): all, or none (its loop over both is the slower one).
+constexpr size_t kZeroCache = 100 * 1024;
 template <typename K>
-static cudaError_t zero_grid(K kernel, int nblk, int *grid, int cap) {
-    const cudaError_t e = root_grid(kernel, grid, cap);
+static cudaError_t zero_grid(K kernel, K with_slots, int nblk, size_t col_bytes, int *grid, int cap, bool *slots,
+                             int *cached) {
+    *slots = nblk <= kSlotBlocks;
+    cudaError_t e = root_grid(*slots ? with_slots : kernel, grid, cap);
     if (e != cudaSuccess) return e;
     const int rounds = (nblk + *grid - 1) / *grid;
     *grid = (nblk + rounds - 1) / rounds;
-    return nblk <= kRootVals * kRootMaxBlocks ? cudaSuccess : cudaErrorInvalidValue;
+    *cached = *slots && rounds * col_bytes <= kZeroCache ? rounds : 0;
+    if (2LL * nblk > kRootPartial) return cudaErrorInvalidValue;
+    return *slots ? set_smem(with_slots, *cached * col_bytes) : cudaSuccess;
 }
 
 cudaError_t launch_hot_pair(int nk, double mu, double tp, double tpp, double t3, double *scratch, double *out,
@@ -1287,7 +1655,10 @@ cudaError_t launch_mu_zero(const GridDev &g, const double2 *S, const double *s2,
                            const double *sinf, double mu0, double T, RootScratch rs, cudaStream_t st) {
     const int nblk = g.n8p / 4;
     int grid = 0;
-    cudaError_t e = zero_grid(k_mu_zero, nblk, &grid, rs.max_blocks);
+    int cached = 0;
+    bool slots = false;
+    const size_t col_bytes = (size_t)4 * (g.nw0 + 1) * sizeof(double2);
+    cudaError_t e = zero_grid(k_mu_zero, k_mu_slots, nblk, col_bytes, &grid, rs.max_blocks, &slots, &cached);
     if (e != cudaSuccess) return e;
     if (rs.reset_mu && (e = cudaMemsetAsync(rs.bar + 4, 0, 2 * sizeof(unsigned) + sizeof(int), st)) != cudaSuccess)
         return e;
@@ -1309,7 +1680,8 @@ cudaError_t launch_mu_zero(const GridDev &g, const double2 *S, const double *s2,
     a.err = reinterpret_cast<int *>(rs.bar + 6);
     a.out = rs.out;
     void *args[] = {&a};
-    e = cudaLaunchCooperativeKernel((const void *)k_mu_zero, dim3(grid), dim3(kRootThreads), args, 0, st);
+    a.cached = cached;
+    e = cudaLaunchCooperativeKernel(slots ? (const void *)k_mu_slots : (const void *)k_mu_zero, dim3(grid), dim3(kRootThreads), args, cached * col_bytes, st);
     if (e != cudaSuccess) return e;
     return launched();
 }
@@ -1319,7 +1691,10 @@ cudaError_t launch_sumrule_zero(const GridDev &g, const double *chiq, const doub
                                 cudaStream_t st, const double *chi0max, double hi_off) {
     const int nblk = g.n8p / 4;
     int grid = 0;
-    cudaError_t e = zero_grid(k_sumrule_zero, nblk, &grid, rs.max_blocks);
+    int cached = 0;
+    bool slots = false;
+    const size_t col_bytes = (size_t)g.nb * sizeof(double4);
+    cudaError_t e = zero_grid(k_sumrule_zero, k_sumrule_slots, nblk, col_bytes, &grid, rs.max_blocks, &slots, &cached);
     if (e != cudaSuccess) return e;
     if (rs.reset_sr && (e = cudaMemsetAsync(rs.bar, 0, 2 * sizeof(unsigned) + sizeof(int), st)) != cudaSuccess)
         return e;
@@ -1345,7 +1720,8 @@ cudaError_t launch_sumrule_zero(const GridDev &g, const double *chiq, const doub
     a.err = reinterpret_cast<int *>(rs.bar + 2);
     a.out = rs.out;
     void *args[] = {&a};
-    e = cudaLaunchCooperativeKernel((const void *)k_sumrule_zero, dim3(grid), dim3(kRootThreads), args, 0, st);
+    a.cached = cached;
+    e = cudaLaunchCooperativeKernel(slots ? (const void *)k_sumrule_slots : (const void *)k_sumrule_zero, dim3(grid), dim3(kRootThreads), args, cached * col_bytes, st);
     if (e != cudaSuccess) return e;
     return launched();
 }
