@@ -376,20 +376,109 @@ __global__ void __launch_bounds__(AlHqPlan<N>::threads) k_al_hq(const AlHqArgs a
     }
 }
 
+// The slice kernels of H: up to 65 lines the slice is complex in shared memory, one
+// transform a line (the lines' real and imaginary parts are what two real lines are to
+// the packed transforms elsewhere), so that H is read and written whole: as two real
+// slices one after the other every 16-byte value took two half-used accesses, and L1
+// was the busiest unit (68%).  129 lines do not fit and keep the two real slices.
+// Per launch of 10 frequencies at 64^2 x 1024: r -> k 437 -> 338 us, q -> r 140 -> 133;
+// 32^2 x 256: 100 -> 58 and 41 -> 26; 128^2 x 256: 179 -> 142 and 59 -> 50.
+template <int NBK>
+struct AlSlice {
+    static constexpr bool cplx = NBK <= 65;
+    static constexpr int L = 2 * (NBK - 1), G = FftPlan<L>::G;
+    using F = SymFft<L >= 64 ? L : 64>;
+    static constexpr bool sym = NBK >= 33;  // as SlicePlan: below, symmetry saves nothing
+    static constexpr int warps = NBK == 65 ? 5 : NBK == 33 ? 4 : 2;
+    static constexpr int threads = cplx ? 32 * warps : SlicePlan<NBK>::threads;
+    static constexpr int blocks = !cplx ? SlicePlan<NBK>::blocks : NBK == 65 ? 2 : NBK == 33 ? 4 : 8;
+    static constexpr size_t scr_off = (size_t)(NBK - 2) * NBK * sizeof(double2);
+    static constexpr size_t scr = (size_t)(sym ? warps * F::per_warp * F::len : threads / G * padded_len(L)) * sizeof(double2);
+    static constexpr size_t tw_off = scr_off + scr;
+    static constexpr size_t bytes = cplx ? tw_off + (sym ? F::ntw : L) * sizeof(double2) : SlicePlan<NBK>::bytes;
+    static_assert(bytes + 1024 <= 233472 / blocks || !cplx, "the CTAs of an SM share its memory");
+};
+template <int NBK>
+__device__ __forceinline__ void al_twiddles(double2 *S, const double2 *__restrict__ tw) {
+    using P = AlSlice<NBK>;
+    double2 *t = reinterpret_cast<double2 *>(reinterpret_cast<char *>(S) + P::tw_off);
+    if constexpr (P::sym)
+        for (int i = threadIdx.x; i < P::F::ntw; i += blockDim.x) t[i] = __ldg(&tw[(i / P::F::G + 1) * (i % P::F::G)]);
+    else
+        for (int i = threadIdx.x; i < P::L; i += blockDim.x) t[i] = __ldg(&tw[i]);
+}
+// DST-I along l (NBK - 2) x DCT-I along m (NBK) of the complex slice S, in place;
+// ends with a barrier
+template <int NBK>
+__device__ __forceinline__ void al_dst_dct(double2 *S) {
+    using P = AlSlice<NBK>;
+    constexpr int L = P::L, NR = NBK - 2;
+    double2 *scr = reinterpret_cast<double2 *>(reinterpret_cast<char *>(S) + P::scr_off);
+    const double2 *tw = reinterpret_cast<const double2 *>(reinterpret_cast<char *>(S) + P::tw_off);
+    auto row_in = [&](int p, int j) -> double2 { return S[p * NBK + (j < NBK ? j : L - j)]; };
+    auto row_out = [&](int p, int k, double2 z) { S[p * NBK + k] = z; };
+    // z = [0, X, 0, -reverse(X)]: its transform is -i Y
+    auto col_in = [&](int p, int j) -> double2 {
+        if (j == 0 || j == NR + 1) return make_double2(0.0, 0.0);
+        const double2 x = S[(j <= NR ? j - 1 : L - j - 1) * NBK + p];
+        return j <= NR ? x : make_double2(-x.x, -x.y);
+    };
+    auto col_out = [&](int p, int k, double2 z) {
+        if (k >= 1 && k <= NR) S[(k - 1) * NBK + p] = make_double2(-z.y, z.x);
+    };
+    if constexpr (P::sym) {
+        sym_lines<L, 1>(scr, tw, NR, row_in, row_out);
+        __syncthreads();
+        sym_lines<L, -1>(scr, tw, NBK, col_in, col_out);
+        __syncthreads();
+    } else {
+        constexpr int G = P::G;
+        const int grp = threadIdx.x / G, t = threadIdx.x % G, ngrp = blockDim.x / G;
+        double2 *x = scr + grp * padded_len(L);
+#pragma unroll 1
+        for (int p = grp; p < NR; p += ngrp) {
+            group_fft_io<L, -1, true>(
+                x, t, tw, grp, [&](int j) { return row_in(p, j); },
+                [&](int k, double2 z) {
+                    if (k < NBK) row_out(p, k, z);
+                });
+            if constexpr (FftPlan<L>::NPASS == 1) group_sync<G>(grp);
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int p = grp; p < NBK; p += ngrp) {
+            group_fft_io<L, -1, true>(
+                x, t, tw, grp, [&](int j) { return col_in(p, j); }, [&](int k, double2 z) { col_out(p, k, z); });
+            if constexpr (FftPlan<L>::NPASS == 1) group_sync<G>(grp);
+        }
+        __syncthreads();
+    }
+}
+
 // H(q, tau_j) -> H(r, tau_j) = DST x DCT[nf H] of the real and imaginary parts
 // (src/cond_opt.cpp:5628-5716); blocks Nw0 + 1 and Nw0 + 2 transform the two
 // end slopes.
 template <int NBK>
-__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
+__global__ void __launch_bounds__(AlSlice<NBK>::threads, AlSlice<NBK>::blocks)
     k_al_q2r(const double2 *__restrict__ HQ, const double2 *__restrict__ dHQ, const double2 *__restrict__ tw,
              int nw0, double nf, double2 *__restrict__ HR, double2 *__restrict__ dHR) {
     constexpr int K4 = (NBK - 2) * NBK, K4p = (K4 + 1) & ~1;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = plan_twiddles<NBK>(S, tw);
     const int b = blockIdx.x, NJ = nw0 + 1;
     const size_t row = (size_t)blockIdx.y * NJ + b, drow = (size_t)blockIdx.y * 2 + (b - NJ);
     const double2 *src = b < NJ ? HQ + row * K4p : dHQ + drow * K4;
-    double *dst = reinterpret_cast<double *>(b < NJ ? HR + row * K4p : dHR + drow * K4);
+    double2 *dst2 = b < NJ ? HR + row * K4p : dHR + drow * K4;
+    if constexpr (AlSlice<NBK>::cplx) {
+        double2 *Z = reinterpret_cast<double2 *>(S);
+        al_twiddles<NBK>(Z, tw);
+        batched<4>(K4, [&](int c) { return src[c]; }, [&](int c, double2 v) { Z[c] = cscale(v, nf); });
+        __syncthreads();
+        al_dst_dct<NBK>(Z);
+        for (int c = threadIdx.x; c < K4; c += blockDim.x) dst2[c] = Z[c];
+        return;
+    }
+    const auto *tws = plan_twiddles<NBK>(S, tw);
+    double *dst = reinterpret_cast<double *>(dst2);
 #pragma unroll 1
     for (int part = 0; part < 2; ++part) {
         for (int c = threadIdx.x; c < K4; c += blockDim.x) S[c] = nf * (part == 0 ? src[c].x : src[c].y);
@@ -408,19 +497,59 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
 //   k = 2, 3: the same for H2, whose end values are H(r, beta), H(r, 0) and
 //   whose end slopes are -dH(r, beta), -dH(r, 0).
 template <int NBK>
-__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
+__global__ void __launch_bounds__(AlSlice<NBK>::threads, AlSlice<NBK>::blocks)
     k_al_r2k(const double2 *__restrict__ HR, const double2 *__restrict__ dHR, const double *__restrict__ Grt,
              const double *__restrict__ er, const double *__restrict__ dG0p, const double2 *__restrict__ tw, int nw0,
              int n8, double mu0, double2 *__restrict__ HK, double2 *__restrict__ H2K, double2 *__restrict__ dHK) {
     constexpr int K4 = (NBK - 2) * NBK, K4p = (K4 + 1) & ~1;
     extern __shared__ __align__(16) double S[];
-    const auto *tws = plan_twiddles<NBK>(S, tw);
     const int b = blockIdx.x, NJ = nw0 + 1;
     HR += (size_t)blockIdx.y * NJ * K4p;
     dHR += (size_t)blockIdx.y * 2 * K4;
     HK += (size_t)blockIdx.y * NJ * K4p;
     H2K += (size_t)blockIdx.y * NJ * K4p;
     dHK += (size_t)blockIdx.y * 4 * K4;
+    if constexpr (AlSlice<NBK>::cplx) {
+        double2 *Z = reinterpret_cast<double2 *>(S);
+        al_twiddles<NBK>(Z, tw);
+        const int nh = b < NJ ? 2 : 1;
+#pragma unroll 1
+        for (int h = 0; h < nh; ++h) {
+            auto put = [&](int c, double2 v) { Z[c] = v; };
+            if (b < NJ) {
+                const double2 *hr = HR + (size_t)(h == 0 ? b : nw0 - b) * K4p;
+                batched<4>(
+                    K4,
+                    [&](int c) {
+                        const int l = c / NBK, m = c % NBK;
+                        return cscale(hr[c], g_minus(Grt, nw0, n8, b, oct_index(l + 1, m)));
+                    },
+                    put);
+            } else {
+                const int k = b - NJ, side = k & 1;  // 0: tau = 0, 1: beta
+                const double2 *hr = HR + (size_t)((k == 0 || k == 3) ? 0 : nw0) * K4p;      // H at 0 / beta
+                const double2 *dr = dHR + (size_t)((k == 0 || k == 3) ? 0 : 1) * K4;        // which dH
+                const double sg = k < 2 ? 1.0 : -1.0;
+                for (int c = threadIdx.x; c < K4; c += blockDim.x) {
+                    const int o = oct_index(c / NBK + 1, c % NBK);
+                    put(c, cadd(cscale(hr[c], dg_minus(er, dG0p, mu0, side, o)),
+                                cscale(dr[c], sg * g_minus(Grt, nw0, n8, side == 0 ? 0 : nw0, o))));
+                }
+            }
+            __syncthreads();
+            al_dst_dct<NBK>(Z);
+            double2 *dst = h == 0 ? HK : H2K;
+            for (int c = threadIdx.x; c < K4; c += blockDim.x) {
+                if (b < NJ)
+                    dst[bidx2(b, c, NJ)] = Z[c];
+                else
+                    dHK[(size_t)(b - NJ) * K4 + c] = Z[c];
+            }
+            __syncthreads();
+        }
+        return;
+    }
+    const auto *tws = plan_twiddles<NBK>(S, tw);
     const int npass = b < NJ ? 4 : 2;
 #pragma unroll 1
     for (int pass = 0; pass < npass; ++pass) {
@@ -640,16 +769,16 @@ struct RunAlHq {
 template <int NBK>
 struct RunAlSlices {
     static cudaError_t run(const GridDev *g, const AlDev *a, const double *dG0p, double mu0, int nfr, cudaStream_t st) {
-        const size_t sm = SlicePlan<NBK>::bytes;
+        const size_t sm = AlSlice<NBK>::bytes;
         cudaError_t e = set_smem(k_al_q2r<NBK>, sm);
         if (e != cudaSuccess) return e;
         if ((e = set_smem(k_al_r2k<NBK>, sm)) != cudaSuccess) return e;
         const double nf = 1.0 / ((double)g->nk0 * g->nk0);
-        k_al_q2r<NBK><<<dim3(g->nw0 + 3, nfr), SlicePlan<NBK>::threads, sm, st>>>(a->HQ, a->dHQ, g->tw_k, g->nw0, nf,
+        k_al_q2r<NBK><<<dim3(g->nw0 + 3, nfr), AlSlice<NBK>::threads, sm, st>>>(a->HQ, a->dHQ, g->tw_k, g->nw0, nf,
                                                                                   a->HR, a->dHR);
         if ((e = launched()) != cudaSuccess) return e;
         // (H(q, tau) is not read any more: G H(k, tau) takes its place)
-        k_al_r2k<NBK><<<dim3(g->nw0 + 5, nfr), SlicePlan<NBK>::threads, sm, st>>>(
+        k_al_r2k<NBK><<<dim3(g->nw0 + 5, nfr), AlSlice<NBK>::threads, sm, st>>>(
             a->HR, a->dHR, a->Grt, g->er, dG0p, g->tw_k, g->nw0, g->n8, mu0, a->HQ, a->H2K, a->dHK);
         return launched();
     }
