@@ -1480,7 +1480,7 @@ __global__ void __launch_bounds__(1024)
 // block reduction of n(mu) - n and dn/dmu in a fixed order; the Newton step
 // is kept inside the bracket [-8, 8] that the sign of n - n0 shrinks, a
 // bisection otherwise; stops when the step is below 1e-15 (1 + |mu|).
-// The Newton form's replacement of the host root search.
+// The Newton form's replacement of the reference's root search.
 __global__ void __launch_bounds__(1024)
     k_mu0_newton(const double *__restrict__ ek, int n8, int nbk, double n, double T,
                  double nk2, double *result, Bp b) {
