@@ -1502,8 +1502,9 @@ int tpsc_sumrule_tangents(tpsc_ctx *ctx, double out[9]) {
     }
     const double T = ctx->T, beta = 1.0 / T, mu0 = g->mu0, U = ctx->U, n = ctx->n, nsr = ctx->nsr;
     const double Usp = ctx->Usp, Uch = ctx->Uch;
-    // the primal FP64 G(r, tau) (the mixed form keeps only its FP32 copy)
-    CK(launch_gslice(d, g->Grt, mu0, T, ctx->st));
+    // the primal FP64 G(r, tau): the FP64 forms' chi0 stage has left it in g->Grt (104 us
+    // at 128^2 x 2048 to form it again); the mixed form keeps only its FP32 copy
+    if (g->g_mixed) CK(launch_gslice(d, g->Grt, mu0, T, ctx->st));
     // per octant point: xi, beta f(xi), d eps/d t' and the density weight
     const int nbk = d.nbk;
     std::vector<double> xi(n8), bf(n8), deps(n8), wf(n8);
@@ -1559,14 +1560,11 @@ int tpsc_sumrule_tangents(tpsc_ctx *ctx, double out[9]) {
         tb.ddq0 = g->t_ddq0;
         tb.ddG0p = g->adj.ddG0p[p - 1];
         tb.ddchir = g->adj.ddchir[p - 1];
-        CK(launch_chi0_tangent(d, tb, mu0, dmu0, T, ctx->st));
+        CK(launch_chi0_tangent(d, tb, mu0, dmu0, T, {ctx->st2, ctx->evf[0], ctx->evf[1]}, ctx->st));
         CK(launch_chi0_tau(d, dchiq, g->t_ddq0, g->t_dcinf, g->t_dcinf2, T, ctx->st, false));
-        CK(launch_sumrule_tan(d, g->chiq, dchiq, g->cinf, g->cinf2, g->t_dcinf, g->t_dcinf2, Usp, -1.0, T,
-                              ctx->red, ctx->st));
-        if ((rc = queue_read_back(ctx, {{ctx->red.result, sizeof(double), 2 * p}}))) return rc;
-        CK(launch_sumrule_tan(d, g->chiq, dchiq, g->cinf, g->cinf2, g->t_dcinf, g->t_dcinf2, Uch, 1.0, T,
-                              ctx->red, ctx->st));
-        if ((rc = queue_read_back(ctx, {{ctx->red.result, sizeof(double), 2 * p + 1}}))) return rc;
+        CK(launch_sumrule_tan(d, g->chiq, dchiq, g->cinf, g->cinf2, g->t_dcinf, g->t_dcinf2, Usp, Uch, T, ctx->red,
+                              ctx->st));
+        if ((rc = queue_read_back(ctx, {{ctx->red.result, 2 * sizeof(double), 2 * p}}))) return rc;
     }
     CK(cudaStreamSynchronize(ctx->st));
     for (int p = 1; p < 3; ++p) {

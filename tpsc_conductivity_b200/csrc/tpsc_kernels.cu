@@ -1097,14 +1097,17 @@ __global__ void __launch_bounds__(kRedThreads)
 // Directional derivative of k_sumrule's trace at fixed U (jdir = nb, tail
 // term by term) in the direction (dchi, dchi0_inf, dchi0_inf2):
 //   sum w T/Nq [1/(1 + h chi)^2 - 1] dchi,  h = sgn U/2,
-// with the same weights (n = 0 halved) and the same tail frequencies.
+// with the same weights (n = 0 halved) and the same tail frequencies, for both sum
+// rules (h = -Usp/2 -> result[0], Uch/2 -> result[1]): chi and dchi, and the tail's
+// divisions, once for the two.  Bound: the dependent divisions of a few rows a
+// thread; 128^2 x 2048: 2 x 16.4 us -> 19.4 us.
 __global__ void __launch_bounds__(kRedThreads)
     k_sumrule_tan(const double4 *__restrict__ chiq, const double4 *__restrict__ dchiq,
                   const double *__restrict__ cinf, const double *__restrict__ cinf2, const double *__restrict__ dcinf,
-                  const double *__restrict__ dcinf2, const double *__restrict__ w16, int nb, double Uv, double sgn,
+                  const double *__restrict__ dcinf2, const double *__restrict__ w16, int nb, double Usp, double Uch,
                   double T, double scale, Reduce r) {
-    const double hu = sgn * Uv / 2.0;
-    double v = 0.0;
+    const double hu[2] = {-Usp / 2.0, Uch / 2.0};
+    double v[2] = {0.0, 0.0};
     const int blk = blockIdx.x;
     const int o0 = 4 * blk;
     const double4 w = *reinterpret_cast<const double4 *>(w16 + o0);
@@ -1114,13 +1117,16 @@ __global__ void __launch_bounds__(kRedThreads)
         const double4 x = col[j], dx = dcol[j];
         const double f = j == 0 ? 0.5 : 1.0;
         const double xs[4] = {x.x, x.y, x.z, x.w}, ds[4] = {dx.x, dx.y, dx.z, dx.w};
-        double s = 0.0;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const double q = 1.0 / (1.0 + hu * xs[c]);
-            s += ww[c] * (q * q - 1.0) * ds[c];
+        for (int i = 0; i < 2; ++i) {
+            double s = 0.0;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const double q = 1.0 / (1.0 + hu[i] * xs[c]);
+                s += ww[c] * (q * q - 1.0) * ds[c];
+            }
+            v[i] += f * s;
         }
-        v += f * s;
     }
     const int nwmax = nb - 1;
     const double tw = 2.0 * 3.141592653589793 * T;
@@ -1132,12 +1138,15 @@ __global__ void __launch_bounds__(kRedThreads)
             const double wn = (nwmax + 1 + t) * tw;
             const double i2 = 1.0 / (wn * wn);
             const double xv = a * i2 + b * i2 * i2, dxv = da * i2 + db * i2 * i2;
-            const double q = 1.0 / (1.0 + hu * xv);
-            v += ww[c] * (q * q - 1.0) * dxv;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const double q = 1.0 / (1.0 + hu[i] * xv);
+                v[i] += ww[c] * (q * q - 1.0) * dxv;
+            }
         }
     }
-    double out[1] = {scale * v};
-    grid_finish<1>(out, r, 0.0);
+    double out[2] = {scale * v[0], scale * v[1]};
+    grid_finish<2>(out, r, 0.0);
 }
 
 // The Newton form's sum-rule evaluation: only the stored frequencies
@@ -2052,12 +2061,12 @@ cudaError_t launch_sumrule(const GridDev &g, const double *chiq, const double *c
 }
 
 cudaError_t launch_sumrule_tan(const GridDev &g, const double *chiq, const double *dchiq, const double *chi0_inf,
-                               const double *chi0_inf2, const double *dchi0_inf, const double *dchi0_inf2, double Uv,
-                               double sign, double T, Reduce r, cudaStream_t st) {
+                               const double *chi0_inf2, const double *dchi0_inf, const double *dchi0_inf2, double Usp,
+                               double Uch, double T, Reduce r, cudaStream_t st) {
     const double Nq = 4.0 * (g.nbk - 1) * (g.nbk - 1);
     k_sumrule_tan<<<g.n8p / 4, kRedThreads, 0, st>>>(reinterpret_cast<const double4 *>(chiq),
                                                      reinterpret_cast<const double4 *>(dchiq), chi0_inf, chi0_inf2,
-                                                     dchi0_inf, dchi0_inf2, g.w16, g.nb, Uv, sign, T, T / Nq, r);
+                                                     dchi0_inf, dchi0_inf2, g.w16, g.nb, Usp, Uch, T, T / Nq, r);
     return launched();
 }
 

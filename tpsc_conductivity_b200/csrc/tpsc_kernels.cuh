@@ -150,16 +150,21 @@ struct TangentBufs {
     double *ddG0p = nullptr; // [n8] or null  d of d/dtau G(r, 0+)
     double *ddchir = nullptr; // [n8] or null d of d/dtau chi0(r, 0)
 };
+// the side stream of the boundary's kernel and the events that fork and join it
+struct TangentSide {
+    cudaStream_t st = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+};
 // dG(r, tau), dchi0(q, tau_j) and d(d/dtau chi0(q, 0)) for the direction in t
 // (mu0 the primal chemical potential, dmu0 its direction)
 cudaError_t launch_chi0_tangent(const GridDev &g, const TangentBufs &t, double mu0, double dmu0, double T,
-                                cudaStream_t st);
-// the directional derivative of the full sum-rule trace (k_sumrule with
-// every frequency and the tail term by term) at U = Uv in the direction
-// (dchiq, dchi0_inf, dchi0_inf2) -> r.result[0]
+                                const TangentSide &side, cudaStream_t st);
+// the directional derivatives of the full sum-rule traces (k_sumrule with
+// every frequency and the tail term by term) of the spin rule at Usp and the
+// charge rule at Uch in the direction (dchiq, dchi0_inf, dchi0_inf2) -> r.result[0..1]
 cudaError_t launch_sumrule_tan(const GridDev &g, const double *chiq, const double *dchiq, const double *chi0_inf,
-                               const double *chi0_inf2, const double *dchi0_inf, const double *dchi0_inf2, double Uv,
-                               double sign, double T, Reduce r, cudaStream_t st);
+                               const double *chi0_inf2, const double *dchi0_inf, const double *dchi0_inf2,
+                               double Usp, double Uch, double T, Reduce r, cudaStream_t st);
 // sums of mom over the frequencies >= j (double-double, rounded once),
 // j = 0..nb -> mom_suf [(nb + 1)][kMomP]; suffix maxima of cmax -> cmax_suf
 // [nb + 1]; the tail moments and tail maximum of launch_tail_moments' result

@@ -76,7 +76,9 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
 // the tangent of k_chi0_boundary: d of d/dtau G(r, 0+) = DCT-I[-(dxi G0 + xi
 // dG0)(k, 0+) / L^2], of d/dtau G(r, 0-) = (hopping or -mu0) - d/dtau G(r, 0+),
 // and of d/dtau chi0(r, 0) by the product rule, then its DCT-I.  der[o] and
-// dmu0 are the directions of the hopping table and of mu0.  One CTA.
+// dmu0 are the directions of the hopping table and of mu0.  One CTA (a chain of two
+// transforms, 27 us at 65 lines, 1/3 of the slices' time), which reads only the first
+// rows of G and dG: it runs on the side stream beside the slices.
 template <int NBK>
 __global__ void __launch_bounds__(kSliceThreads, 1)
     k_chi0_boundary_tan(const double *__restrict__ ek, const double *__restrict__ er, const double *__restrict__ der,
@@ -131,7 +133,7 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
 template <int NBK>
 struct RunChi0Tan {
     static cudaError_t run(const GridDev *g, const TangentBufs *t, double mu0, double dmu0, double T,
-                           cudaStream_t st) {
+                           const TangentSide *side, cudaStream_t st) {
         const size_t sm = SlicePlan<NBK>::bytes, smw = SliceSmem<NBK, SliceGroups<NBK>::wide>::bytes;
         cudaError_t e;
         if ((e = set_smem(k_gslice_tan<NBK>, sm)) != cudaSuccess) return e;
@@ -140,20 +142,24 @@ struct RunChi0Tan {
         const double nk02 = (double)g->nk0 * g->nk0;
         k_gslice_tan<NBK><<<g->nw0 + 1, SlicePlan<NBK>::threads, sm, st>>>(g->gk, t->fd, g->tw_k, g->n8, g->nw0, T, t->dGrt);
         if ((e = launched()) != cudaSuccess) return e;
+        if ((e = cudaEventRecord(side->fork, st)) != cudaSuccess) return e;
+        if ((e = cudaStreamWaitEvent(side->st, side->fork, 0)) != cudaSuccess) return e;
+        k_chi0_boundary_tan<NBK><<<1, kSliceThreads, smw, side->st>>>(
+            g->ek, g->er, t->der, t->fd, g->tw_k, t->Grt, t->dGrt, t->dG0p, g->n8, mu0, dmu0, T, nk02, t->ddq0,
+            t->ddG0p, t->ddchir);
+        if ((e = launched()) != cudaSuccess) return e;
         k_chi0_slice_tan<NBK><<<g->nb, SlicePlan<NBK>::threads, sm, st>>>(t->Grt, t->dGrt, g->tw_k, g->n8, g->nw0, t->dchiq);
         if ((e = launched()) != cudaSuccess) return e;
-        k_chi0_boundary_tan<NBK><<<1, kSliceThreads, smw, st>>>(g->ek, g->er, t->der, t->fd, g->tw_k, t->Grt, t->dGrt,
-                                                               t->dG0p, g->n8, mu0, dmu0, T, nk02, t->ddq0,
-                                                               t->ddG0p, t->ddchir);
-        return launched();
+        if ((e = cudaEventRecord(side->join, side->st)) != cudaSuccess) return e;
+        return cudaStreamWaitEvent(st, side->join, 0);
     }
 };
 
 }  // namespace
 
 cudaError_t launch_chi0_tangent(const GridDev &g, const TangentBufs &t, double mu0, double dmu0, double T,
-                                cudaStream_t st) {
-    return dispatch_nbk<RunChi0Tan>(g.nbk, &g, &t, mu0, dmu0, T, st);
+                                const TangentSide &side, cudaStream_t st) {
+    return dispatch_nbk<RunChi0Tan>(g.nbk, &g, &t, mu0, dmu0, T, &side, st);
 }
 
 }  // namespace tpsc
