@@ -232,7 +232,9 @@ int tpsc_find_mu(tpsc_ctx *ctx);
  * traceSelfG -> mu -> traceSelfG2, i.e. green::calc_Self_FFT_spline +
  * traceSelfG + find_mu (src/tpsc_main.cpp:71-75) without the half-grid
  * Usp/Uch pre-pass (which only feeds the difRel diagnostics) and without
- * file output. */
+ * file output.  A solve whose Usp or Uch is not found leaves chi0 and nothing
+ * after it: the calls that need roots, V, Sigma or mu answer TPSC_ERR_STATE
+ * until a solve succeeds. */
 int tpsc_solve(tpsc_ctx *ctx);
 
 /* ---- results ------------------------------------------------------------ */

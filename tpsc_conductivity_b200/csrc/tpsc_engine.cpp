@@ -201,6 +201,7 @@ struct tpsc_ctx {
     int nk0 = 0, Nw0 = 0;
     double n = 0, T = 0, tp = 0, tpp = 0, t3 = 0, U = 0, nsr = 0;
     double Usp = 0, Uch = 0;
+    double found[2] = {0, 0};  // the last Usp, Uch that a search found, whatever the model (dres holds them)
     double mu_shift = 0;  // added to the density root mu0 (tpsc_set_mu_shift)
     std::map<std::pair<int, int>, Grid *> grids;
     Grid *cur = nullptr;
@@ -575,17 +576,30 @@ int set_roots(tpsc_ctx *ctx, const double *r, unsigned err) {
     if (err) return fail(ctx, TPSC_ERR_CUDA, "device root search: grid barrier timed out");
     if (r[4] != 1.0) return fail(ctx, TPSC_ERR_NO_ROOT, "Usp not found");
     if (r[5] != 1.0) return fail(ctx, TPSC_ERR_NO_ROOT, "Uch not found");
-    ctx->Usp = r[0];
-    ctx->Uch = r[1];
+    ctx->Usp = ctx->found[0] = r[0];
+    ctx->Uch = ctx->found[1] = r[1];
     ctx->scal[TPSC_S_EVALS_SP] = r[2];
     ctx->scal[TPSC_S_EVALS_CH] = r[3];
     ctx->scal[TPSC_S_USP] = ctx->Usp;
     ctx->scal[TPSC_S_UCH] = ctx->Uch;
     return TPSC_OK;
 }
+// A search for Usp, Uch that failed: what was formed from its last iterates (a
+// solve queues every stage before it reads a result) is not a result, and
+// ctx->dres holds the last roots that were found again.
+int drop_roots(tpsc_ctx *ctx, int rc) {
+    Grid *g = ctx->cur;
+    g->have_U = g->have_V = g->have_S = false;
+    ctx->scal[TPSC_S_EVALS_MU] = 0;
+    const std::string msg = ctx->err;
+    launch_store(ctx->dres, ctx->found, 2, ctx->st);
+    ctx->err = msg;
+    return rc;
+}
 // r = (Tr Sigma G0, its asymptotic part, mu, evals, ok, Tr Sigma G at mu, -, Sigma_inf)
 // of the mu search, err its barrier flag; traces: r[0..1] were formed
 int set_mu(tpsc_ctx *ctx, const double *r, int err, bool traces) {
+    ctx->scal[TPSC_S_EVALS_MU] = 0;  // no mu until it is found
     if (err) return fail(ctx, TPSC_ERR_CUDA, "device mu search: grid barrier timed out");
     ctx->scal[TPSC_S_SIGMA_INF] = r[7];
     if (traces) {
@@ -725,7 +739,7 @@ int sumrule(tpsc_ctx *ctx, int channel, double Uv, double *tr, double *dtr) {
 
 // chi::find_Usp_Uch(nq0, nw0, Usc) on the current grid after chi0 (src/chi.cpp:850-876)
 // read: take the roots back now; a solve defers that to its one readback at
-// the end, the interval's end then coming from the device chi0max
+// the end (solve_finish), the interval's end then coming from the device chi0max
 int roots_Usp_Uch(tpsc_ctx *ctx, double Usc[2], bool read = true) {
     const double n = ctx->n, U = ctx->U, nsr = ctx->nsr;
     int rc = TPSC_OK;
@@ -744,15 +758,15 @@ int roots_Usp_Uch(tpsc_ctx *ctx, double Usc[2], bool read = true) {
         CK(launch_sumrule_zero(g->d, g->chiq, g->cinf, g->cinf2, ctx->T, n, nsr, U, hi, rs, ctx->st, chi0max, off));
     }
     ctx->roots.reset_sr = true;
-    ctx->cur->have_U = true;
     if (!read) return TPSC_OK;
     // the results and the barrier's error flag in one readback
     if ((rc = read_back(ctx, {{ctx->dres, 6 * sizeof(double), 0}, {ctx->roots.bar + 2, sizeof(unsigned), 6}})))
-        return rc;
+        return drop_roots(ctx, rc);
     unsigned err;
     std::memcpy(&err, ctx->h_res + 6, sizeof(unsigned));
     ctx->roots.reset_sr = err != 0;
-    if ((rc = set_roots(ctx, ctx->h_res, err))) return rc;
+    if ((rc = set_roots(ctx, ctx->h_res, err))) return drop_roots(ctx, rc);
+    g->have_U = true;
     Usc[0] = ctx->Usp;
     Usc[1] = ctx->Uch;
     return TPSC_OK;
@@ -904,7 +918,8 @@ int mark(tpsc_ctx *ctx, int i) {
 // host round trip (the roots, the vertex and Sigma read their inputs on the
 // device), ending in the gather of everything the host checks into ctx->h_res;
 // solve_finish waits for it and checks chi0max, the sum-rule roots, the mu
-// search and their barrier flags in stage order.
+// search and their barrier flags in stage order.  Only there it is known
+// whether V and Sigma are those of roots that were found.
 int solve_queue(tpsc_ctx *ctx) {
     double Usc[2];
     int rc;
@@ -931,17 +946,17 @@ int solve_queue(tpsc_ctx *ctx) {
 }
 
 int solve_finish(tpsc_ctx *ctx) {
-    CK(cudaStreamSynchronize(ctx->st));
     int rc;
+    if (cudaError_t e = cudaStreamSynchronize(ctx->st)) return drop_roots(ctx, cuda_fail(ctx, e, "solve"));
     const double *h = ctx->h_res;
-    if ((rc = set_chi0max(ctx, h))) return rc;
     unsigned err_sr;
     std::memcpy(&err_sr, h + 9, sizeof(unsigned));
     int err_mu;
     std::memcpy(&err_mu, h + 16, sizeof(int));
     ctx->roots.reset_sr = err_sr != 0;
     ctx->roots.reset_mu = err_mu != 0;
-    if ((rc = set_roots(ctx, h + 3, err_sr))) return rc;
+    if ((rc = set_chi0max(ctx, h)) || (rc = set_roots(ctx, h + 3, err_sr))) return drop_roots(ctx, rc);
+    ctx->cur->have_U = true;
     set_dblocc(ctx);
     double r[8];
     for (int i = 0; i < 6; ++i) r[i] = h[10 + i];
@@ -954,7 +969,7 @@ int solve_finish(tpsc_ctx *ctx) {
 void solve_state(tpsc_ctx *ctx) {
     Grid *g = ctx->cur;
     g->g_mixed = mixed(ctx);
-    g->have_chi0 = g->have_U = g->have_V = g->have_S = true;
+    g->have_chi0 = g->have_V = g->have_S = true;
     g->have_mom = (ctx->form & TPSC_FORM_NEWTON) != 0;
     g->have_mom_host = false;
     ctx->roots.reset_sr = ctx->roots.reset_mu = true;
@@ -1032,7 +1047,7 @@ int run_solve(tpsc_ctx *ctx) {
     }
     ctx->seen_key = key;
     ctx->seen_grid = g;
-    if ((rc = solve_queue(ctx))) return rc;
+    if ((rc = solve_queue(ctx))) return drop_roots(ctx, rc);
     g->warm_forms |= fbit;
     return solve_finish(ctx);
 }
