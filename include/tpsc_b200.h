@@ -77,7 +77,12 @@ enum tpsc_scalar {
  *    in FP32 with compensated twiddles (G stored in FP32); Sigma's
  *    transforms, every tau transform, the sum rules, traces, roots and the
  *    continuation in FP64.  Sigma within ~1e-6 of the FP64 forms.
- * Neither NEWTON nor MIXED has a counterpart in the reference. */
+ * Neither NEWTON nor MIXED has a counterpart in the reference.
+ * In every form the searches for Usp, Uch and mu are cooperative launches
+ * whose blocks exchange values; a wait for another block ends after 1.5 s of
+ * wall clock.  The search (in tpsc_solve the solve) is then repeated in one
+ * block, which waits for no other; it fails with TPSC_ERR_CUDA only if that
+ * fails too. */
 enum tpsc_form { TPSC_FORM_REFERENCE = 0, TPSC_FORM_NEWTON = 1, TPSC_FORM_MIXED = 2 };
 
 /* Create a context on CUDA device `device`.  Returns NULL and sets *status on
@@ -420,6 +425,11 @@ int tpsc_fma_peak(int bits, double *tflops);
  * with it; *ms: the kernel's time.  Returns TPSC_OK when the launch itself
  * ran (the flag reports the barrier). */
 int tpsc_barrier_probe(tpsc_ctx *ctx, int withhold, int *err_flag, int *timed_out, int *blocks, double *ms);
+/* Check of what follows such a wait (on the host; nothing waits): the next
+ * `count` error flags that root searches of the context read back count as
+ * set.  A solve reads two (the sum rules', mu's), find_Usp_Uch_grid and
+ * find_mu one. */
+int tpsc_inject_wait_timeouts(tpsc_ctx *ctx, int count);
 
 /* Number of CUDA kernels the library has launched (all contexts) since it was
  * loaded. */

@@ -190,6 +190,8 @@ struct tpsc_ctx {
     Reduce red;
     Reduce redm;              // moment sums: partial [(2 kMomP + 1) kMaxBlocks], result [32]
     RootScratch roots;        // the device root searches' state
+    bool ran_out = false;     // a wait of the last root search that was read back ran out
+    int inject_timeouts = 0;  // tpsc_inject_wait_timeouts
     // device results the later stages read without a host round trip:
     // [0..5] Usp, Uch, evals_sp, evals_ch, ok_sp, ok_ch (the vertex reads [0..1])
     double *dres = nullptr;
@@ -584,6 +586,33 @@ int set_roots(tpsc_ctx *ctx, const double *r, unsigned err) {
     ctx->scal[TPSC_S_UCH] = ctx->Uch;
     return TPSC_OK;
 }
+// the error flag of a search's waits, read back to p
+unsigned wait_flag(tpsc_ctx *ctx, const double *p) {
+    unsigned f;
+    std::memcpy(&f, p, sizeof(f));
+    if (ctx->inject_timeouts > 0) {
+        --ctx->inject_timeouts;
+        f = 1;
+    }
+    if (f) ctx->ran_out = true;
+    return f;
+}
+// f(), and once more with the root searches in one block, which waits for no other,
+// when a wait between their blocks ran out: the grid's blocks were then not on the GPU
+// together for more than a second (another context's grids, time slicing, a debugger).
+// The reference form's sums are in block order: the same bits whatever the grid.
+template <class F>
+int with_waits(tpsc_ctx *ctx, const F &f) {
+    ctx->ran_out = false;
+    int rc = f();
+    if (!rc || !ctx->ran_out) return rc;
+    const int cap = ctx->roots.max_blocks;
+    ctx->roots.max_blocks = 1;
+    ctx->err.clear();
+    rc = f();
+    ctx->roots.max_blocks = cap;
+    return rc;
+}
 // A search for Usp, Uch that failed: what was formed from its last iterates (a
 // solve queues every stage before it reads a result) is not a result, and
 // ctx->dres holds the last roots that were found again.
@@ -598,7 +627,7 @@ int drop_roots(tpsc_ctx *ctx, int rc) {
 }
 // r = (Tr Sigma G0, its asymptotic part, mu, evals, ok, Tr Sigma G at mu, -, Sigma_inf)
 // of the mu search, err its barrier flag; traces: r[0..1] were formed
-int set_mu(tpsc_ctx *ctx, const double *r, int err, bool traces) {
+int set_mu(tpsc_ctx *ctx, const double *r, unsigned err, bool traces) {
     ctx->scal[TPSC_S_EVALS_MU] = 0;  // no mu until it is found
     if (err) return fail(ctx, TPSC_ERR_CUDA, "device mu search: grid barrier timed out");
     ctx->scal[TPSC_S_SIGMA_INF] = r[7];
@@ -740,7 +769,7 @@ int sumrule(tpsc_ctx *ctx, int channel, double Uv, double *tr, double *dtr) {
 // chi::find_Usp_Uch(nq0, nw0, Usc) on the current grid after chi0 (src/chi.cpp:850-876)
 // read: take the roots back now; a solve defers that to its one readback at
 // the end (solve_finish), the interval's end then coming from the device chi0max
-int roots_Usp_Uch(tpsc_ctx *ctx, double Usc[2], bool read = true) {
+int search_Usp_Uch(tpsc_ctx *ctx, double Usc[2], bool read) {
     const double n = ctx->n, U = ctx->U, nsr = ctx->nsr;
     int rc = TPSC_OK;
     // both roots in one cooperative launch (tpsc_roots.cu), into ctx->dres,
@@ -762,14 +791,17 @@ int roots_Usp_Uch(tpsc_ctx *ctx, double Usc[2], bool read = true) {
     // the results and the barrier's error flag in one readback
     if ((rc = read_back(ctx, {{ctx->dres, 6 * sizeof(double), 0}, {ctx->roots.bar + 2, sizeof(unsigned), 6}})))
         return drop_roots(ctx, rc);
-    unsigned err;
-    std::memcpy(&err, ctx->h_res + 6, sizeof(unsigned));
+    const unsigned err = wait_flag(ctx, ctx->h_res + 6);
     ctx->roots.reset_sr = err != 0;
     if ((rc = set_roots(ctx, ctx->h_res, err))) return drop_roots(ctx, rc);
     g->have_U = true;
     Usc[0] = ctx->Usp;
     Usc[1] = ctx->Uch;
     return TPSC_OK;
+}
+
+int roots_Usp_Uch(tpsc_ctx *ctx, double Usc[2]) {
+    return with_waits(ctx, [&]() { return search_Usp_Uch(ctx, Usc, true); });
 }
 
 void set_dblocc(tpsc_ctx *ctx) {
@@ -926,7 +958,7 @@ int solve_queue(tpsc_ctx *ctx) {
     if ((rc = mark(ctx, 0))) return rc;
     if ((rc = run_chi0(ctx, false))) return rc;
     if ((rc = mark(ctx, 1))) return rc;
-    if ((rc = roots_Usp_Uch(ctx, Usc, false))) return rc;
+    if ((rc = search_Usp_Uch(ctx, Usc, false))) return rc;
     if ((rc = mark(ctx, 2))) return rc;
     if ((rc = run_vertex(ctx))) return rc;
     if ((rc = mark(ctx, 3))) return rc;
@@ -949,10 +981,7 @@ int solve_finish(tpsc_ctx *ctx) {
     int rc;
     if (cudaError_t e = cudaStreamSynchronize(ctx->st)) return drop_roots(ctx, cuda_fail(ctx, e, "solve"));
     const double *h = ctx->h_res;
-    unsigned err_sr;
-    std::memcpy(&err_sr, h + 9, sizeof(unsigned));
-    int err_mu;
-    std::memcpy(&err_mu, h + 16, sizeof(int));
+    const unsigned err_sr = wait_flag(ctx, h + 9), err_mu = wait_flag(ctx, h + 16);
     ctx->roots.reset_sr = err_sr != 0;
     ctx->roots.reset_mu = err_mu != 0;
     if ((rc = set_chi0max(ctx, h)) || (rc = set_roots(ctx, h + 3, err_sr))) return drop_roots(ctx, rc);
@@ -984,7 +1013,7 @@ void solve_state(tpsc_ctx *ctx) {
 // happen outside a capture); a new capture updates the executable graph in
 // place when its topology allows.  A capture that fails turns graphs off for
 // the context and the solve runs as direct launches.
-int run_solve(tpsc_ctx *ctx) {
+int launch_solve(tpsc_ctx *ctx) {
     Grid *g = ctx->cur;
     const GridDev &d = g->d;
     if (mixed(ctx) && !g->Grt32) CK(dalloc(g, &g->Grt32, (size_t)(d.nw0 + 1) * d.n8));
@@ -998,7 +1027,8 @@ int run_solve(tpsc_ctx *ctx) {
     key.rsr = ctx->roots.reset_sr;
     key.rmu = ctx->roots.reset_mu;
     const unsigned fbit = 1u << (ctx->form & 3);
-    const bool graphs = ctx->graph_mode > 0 && !ctx->graph_off && (g->warm_forms & fbit);
+    // (a solve that is repeated in one block is not worth a graph)
+    const bool graphs = ctx->graph_mode > 0 && !ctx->graph_off && (g->warm_forms & fbit) && !ctx->ran_out;
     int rc = TPSC_OK;
     if (graphs && g->graph_exec && key == g->graph_key) {
         CK(cudaGraphLaunch(g->graph_exec, ctx->st));
@@ -1052,9 +1082,13 @@ int run_solve(tpsc_ctx *ctx) {
     return solve_finish(ctx);
 }
 
+int run_solve(tpsc_ctx *ctx) {
+    return with_waits(ctx, [&]() { return launch_solve(ctx); });
+}
+
 // green::find_mu with traceSelfG2 (src/green.cpp:3185-3282); in the Newton form
 // the traces of traceSelfG come with it
-int find_mu(tpsc_ctx *ctx) {
+int search_mu(tpsc_ctx *ctx) {
     Grid *g = ctx->cur;
     if (!g || !g->have_S) return fail(ctx, TPSC_ERR_STATE, "the self-energy has not been computed");
     const bool traces = (ctx->form & TPSC_FORM_NEWTON) != 0;
@@ -1065,10 +1099,12 @@ int find_mu(tpsc_ctx *ctx) {
                               {ctx->roots.bar + 6, sizeof(int), 6},
                               {g->sinf, sizeof(double), 7}})))
         return rc;
-    int err;
-    std::memcpy(&err, ctx->h_res + 6, sizeof(int));
+    const unsigned err = wait_flag(ctx, ctx->h_res + 6);
     ctx->roots.reset_mu = err != 0;
     return set_mu(ctx, ctx->h_res, err, traces);
+}
+int find_mu(tpsc_ctx *ctx) {
+    return with_waits(ctx, [&]() { return search_mu(ctx); });
 }
 
 // Device state of the correlator on grid g for n_theta bins: the K4 arrays
@@ -2664,6 +2700,12 @@ int tpsc_chijj(tpsc_ctx *ctx, int n_theta) {
     if (g->d.nk0 < 8) return fail(ctx, TPSC_ERR_ARG, "need nk0 >= 8");
     g->cond_bins = 0;
     return run_cond(ctx, n_theta);
+}
+
+int tpsc_inject_wait_timeouts(tpsc_ctx *ctx, int count) {
+    if (!ctx || count < 0) return fail(ctx, TPSC_ERR_ARG, "need a context and count >= 0");
+    ctx->inject_timeouts = count;
+    return TPSC_OK;
 }
 
 int tpsc_barrier_probe(tpsc_ctx *ctx, int withhold, int *err_flag, int *timed_out, int *blocks, double *ms) {
