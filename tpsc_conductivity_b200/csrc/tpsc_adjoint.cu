@@ -1225,9 +1225,9 @@ __global__ void __launch_bounds__(256) k_adj_sums(const double *__restrict__ par
     const int slot = blockIdx.x;
     KSum acc;
     for (int r = threadIdx.x; r < nrows; r += blockDim.x) acc.add(part[(size_t)r * kAdjW + slot]);
-    double v[1] = {acc.value()};
+    KSum v[1] = {acc};
     __shared__ double tot[1];
-    block_sum<1>(v, tot);
+    block_ksum<1>(v, tot);
     if (threadIdx.x == 0) out[slot] = tot[0];
 }
 

@@ -718,8 +718,8 @@ __global__ void __launch_bounds__(128) k_al_finish(const double *__restrict__ co
     KSum s;
     for (int c = threadIdx.x; c < K4; c += blockDim.x)
         if (v == 0 || (bin ? bin[c] : 0) == v - 1) s.add(colv[c]);
-    double x[1] = {s.value()};
-    block_sum<1>(x, tot);
+    KSum x[1] = {s};
+    block_ksum<1>(x, tot);
     if (threadIdx.x == 0) out[(size_t)blockIdx.y * gridDim.x + v] = tot[0];
 }
 

@@ -586,8 +586,8 @@ __global__ void __launch_bounds__(CondTauPlan<N>::threads, CondTauPlan<N>::block
                 s0[2 + tid] = q.dGp * q.Jt0 + q.Gt0 * q.dJ0;
                 sN[2 + tid] = q.dGm * Jbeta - (q.Gt0 + 1.0) * q.dJb;
             }
-            double v2[2] = {va.value(), vb.value()};
-            block_sum<2>(v2, sV);
+            KSum v2[2] = {va, vb};
+            block_ksum<2>(v2, sV);
         }
         // ---- splines and FFT_{-} of both: the bubble's moments from the half
         // spline (odd about beta/2), the Maki-Thompson moment from the G J
@@ -601,15 +601,15 @@ __global__ void __launch_bounds__(CondTauPlan<N>::threads, CondTauPlan<N>::block
                 ma.add(w * m.x);
                 mb.add(w * m.y);
             }
-            double2 m = make_double2(ma.value(), mb.value());
             constexpr int W = G < 32 ? G : 32;
             const unsigned lanes = G < 32 ? (1u << G) - 1u : 0xffffffffu;
-            for (int off = W / 2; off > 0; off >>= 1) {
-                m.x += __shfl_down_sync(lanes, m.x, off, W);
-                m.y += __shfl_down_sync(lanes, m.y, off, W);
+            ma.join_lanes<W>(lanes);
+            mb.join_lanes<W>(lanes);
+            __shared__ double2 red[2][(G + 31) / 32];
+            if (t % 32 == 0) {
+                red[0][t / 32] = make_double2(ma.s, ma.c);
+                red[1][t / 32] = make_double2(mb.s, mb.c);
             }
-            __shared__ double2 red[(G + 31) / 32];
-            if (t % 32 == 0) red[t / 32] = m;
             auto in = [&](int j) -> double2 {
                 const bool lo = j < NO;
                 const int jj = lo ? j : N - 1 - j;
@@ -619,12 +619,10 @@ __global__ void __launch_bounds__(CondTauPlan<N>::threads, CondTauPlan<N>::block
             };
             group_fft_io<N, -1, false, true>(X1, t, (const TwoLevelTw *)tw2, 0, in, ScratchIO{X1});
             if (t < 2) {
-                double sM = 0.0;
-                for (int w = 0; w < (G + 31) / 32; ++w) sM += part_of(red[w], t);
-                cs[t].integ = h * sV[t] - h * h * h / 12.0 * sM;
-                if (G == 1) {
-                    sM = red[0].y;
-                    cs[1].integ = h * sV[1] - h * h * h / 12.0 * sM;
+                for (int q = t; q < 2; q += G) {
+                    KSum sM;
+                    for (int w = 0; w < (G + 31) / 32; ++w) sM.join(red[q][w].x, red[q][w].y);
+                    cs[q].integ = h * sV[q] - h * h * h / 12.0 * sM.value();
                 }
             }
         } else if (grp == 1) {
@@ -739,9 +737,9 @@ __global__ void __launch_bounds__(32 * kCondFinishWarps)
         KSum s;
         for (int b = threadIdx.x; b < nblk + nlines; b += blockDim.x)
             s.add(b < nblk ? partial[(size_t)b * pw + pw - 1] : lines[b - nblk]);
-        double v[1] = {s.value()};
+        KSum v[1] = {s};
         __shared__ double tot[1];
-        block_sum<1>(v, tot);
+        block_ksum<1>(v, tot);
         if (threadIdx.x == 0) out[(size_t)nbins * PWB + PWB] = tot[0];
         return;
     }

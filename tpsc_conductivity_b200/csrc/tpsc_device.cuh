@@ -62,6 +62,13 @@ __device__ __forceinline__ int oct_weight(int base, int l, int m, int nbk) {
     return w;
 }
 
+// error-free sum of two doubles (Knuth's TwoSum): a + b = s + e exactly
+__device__ __forceinline__ void two_sum(double a, double b, double &s, double &e) {
+    s = a + b;
+    const double bp = s - a;
+    e = (a - (s - bp)) + (b - bp);
+}
+
 // ---------------------------------------------------------------------------
 // compensated (Kahan-Babuska) summation
 // ---------------------------------------------------------------------------
@@ -74,6 +81,22 @@ struct KSum {
         else
             c += (x - t) + s;
         s = t;
+    }
+    // another compensated sum, by TwoSum
+    __device__ __forceinline__ void join(double s2, double c2) {
+        double t, r;
+        two_sum(s, s2, t, r);
+        s = t;
+        c += c2 + r;
+    }
+    // the sums of a segment of W lanes (W a power of two, `lanes` its mask), in its first lane
+    template <int W>
+    __device__ __forceinline__ void join_lanes(unsigned lanes) {
+#pragma unroll
+        for (int off = W / 2; off > 0; off >>= 1) {
+            const double s2 = __shfl_down_sync(lanes, s, off, W), c2 = __shfl_down_sync(lanes, c, off, W);
+            join(s2, c2);
+        }
     }
     __device__ __forceinline__ double value() const { return s + c; }
 };
@@ -444,13 +467,6 @@ __device__ void spline_second_derivatives(double *A, int lda, int NJ, double h, 
     __syncthreads();
 }
 
-// error-free sum of two doubles (Knuth's TwoSum): a + b = s + e exactly
-__device__ __forceinline__ void two_sum(double a, double b, double &s, double &e) {
-    s = a + b;
-    const double bp = s - a;
-    e = (a - (s - bp)) + (b - bp);
-}
-
 // per-column sum of y[i0..i1) over the TPC threads of each column -> out[c]:
 // compensated per-thread sums, then a fixed shuffle tree that adds the pairs
 // (sum, compensation) with TwoSum, then the column's warps in order.  TPC is
@@ -461,28 +477,14 @@ __device__ void column_sums(const double *A, int lda, int i0, int i1, double *ou
     const int c = threadIdx.x / TPC, k = threadIdx.x % TPC;
     KSum acc;
     for (int i = i0 + k; i < i1; i += TPC) acc.add(A[c * lda + i]);
-    double s = acc.s, e = acc.c;
-    for (int off = 16; off > 0; off >>= 1) {
-        const double s2 = __shfl_down_sync(0xffffffffu, s, off);
-        const double e2 = __shfl_down_sync(0xffffffffu, e, off);
-        double t, r;
-        two_sum(s, s2, t, r);
-        s = t;
-        e += e2 + r;
-    }
+    acc.join_lanes<32>(0xffffffffu);
     __shared__ double2 part[32];
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = make_double2(s, e);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = make_double2(acc.s, acc.c);
     __syncthreads();
     if (k == 0) {
         const int w0 = threadIdx.x >> 5, nw = TPC >> 5;
-        double S = part[w0].x, E = part[w0].y;
-        for (int q = 1; q < nw; ++q) {
-            double t, r;
-            two_sum(S, part[w0 + q].x, t, r);
-            S = t;
-            E += part[w0 + q].y + r;
-        }
-        out[c] = S + E;
+        for (int q = 1; q < nw; ++q) acc.join(part[w0 + q].x, part[w0 + q].y);
+        out[c] = acc.value();
     }
     __syncthreads();
 }
@@ -898,6 +900,26 @@ __device__ void block_sum(double (&v)[NV], double *out) {
         double s = 0.0;
         for (int w = 0; w < nw; ++w) s += red[w][threadIdx.x];
         out[threadIdx.x] = s;
+    }
+    __syncthreads();
+}
+// block_sum of compensated sums: the compensations are carried through the tree (a
+// plain tree after compensated threads rounds once per level)
+template <int NV>
+__device__ void block_ksum(KSum (&v)[NV], double *out) {
+    __shared__ double2 red[32][NV];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        v[k].template join_lanes<32>(0xffffffffu);
+        if (lane == 0) red[warp][k] = make_double2(v[k].s, v[k].c);
+    }
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        const int nw = (blockDim.x + 31) >> 5;
+        KSum a;
+        for (int w = 0; w < nw; ++w) a.join(red[w][threadIdx.x].x, red[w][threadIdx.x].y);
+        out[threadIdx.x] = a.value();
     }
     __syncthreads();
 }

@@ -820,22 +820,24 @@ struct Tau3Group {
             }
     }
     __device__ void sync() { group_sync<Tau3Plan<N>::G>(grp); }
-    // sum of v over the group's threads, in its thread 0; red: one entry per warp of the block
-    __device__ double2 sum(double2 v, double2 *red) {
+    // sums of a and c over the group's threads, in its thread 0; red: one entry per warp of the block
+    __device__ double2 sum(KSum a, KSum c, double4 *red) {
         constexpr int G = Tau3Plan<N>::G, W = G < 32 ? G : 32;
         const unsigned lanes = G < 32 ? ((1u << W) - 1u) << ((threadIdx.x & 31) / W * W) : 0xffffffffu;
-        for (int off = W / 2; off > 0; off >>= 1) {
-            v.x += __shfl_down_sync(lanes, v.x, off, W);
-            v.y += __shfl_down_sync(lanes, v.y, off, W);
-        }
+        a.join_lanes<W>(lanes);
+        c.join_lanes<W>(lanes);
         if constexpr (G > 32) {
-            if (t % 32 == 0) red[threadIdx.x / 32] = v;
+            if (t % 32 == 0) red[threadIdx.x / 32] = make_double4(a.s, a.c, c.s, c.c);
             sync();
             if (t == 0)
-                for (int w = 1; w < G / 32; ++w) v = cadd(v, red[threadIdx.x / 32 + w]);
+                for (int w = 1; w < G / 32; ++w) {
+                    const double4 r = red[threadIdx.x / 32 + w];
+                    a.join(r.x, r.y);
+                    c.join(r.z, r.w);
+                }
             sync();
         }
-        return v;
+        return make_double2(a.value(), c.value());
     }
 };
 // the two columns of a packed transform at bins n and its partner
@@ -919,7 +921,7 @@ __global__ void __launch_bounds__(Tau3Plan<N>::threads, Tau3Plan<N>::blocks)
     chi0_inf2 = at(chi0_inf2, b.arena);
     T = bpar(b, kPpT, T);
     extern __shared__ __align__(16) double2 smem3[];
-    __shared__ double2 red[Tau3Plan<N>::threads / 32];
+    __shared__ double4 red[Tau3Plan<N>::threads / 32];
     Tau3Group<N> q(smem3);
     tau_tables(q.tw2, q.tw2 + 1, tw, tw, N);
     __syncthreads();
@@ -940,7 +942,7 @@ __global__ void __launch_bounds__(Tau3Plan<N>::threads, Tau3Plan<N>::blocks)
             a.add(w * v.x);
             c.add(w * v.y);
         }
-        return q.sum(make_double2(a.value(), c.value()), red);
+        return q.sum(a, c, red);
     };
     const double h = 1.0 / (N * T), ih = 1.0 / h;
     const double2 sV = trapezoid();
