@@ -441,8 +441,9 @@ __global__ void __launch_bounds__(kRootThreads) k_sumrule_roots(SumRootArgs a) {
 // so that this part of Tr(G - G0) at mu is Re sum_m (mu0 - mu)^m C_m - G0 to
 // a relative kMuSeriesMax^kMuMomP while |mu - mu0| <= kMuSeriesMax |z|.
 //
-// C_m for m >= kMuMomF64 is formed and summed in FP32 (per thread, ~32 terms;
-// the block and grid sums are FP64): its term (mu0 - mu)^m C_m is at most
+// C_m for m >= kMuMomF64 is formed and summed in FP32 (per thread: 32 terms of the
+// stored frequencies, a column's Nw0/64 + 1 of the tail term by term; the sums of
+// columns, blocks and the grid are FP64): its term (mu0 - mu)^m C_m is at most
 // kMuSeriesMax^m = 8e-7 of the leading one per point, so an FP32 relative
 // error ~1e-6 on it moves Tr(G - G0) by < 1e-12 of its leading term.  The
 // point constants live in shared memory and Tr Sigma G0, its Hartree part and
@@ -491,10 +492,11 @@ __global__ void __launch_bounds__(kMomThreads, 2)
     double tsg = 0.0, har = 0.0, g0 = 0.0;
     double m64[2 * P64];
     float m32[2 * P32];
+    double t32[2 * P32];  // the tail's columns
 #pragma unroll
     for (int k = 0; k < 2 * P64; ++k) m64[k] = 0.0;
 #pragma unroll
-    for (int k = 0; k < 2 * P32; ++k) m32[k] = 0.0f;
+    for (int k = 0; k < 2 * P32; ++k) t32[k] = m32[k] = 0.0f;
     // z = i w_n - x - Sigma with x = eps - mu0; inv = 1 / (w_n^2 + x^2)
     // rr = 1/|z|^2 (|z| >= w_n > 0)
     auto moments_rr = [&](double zx, double zy, double rr, double x, double w, double inv) {
@@ -683,6 +685,11 @@ __global__ void __launch_bounds__(kMomThreads, 2)
                         moments(wn, -a3 * i2 + a5 * i2 * i2, -sinf * i1 + a4 * i2 * i1, xc, wc,
                                 1.0 / (wn * wn + xc * xc));
                     }
+#pragma unroll
+                    for (int k = 0; k < 2 * P32; ++k) {
+                        t32[k] += m32[k];
+                        m32[k] = 0.0f;
+                    }
                 }
         }
         sre += __shfl_down_sync(0xffffffffu, sre, 16);
@@ -695,8 +702,8 @@ __global__ void __launch_bounds__(kMomThreads, 2)
                     m64[2 * m] += rm;
                     m64[2 * m + 1] += imm;
                 } else {
-                    m32[2 * (m - P64)] += (float)rm;
-                    m32[2 * (m - P64) + 1] += (float)imm;
+                    t32[2 * (m - P64)] += rm;
+                    t32[2 * (m - P64) + 1] += imm;
                 }
             }
         }
@@ -709,7 +716,7 @@ __global__ void __launch_bounds__(kMomThreads, 2)
 #pragma unroll
     for (int k = 0; k < 2 * P64; ++k) acc[2 + k] = m64[k];
 #pragma unroll
-    for (int k = 0; k < 2 * P32; ++k) acc[2 + 2 * P64 + k] = (double)m32[k];
+    for (int k = 0; k < 2 * P32; ++k) acc[2 + 2 * P64 + k] = m32[k] + t32[k];
     acc[2 + 2 * kMuMomP] = g0;
     block_store<NV>(acc, partial);
 }
