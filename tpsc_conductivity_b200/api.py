@@ -386,9 +386,11 @@ def _scalar_names():
     return SCALAR_NAMES
 
 
-def solve_points(params, ctx=None, streams=2):
+def solve_points(params, ctx=None, streams=None):
     """tpsc_solve_points: the rows (nk0, Nw0, n, T, tp, tpp, t3, U) solved by
     shape groups in the Newton-form mixed solve, one graph launch per group.
+    ``streams`` sets how many streams the groups go over
+    (tpsc_set_group_streams); None leaves the context's, 4 at first.
     Returns (scalars [npts, TPSC_S_COUNT], status [npts], wall ms)."""
     ctx = ctx or Context()
     p = np.ascontiguousarray(params, dtype=np.float64)
@@ -396,7 +398,8 @@ def solve_points(params, ctx=None, streams=2):
     res = np.zeros((n, len(_scalar_names())))
     st = np.zeros(n, dtype=np.int32)
     ms = np.zeros(1)
-    ctx.call("tpsc_set_group_streams", int(streams))
+    if streams is not None:
+        ctx.call("tpsc_set_group_streams", int(streams))
     ctx.call("tpsc_solve_points", n, _dptr(p), _dptr(res), st.ctypes.data_as(_lib._ip), _dptr(ms))
     return res, st, float(ms[0])
 
