@@ -123,12 +123,14 @@ int tpsc_set_nsr(tpsc_ctx *ctx, double nsr);
 int tpsc_set_graph_mode(tpsc_ctx *ctx, int mode);
 
 /* Tilings of the three tau transforms (chi0, V, Sigma), process-wide per
- * Nw0: tile 0 one column pair per CTA (two CTAs per SM, the default), 1 four
- * columns per CTA.  tpsc_tune_tau_tiles times both on the current grid after
- * a solve (reps runs each) and keeps the faster of each; ms (may be NULL)
+ * Nw0: tile 0 the default (up to Nw0 = 2048 several column pairs per CTA, an
+ * FFT group each; at 4096, and for chi0 in the FP64 forms, one column pair
+ * per CTA), 1 four columns per CTA.  tpsc_tune_tau_tiles times both on the
+ * current grid after a solve (reps runs each) and keeps the faster of each,
+ * chi0's for the precision of the context's form; ms (may be NULL)
  * receives the mean times, ms[2 kind + tile].  The transforms run in place,
  * so the next solve recomputes the grid's stages.  tpsc_set_tau_tile sets
- * one tiling (kind 0 chi0, 1 V, 2 Sigma). */
+ * one tiling (kind 0 chi0, in every form, 1 V, 2 Sigma). */
 int tpsc_tune_tau_tiles(tpsc_ctx *ctx, int reps, double ms[6]);
 /* The same tuner over the FFT plan as well: tile 2 = one column pair per CTA
  * with radix-8 FFT passes (twice the threads in the FFT; Nw0 <= 2048), timed

@@ -2310,10 +2310,16 @@ int tpsc_get_sigma_tau(tpsc_ctx *ctx, int j, double *out) {
     return TPSC_OK;
 }
 
+// the slot of a transform's tiling in the context's form
+static int tau_slot(const tpsc_ctx *ctx, int kind) {
+    return kind == kTauChi0 && !mixed(ctx) ? kTauChi0Keep : kind;
+}
+
 // The tiling of the three tau transforms for the current grid's Nw0, picked
-// by timing: each transform runs in both tilings (one column pair per CTA,
-// four columns per CTA) reps times on this grid's buffers after one warm-up,
-// and the faster stays (process-wide).  ms[2 kind + tile] receives the mean
+// by timing: each transform runs in both tilings (the default, see
+// tpsc_set_tau_tile, and four columns per CTA) reps times on this grid's
+// buffers after one warm-up, and the faster stays (process-wide, chi0's for
+// the form's precision).  ms[2 kind + tile] receives the mean
 // times (kind 0 chi0, 1 V, 2 Sigma).  The transforms run in place, so the
 // grid's stage results are stale afterwards: the next solve recomputes them.
 int tpsc_tune_tau_tiles(tpsc_ctx *ctx, int reps, double ms[6]) {
@@ -2329,7 +2335,7 @@ int tpsc_tune_tau_tiles(tpsc_ctx *ctx, int reps, double ms[6]) {
         double best = 0.0;
         int pick = 0;
         for (int tile = 0; tile < 2; ++tile) {
-            set_tau_tile(kind, d.nw0, tile);
+            set_tau_tile(tau_slot(ctx, kind), d.nw0, tile);
             auto run = [&]() -> cudaError_t {
                 if (kind == kTauChi0) return launch_chi0_tau(d, g->chiq, g->dchiqt0, g->cinf, g->cinf2, ctx->T, ctx->st, !mixed(ctx));
                 if (kind == kTauVertex) return launch_vertex_tau(d, g->V, g->chirt, ctx->U, ctx->dres, ctx->st);
@@ -2349,16 +2355,16 @@ int tpsc_tune_tau_tiles(tpsc_ctx *ctx, int reps, double ms[6]) {
                 pick = tile;
             }
         }
-        set_tau_tile(kind, d.nw0, pick);
+        set_tau_tile(tau_slot(ctx, kind), d.nw0, pick);
     }
     g->have_chi0 = g->have_V = g->have_S = g->have_mom = g->have_U = false;
     return TPSC_OK;
 }
 
 // The FFT plan and tiling of the three tau transforms for the current grid's
-// Nw0: one column pair per CTA with radix-16 passes (0), four columns per CTA
-// (1), one pair per CTA with radix-8 passes (2, Nw0 <= 2048: twice the
-// threads in the FFT, one more pass) -- each timed as in
+// Nw0: the default with radix-16 passes (0), four columns per CTA (1), one
+// pair per CTA with radix-8 passes (2, Nw0 <= 2048: twice the threads in the
+// FFT, one more pass) -- each timed as in
 // tpsc_tune_tau_tiles, the fastest kept; ms[3 kind + plan] (plan 2 is 0
 // where it does not apply).
 int tpsc_tune_tau_plans(tpsc_ctx *ctx, int reps, double ms[9]) {
@@ -2377,7 +2383,7 @@ int tpsc_tune_tau_plans(tpsc_ctx *ctx, int reps, double ms[9]) {
         for (int plan = 0; plan < 3; ++plan) {
             if (ms) ms[3 * kind + plan] = 0.0;
             if (plan >= nplans) continue;
-            set_tau_tile(kind, d.nw0, plan);
+            set_tau_tile(tau_slot(ctx, kind), d.nw0, plan);
             auto run = [&]() -> cudaError_t {
                 if (kind == kTauChi0) return launch_chi0_tau(d, g->chiq, g->dchiqt0, g->cinf, g->cinf2, ctx->T, ctx->st, !mixed(ctx));
                 if (kind == kTauVertex) return launch_vertex_tau(d, g->V, g->chirt, ctx->U, ctx->dres, ctx->st);
@@ -2397,19 +2403,21 @@ int tpsc_tune_tau_plans(tpsc_ctx *ctx, int reps, double ms[9]) {
                 pick = plan;
             }
         }
-        set_tau_tile(kind, d.nw0, pick);
+        set_tau_tile(tau_slot(ctx, kind), d.nw0, pick);
     }
     g->have_chi0 = g->have_V = g->have_S = g->have_mom = g->have_U = false;
     return TPSC_OK;
 }
 
-// the tiling of one tau transform for one Nw0 (kind 0 chi0, 1 V, 2 Sigma;
-// tile 0 one column pair per CTA, 1 four columns per CTA, 2 one pair per CTA
-// with radix-8 FFT passes, Nw0 <= 2048)
+// the tiling of one tau transform for one Nw0 (kind 0 chi0, in every form, 1 V,
+// 2 Sigma; tile 0 the default: up to Nw0 = 2048 several column pairs per CTA, one
+// FFT group each, at 4096 and for the FP64 forms' chi0 one pair per CTA; 1 four
+// columns per CTA; 2 one pair per CTA with radix-8 FFT passes, Nw0 <= 2048)
 int tpsc_set_tau_tile(int kind, int nw0, int tile) {
     if (kind < 0 || kind > 2 || tile < 0 || tile > 2 || !supported_grid(8, nw0) || (tile == 2 && nw0 > 2048))
         return fail(nullptr, TPSC_ERR_ARG, "need kind 0..2, tile 0..2 (2: Nw0 <= 2048) and a supported Nw0");
     set_tau_tile(kind, nw0, tile);
+    if (kind == kTauChi0) set_tau_tile(kTauChi0Keep, nw0, tile);
     return TPSC_OK;
 }
 

@@ -35,7 +35,7 @@ static std::atomic<long long> g_launches{0};
 // tpsc_tune_tau_plans): 0 one column pair per CTA, radix-16 FFT passes;
 // 1 four columns per CTA (k_*_tau); 2 one pair per CTA with radix-8 passes
 // (k_*_tau2<N, 8>, N <= 2048; 0 elsewhere)
-static std::atomic<int> g_tau_tile[3][13];
+static std::atomic<int> g_tau_tile[4][13];
 static std::atomic<long long> g_tau_tiles_version{0};
 static int tile_index(int n) {
     int k = 0;
@@ -1845,11 +1845,11 @@ dim3 tau3_grid(const GridDev &g, const Bp &b) {
 }
 template <int N>
 struct RunChi0Tau {
-    // (a batched launch, b->pp set, always takes the pair-per-CTA kernel)
+    // (a batched launch, b->pp set, has no four-column tiling: the default instead)
     static cudaError_t run(const GridDev *g, double *chiq, const double *dchiqt0, double *cinf, double *cinf2,
                            double T, bool keep, const Bp *b, cudaStream_t st) {
         cudaError_t e;
-        const int tile = tau_tile(kTauChi0, N);
+        const int tile = tau_tile(keep ? kTauChi0Keep : kTauChi0, N);
         if constexpr (N <= kTau3Max) {
             if (!keep && (tile == 0 || (tile == 1 && b->pp))) {
                 const size_t sm = Tau3Plan<N>::bytes;

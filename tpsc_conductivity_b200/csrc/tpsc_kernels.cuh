@@ -469,7 +469,9 @@ cudaError_t launch_store(double *dst, const double *v, int n, cudaStream_t st);
 // tiling of the tau transforms (chi0, V, Sigma) per N, process-wide: 0 one
 // column pair per CTA (the default), 1 four columns per CTA; the version
 // counts the changes
-constexpr int kTauChi0 = 0, kTauVertex = 1, kTauSigma = 2;
+// (chi0's tiling apart for launches that keep the order of sums, the FP64 forms': their
+// default is another kernel, so that a tiling timed in one form says nothing of the other)
+constexpr int kTauChi0 = 0, kTauVertex = 1, kTauSigma = 2, kTauChi0Keep = 3;
 int tau_tile(int kind, int n);
 void set_tau_tile(int kind, int n, int tile);
 long long tau_tiles_version();
