@@ -804,7 +804,7 @@ int al_batch(const GridDev &g, int K4, int nfreq) {
     // 1024 (96 frequencies): 10 a launch 14.2 ms, 5 15.1, 2 16.4, 1 18.9; 32^2 x
     // 256 (40): 14 a launch 1.2 ms, 2 2.0, 1 3.2.
     const size_t bytes = (size_t)3 * (g.nw0 + 1) * ((K4 + 1) & ~1) * sizeof(double2);
-    const int fill = (148 * 64 + K4 - 1) / K4, room = (int)std::max<size_t>(1, ((size_t)1 << 30) / bytes);
+    const int fill = (sm_count() * 64 + K4 - 1) / K4, room = (int)std::max<size_t>(1, ((size_t)1 << 30) / bytes);
     return std::max(1, std::min({fill, room, nfreq, 40}));
 }
 

@@ -313,16 +313,21 @@ __device__ __forceinline__ void prefetch_l2_blockrow(const double *a, int j, int
         asm volatile("prefetch.global.L2 [%0];" ::"l"(a + ((size_t)b * NJ + j) * 4));
 }
 
+// SMs of the current device (148 on a whole B200; 0 on an error)
+inline int sm_count() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    return sms;
+}
 // CTAs that one launch of `kernel` holds on the GPU at once: a slice kernel's
 // CTA j prefetches the inputs of slice j + this, which the same launch reaches
 // about one wave later
 template <class K>
 int resident_ctas(K kernel, int threads, size_t smem) {
-    int dev = 0, sms = 0, per = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    int per = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem) != cudaSuccess) return 0;
-    return sms * per;
+    return sm_count() * per;
 }
 
 // Fill a symmetric NBK x NBK slice from the octant points: value(o) does all

@@ -2052,7 +2052,7 @@ cudaError_t launch_sumrule(const GridDev &g, const double *chiq, const double *c
     const int nblk = g.n8p / 4;
     if (jdir < g.nb && !tail) {
         // low frequencies only: a short grid over the flattened (block, j) index
-        const int grid = (int)std::min<long long>(2 * 148, ((long long)nblk * jdir + kRedThreads - 1) / kRedThreads);
+        const int grid = (int)std::min<long long>(std::max(1, 2 * sm_count()), ((long long)nblk * jdir + kRedThreads - 1) / kRedThreads);
         k_sumrule_low<<<std::max(grid, 1), kRedThreads, 0, st>>>(reinterpret_cast<const double4 *>(chiq), g.w16,
                                                                   g.nb, nblk, jdir, Uv, sign, T / Nq, r);
         return launched();
@@ -2237,7 +2237,7 @@ cudaError_t launch_trace_diff_G(const GridDev &g, const double2 *S, const double
     if (jdir < 0 || jdir > NO) jdir = NO;
     const int nblk = g.n8p / 4;
     if (!tail) {
-        const int grid = (int)std::min<long long>(2 * 148, ((long long)nblk * jdir + kRedThreads - 1) / kRedThreads);
+        const int grid = (int)std::min<long long>(std::max(1, 2 * sm_count()), ((long long)nblk * jdir + kRedThreads - 1) / kRedThreads);
         k_trace_diff_G_low<<<std::max(grid, 1), kRedThreads, 0, st>>>(S, s2, s3, sinf, g.ek, g.w16, g.nw0, nblk, mu0,
                                                                        pmu, T, jdir, r);
         return launched();

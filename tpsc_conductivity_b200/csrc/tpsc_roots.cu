@@ -1106,7 +1106,8 @@ __global__ void __launch_bounds__(kRootThreads, 2) k_mu_zero(MuRootArgs a) {
 // after it had read e.  kSlotCopies copies of a set, each for as many readers, as one
 // would be polled by every SM at once.  With more column blocks every block would
 // poll (and wait for) hundreds of slots: there the kernels above are faster
-// (537 column blocks: 348 and 324 us a search, with slots 373 and 355).
+// (537 column blocks: 348 and 324 us a search, with slots 373 and 355).  The lattices
+// have 4, 12, 39, 141, 537 and 2097 column blocks: any bound from 141 to 536 is this rule.
 constexpr int kSlotBlocks = 148, kSlotCopies = 8, kSlotStride = 160;
 static_assert(2 * 2 * kSlotCopies * kSlotStride <= kRootPartial && kSlotStride >= kSlotBlocks, "slots do not fit");
 __device__ __forceinline__ void slot_store(ulonglong2 *p, double x, unsigned n) {
@@ -1603,7 +1604,7 @@ cudaError_t launch_sigma_moments(const GridDev &g, const double2 *S, const doubl
     // leave four blocks per SM: fewer reductions and, at small cutoffs, full blocks;
     // at 129 lines and more than 1024 frequencies, or one point of 65 lines and
     // less, one each, as a grid without its last blocks would be slower
-    const int nblk = g.n8p / 4, fill = 4 * 148;
+    const int nblk = g.n8p / 4, fill = std::max(1, 4 * sm_count());
     auto per = [&](int units, int most) {
         int k = 1;
         while (2 * k <= most && (long long)units * b.P >= 2LL * k * fill) k *= 2;
