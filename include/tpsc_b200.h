@@ -73,10 +73,10 @@ enum tpsc_scalar {
  *    high frequencies of the sum rules and of Tr(G-G0) enter as power series
  *    from moments computed once per search (truncation below 1e-19 of the
  *    leading term).  Same roots to ~1e-14, several times fewer passes;
- *  TPSC_FORM_MIXED (2): the G(r, tau), chi0(q, tau) and V(q) slice transforms
- *    in FP32 with compensated twiddles (G stored in FP32); Sigma's
- *    transforms, every tau transform, the sum rules, traces, roots and the
- *    continuation in FP64.  Sigma within ~1e-6 of the FP64 forms.
+ *  TPSC_FORM_MIXED (2): the slice transforms of G(r, tau), chi0(q, tau), V(q)
+ *    and Sigma in FP32 with compensated twiddles (G stored in FP32, Sigma's
+ *    near field in FP64); every tau transform, the sum rules, traces, roots
+ *    and the continuation in FP64.  Sigma within ~1e-6 of the FP64 forms.
  * Neither NEWTON nor MIXED has a counterpart in the reference.
  * In every form the searches for Usp, Uch and mu are cooperative launches
  * whose blocks exchange values; a wait for another block ends after 1.5 s of
@@ -111,8 +111,8 @@ int tpsc_set_form(tpsc_ctx *ctx, int form);
  * src/chi.cpp:931-981) keeps its constructor's nsr. */
 int tpsc_set_nsr(tpsc_ctx *ctx, double nsr);
 
-/* CUDA graphs for Newton-form solves (no counterpart in the reference, whose
- * solve runs on the host).  A Newton-form tpsc_solve queues its launches with
+/* CUDA graphs for solves (no counterpart in the reference, whose solve runs
+ * on the host).  A tpsc_solve, in any form, queues its launches with
  * no host round trip, so the whole solve from the chi0 stage to the final
  * readback can run as one captured graph.  mode 0: direct launches; 1
  * (default): a solve whose launches repeat those of the previous solve
@@ -318,8 +318,9 @@ int tpsc_get_chijj(tpsc_ctx *ctx, double *chijj1, double *chijj2, double *kx0, d
  * grid of mmin (src/cond_opt.cpp:5123-5155): every n up to (Nw0/2)/2^mmin,
  * then mmin blocks of (Nw0/2)/2^(mmin+1) points whose spacing doubles; the
  * entry n = 0 is not computed and stays 0, as in the reference.  n_theta >= 1
- * angle bins as in tpsc_chijj; 0 <= mmin <= 24.  Each grid frequency costs
- * about one and a half tpsc_chijj. */
+ * angle bins as in tpsc_chijj; 0 <= mmin <= 24.  Its tables and a batch of
+ * frequencies take 0.6 GB at 64^2 x 1024, 1.4 GB at 128^2 x 2048 and 8.1 GB at
+ * 256^2 x 4096 on the device, kept with the grid. */
 int tpsc_chijj3(tpsc_ctx *ctx, int mmin, int n_theta);
 /* Results of the last tpsc_chijj3: *n_freq = N, the grid size; then, where the
  * pointer is not NULL (cap >= N is required for those), ind_freq [N] the
@@ -480,7 +481,7 @@ void tpsc_batch_destroy(tpsc_batch *b);
 const char *tpsc_batch_last_error(const tpsc_batch *b);
 int tpsc_batch_streams(const tpsc_batch *b, int *nstreams);
 /* tpsc_set_graph_mode of every context of the batch (default 1); with 2,
- * each Newton-form point runs as one graph launch, the graph of its grid
+ * each point runs as one graph launch, the graph of its grid
  * updated in place for the point's model; with 3, a Newton + mixed sweep runs
  * by shape groups, one launch per stage over every point of a group, one
  * graph launch per group (tpsc_solve_points on the first context). */

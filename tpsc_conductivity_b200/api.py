@@ -63,7 +63,7 @@ class Green:
         self.ctx.call("tpsc_set_form", int(form))
 
     def set_graph_mode(self, mode):
-        """CUDA graphs for Newton-form solves of the context: 0 off, 1 replay a
+        """CUDA graphs for the solves of the context: 0 off, 1 replay a
         repeated solve (default), 2 capture every solve."""
         self.ctx.call("tpsc_set_graph_mode", int(mode))
 
@@ -478,7 +478,7 @@ class Batch:
         return rows, st, ms.value
 
     def set_graph_mode(self, mode):
-        """tpsc_set_graph_mode of every solver context (2: each Newton-form
+        """tpsc_set_graph_mode of every solver context (2: each
         point is one graph launch, updated in place per point; 3: a Newton +
         mixed sweep by shape groups, one graph launch per (nk0, Nw0) group
         whose kernels each run over all its points)."""

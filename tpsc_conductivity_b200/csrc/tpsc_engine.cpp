@@ -1568,7 +1568,7 @@ int tpsc_sumrule_tangents(tpsc_ctx *ctx, double out[9]) {
             const double ez = std::exp(-std::fabs(z)), f = z > 0 ? ez / (1.0 + ez) : 1.0 / (1.0 + ez);
             bf[o] = beta * f;
             deps[o] = -4.0 * g->ktab[l] * g->ktab[m];
-            // the density's weight (k_density) times df/dxi = -beta f (1 - f)
+            // the density's weight (density_total) times df/dxi = -beta f (1 - f)
             double w = 8;
             if (l == 0 || l == nbk - 1) w /= 2;
             if (m == 0 || m == nbk - 1) w /= 2;

@@ -1183,10 +1183,10 @@ __global__ void __launch_bounds__(kRedThreads)
 // Per-frequency moments of chi0 for the sum-rule series of the Newton form:
 // mom[j][k] = sum_q w_q f_j chi(q, iq_j)^(k+2), k < kMomP (f_0 = 1/2, else 1),
 // and cmax[j] = max_q |chi(q, iq_j)|.  One block per frequency j, a fixed
-// reduction order (deterministic).  With |h chi| < kTailSeriesMax for every
+// reduction order (deterministic).  With |h chi| < kMomSeriesMax for every
 // q at frequencies j >= jdir,
 //   sum_{q, j >= jdir} w f [chi/(1 + h chi) - chi] = sum_{m=1}^{kMomP} (-h)^m M_{m+1}
-// up to a relative (kTailSeriesMax)^kMomP.
+// up to a relative (kMomSeriesMax)^kMomP.
 __global__ void __launch_bounds__(256)
     k_chi0_moments(const double4 *__restrict__ chiq, const double *__restrict__ w16, int nb, int nblk,
                    double *__restrict__ mom, double *__restrict__ cmax, Bp b) {

@@ -1,6 +1,8 @@
-// tpsc_roots.cu -- the Newton form's root searches on the device.
+// tpsc_roots.cu -- the root searches on the device: the Newton form's, then the
+// reference form's (find_zero, tpsc_findzero.h, over the same grid-wide sums) and
+// the Fermi-surface hot spot's.
 //
-// The sum-rule roots Usp and Uch (chi::find_Usp_Uch(nq0, nw0, Usc),
+// The Newton form's: the sum-rule roots Usp and Uch (chi::find_Usp_Uch(nq0, nw0, Usc),
 // src/chi.cpp:846-876) as one cooperative kernel: every block sums its share
 // of the stored frequencies below the series cut, a grid barrier, then every
 // block adds the partials and the high-frequency moment series and takes the
@@ -10,8 +12,8 @@
 //
 // The grid barrier spins on a generation counter with a wall-time bound:
 // the launch is cooperative (every block resident), so the bound only ends
-// a wait that could not otherwise end; it then sets the error flag, every
-// block leaves, and the host reports the failure.
+// a wait for blocks that are off the GPU all that time; it then sets the error
+// flag, every block leaves, and the host repeats the search in one block.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -132,12 +134,13 @@ struct SumRootArgs {
     double T, scale, n, nsr, U, hi_sp;
     const double *chi0max;  // device max chi0(q, 0), or null: hi_sp as given
     double hi_off;          // hi_sp = 2 / chi0max - hi_off
-    double *partial;  // [2][2 kRootMaxBlocks]: two buffers of (value, derivative) per block
+    double *partial;  // [kRootPartial]: two buffers of kRootVals values per block, or of one per
+                      // column block (k_sumrule_zero), or the slots (k_sumrule_slots)
     unsigned *bar;    // [2], zero at launch
     int *err;         // zero at launch
     double *out;      // Usp, Uch, evals_sp, evals_ch, ok_sp, ok_ch
     Bp b;             // batched launch: point blockIdx.z, blocks blockIdx.x of gridDim.x per point
-    int cached;  // (k_sumrule_zero) column blocks of a block whose rows are kept in its shared memory
+    int cached;       // (k_sumrule_slots) column blocks of a block whose rows are kept in its shared memory
 };
 
 // the value and its derivatives, each summed in a fixed order, into
@@ -492,11 +495,14 @@ __global__ void __launch_bounds__(kMomThreads, 2)
     double tsg = 0.0, har = 0.0, g0 = 0.0;
     double m64[2 * P64];
     float m32[2 * P32];
-    double t32[2 * P32];  // the tail's columns
 #pragma unroll
     for (int k = 0; k < 2 * P64; ++k) m64[k] = 0.0;
 #pragma unroll
-    for (int k = 0; k < 2 * P32; ++k) t32[k] = m32[k] = 0.0f;
+    for (int k = 0; k < 2 * P32; ++k) m32[k] = 0.0f;
+    // a tail block's FP64 sums of the FP32 moments over its columns, a thread's at
+    // t32[k][threadIdx.x], in place of the Sigma rows (in registers they spilled)
+    double(*const t32)[kMomThreads] = reinterpret_cast<double(*)[kMomThreads]>(s_row);
+    static_assert(sizeof(s_row) >= 2 * P32 * kMomThreads * sizeof(double), "the tail's sums do not fit");
     // z = i w_n - x - Sigma with x = eps - mu0; inv = 1 / (w_n^2 + x^2)
     // rr = 1/|z|^2 (|z| >= w_n > 0)
     auto moments_rr = [&](double zx, double zy, double rr, double x, double w, double inv) {
@@ -618,6 +624,8 @@ __global__ void __launch_bounds__(kMomThreads, 2)
         const int lane = threadIdx.x & 31, sub = lane & 15, half = threadIdx.x >> 4;
         const double w_no = (2 * NO + 1) * pt;
         double sre = 0.0, sim = 0.0;  // lanes sub < kMuMomP: w C_sub, sub = kMuMomP: w G0
+#pragma unroll
+        for (int k = 0; k < 2 * P32; ++k) t32[k][threadIdx.x] = 0.0;
         for (int r = 0; r < per_t; ++r) {
             const int o = ((blockIdx.x - nsb) * per_t + r) * kMomTailCols + half;
             const double w = o < 4 * nblk ? __ldg(&w16[o]) : 0.0;
@@ -687,7 +695,7 @@ __global__ void __launch_bounds__(kMomThreads, 2)
                     }
 #pragma unroll
                     for (int k = 0; k < 2 * P32; ++k) {
-                        t32[k] += m32[k];
+                        t32[k][threadIdx.x] += m32[k];
                         m32[k] = 0.0f;
                     }
                 }
@@ -702,8 +710,8 @@ __global__ void __launch_bounds__(kMomThreads, 2)
                     m64[2 * m] += rm;
                     m64[2 * m + 1] += imm;
                 } else {
-                    t32[2 * (m - P64)] += rm;
-                    t32[2 * (m - P64) + 1] += imm;
+                    t32[2 * (m - P64)][threadIdx.x] += rm;
+                    t32[2 * (m - P64) + 1][threadIdx.x] += imm;
                 }
             }
         }
@@ -716,7 +724,7 @@ __global__ void __launch_bounds__(kMomThreads, 2)
 #pragma unroll
     for (int k = 0; k < 2 * P64; ++k) acc[2 + k] = m64[k];
 #pragma unroll
-    for (int k = 0; k < 2 * P32; ++k) acc[2 + 2 * P64 + k] = m32[k] + t32[k];
+    for (int k = 0; k < 2 * P32; ++k) acc[2 + 2 * P64 + k] = (int)blockIdx.x < nsb ? m32[k] : t32[k][threadIdx.x];
     acc[2 + 2 * kMuMomP] = g0;
     block_store<NV>(acc, partial);
 }
@@ -727,12 +735,12 @@ struct MuRootArgs {
     const double *mom;  // the k_sigma_moments results
     int nw0, nblk, jc;
     double mu0, T, nk02, wc;  // wc = w_jc
-    double *partial;  // [2][2 kRootMaxBlocks]
+    double *partial;  // as above
     unsigned *bar;
     int *err;
     double *out;  // mu, evals, ok, Tr Sigma G at mu
     Bp b;         // batched launch: point blockIdx.z
-    int cached;  // (k_mu_zero) as above, Sigma
+    int cached;   // (k_mu_slots) as above, Sigma
 };
 
 // the four octant points of column block blk at frequency j of
@@ -1101,9 +1109,9 @@ __global__ void __launch_bounds__(kRootThreads, 2) k_mu_zero(MuRootArgs a) {
 // is two 64-bit words, each half of the value and the number of the evaluation: a word
 // is stored and loaded whole, so that no order between words or slots matters and the
 // accesses are relaxed (with an empty-slot value instead of the number the stores had to
-// release and the loads to acquire, and every kernel's L1 was emptied: 5% slower).  Two sets of slots in turn: a block
-// stores evaluation e + 2 after it has read all of e + 1, which every block stored
-// after it had read e.  kSlotCopies copies of a set, each for as many readers, as one
+// release and the loads to acquire, and every kernel's L1 was emptied: 5% slower).
+// Two sets of slots in turn: a block stores evaluation e + 2 after it has read all of
+// e + 1, which every block stored after it had read e.  kSlotCopies copies of a set, each for as many readers, as one
 // would be polled by every SM at once.  With more column blocks every block would
 // poll (and wait for) hundreds of slots: there the kernels above are faster
 // (537 column blocks: 348 and 324 us a search, with slots 373 and 355).  The lattices
