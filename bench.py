@@ -406,9 +406,9 @@ def our_arm(a, world, rank, local_rank):
                    "parallelism": "replicas" if world > 1 else "single GPU",
                    "l2": "512 MB flush before every step; working set ~2.4 GB per solve",
                    "sumrule_evals": int(sc["evals_sp"] + sc["evals_ch"]), "mu_evals": int(sc["evals_mu"]),
-                   "launch": "Newton-form solves replay one captured CUDA graph (tpsc_set_graph_mode 1: "
-                             "same kernels and arguments as direct launches); the FP64 drop-in with the "
-                             "reference's root searches runs direct launches with its host round trips"},
+                   "launch": "solves of every form replay one captured CUDA graph (tpsc_set_graph_mode 1: "
+                             "same kernels and arguments as direct launches); the FP64 drop-in runs the "
+                             "reference's root searches on the device"},
         "solve_graph": graph_stats,
         "tau_tiles": tau_tiles,
         "slice_plans": slice_plans,
