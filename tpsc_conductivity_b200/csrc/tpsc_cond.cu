@@ -367,7 +367,7 @@ __device__ __forceinline__ double part_of(double2 z, int q) { return q == 0 ? z.
 // transforms' latencies at 16 warps per SM.  One transform at a time in 128 or
 // 256 threads at 240 registers (8 warps per SM), with four exponentials, five
 // more divisions per point and the roots' Newton polish in the pair loop took
-// 8290 us at 256^2 x 4096 and 937 at 128^2 x 2048; this takes 3265 and 453.
+// 8290 us at 256^2 x 4096 and 937 at 128^2 x 2048; this takes 3300 and 461.
 // The tails' exponentials exp(-|r| tau_j) are products of two table entries
 // (formed per pair) when the roots are real, as they are for Sigma_inf > 0.
 template <int N>
