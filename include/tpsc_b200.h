@@ -123,9 +123,9 @@ int tpsc_set_nsr(tpsc_ctx *ctx, double nsr);
 int tpsc_set_graph_mode(tpsc_ctx *ctx, int mode);
 
 /* Tilings of the three tau transforms (chi0, V, Sigma), process-wide per
- * Nw0: tile 0 the default (up to Nw0 = 2048 several column pairs per CTA, an
- * FFT group each; at 4096, and for chi0 in the FP64 forms, one column pair
- * per CTA), 1 four columns per CTA.  tpsc_tune_tau_tiles times both on the
+ * Nw0: tile 0 the default (one column pair per CTA, or, of launches beyond one
+ * wave of those up to Nw0 = 2048, several pairs per CTA, an FFT group each; not
+ * chi0 in the FP64 forms), 1 four columns per CTA.  tpsc_tune_tau_tiles times both on the
  * current grid after a solve (reps runs each) and keeps the faster of each,
  * chi0's for the precision of the context's form; ms (may be NULL)
  * receives the mean times, ms[2 kind + tile].  The transforms run in place,

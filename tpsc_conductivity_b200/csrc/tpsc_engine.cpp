@@ -2410,9 +2410,10 @@ int tpsc_tune_tau_plans(tpsc_ctx *ctx, int reps, double ms[9]) {
 }
 
 // the tiling of one tau transform for one Nw0 (kind 0 chi0, in every form, 1 V,
-// 2 Sigma; tile 0 the default: up to Nw0 = 2048 several column pairs per CTA, one
-// FFT group each, at 4096 and for the FP64 forms' chi0 one pair per CTA; 1 four
-// columns per CTA; 2 one pair per CTA with radix-8 FFT passes, Nw0 <= 2048)
+// 2 Sigma; tile 0 the default: one pair per CTA, or, of launches beyond one wave of
+// those up to Nw0 = 2048, several pairs per CTA, one FFT group each (not the FP64
+// forms' chi0); 1 four columns per CTA; 2 one pair per CTA with radix-8 FFT passes,
+// Nw0 <= 2048)
 int tpsc_set_tau_tile(int kind, int nw0, int tile) {
     if (kind < 0 || kind > 2 || tile < 0 || tile > 2 || !supported_grid(8, nw0) || (tile == 2 && nw0 > 2048))
         return fail(nullptr, TPSC_ERR_ARG, "need kind 0..2, tile 0..2 (2: Nw0 <= 2048) and a supported Nw0");

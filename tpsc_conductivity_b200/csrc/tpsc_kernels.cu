@@ -775,13 +775,18 @@ __global__ void __launch_bounds__(256, 2)
 // tau transforms by groups: a pair of columns is one complex column in a buffer
 // of its own, splined (spline_complex) and transformed in place by one FFT group
 // of G = N/16 threads; a CTA of 128 threads takes 128/G pairs, so that every
-// thread transforms whatever N is, and its barriers are the groups' own.  Pair kernels of 256 threads (k_*_tau2) left all but N/16
-// of them idle in the transform and swept columns of 65 nodes in chunks of one
-// row with 30 warm-up rows.  64 points of the parameter sweep, one launch: chi0 at
+// thread transforms whatever N is, and its barriers are the groups' own.  Pair
+// kernels of 256 threads (k_*_tau2) leave all but N/16 of them idle in the
+// transform and sweep columns of 65 nodes in chunks of one row with 30 warm-up
+// rows.  64 points of the parameter sweep, one launch: chi0 at
 // Nw0 = 256 189 -> 39 us, Sigma 183 -> 39, at 1024 256 -> 115 and 253 -> 132;
 // 128^2 x 2048: chi0 58 -> 45, Sigma 65 -> 55, V 30 -> 26.  At Nw0 = 4096, where
 // the pair kernels' 256 threads all transform, they stay: Sigma 380 us against
 // 399, chi0 306 against 316, V 182 against 189 (half the threads sweep here).
+// They also stay for a launch whose pairs they hold at once (tau_groups): there
+// only the time of one pair counts, and the more threads have the shorter chains.
+// One point, group -> pair kernel: 16^2 x 64 V 10.0 -> 5.3 us, Sigma 16.7 -> 12.1,
+// chi0 15.5 -> 12.7; 64^2 x 1024 V 11.7 -> 8.2, Sigma 20.3 -> 15.8, chi0 18.2 -> 15.0.
 // ---------------------------------------------------------------------------
 constexpr int kTau3Max = 2048;
 template <int N>
@@ -1843,6 +1848,10 @@ template <int N>
 dim3 tau3_grid(const GridDev &g, const Bp &b) {
     return dim3((g.n8p / 2 + Tau3Plan<N>::pairs - 1) / Tau3Plan<N>::pairs, 1, b.P);
 }
+// more column pairs than one wave of the pair kernels (256 threads, two CTAs an SM) takes
+inline bool tau_groups(const GridDev &g, const Bp &b) {
+    return (long long)(g.n8p / 2) * b.P > 2LL * sm_count();
+}
 template <int N>
 struct RunChi0Tau {
     // (a batched launch, b->pp set, has no four-column tiling: the default instead)
@@ -1851,7 +1860,7 @@ struct RunChi0Tau {
         cudaError_t e;
         const int tile = tau_tile(keep ? kTauChi0Keep : kTauChi0, N);
         if constexpr (N <= kTau3Max) {
-            if (!keep && (tile == 0 || (tile == 1 && b->pp))) {
+            if (!keep && (tile == 0 || (tile == 1 && b->pp)) && tau_groups(*g, *b)) {
                 const size_t sm = Tau3Plan<N>::bytes;
                 if ((e = set_smem(k_chi0_tau3<N>, sm)) != cudaSuccess) return e;
                 k_chi0_tau3<N><<<tau3_grid<N>(*g, *b), Tau3Plan<N>::threads, sm, st>>>(
@@ -1901,14 +1910,15 @@ struct RunVertexTau {
             }
         }
         if constexpr (N <= kTau3Max) {
-            if (tile != 1 || b->pp) {
+            if ((tile != 1 || b->pp) && tau_groups(*g, *b)) {
                 const size_t sm = Tau3Plan<N>::bytes;
                 if ((e = set_smem(k_vertex_tau3<N>, sm)) != cudaSuccess) return e;
                 k_vertex_tau3<N><<<tau3_grid<N>(*g, *b), Tau3Plan<N>::threads, sm, st>>>(Vr, chirt, g->tw_w, U, Usc, g->n8,
                                                                                           g->n8p, *b);
                 return launched();
             }
-        } else if (tile != 1 || b->pp) {
+        }
+        if (tile != 1 || b->pp) {
             const size_t sm = Tau2Smem<N>::bytes;
             if ((e = set_smem(k_vertex_tau2<N>, sm)) != cudaSuccess) return e;
             k_vertex_tau2<N><<<dim3(g->n8p / 2, 1, b->P), 256, sm, st>>>(Vr, chirt, g->tw_w, U, Usc, g->n8, *b);
@@ -1937,17 +1947,19 @@ struct RunSigmaTau {
             }
         }
         if constexpr (N <= kTau3Max) {
-            if (tile != 1 || b->pp) {
+            if ((tile != 1 || b->pp) && tau_groups(*g, *b)) {
                 const size_t sm = Tau3Plan<N>::bytes;
                 if ((e = set_smem(k_sigma_tau3<N>, sm)) != cudaSuccess) return e;
                 k_sigma_tau3<N><<<tau3_grid<N>(*g, *b), Tau3Plan<N>::threads, sm, st>>>(
                     sigt, dS, S, s2, s3, s4, sinf, g->spl_full, g->tw_w, g->ht_w, T, g->n8, g->n8p, *b);
                 return launched();
             }
-        } else if (tile != 1 || b->pp) {
+        }
+        if (tile != 1 || b->pp) {
             const size_t sm = Tau2Smem<N>::bytes;
             if ((e = set_smem(k_sigma_tau2<N>, sm)) != cudaSuccess) return e;
-            k_sigma_tau2<N><<<dim3(g->n8p / 2, 1, b->P), 256, sm, st>>>(sigt, dS, S, s2, s3, s4, sinf, g->spl_full, g->tw_w, g->ht_w, T, g->n8, g->n8p, *b);
+            k_sigma_tau2<N><<<dim3(g->n8p / 2, 1, b->P), 256, sm, st>>>(sigt, dS, S, s2, s3, s4, sinf, g->spl_full,
+                                                                       g->tw_w, g->ht_w, T, g->n8, g->n8p, *b);
             return launched();
         }
         const size_t sm = TauSmem<N>::bytes(N + 1);
