@@ -256,6 +256,33 @@ struct SlicePlan {
     static_assert(bytes <= 232448, "slice does not fit in shared memory");
 };
 
+// SMs of the current device (148 on a whole B200; 0 on an error)
+inline int sm_count() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    return sms;
+}
+// A slice launch that PER blocks of kSliceThreads an SM hold at once, up to 65 lines: its
+// time is one slice's, and 352 threads instead of the plan's 64 to 192 shorten the loops
+// that fill and store it (the transform has no more groups than line pairs to give it).
+// The plan's block -> the wide one, one point: 64^2 x 64 G 11.4 -> 7.5 us (FP32) and 8.6 ->
+// 6.3 (FP64), V 8.8 -> 7.7 and 10.0 -> 7.1, chi0 8.5 -> 6.9, Sigma 8.6 -> 7.5; 32^2 x 64
+// G 6.7 -> 5.5; 128^2 x 64 G 15.0 -> 11.6.
+template <class P, int PER>
+struct WidePlan : P {
+    static constexpr int threads = kSliceThreads, blocks = PER;
+    static_assert(P::threads <= kSliceThreads, "a wide block");
+};
+// f(plan) with the plan of a launch of `slices` slices
+template <int NBK, class P, int PER, class F>
+cudaError_t with_plan(long long slices, const F &f) {
+    if constexpr (NBK <= 65) {
+        if (slices <= (long long)PER * sm_count()) return f(WidePlan<P, PER>{});
+    }
+    return f(P{});
+}
+
 // the twiddles of the plan's transform in shared memory (the first
 // __syncthreads of the kernel publishes them)
 template <int NBK, bool KEEP = false>
@@ -316,13 +343,6 @@ __device__ __forceinline__ void prefetch_l2_blockrow(const double *a, int j, int
         asm volatile("prefetch.global.L2 [%0];" ::"l"(a + ((size_t)b * NJ + j) * 4));
 }
 
-// SMs of the current device (148 on a whole B200; 0 on an error)
-inline int sm_count() {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    return sms;
-}
 // CTAs that one launch of `kernel` holds on the GPU at once: a slice kernel's
 // CTA j prefetches the inputs of slice j + this, which the same launch reaches
 // about one wave later

@@ -97,8 +97,8 @@ __global__ void k_gk_table(const double *__restrict__ ek, int n8, double mu0, do
 // needs G(r, tau) and G(r, -tau) (src/chi0.cpp:462-495); G(r,-tau) =
 // -G(r, beta - tau), so one table serves both stages.  Plain layout
 // Grt[j * n8 + o].
-template <int NBK>
-__global__ void __launch_bounds__(SlicePlan<NBK, true>::threads, SlicePlan<NBK, true>::blocks)
+template <int NBK, class P>
+__global__ void __launch_bounds__(P::threads, P::blocks)
     k_gslice(const double2 *__restrict__ gk, const double2 *__restrict__ tw,
              int n8, int nw0, double T, double *__restrict__ Grt) {
     extern __shared__ __align__(16) double S[];
@@ -123,8 +123,8 @@ __global__ void __launch_bounds__(SlicePlan<NBK, true>::threads, SlicePlan<NBK, 
 // chi0(r, tau_j) = -2 G(r, tau_j) G(r, -tau_j) and its DCT-I chi0(q, tau_j),
 // j = 0..Nw0/2 (src/chi0.cpp:393-418, 497-517, 545-558).  tau = 0 uses
 // G(r,0-) = G(r,0+) + delta_r0, tau = beta/2 uses 2 G^2.
-template <int NBK>
-__global__ void __launch_bounds__(SlicePlan<NBK, true>::threads, SlicePlan<NBK, true>::blocks)
+template <int NBK, class P>
+__global__ void __launch_bounds__(P::threads, P::blocks)
     k_chi0_slice(const double *__restrict__ Grt, const double2 *__restrict__ tw,
                  int n8, int nw0, double *__restrict__ chirt, double *__restrict__ chiq) {
     extern __shared__ __align__(16) double S[];
@@ -132,14 +132,14 @@ __global__ void __launch_bounds__(SlicePlan<NBK, true>::threads, SlicePlan<NBK, 
     const int j = blockIdx.x;
     const int nb = nw0 / 2 + 1;
     // G(r, tau_j) and G(r, beta - tau_j) staged in the slice / scratch area
-    static_assert(2 * StageRows<NBK>::drow_bytes <= SlicePlan<NBK, true>::tw_off, "inputs must fit");
+    static_assert(2 * StageRows<NBK>::drow_bytes <= P::tw_off, "inputs must fit");
     double *gp = S;
     double *gm = S + StageRows<NBK>::drow_bytes / sizeof(double);
     stage_drow<NBK>(gp, Grt + (size_t)j * n8);
     stage_drow<NBK>(gm, Grt + (size_t)(nw0 - j) * n8);
     cp_async_wait_all();
     __syncthreads();
-    fill_from_staged<NBK, SlicePlan<NBK, true>::threads>(S, [&](int o) -> double {
+    fill_from_staged<NBK, P::threads>(S, [&](int o) -> double {
         const double a = gp[o];
         double c;
         if (j == 0)
@@ -222,8 +222,8 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
 
 // V(q, iqn) = (T/L^2) U [3 Usp (chisp - chi0) + Uch (chich - chi0)] / 8 and
 // its DCT-I over q, one bosonic frequency per CTA (src/chi.cpp:89-115).
-template <int NBK>
-__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
+template <int NBK, class P>
+__global__ void __launch_bounds__(P::threads, P::blocks)
     k_vertex_q(const double *__restrict__ chiq, const double2 *__restrict__ tw,
                int n8, int nb, double normFact, double U, const double *__restrict__ Usc, double *__restrict__ Vr) {
     extern __shared__ __align__(16) double S[];
@@ -231,12 +231,12 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
     const int j = blockIdx.x;
     const double Usp = Usc[0], Uch = Usc[1];
     // chi0(q, iq_j) staged in the slice / scratch area
-    static_assert(StageRows<NBK>::blockrow_bytes <= SlicePlan<NBK>::tw_off, "inputs must fit");
+    static_assert(StageRows<NBK>::blockrow_bytes <= P::tw_off, "inputs must fit");
     double *cs = S;
     stage_blockrow<NBK>(cs, chiq, j, nb);
     cp_async_wait_all();
     __syncthreads();
-    fill_from_staged<NBK, SlicePlan<NBK>::threads>(S, [&](int o) -> double {
+    fill_from_staged<NBK, P::threads>(S, [&](int o) -> double {
         const double c0 = cs[o];
         const double sp = c0 / (1.0 - Usp * c0 / 2.0);
         const double ch = c0 / (1.0 + Uch * c0 / 2.0);
@@ -303,8 +303,8 @@ __global__ void __launch_bounds__(kSliceThreads, 1)
 // Sigma(k, tau_j) = DCT-I[ G(r, tau_j) V(r, tau_j) ], j = 0..Nw0, with
 // V(r, tau_j) = V(r, beta - tau_j) for tau_j > beta/2 (src/green.cpp:1822-1885),
 // in FP64 (the mixed form's FP32 slice is k_sigma_slice32).
-template <int NBK>
-__global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::blocks)
+template <int NBK, class P>
+__global__ void __launch_bounds__(P::threads, P::blocks)
     k_sigma_slice(const double *__restrict__ Grt, const double *__restrict__ V,
                   const double2 *__restrict__ tw, int n8, int nw0, int ahead, double *__restrict__ sigt) {
     extern __shared__ __align__(16) double S[];
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
         prefetch_l2_blockrow(V, jn < nb ? jn : nw0 - jn, nb, (n8 + 3) / 4);
     }
     // V(r, tau_j) and G(r, tau_j) staged in the slice / scratch area
-    static_assert(StageRows<NBK>::blockrow_bytes + StageRows<NBK>::drow_bytes <= SlicePlan<NBK>::tw_off,
+    static_assert(StageRows<NBK>::blockrow_bytes + StageRows<NBK>::drow_bytes <= P::tw_off,
                   "inputs must fit");
     double *vs = S;
     double *gs = S + StageRows<NBK>::blockrow_bytes / sizeof(double);
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(SlicePlan<NBK>::threads, SlicePlan<NBK>::block
     stage_drow<NBK>(gs, Grt + (size_t)j * n8);
     cp_async_wait_all();
     __syncthreads();
-    fill_from_staged<NBK, SlicePlan<NBK>::threads>(S, [&](int o) -> double { return gs[o] * vs[o]; });
+    fill_from_staged<NBK, P::threads>(S, [&](int o) -> double { return gs[o] * vs[o]; });
     __syncthreads();
     plan_dct2<NBK>(S, tws);
     for (int o = threadIdx.x; o < n8; o += blockDim.x) {
@@ -1771,14 +1771,17 @@ __global__ void k_store(StoreVals s, double *__restrict__ dst) {
 template <int NBK>
 struct RunGslice {
     static cudaError_t run(const GridDev *g, double *Grt, double mu0, double T, cudaStream_t st) {
-        const size_t sm = SlicePlan<NBK, true>::bytes;
-        cudaError_t e = set_smem(k_gslice<NBK>, sm);
-        if (e != cudaSuccess) return e;
         const double nk02 = (double)g->nk0 * g->nk0;
         k_gk_table<<<(g->n8 + 255) / 256, 256, 0, st>>>(g->ek, g->n8, mu0, T, nk02, g->gk, Bp{});
-        if ((e = launched()) != cudaSuccess) return e;
-        k_gslice<NBK><<<g->nw0 + 1, SlicePlan<NBK, true>::threads, sm, st>>>(g->gk, g->tw_k, g->n8, g->nw0, T, Grt);
-        return launched();
+        cudaError_t e = launched();
+        if (e != cudaSuccess) return e;
+        return with_plan<NBK, SlicePlan<NBK, true>, 1>(g->nw0 + 1, [&](auto plan) {
+            using P = decltype(plan);
+            cudaError_t err = set_smem(k_gslice<NBK, P>, P::bytes);
+            if (err != cudaSuccess) return err;
+            k_gslice<NBK, P><<<g->nw0 + 1, P::threads, P::bytes, st>>>(g->gk, g->tw_k, g->n8, g->nw0, T, Grt);
+            return launched();
+        });
     }
 };
 template <int NBK>
@@ -1798,23 +1801,27 @@ struct RunChi0Boundary {
 template <int NBK>
 struct RunChi0Slice {
     static cudaError_t run(const GridDev *g, const double *Grt, double *chirt, double *chiq, cudaStream_t st) {
-        const size_t sm = SlicePlan<NBK, true>::bytes;
-        cudaError_t e = set_smem(k_chi0_slice<NBK>, sm);
-        if (e != cudaSuccess) return e;
-        k_chi0_slice<NBK><<<g->nb, SlicePlan<NBK, true>::threads, sm, st>>>(Grt, g->tw_k, g->n8, g->nw0, chirt, chiq);
-        return launched();
+        return with_plan<NBK, SlicePlan<NBK, true>, 1>(g->nb, [&](auto plan) {
+            using P = decltype(plan);
+            cudaError_t e = set_smem(k_chi0_slice<NBK, P>, P::bytes);
+            if (e != cudaSuccess) return e;
+            k_chi0_slice<NBK, P><<<g->nb, P::threads, P::bytes, st>>>(Grt, g->tw_k, g->n8, g->nw0, chirt, chiq);
+            return launched();
+        });
     }
 };
 template <int NBK>
 struct RunVertexQ {
     static cudaError_t run(const GridDev *g, const double *chiq, double *Vr, double U, const double *Usc, double T,
                            cudaStream_t st) {
-        const size_t sm = SlicePlan<NBK>::bytes;
-        cudaError_t e = set_smem(k_vertex_q<NBK>, sm);
-        if (e != cudaSuccess) return e;
         const double normFact = T / ((double)g->nk0 * g->nk0);
-        k_vertex_q<NBK><<<g->nb, SlicePlan<NBK>::threads, sm, st>>>(chiq, g->tw_k, g->n8, g->nb, normFact, U, Usc, Vr);
-        return launched();
+        return with_plan<NBK, SlicePlan<NBK>, 1>(g->nb, [&](auto plan) {
+            using P = decltype(plan);
+            cudaError_t e = set_smem(k_vertex_q<NBK, P>, P::bytes);
+            if (e != cudaSuccess) return e;
+            k_vertex_q<NBK, P><<<g->nb, P::threads, P::bytes, st>>>(chiq, g->tw_k, g->n8, g->nb, normFact, U, Usc, Vr);
+            return launched();
+        });
     }
 };
 template <int NBK>
@@ -1835,12 +1842,14 @@ struct RunSigmaBoundary {
 template <int NBK>
 struct RunSigmaSlice {
     static cudaError_t run(const GridDev *g, const double *Grt, const double *V, double *sigt, cudaStream_t st) {
-        const size_t sm = SlicePlan<NBK>::bytes;
-        cudaError_t e = set_smem(k_sigma_slice<NBK>, sm);
-        if (e != cudaSuccess) return e;
-        const int ahead = resident_ctas(k_sigma_slice<NBK>, SlicePlan<NBK>::threads, sm);
-        k_sigma_slice<NBK><<<g->nw0 + 1, SlicePlan<NBK>::threads, sm, st>>>(Grt, V, g->tw_k, g->n8, g->nw0, ahead, sigt);
-        return launched();
+        return with_plan<NBK, SlicePlan<NBK>, 1>(g->nw0 + 1, [&](auto plan) {
+            using P = decltype(plan);
+            cudaError_t e = set_smem(k_sigma_slice<NBK, P>, P::bytes);
+            if (e != cudaSuccess) return e;
+            const int ahead = resident_ctas(k_sigma_slice<NBK, P>, P::threads, P::bytes);
+            k_sigma_slice<NBK, P><<<g->nw0 + 1, P::threads, P::bytes, st>>>(Grt, V, g->tw_k, g->n8, g->nw0, ahead, sigt);
+            return launched();
+        });
     }
 };
 

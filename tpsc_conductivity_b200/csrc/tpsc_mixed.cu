@@ -110,8 +110,8 @@ __device__ __forceinline__ void dst_dct_slice32(float *S, const float4 *tws) {
 // G(r, tau_j) = DCT-I[ G0(k, tau_j) / L^2 ] in FP32 (the FP64 k_gslice's
 // stage, src/green.cpp:1830-1841 and src/chi0.cpp:462-495): G0 formed in
 // FP64, rounded once to float; Grt32[j * n8 + o].
-template <int NBK>
-__global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::blocks)
+template <int NBK, class P>
+__global__ void __launch_bounds__(P::threads, P::blocks)
     k_gslice32(const double2 *__restrict__ gk, const float4 *__restrict__ tw,
                int n8, int nw0, double T, float *__restrict__ Grt, Bp b) {
     extern __shared__ __align__(16) float S32[];
@@ -139,8 +139,8 @@ __global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::b
 // chi0(r, tau_j) = -2 G(r, tau_j) G(r, -tau_j) from the FP32 G (the product
 // is exact in FP64 and kept there for the tau transforms), its DCT-I in FP32
 // -> chi0(q, tau_j) in FP64 (src/chi0.cpp:393-418, 497-517, 545-558).
-template <int NBK>
-__global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::blocks)
+template <int NBK, class P>
+__global__ void __launch_bounds__(P::threads, P::blocks)
     k_chi0_slice32(const float *__restrict__ Grt, const float4 *__restrict__ tw,
                    int n8, int nw0, int ahead, double *__restrict__ chirt, double *__restrict__ chiq, Bp b) {
     extern __shared__ __align__(16) float S32[];
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::b
     stage_frow<NBK>(gm, Grt + (size_t)(nw0 - j) * n8);
     cp_async_wait_all();
     __syncthreads();
-    fill_from_staged<NBK, Slice32Plan<NBK>::threads>(S32, [&](int o) -> float {
+    fill_from_staged<NBK, P::threads>(S32, [&](int o) -> float {
         const double a = gp[o];
         double c;
         if (j == 0)
@@ -187,8 +187,8 @@ __global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::b
 // (src/chi.cpp:89-115).  With a = Usp/2, b = Uch/2,
 //   chi_sp - chi0 = a chi0^2 / (1 - a chi0),  chi_ch - chi0 = -b chi0^2 / (1 + b chi0),
 // so that V takes one FP64 division per point.
-template <int NBK>
-__global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::blocks)
+template <int NBK, class P>
+__global__ void __launch_bounds__(P::threads, P::blocks)
     k_vertex_q32(const double *__restrict__ chiq, const float4 *__restrict__ tw,
                  int n8, int nb, int ahead, double normFact, double U, const double *__restrict__ Usc,
                  double *__restrict__ Vr, Bp b) {
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::b
     stage_blockrow<NBK>(cs, chiq, j, nb);
     cp_async_wait_all();
     __syncthreads();
-    fill_from_staged<NBK, Slice32Plan<NBK>::threads>(S32, [&](int o) -> float {
+    fill_from_staged<NBK, P::threads>(S32, [&](int o) -> float {
         const double c0 = cs[o];
         const double a = 0.5 * Usp, b = 0.5 * Uch;
         const double ds = 1.0 - a * c0, dc = 1.0 + b * c0;
@@ -246,8 +246,8 @@ struct SigmaSlice32Smem {
 // FP32, the near field's transform added in FP64 (cos(pi a t / (nbk - 1)) by
 // the Chebyshev recurrence from the FP64 twiddle table entry tw64[t],
 // tw64[m] = exp(-2 pi i m / L), L = 2 (nbk - 1)).
-template <int NBK>
-__global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::blocks)
+template <int NBK, class P>
+__global__ void __launch_bounds__(P::threads, P::blocks)
     k_sigma_slice32(const float *__restrict__ Grt, const double *__restrict__ V, const float4 *__restrict__ tw,
                     const double2 *__restrict__ tw64, int n8, int nw0, int ahead, double *__restrict__ sigt, Bp b) {
     Grt = at(Grt, b.arena);
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(Slice32Plan<NBK>::threads, Slice32Plan<NBK>::b
     cp_async_wait_all();
     __syncthreads();
     // octant points o < NOCT are exactly those with l <= R
-    fill_from_staged<NBK, Slice32Plan<NBK>::threads>(S32, [&](int o) -> float {
+    fill_from_staged<NBK, P::threads>(S32, [&](int o) -> float {
         const double x = (double)gs[o] * vs[o];
         if (o < NOCT) {
             xn[o] = x;
@@ -377,13 +377,16 @@ struct RunGslice32 {
     static cudaError_t run(const GridDev *g, float *Grt, double mu0, double T, const Bp *b, cudaStream_t st) {
         const int plan = slice_plan(kSliceG, NBK);
         if (plan == kSliceDirect && g->dct32) return launch_gslice_dct(*g, Grt, mu0, T, st, *b);
-        const size_t sm = Slice32Plan<NBK>::bytes;
-        cudaError_t e = set_smem(k_gslice32<NBK>, sm);
+        cudaError_t e = launch_gk_table(*g, mu0, T, st, *b);
         if (e != cudaSuccess) return e;
-        if ((e = launch_gk_table(*g, mu0, T, st, *b)) != cudaSuccess) return e;
-        k_gslice32<NBK><<<dim3(g->nw0 + 1, 1, b->P), Slice32Plan<NBK>::threads, sm, st>>>(g->gk, g->tw_k32, g->n8, g->nw0, T,
-                                                                               Grt, *b);
-        return launched();
+        return with_plan<NBK, Slice32Plan<NBK>, 2>((long long)(g->nw0 + 1) * b->P, [&](auto p) {
+            using P = decltype(p);
+            cudaError_t err = set_smem(k_gslice32<NBK, P>, P::bytes);
+            if (err != cudaSuccess) return err;
+            k_gslice32<NBK, P><<<dim3(g->nw0 + 1, 1, b->P), P::threads, P::bytes, st>>>(g->gk, g->tw_k32, g->n8, g->nw0,
+                                                                                       T, Grt, *b);
+            return launched();
+        });
     }
 };
 template <int NBK>
@@ -392,13 +395,15 @@ struct RunChi0Slice32 {
                            cudaStream_t st) {
         const int plan = slice_plan(kSliceChi0, NBK);
         if (plan == kSliceDirect && g->dct32) return launch_chi0_slice_dct(*g, Grt, chirt, chiq, st, *b);
-        const size_t sm = Slice32Plan<NBK>::bytes;
-        cudaError_t e = set_smem(k_chi0_slice32<NBK>, sm);
-        if (e != cudaSuccess) return e;
-        const int ahead = b->P > 1 ? 0 : resident_ctas(k_chi0_slice32<NBK>, Slice32Plan<NBK>::threads, sm);
-        k_chi0_slice32<NBK><<<dim3(g->nb, 1, b->P), Slice32Plan<NBK>::threads, sm, st>>>(Grt, g->tw_k32, g->n8, g->nw0, ahead,
-                                                                              chirt, chiq, *b);
-        return launched();
+        return with_plan<NBK, Slice32Plan<NBK>, 2>((long long)g->nb * b->P, [&](auto p) {
+            using P = decltype(p);
+            cudaError_t e = set_smem(k_chi0_slice32<NBK, P>, P::bytes);
+            if (e != cudaSuccess) return e;
+            const int ahead = b->P > 1 ? 0 : resident_ctas(k_chi0_slice32<NBK, P>, P::threads, P::bytes);
+            k_chi0_slice32<NBK, P><<<dim3(g->nb, 1, b->P), P::threads, P::bytes, st>>>(Grt, g->tw_k32, g->n8, g->nw0,
+                                                                                      ahead, chirt, chiq, *b);
+            return launched();
+        });
     }
 };
 template <int NBK>
@@ -408,14 +413,16 @@ struct RunVertexQ32 {
         const int plan = slice_plan(kSliceVertex, NBK);
         if (plan == kSliceTensor && g->dct_tc) return launch_vertex_q_tc(*g, chiq, Vr, U, Usc, T, st, *b);
         if (plan == kSliceDirect && g->dct32) return launch_vertex_q_dct(*g, chiq, Vr, U, Usc, T, st, *b);
-        const size_t sm = Slice32Plan<NBK>::bytes;
-        cudaError_t e = set_smem(k_vertex_q32<NBK>, sm);
-        if (e != cudaSuccess) return e;
         const double normFact = T / ((double)g->nk0 * g->nk0);
-        const int ahead = b->P > 1 ? 0 : resident_ctas(k_vertex_q32<NBK>, Slice32Plan<NBK>::threads, sm);
-        k_vertex_q32<NBK><<<dim3(g->nb, 1, b->P), Slice32Plan<NBK>::threads, sm, st>>>(chiq, g->tw_k32, g->n8, g->nb, ahead,
-                                                                            normFact, U, Usc, Vr, *b);
-        return launched();
+        return with_plan<NBK, Slice32Plan<NBK>, 2>((long long)g->nb * b->P, [&](auto p) {
+            using P = decltype(p);
+            cudaError_t e = set_smem(k_vertex_q32<NBK, P>, P::bytes);
+            if (e != cudaSuccess) return e;
+            const int ahead = b->P > 1 ? 0 : resident_ctas(k_vertex_q32<NBK, P>, P::threads, P::bytes);
+            k_vertex_q32<NBK, P><<<dim3(g->nb, 1, b->P), P::threads, P::bytes, st>>>(chiq, g->tw_k32, g->n8, g->nb, ahead,
+                                                                                    normFact, U, Usc, Vr, *b);
+            return launched();
+        });
     }
 };
 
@@ -427,12 +434,15 @@ struct RunSigmaSlice32 {
         if (plan == kSliceTensor && g->dct_tc) return launch_sigma_slice_tc(*g, Grt, V, sigt, st, *b);
         if (plan == kSliceDirect && g->dct32) return launch_sigma_slice_dct(*g, Grt, V, sigt, st, *b);
         const size_t sm = SigmaSlice32Smem<NBK>::bytes;
-        cudaError_t e = set_smem(k_sigma_slice32<NBK>, sm);
-        if (e != cudaSuccess) return e;
-        const int ahead = b->P > 1 ? 0 : resident_ctas(k_sigma_slice32<NBK>, Slice32Plan<NBK>::threads, sm);
-        k_sigma_slice32<NBK><<<dim3(g->nw0 + 1, 1, b->P), Slice32Plan<NBK>::threads, sm, st>>>(Grt, V, g->tw_k32, g->tw_k, g->n8,
-                                                                                    g->nw0, ahead, sigt, *b);
-        return launched();
+        return with_plan<NBK, Slice32Plan<NBK>, 2>((long long)(g->nw0 + 1) * b->P, [&](auto p) {
+            using P = decltype(p);
+            cudaError_t e = set_smem(k_sigma_slice32<NBK, P>, sm);
+            if (e != cudaSuccess) return e;
+            const int ahead = b->P > 1 ? 0 : resident_ctas(k_sigma_slice32<NBK, P>, P::threads, sm);
+            k_sigma_slice32<NBK, P><<<dim3(g->nw0 + 1, 1, b->P), P::threads, sm, st>>>(Grt, V, g->tw_k32, g->tw_k, g->n8,
+                                                                                      g->nw0, ahead, sigt, *b);
+            return launched();
+        });
     }
 };
 
