@@ -499,8 +499,11 @@ __global__ void __launch_bounds__(kMomThreads, 2)
     for (int k = 0; k < 2 * P64; ++k) m64[k] = 0.0;
 #pragma unroll
     for (int k = 0; k < 2 * P32; ++k) m32[k] = 0.0f;
-    // a tail block's FP64 sums of the FP32 moments over its columns, a thread's at
-    // t32[k][threadIdx.x], in place of the Sigma rows (in registers they spilled)
+    // the FP32 moments of a tail block: their sums, and those of its columns term by term
+    // (a thread's at t32[k][threadIdx.x], in place of the Sigma rows: in registers they
+    // spilled)
+    double a32[2 * P32];
+    bool slow_any = false;
     double(*const t32)[kMomThreads] = reinterpret_cast<double(*)[kMomThreads]>(s_row);
     static_assert(sizeof(s_row) >= 2 * P32 * kMomThreads * sizeof(double), "the tail's sums do not fit");
     // z = i w_n - x - Sigma with x = eps - mu0; inv = 1 / (w_n^2 + x^2)
@@ -624,8 +627,6 @@ __global__ void __launch_bounds__(kMomThreads, 2)
         const int lane = threadIdx.x & 31, sub = lane & 15, half = threadIdx.x >> 4;
         const double w_no = (2 * NO + 1) * pt;
         double sre = 0.0, sim = 0.0;  // lanes sub < kMuMomP: w C_sub, sub = kMuMomP: w G0
-#pragma unroll
-        for (int k = 0; k < 2 * P32; ++k) t32[k][threadIdx.x] = 0.0;
         for (int r = 0; r < per_t; ++r) {
             const int o = ((blockIdx.x - nsb) * per_t + r) * kMomTailCols + half;
             const double w = o < 4 * nblk ? __ldg(&w16[o]) : 0.0;
@@ -695,9 +696,10 @@ __global__ void __launch_bounds__(kMomThreads, 2)
                     }
 #pragma unroll
                     for (int k = 0; k < 2 * P32; ++k) {
-                        t32[k][threadIdx.x] += m32[k];
+                        t32[k][threadIdx.x] = m32[k] + (slow_any ? t32[k][threadIdx.x] : 0.0);
                         m32[k] = 0.0f;
                     }
+                    slow_any = true;
                 }
         }
         sre += __shfl_down_sync(0xffffffffu, sre, 16);
@@ -705,26 +707,30 @@ __global__ void __launch_bounds__(kMomThreads, 2)
 #pragma unroll
         for (int m = 0; m < kMuMomP; ++m) {
             const double rm = __shfl_sync(0xffffffffu, sre, m), imm = __shfl_sync(0xffffffffu, sim, m);
-            if (lane == 0) {
-                if (m < P64) {
-                    m64[2 * m] += rm;
-                    m64[2 * m + 1] += imm;
-                } else {
-                    t32[2 * (m - P64)][threadIdx.x] += rm;
-                    t32[2 * (m - P64) + 1][threadIdx.x] += imm;
-                }
+            if (m < P64) {
+                m64[2 * m] += lane == 0 ? rm : 0.0;
+                m64[2 * m + 1] += lane == 0 ? imm : 0.0;
+            } else {
+                a32[2 * (m - P64)] = lane == 0 ? rm : 0.0;
+                a32[2 * (m - P64) + 1] = lane == 0 ? imm : 0.0;
             }
         }
+        if (slow_any)
+#pragma unroll
+            for (int k = 0; k < 2 * P32; ++k) a32[k] += t32[k][threadIdx.x];
         const double gt = __shfl_sync(0xffffffffu, sre, kMuMomP);
         if (lane == 0) g0 += gt;
     }
+    if ((int)blockIdx.x < nsb)
+#pragma unroll
+        for (int k = 0; k < 2 * P32; ++k) a32[k] = m32[k];
     double acc[NV];
     acc[0] = tsg * T / nk02;
     acc[1] = har * sinf * T / nk02 + fermi;
 #pragma unroll
     for (int k = 0; k < 2 * P64; ++k) acc[2 + k] = m64[k];
 #pragma unroll
-    for (int k = 0; k < 2 * P32; ++k) acc[2 + 2 * P64 + k] = (int)blockIdx.x < nsb ? m32[k] : t32[k][threadIdx.x];
+    for (int k = 0; k < 2 * P32; ++k) acc[2 + 2 * P64 + k] = a32[k];
     acc[2 + 2 * kMuMomP] = g0;
     block_store<NV>(acc, partial);
 }
