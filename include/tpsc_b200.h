@@ -482,7 +482,8 @@ const char *tpsc_batch_last_error(const tpsc_batch *b);
 int tpsc_batch_streams(const tpsc_batch *b, int *nstreams);
 /* tpsc_set_graph_mode of every context of the batch (default 1); with 2,
  * each point runs as one graph launch, the graph of its grid
- * updated in place for the point's model; with 3, a Newton + mixed sweep runs
+ * updated in place for the point's model (but for the reference form's larger
+ * lattices on five contexts or more, whose searches the host drives); with 3, a Newton + mixed sweep runs
  * by shape groups, one launch per stage over every point of a group, one
  * graph launch per group (tpsc_solve_points on the first context). */
 int tpsc_batch_set_graph_mode(tpsc_batch *b, int mode);

@@ -700,14 +700,17 @@ __device__ __forceinline__ double4 ld_stream4(const double4 *p) {
 
 // one term of Tr(G - G0) (green::traceDiffG, src/green.cpp:3108-3182) and its
 // derivative with respect to the chemical potential pmu: w Re[G - G0] with
-// G = 1/(i w_n - e + pmu - Sigma), G0 = 1/(i w_n - e + mu0)
+// G = 1/(i w_n - e + pmu - Sigma), G0 = 1/(i w_n - e + mu0).  The value's products are
+// fused here, not by the compiler, which does it by what stands beside them: find_zero
+// ends at the last bits of the sum, and a search on the host then took other steps (9
+// evaluations for 20) than the device's.
 __device__ __forceinline__ void trdiff_term(double wn, double rS, double iS, double e, double mu0, double pmu,
                                             double w, double &v, double &dv) {
-    const double a = e - pmu + rS, d = e - mu0, g = mu0 - pmu + rS;
-    const double A2 = (wn - iS) * (wn - iS) + a * a;
-    const double num = g * a * d + iS * (iS - 2 * wn) * d - wn * wn * g;
-    const double inv = w / (A2 * (wn * wn + d * d));
-    v += inv * num;
+    const double a = e - pmu + rS, d = e - mu0, g = mu0 - pmu + rS, y = wn - iS, wn2 = __dmul_rn(wn, wn);
+    const double A2 = fma(y, y, __dmul_rn(a, a));
+    const double num = fma(-wn2, g, fma(__dmul_rn(g, a), d, __dmul_rn(__dmul_rn(iS, fma(-2.0, wn, iS)), d)));
+    const double inv = w / __dmul_rn(A2, fma(d, d, wn2));
+    v = fma(inv, num, v);
     dv += inv * (wn * wn - (a + g) * d + num * 2.0 * a / A2);
 }
 // the same with the second derivative: d2/dpmu2 w Re G = 2 w Re G^3, and
@@ -717,6 +720,21 @@ __device__ __forceinline__ void trdiff_term(double wn, double rS, double iS, dou
     trdiff_term(wn, rS, iS, e, mu0, pmu, w, v, dv);
     const double x = pmu - e - rS, y = wn - iS, r = 1.0 / (x * x + y * y);
     d2v += 2.0 * w * x * (x * x - 3.0 * y * y) * (r * r * r);
+}
+
+// Sigma in those terms: as sigma_full, and its asymptotic tail, rounded the same way
+// wherever they are formed
+__device__ __forceinline__ void trdiff_sigma(double i1, double sinf, double c2, double c3, double2 Sv, double &rS,
+                                             double &iS) {
+    const double i2 = __dmul_rn(i1, i1), i4 = __dmul_rn(i2, i2);
+    rS = fma(Sv.x, i4, -__dmul_rn(c2, i2));
+    iS = fma(Sv.y, i4, fma(__dmul_rn(c3, i2), i1, -__dmul_rn(sinf, i1)));
+}
+__device__ __forceinline__ void trdiff_sigma_tail(double i1, double sinf, double c2, double c3, double c4, double &rS,
+                                                  double &iS) {
+    const double i2 = __dmul_rn(i1, i1);
+    rS = fma(__dmul_rn(c4, i2), i2, -__dmul_rn(c2, i2));
+    iS = fma(__dmul_rn(c3, i2), i1, -__dmul_rn(sinf, i1));
 }
 
 // a row of four: streamed (read once), or left in the caches for the next pass
@@ -809,7 +827,7 @@ __device__ __forceinline__ void trace_diff_block(const double2 *__restrict__ S, 
     const double pt = 3.141592653589793 * T;
     const double4 *row = reinterpret_cast<const double4 *>(S + (size_t)blk * 4 * NO);
     for (int j = threadIdx.x; j < jdir; j += blockDim.x) {
-        const double wn = (2 * j + 1) * pt;
+        const double wn = __dmul_rn(2 * j + 1, pt);
         const double i1 = 1.0 / wn;
         const double4 p = ld_row<STREAM>(&row[2 * j]), q = ld_row<STREAM>(&row[2 * j + 1]);
         const double2 sv[4] = {make_double2(p.x, p.y), make_double2(p.z, p.w), make_double2(q.x, q.y),
@@ -818,19 +836,19 @@ __device__ __forceinline__ void trace_diff_block(const double2 *__restrict__ S, 
         for (int c = 0; c < 4; ++c) {
             if (ww[c] == 0.0) continue;
             double rS, iS;
-            sigma_full(i1, sinf, c2[c], c3[c], sv[c], rS, iS);
+            trdiff_sigma(i1, sinf, c2[c], c3[c], sv[c], rS, iS);
             trdiff_term(wn, rS, iS, e[c], mu0, pmu, ww[c], v, dv);
         }
     }
     for (int t = threadIdx.x; tail && t <= NO; t += blockDim.x) {
         const int j = NO + t;
-        const double wn = (2 * j + 1) * pt;
-        const double i1 = 1.0 / wn, i2 = i1 * i1;
+        const double wn = __dmul_rn(2 * j + 1, pt);
+        const double i1 = 1.0 / wn;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             if (ww[c] == 0.0) continue;
-            const double rS = -c2[c] * i2 + c4[c] * i2 * i2;
-            const double iS = -sinf * i1 + c3[c] * i2 * i1;
+            double rS, iS;
+            trdiff_sigma_tail(i1, sinf, c2[c], c3[c], c4[c], rS, iS);
             trdiff_term(wn, rS, iS, e[c], mu0, pmu, ww[c], v, dv);
         }
     }

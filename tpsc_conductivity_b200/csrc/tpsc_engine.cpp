@@ -766,6 +766,43 @@ int sumrule(tpsc_ctx *ctx, int channel, double Uv, double *tr, double *dtr) {
     return TPSC_OK;
 }
 
+// whether the host drives the root searches of the context on grid g: the reference
+// form's, where the other contexts of a batch leave the device search too few blocks
+bool host_search(const tpsc_ctx *ctx, const Grid *g) {
+    return !(ctx->form & TPSC_FORM_NEWTON) && !ctx->ran_out && zero_by_host(g->d, ctx->roots.max_blocks);
+}
+// find_Usp_Uch by find_zero over the kernels of one evaluation, a round trip each; after
+// the chi0 stage has been read back
+int host_Usp_Uch(tpsc_ctx *ctx) {
+    const double n = ctx->n, U = ctx->U, nsr = ctx->nsr;
+    double r[6] = {0, 0, 0, 0, 0, 0};
+    int rc = TPSC_OK;
+    for (int ch = 0; ch < 2; ++ch) {
+        // chi::sum_rule_sp (src/chi.cpp:833-836), then sum_rule_ch (840-843)
+        auto f = [&](double Uv, double &y) -> bool {
+            double tr;
+            if ((rc = sumrule(ctx, ch, Uv, &tr, nullptr))) return false;
+            y = ch == 0 ? tr + n - n * n / 2.0 - nsr + Uv * nsr * nsr / (2.0 * U)
+                        : tr + n - n * n / 2.0 - (nsr + r[0] * nsr * nsr / (2.0 * U) - nsr * nsr);
+            return true;
+        };
+        const double init[3] = {ch == 0 ? U / 2.0 : 0.0, 0.0,
+                                ch == 0 ? 2.0 / ctx->scal[TPSC_S_CHI0MAX] - 2 * EPS : 1000.0 * U};
+        int nev;
+        bool gone;
+        const bool ok = find_zero(f, init, &r[ch], nullptr, &nev, &gone);
+        if (gone) return drop_roots(ctx, rc);
+        r[2 + ch] = nev;
+        r[4 + ch] = ok;
+        if (!ok) break;
+    }
+    if ((rc = set_roots(ctx, r, 0))) return drop_roots(ctx, rc);
+    ctx->cur->have_U = true;
+    // where the vertex and Sigma kernels read them
+    CK(launch_store(ctx->dres, r, 2, ctx->st));
+    return TPSC_OK;
+}
+
 // chi::find_Usp_Uch(nq0, nw0, Usc) on the current grid after chi0 (src/chi.cpp:850-876)
 // read: take the roots back now; a solve defers that to its one readback at
 // the end (solve_finish), the interval's end then coming from the device chi0max
@@ -775,6 +812,12 @@ int search_Usp_Uch(tpsc_ctx *ctx, double Usc[2], bool read) {
     // both roots in one cooperative launch (tpsc_roots.cu), into ctx->dres,
     // where the vertex and Sigma kernels read them
     Grid *g = ctx->cur;
+    if (host_search(ctx, g)) {
+        if ((rc = host_Usp_Uch(ctx))) return rc;
+        Usc[0] = ctx->Usp;
+        Usc[1] = ctx->Uch;
+        return TPSC_OK;
+    }
     RootScratch rs = ctx->roots;
     rs.out = ctx->dres;
     const double hi = read ? 2.0 / ctx->scal[TPSC_S_CHI0MAX] - 2 * EPS : 0.0, off = read ? 0.0 : 2 * EPS;
@@ -875,6 +918,34 @@ int trace_diff_G(tpsc_ctx *ctx, double pmu, double *tr, double *dtr = nullptr) {
     *tr = r[0];
     if (dtr) *dtr = r[1];
     return TPSC_OK;
+}
+
+// find_mu and traceSelfG2 as host_Usp_Uch
+int trace_value_G(tpsc_ctx *ctx, double pmu, double *tr) {
+    Grid *g = ctx->cur;
+    CK(launch_trace_value_G(g->d, g->S, g->s2, g->s3, g->s4, g->sinf, g->mu0, pmu, ctx->T, ctx->red, ctx->st));
+    return read_result(ctx, 1, tr);
+}
+int host_mu(tpsc_ctx *ctx) {
+    Grid *g = ctx->cur;
+    int rc = TPSC_OK;
+    ctx->scal[TPSC_S_EVALS_MU] = 0;
+    auto f = [&](double m, double &y) -> bool { return (rc = trace_value_G(ctx, m, &y)) == TPSC_OK; };
+    const double init[3] = {0.0, -10.0, 10.0}, lims[2] = {-20.0, 20.0};
+    double r[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    int nev;
+    bool gone;
+    const bool ok = find_zero(f, init, &r[2], lims, &nev, &gone);
+    if (gone) return rc;
+    r[3] = nev;
+    r[4] = ok;
+    if (ok) {
+        CK(launch_trace_self_G2(g->d, g->S, g->s2, g->s3, g->sinf, r[2], ctx->T, ctx->red, ctx->st));
+        if ((rc = read_result(ctx, 1, &r[5]))) return rc;
+    }
+    if ((rc = read_back(ctx, {{g->sinf, sizeof(double), 0}}))) return rc;
+    r[7] = ctx->h_res[0];
+    return set_mu(ctx, r, 0, false);
 }
 
 // The find_mu series covers the frequencies from jc = first n with
@@ -994,6 +1065,25 @@ int solve_finish(tpsc_ctx *ctx) {
     return set_mu(ctx, r, err_mu, true);
 }
 
+// The solve with searches that the host drives: stage by stage.
+int host_solve(tpsc_ctx *ctx) {
+    double out[2];
+    int rc;
+    if ((rc = mark(ctx, 0))) return rc;
+    if ((rc = run_chi0(ctx))) return drop_roots(ctx, rc);
+    if ((rc = mark(ctx, 1))) return rc;
+    if ((rc = host_Usp_Uch(ctx))) return rc;
+    set_dblocc(ctx);
+    if ((rc = mark(ctx, 2))) return rc;
+    if ((rc = run_vertex(ctx))) return rc;
+    if ((rc = mark(ctx, 3))) return rc;
+    if ((rc = run_self(ctx, false))) return rc;
+    if ((rc = mark(ctx, 4))) return rc;
+    if ((rc = trace_self_G(ctx, out))) return rc;
+    if ((rc = host_mu(ctx))) return rc;
+    return mark(ctx, 5);
+}
+
 // the host state solve_queue leaves behind (a replayed graph only launches)
 void solve_state(tpsc_ctx *ctx) {
     Grid *g = ctx->cur;
@@ -1017,6 +1107,7 @@ int launch_solve(tpsc_ctx *ctx) {
     Grid *g = ctx->cur;
     const GridDev &d = g->d;
     if (mixed(ctx) && !g->Grt32) CK(dalloc(g, &g->Grt32, (size_t)(d.nw0 + 1) * d.n8));
+    if (host_search(ctx, g)) return host_solve(ctx);
     SolveKey key;
     key.form = ctx->form;
     key.cap = ctx->roots.max_blocks;
@@ -1091,6 +1182,7 @@ int run_solve(tpsc_ctx *ctx) {
 int search_mu(tpsc_ctx *ctx) {
     Grid *g = ctx->cur;
     if (!g || !g->have_S) return fail(ctx, TPSC_ERR_STATE, "the self-energy has not been computed");
+    if (host_search(ctx, g)) return host_mu(ctx);
     const bool traces = (ctx->form & TPSC_FORM_NEWTON) != 0;
     int rc = queue_mu_search(ctx, traces);
     if (rc) return rc;

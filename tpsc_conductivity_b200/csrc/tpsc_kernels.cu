@@ -1312,14 +1312,18 @@ __global__ void __launch_bounds__(256)
 // Stored frequencies j < jdir term by term (jdir = Nw0/2: all), and the
 // tail Nw0/2 <= j <= Nw0 when `tail` is set; the Newton form covers the
 // rest with the series of k_sigma_moments.
+// DERIV = false: the value alone.
+template <bool DERIV>
 __global__ void __launch_bounds__(kRedThreads)
     k_trace_diff_G(const double2 *__restrict__ S, const double *__restrict__ s2, const double *__restrict__ s3,
                    const double *__restrict__ s4, const double *__restrict__ sinfp, const double *__restrict__ ek,
                    const double *__restrict__ w16, int nw0, double mu0, double pmu, double T, int jdir, int tail,
                    Reduce r) {
-    double out[2];
-    trace_diff_block<true>(S, s2, s3, s4, sinfp, ek, w16, blockIdx.x, nw0, mu0, pmu, T, jdir, tail, out[0], out[1]);
-    grid_finish<2>(out, r, 0.0);
+    double out[1 + DERIV], v, dv;
+    trace_diff_block<true>(S, s2, s3, s4, sinfp, ek, w16, blockIdx.x, nw0, mu0, pmu, T, jdir, tail, v, dv);
+    out[0] = v;
+    if (DERIV) out[DERIV] = dv;
+    grid_finish<1 + DERIV>(out, r, 0.0);
 }
 
 // The Newton form's Tr(G - G0) evaluation: only the stored frequencies
@@ -1400,6 +1404,16 @@ __global__ void __launch_bounds__(kRedThreads)
     }
     double out[2] = {v.value(), v2.value()};
     grid_finish<2>(out, r, 0.0);
+}
+
+// Tr Sigma G (green::traceSelfG2, src/green.cpp:2929-2976) by itself, for the searches
+// that the host drives
+__global__ void __launch_bounds__(kRedThreads)
+    k_trace_self_G2(const double2 *__restrict__ S, const double *__restrict__ s2, const double *__restrict__ s3,
+                    const double *__restrict__ sinfp, const double *__restrict__ ek, const double *__restrict__ w16,
+                    int nw0, double mu, double T, double nk02, Reduce r) {
+    double out[1] = {trace_self2_block<true>(S, s2, s3, sinfp, ek, w16, blockIdx.x, nw0, mu, T, nk02)};
+    grid_finish<1>(out, r, 0.0);
 }
 
 // raw and tail parts of chi0::traceChi0 (src/chi0.cpp:1498-1584)
@@ -2263,8 +2277,16 @@ cudaError_t launch_trace_diff_G(const GridDev &g, const double2 *S, const double
                                                                        pmu, T, jdir, r);
         return launched();
     }
-    k_trace_diff_G<<<nblk, kRedThreads, 0, st>>>(S, s2, s3, s4, sinf, g.ek, g.w16, g.nw0, mu0, pmu, T, jdir, tail,
+    k_trace_diff_G<true><<<nblk, kRedThreads, 0, st>>>(S, s2, s3, s4, sinf, g.ek, g.w16, g.nw0, mu0, pmu, T, jdir, tail,
                                                   r);
+    return launched();
+}
+
+cudaError_t launch_trace_value_G(const GridDev &g, const double2 *S, const double *s2, const double *s3,
+                                 const double *s4, const double *sinf, double mu0, double pmu, double T, Reduce r,
+                                 cudaStream_t st) {
+    k_trace_diff_G<false><<<g.n8p / 4, kRedThreads, 0, st>>>(S, s2, s3, s4, sinf, g.ek, g.w16, g.nw0, mu0, pmu, T,
+                                                             g.nw0 / 2, 1, r);
     return launched();
 }
 
@@ -2273,6 +2295,17 @@ cudaError_t launch_trace_self_G(const GridDev &g, const double2 *S, const double
     const double nk02 = 4.0 * (g.nbk - 1) * (g.nbk - 1);
     k_trace_self_G<<<g.n8p / 4, kRedThreads, 0, st>>>(S, s2, s3, sinf, g.ek, g.w16, g.nw0, mu0, T, nk02, r);
     return launched();
+}
+
+cudaError_t launch_trace_self_G2(const GridDev &g, const double2 *S, const double *s2, const double *s3,
+                                 const double *sinf, double mu, double T, Reduce r, cudaStream_t st) {
+    const double nk02 = 4.0 * (g.nbk - 1) * (g.nbk - 1);
+    k_trace_self_G2<<<g.n8p / 4, kRedThreads, 0, st>>>(S, s2, s3, sinf, g.ek, g.w16, g.nw0, mu, T, nk02, r);
+    return launched();
+}
+
+bool zero_by_host(const GridDev &g, int max_blocks) {
+    return max_blocks > 0 && 2 * max_blocks < sm_count() && g.n8p / 4 > 4 * max_blocks;
 }
 
 cudaError_t launch_pade_sigma(const GridDev &g, const double2 *S, const double *s2, const double *s3,

@@ -199,8 +199,25 @@ cudaError_t launch_sigma_tau(const GridDev &g, const double *sigt, const double 
 cudaError_t launch_trace_diff_G(const GridDev &g, const double2 *S, const double *s2, const double *s3,
                                 const double *s4, const double *sinf, double mu0, double pmu, double T, Reduce r,
                                 cudaStream_t st, int jdir = -1);
+// the value alone, all frequencies
+cudaError_t launch_trace_value_G(const GridDev &g, const double2 *S, const double *s2, const double *s3,
+                                 const double *s4, const double *sinf, double mu0, double pmu, double T, Reduce r,
+                                 cudaStream_t st);
 cudaError_t launch_trace_self_G(const GridDev &g, const double2 *S, const double *s2, const double *s3,
                                 const double *sinf, double mu0, double T, Reduce r, cudaStream_t st);
+
+cudaError_t launch_trace_self_G2(const GridDev &g, const double2 *S, const double *s2, const double *s3,
+                                 const double *sinf, double mu, double T, Reduce r, cudaStream_t st);
+// Whether the host drives the reference form's searches: their cooperative grid is
+// capped at max_blocks, fewer than half the SMs and a quarter of the column blocks.  A
+// search of a few blocks has too few warps for its reads, which with many contexts come
+// from HBM, where the kernel of one evaluation by itself takes the whole GPU.  Batches
+// of reference-form solves, device search -> host's: 16 of 256^2 x 1024 on 16 contexts 124
+// -> 39 ms, on 8 75 -> 39 (on 4, 74 blocks each, the device's 50); 32 of 128^2 x 1024 on
+// 16 68 -> 22, on 8 36 -> 22; 64 of 64^2 x 512 on 16 23 -> 14.  On 8 contexts (37 blocks
+// of 141) the device takes 14 ms for these where host-driven searches took 23, and 9
+// where they took 17 for 64 of 32^2 x 256 on 16 (18 of 39).
+bool zero_by_host(const GridDev &g, int max_blocks);
 
 // ---- the Newton form's root searches on the device (tpsc_roots.cu) ----------
 constexpr int kRootMaxBlocks = 1024;

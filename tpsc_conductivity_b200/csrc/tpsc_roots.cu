@@ -1376,7 +1376,7 @@ __device__ __noinline__ void trace_diff_values(const MuRootArgs &a, const double
             e[c] = ww[c] != 0.0 ? a.ek[4 * blk + c] : 0.0;
         }
         auto row = [&](int j) {
-            const double wn = (2 * j + 1) * pt;
+            const double wn = __dmul_rn(2 * j + 1, pt);
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 if (ww[c] == 0.0) continue;
@@ -1401,13 +1401,11 @@ __global__ void __launch_bounds__(kRootThreads, 2) k_mu_slots(MuRootArgs a) {
                 const int j = i >> 2, c = i & 3, o = 4 * blk + c;
                 double rS = 0.0, iS = 0.0;
                 if (a.w16[o] != 0.0) {
-                    const double wn = (2 * j + 1) * pt, i1 = 1.0 / wn, i2 = i1 * i1;
-                    if (j < NO) {
-                        sigma_full(i1, sinf, a.s2[o], a.s3[o], a.S[((size_t)blk * NO + j) * 4 + c], rS, iS);
-                    } else {
-                        rS = -a.s2[o] * i2 + a.s4[o] * i2 * i2;
-                        iS = -sinf * i1 + a.s3[o] * i2 * i1;
-                    }
+                    const double i1 = 1.0 / __dmul_rn(2 * j + 1, pt);
+                    if (j < NO)
+                        trdiff_sigma(i1, sinf, a.s2[o], a.s3[o], a.S[((size_t)blk * NO + j) * 4 + c], rS, iS);
+                    else
+                        trdiff_sigma_tail(i1, sinf, a.s2[o], a.s3[o], a.s4[o], rS, iS);
                 }
                 zself[((size_t)lb * 4 + c) * R + j] = make_double2(rS, iS);
             }
